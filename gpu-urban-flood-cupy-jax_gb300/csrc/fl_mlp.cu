@@ -22,17 +22,13 @@
 // Every mbarrier wait is bounded in time; a wait that gives up records an
 // error flag, drains the outstanding MMAs (bounded again), frees TMEM and
 // returns.
-#include <cuda_bf16.h>
-
 #include <algorithm>
 
-#include "fl_device.cuh"
+#include "fl_umma.cuh"
 
 namespace fl {
 
-constexpr int MM_BM = 128, MM_BN = 128, MM_BK = 64, MM_STAGES = 4, MM_THREADS = 128;
-constexpr int MM_CHUNK_BYTES = MM_BM * MM_BK * 2;  // 16 KB per operand per stage
-constexpr uint64_t MM_WAIT_NS = 1000000000ull;
+constexpr int MM_STAGES = 4, MM_THREADS = 128;
 
 struct GemmSeg {
     const __nv_bfloat16 *base;
@@ -59,49 +55,6 @@ struct GemmArgs {
     int32_t wide;                    // bias / residual / outputs allow 32-byte accesses (persistent kernel)
     int32_t *error;                  // set to FL_E_TIMEOUT if a wait gave up
 };
-
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);  // start address (16-byte units)
-    d |= (uint64_t)1 << 16;                    // leading byte offset (unused by swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;          // stride byte offset: 8 rows x 128 B
-    d |= (uint64_t)1 << 46;                    // descriptor version
-    d |= (uint64_t)2 << 61;                    // 128-byte swizzle
-    return d;
-}
-
-// kind::f16 instruction descriptor: fp32 accumulator, bf16 A and B, both
-// K-major, M = 128, N = 128.
-__device__ __forceinline__ uint32_t umma_idesc_bf16_128x128() {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MM_BN >> 3) << 17) | ((uint32_t)(MM_BM >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.u32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(d_tmem),
-        "l"(a), "l"(b), "r"(idesc), "r"(acc));
-}
-
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
 
 // Copy one 64-wide chunk (128 rows x 128 B) into the swizzled stage layout:
 // 16-byte piece c of row R lands at R * 128 + ((c ^ (R & 7)) * 16).
@@ -337,28 +290,6 @@ __device__ __forceinline__ void warp_load_chunk_a(const GemmArgs &g, const TileR
         else
             asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "r"(0u) : "memory");
     }
-}
-
-// 32-byte global accesses (8 x 32 bits; the address is 32-byte aligned).
-__device__ __forceinline__ void ld8f(const float *p, float *d) {
-    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]), "=f"(d[4]), "=f"(d[5]), "=f"(d[6]), "=f"(d[7])
-                 : "l"(p));
-}
-__device__ __forceinline__ void st8f(float *p, const float *s) {
-    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(s[0]), "f"(s[1]), "f"(s[2]),
-                 "f"(s[3]), "f"(s[4]), "f"(s[5]), "f"(s[6]), "f"(s[7])
-                 : "memory");
-}
-__device__ __forceinline__ void st8u(void *p, const uint32_t *s) {
-    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(s[0]), "r"(s[1]), "r"(s[2]),
-                 "r"(s[3]), "r"(s[4]), "r"(s[5]), "r"(s[6]), "r"(s[7])
-                 : "memory");
-}
-
-__device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    return *(uint32_t *)&h;
 }
 
 // The epilogue of one row's 32 columns [nb, nb + 32).  With g.wide, 16
@@ -643,7 +574,7 @@ int set_error(int code, const char *fmt, ...);
 void add_launches(int64_t n);
 
 // Per-device error flag of the GEMM kernel's bounded waits.
-static int gemm_error_flag(int32_t **out) {
+int gemm_error_flag(int32_t **out) {
     constexpr int MAX_DEVICES = 64;
     static std::mutex mu;
     static int32_t *flag[MAX_DEVICES] = {};

@@ -131,6 +131,23 @@ class FlGemmDesc(C.Structure):
     ]
 
 
+class FlDenseRef(C.Structure):
+    _fields_ = [("w", C.c_void_p), ("ldw", C.c_int64), ("b", C.c_void_p)]
+
+
+class FlMpnnForwardDesc(C.Structure):
+    _fields_ = [
+        ("cells", C.c_int32), ("edges", C.c_int32), ("layers", C.c_int32),
+        ("src", C.c_void_p), ("recv_start", C.c_void_p), ("x", C.c_void_p), ("ef", C.c_void_p),
+        ("ldx", C.c_int64), ("lde", C.c_int64),
+        ("enc_n", FlDenseRef * 2), ("enc_e", FlDenseRef * 2), ("dec", FlDenseRef * 2),
+        ("edge", C.POINTER(FlDenseRef)), ("node", C.POINTER(FlDenseRef)),
+        ("zn", C.c_void_p), ("ze", C.c_void_p), ("e", C.c_void_p), ("zd", C.c_void_p),
+        ("h_bf", C.POINTER(C.c_void_p)), ("agg", C.POINTER(C.c_void_p)), ("z1e", C.POINTER(C.c_void_p)),
+        ("z1n", C.POINTER(C.c_void_p)), ("h_f32", C.c_void_p * 2), ("y", C.c_void_p),
+    ]
+
+
 _lib = None
 
 # symbol -> (restype, argtypes)
@@ -163,6 +180,7 @@ _SIGNATURES = {
     "fl_time_kernel": (C.c_int, [C.c_void_p, C.c_int32, C.c_int32, C.c_void_p, f64p]),
     "fl_launch_count": (C.c_int64, []),
     "fl_gemm_bf16": (C.c_int, [C.POINTER(FlGemmDesc), C.c_void_p]),
+    "fl_mpnn_forward": (C.c_int, [C.POINTER(FlMpnnForwardDesc), C.c_void_p]),
     "fl_gemm_status": (C.c_int, [C.c_void_p]),
     "fl_wait_selftest": (C.c_int, [C.c_double, i32p, f64p]),
     "fl_transpose_bf16": (C.c_int, [C.POINTER(FlGemmSegment), C.c_int32, C.c_int32, C.c_void_p, C.c_int64,

@@ -9,9 +9,11 @@ Architecture (hidden width H = 128, every MLP Linear-ReLU-Linear):
       h_i <- h_i + MLP_n([h_i, a_i])          residual node update
   decoder       h -> 64 outputs (two used: next-hour depth change, hour max above it)
 
-Every dense product runs on the tcgen05 GEMM (bf16 operands, fp32
-accumulation in TMEM); the concatenated edge-MLP input is gathered inside the
-GEMM.  The backward pass is written out by hand: dX = dZ W on the GEMM with
+Every dense product runs on the tensor cores (tcgen05, bf16 operands, fp32
+accumulation in TMEM).  On a triangle mesh's dual graph the forward pass is a
+native call of fused blocks (messages and their sum per layer, two-layer
+MLPs); a graph with more than three edges into a cell runs it product by
+product, the concatenated edge-MLP input gathered inside the GEMM.  The backward pass is written out by hand: dX = dZ W on the GEMM with
 the transposed weight copy, dW = dZ^T X as a split-K GEMM over rows of
 transposed bf16 copies, bias gradients as column sums, input gradients
 scattered back to cells with fixed-order CSR sums.  Weights are fp32 masters
@@ -32,6 +34,7 @@ FIN = 64
 FOUT = 64
 N_NODE_FEATURES = 12
 N_EDGE_FEATURES = 4
+MAX_IN = 3  # incoming dual edges per cell that the fused blocks take (a triangle has three edges)
 
 
 def round64(x: int) -> int:
@@ -87,6 +90,7 @@ class DualGraph:
         self.send_start = t(send_start.astype(np.int32), torch.int32)
         self.row_start = t(np.arange(self.E + 1, dtype=np.int32), torch.int32)  # identity segments (row copies)
         self.indeg = t(self.indeg_h, torch.float32)
+        self.max_in = int(self.indeg_h.max()) if self.C else 0
         self.ef_bf = t(ef, torch.float32).to(torch.bfloat16).contiguous()
 
     def replicate(self, copies: int) -> "DualGraph":
@@ -100,6 +104,7 @@ class DualGraph:
         off_c = (np.arange(k, dtype=np.int64) * C)[:, None]
         off_e = (np.arange(k, dtype=np.int64) * E)[:, None]
         g.C, g.E = C * k, E * k
+        g.max_in = self.max_in
         g.src_h = (self.src_h[None, :] + off_c).reshape(-1).astype(np.int32)
         g.dst_h = (self.dst_h[None, :] + off_c).reshape(-1).astype(np.int32)
         rs = self.recv_start.cpu().numpy().astype(np.int64)
@@ -171,18 +176,18 @@ class Workspace:
         bf = lambda *s: torch.empty(*s, device=device, dtype=torch.bfloat16)  # noqa: E731
         f32 = lambda *s: torch.empty(*s, device=device, dtype=torch.float32)  # noqa: E731
         self.C, self.E, self.train = C, E, train
+        self._bf, self._f32 = bf, f32
+        self.n_layers = n_layers
         keep = n_layers if train else 1  # inference reuses one set of layer buffers
-        self.zn, self.ze, self.e_bf = bf(C, H), bf(E, H), bf(E, H)
+        self.e_bf = bf(E, H)
         self.h_bf = [bf(C, H) for _ in range(n_layers + 1 if train else 2)]
         self.h_f32 = [f32(C, H), f32(C, H)]
-        self.z1e = [bf(E, H) for _ in range(keep)]
         self.agg_bf = [bf(C, H) for _ in range(keep)]
-        self.z1n = [bf(C, H) for _ in range(keep)]
-        self.zd = bf(C, H)
         self.y = f32(C, FOUT)
-        self.m_f32 = f32(E, H)
+        self.zn = self.ze = self.zd = self.z1e = self.z1n = self.m_f32 = None
         if not train:
             return
+        self.hidden()
         # backward scratch
         self.dz_bf_e = bf(E, H)
         self.dzf_e = f32(E, H)
@@ -198,6 +203,21 @@ class Workspace:
         self.tB = bf(3 * H, Mp)      # X^T
         self.cs_scratch = f32(256 * 3 * H * H)
         self.part = f32(512 * H * 3 * H)
+
+    def hidden(self, messages: bool = False):
+        """The MLPs' hidden activations (training; the blocks of the forward
+        pass keep them on chip otherwise) and the fp32 messages (products
+        run one by one)."""
+
+        if self.zn is None:
+            C, E, bf = self.C, self.E, self._bf
+            keep = self.n_layers if self.train else 1
+            self.zn, self.ze, self.zd = bf(C, H), bf(E, H), bf(C, H)
+            self.z1e = [bf(E, H) for _ in range(keep)]
+            self.z1n = [bf(C, H) for _ in range(keep)]
+        if messages and self.m_f32 is None:
+            self.m_f32 = self._f32(self.E, H)
+        return self
 
 
 class MPNN:
@@ -239,6 +259,10 @@ class MPNN:
         into the workspace).  train=False keeps no activations for backward."""
 
         ws = self.workspace(g, train)
+        if getattr(g, "max_in", MAX_IN + 1) <= MAX_IN:
+            ops.mpnn_forward(self, g, x_bf, ws)
+            return ws.y
+        ws.hidden(messages=True)
         C, E = g.C, g.E
         a, b = self.enc_n
         ops.gemm([(x_bf, None, FIN)], a.w_bf, bias=a.b, out_bf16=ws.zn, relu=True)

@@ -70,6 +70,47 @@ def gemm(segments, b, *, bias=None, residual=None, out_f32=None, out_bf16=None, 
     N.check(lib.fl_gemm_bf16(C.byref(d), _stream()), "fl_gemm_bf16")
 
 
+def _dense_refs(layers):
+    arr = (N.FlDenseRef * max(len(layers), 1))()
+    for r, d in zip(arr, layers):
+        r.w, r.ldw, r.b = d.w_bf.data_ptr(), d.w_bf.stride(0), d.b.data_ptr()
+    return arr
+
+
+def _pointers(tensors, n):
+    """n pointers, cycling through the tensors (None: NULL pointers)."""
+
+    ts = [t.data_ptr() for t in tensors] if tensors else [None]
+    return (C.c_void_p * max(n, 1))(*[ts[k % len(ts)] for k in range(n)])
+
+
+def mpnn_forward(net, g, x, ws):
+    """The network's forward pass over graph g (at most three edges into a
+    cell) into workspace ws; hidden activations are kept where ws has them."""
+
+    import torch
+
+    if x.dtype != torch.bfloat16 or x.dim() != 2 or x.stride(1) != 1:
+        raise ValueError("A segments must be row-major bf16 matrices")
+    if x.shape[0] != g.C or x.shape[1] < 64:
+        raise ValueError(f"inputs have shape {tuple(x.shape)}, expected ({g.C}, 64)")
+    L = net.n_layers
+    d = N.FlMpnnForwardDesc()
+    d.cells, d.edges, d.layers = g.C, g.E, L
+    d.src, d.recv_start = _ptr(g.src), _ptr(g.recv_start)
+    d.x, d.ldx = _ptr(x), x.stride(0)
+    d.ef, d.lde = _ptr(g.ef_bf), g.ef_bf.stride(0)
+    d.enc_n, d.enc_e, d.dec = _dense_refs(net.enc_n), _dense_refs(net.enc_e), _dense_refs(net.dec)
+    d.edge = _dense_refs([m for pair in net.edge for m in pair])
+    d.node = _dense_refs([m for pair in net.node for m in pair])
+    d.zn, d.ze, d.e, d.zd = _ptr(ws.zn), _ptr(ws.ze), _ptr(ws.e_bf), _ptr(ws.zd)
+    d.h_bf = _pointers(ws.h_bf, L + 1)
+    d.agg, d.z1e, d.z1n = _pointers(ws.agg_bf, L), _pointers(ws.z1e, L), _pointers(ws.z1n, L)
+    d.h_f32[0], d.h_f32[1] = ws.h_f32[0].data_ptr(), ws.h_f32[1].data_ptr()
+    d.y = _ptr(ws.y)
+    N.check(N.load().fl_mpnn_forward(C.byref(d), _stream()), "fl_mpnn_forward")
+
+
 def status():
     N.check(N.load().fl_gemm_status(_stream()), "fl_gemm_status")
 

@@ -433,6 +433,38 @@ FL_API int fl_adam(float *w, float *m1, float *m2, const float *g, int32_t rows,
                    void *stream);
 FL_API int fl_cast_bf16(const float *src, int64_t lds, int32_t m, int32_t n, void *dst, int64_t ldd, void *stream);
 
+/* The surrogate network's forward pass in fused blocks (no counterpart in the
+ * reference): encoders, `layers` processor layers, decoder, in 3 + 2 x layers
+ * launches.  Directed dual edges are sorted by receiving cell (recv_start is
+ * the CSR over them, at most three per cell; src the sending cells); hidden
+ * width 128, 64 padded input features per cell and edge, 64 padded outputs.
+ * Results are those of one fl_gemm_bf16 per product with fl_segment_sum in
+ * between, bit for bit.  x [cells, ldx] and ef [edges, lde]: bf16 inputs.  e:
+ * bf16 [edges, 128]; h_f32: two fp32 [cells, 128]; h_bf: layers + 1 and agg:
+ * layers bf16 [cells, 128] buffers (inference may alternate between two, and
+ * repeat one).  zn, ze, zd and the entries of z1e and z1n keep the hidden
+ * activations for a backward pass, or are NULL.  y: fp32 [cells, 64]. */
+typedef struct {
+    const void *w; /* bf16 [n_out, ldw], input features contiguous */
+    int64_t ldw;
+    const float *b;
+} FlDenseRef;
+
+typedef struct {
+    int32_t cells, edges, layers;
+    const int32_t *src, *recv_start;
+    const void *x, *ef;
+    int64_t ldx, lde;
+    FlDenseRef enc_n[2], enc_e[2], dec[2];
+    const FlDenseRef *edge, *node; /* two per layer */
+    void *zn, *ze, *e, *zd;
+    void *const *h_bf, *const *agg, *const *z1e, *const *z1n;
+    float *h_f32[2];
+    float *y;
+} FlMpnnForwardDesc;
+
+FL_API int fl_mpnn_forward(const FlMpnnForwardDesc *desc, void *stream);
+
 /* Self-test of the bounded device waits (no reference counterpart): one
  * warp waits on an mbarrier that nothing arrives on; *status receives
  * FL_E_TIMEOUT once the wait gives up after limit_s (at most 5 s), and the

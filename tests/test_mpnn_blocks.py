@@ -1,0 +1,66 @@
+"""The network's fused blocks against the same network run product by product
+(the path of graphs with more than three edges into a cell), which the oracle
+tests pin: the blocks keep every rounding point and the order of every sum, so
+the results are the same bits."""
+
+import copy
+
+import numpy as np
+import pytest
+
+# cells: 2 (one partial tile), 128 (one full tile), 162 and 20,402 (a remainder; more tiles than SMs)
+GRIDS = [1, 8, 9, 101]
+
+
+def _case(n, layers, copies=1):
+    torch = pytest.importorskip("torch")
+    from floodgb import native
+    from floodgb.build import build_library
+    from floodgb.surrogate.model import FIN, MPNN, DualGraph
+    from floodgb.synthetic import make_grid_city
+
+    build_library()
+    native.load()
+    if native.device_count() < 1:
+        pytest.skip("no CUDA device")
+    g = DualGraph(make_grid_city(n=n, size_m=10.0 * n, seed=4).city.topologies.surface_topology)
+    if copies > 1:
+        g = g.replicate(copies)
+    assert g.max_in <= 3
+    plain = copy.copy(g)
+    plain.max_in = 99  # product by product
+    net, ref = MPNN(n_layers=layers, seed=3), MPNN(n_layers=layers, seed=3)
+    rng = np.random.default_rng(n)
+    for d, r in zip(net.layers(), ref.layers()):
+        b = torch.as_tensor(rng.normal(0, 0.1, d.n_out).astype(np.float32), device="cuda")
+        d.b.copy_(b)
+        r.b.copy_(b)
+    wide = torch.as_tensor(rng.normal(size=(g.C, FIN + 8)).astype(np.float32), device="cuda").to(torch.bfloat16)
+    return torch, g, plain, net, ref, wide[:, 8:]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", GRIDS)
+@pytest.mark.parametrize("train", [False, True])
+def test_forward_blocks_give_the_products_bits(n, train):
+    torch, g, plain, net, ref, x = _case(n, 3, copies=2 if n == 9 else 1)
+    y = net.forward(g, x, train=train).clone()
+    want = ref.forward(plain, x, train=train)
+    assert bool(torch.isfinite(want).all()) and float(want.abs().max()) > 0
+    assert torch.equal(y, want)
+    if train:
+        a, b = net.ws, ref.ws
+        for k in ("zn", "ze", "e_bf", "zd"):
+            assert torch.equal(getattr(a, k), getattr(b, k)), k
+        for k in ("z1e", "agg_bf", "z1n", "h_bf"):
+            for p, q in zip(getattr(a, k), getattr(b, k)):
+                assert torch.equal(p, q), k
+
+
+@pytest.mark.gpu
+def test_forward_rejects_inputs_of_another_shape():
+    torch, g, _, net, _, x = _case(8, 1)
+    with pytest.raises(ValueError):
+        net.forward(g, x[:-1], train=False)
+    with pytest.raises(ValueError):
+        net.forward(g, x.float(), train=False)
