@@ -30,18 +30,10 @@
 // are those of the separate products, so both give the same bits.
 //
 // Every mbarrier wait is bounded; one that gives up sets the error flag.
-#include <algorithm>
-#include <atomic>
-
-#include "fl_umma.cuh"
+#include "fl_mpnn.cuh"
 
 namespace fl {
 
-int set_error(int code, const char *fmt, ...);
-void add_launches(int64_t n);
-int gemm_error_flag(int32_t **out);
-
-constexpr int MF_H = 128;  // hidden width
 constexpr int MF_PROD_WARPS = 4, MF_EPI_WARPS = 8, MF_THREADS = 32 * (MF_PROD_WARPS + 1 + MF_EPI_WARPS);
 constexpr int MF_CHUNKS = 14;  // 16 KB chunks of shared memory
 constexpr int MF_SMEM = MF_CHUNKS * MM_CHUNK_BYTES + 1024 /* biases */ + 256 /* barriers */ + 1024 /* alignment */;
@@ -74,27 +66,6 @@ struct Mlp2Args {
     int32_t n2, M, ring;
     int32_t *error;
 };
-
-// Producer warp's part of a 128-row chunk: its 32 rows, four whole 128-byte
-// row pieces per instruction.  `own`: this lane's row pointer (nullptr: the
-// row is left as it is), at the chunk's first column.
-__device__ __forceinline__ void warp_copy_rows(const __nv_bfloat16 *own, uint32_t sdst, int pw, int lane) {
-    const int c = lane & 7;
-    const uint64_t p = (uint64_t)own;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int rr = 4 * i + (lane >> 3);
-        const uint64_t row = __shfl_sync(0xffffffffu, p, rr);
-        const int R = 32 * pw + rr;
-        if (row) cp_async16(sdst + (uint32_t)(R * 128 + ((c ^ (R & 7)) << 4)), (const __nv_bfloat16 *)row + c * 8);
-    }
-}
-
-// A bounded wait of a whole warp: one outcome for all lanes, which then go on
-// together (the TMEM accesses that follow are warp-wide).
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
-    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, MM_WAIT_NS));
-}
 
 // relu(v + bias) of 32 columns as 16 bf16 pairs; bias in shared memory.
 __device__ __forceinline__ void relu_pack32(const uint32_t (&v)[32], const float *bias, uint32_t *out) {
@@ -595,33 +566,6 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_mlp2(const __grid_constant__ 
     if (warp == MF_PROD_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
 }
 
-// Raise a kernel's dynamic shared memory limit once per device.
-static cudaError_t allow_smem(const void *fn, int bytes, int dev, std::atomic<uint64_t> &done) {
-    if (dev < 64 && (done.load(std::memory_order_acquire) >> dev & 1u)) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess && dev < 64) done.fetch_or(1ull << dev, std::memory_order_release);
-    return e;
-}
-
-// The pass's launches after the first are programmatic dependents of the one
-// before: a block's set-up (TMEM, weights) overlaps the previous kernel's
-// last tiles.  A kernel lets its dependent start only after its own wait, so
-// a prefetch of weights never overtakes a kernel before the pass.
-template <class Args>
-static cudaError_t launch_block(void (*kernel)(Args), const Args &a, int rows, int sms, bool dependent, cudaStream_t st) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)std::max(1, std::min((rows + MM_BM - 1) / MM_BM, sms)));
-    cfg.blockDim = dim3(MF_THREADS);
-    cfg.dynamicSmemBytes = MF_SMEM;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = dependent ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, a);
-}
-
 }  // namespace fl
 
 using namespace fl;
@@ -690,7 +634,7 @@ extern "C" FL_API int fl_mpnn_forward(const FlMpnnForwardDesc *d, void *stream) 
         m.M = rows;
         m.ring = std::min(M2_MAX_RING, MF_CHUNKS - 2 - (k0 + k1) / 64);
         m.error = err;
-        e = launch_block(k_mlp2, m, rows, sms, launched > 0, st);
+        e = launch_blocks(k_mlp2, m, (rows + MM_BM - 1) / MM_BM, sms, MF_THREADS, MF_SMEM, launched > 0, st);
         ++launched;
     };
     mlp(d->x, d->ldx, 64, nullptr, 0, d->enc_n[0], d->enc_n[1], MF_H, d->cells, nullptr, d->zn, d->h_f32[0], d->h_bf[0]);
@@ -711,7 +655,7 @@ extern "C" FL_API int fl_mpnn_forward(const FlMpnnForwardDesc *d, void *stream) 
         q.agg = (bf *)d->agg[l];
         q.C = d->cells;
         q.error = err;
-        e = launch_block(k_edge_fwd, q, d->cells, sms, true, st);
+        e = launch_blocks(k_edge_fwd, q, (d->cells + MM_BM - 1) / MM_BM, sms, MF_THREADS, MF_SMEM, true, st);
         ++launched;
         mlp(d->h_bf[l], MF_H, 128, d->agg[l], 128, d->node[2 * l], d->node[2 * l + 1], MF_H, d->cells, d->h_f32[l & 1],
             d->z1n ? d->z1n[l] : nullptr, d->h_f32[(l & 1) ^ 1], d->h_bf[l + 1]);

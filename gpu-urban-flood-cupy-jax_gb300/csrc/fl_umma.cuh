@@ -23,6 +23,25 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr) {
     return d;
 }
 
+// Operand stored with its M (N) index contiguous, 128-byte swizzle: 64 of them
+// (128 bytes) per K row, 8-row groups 1024 bytes apart, the next 64 of them
+// `block` bytes on.
+__device__ __forceinline__ uint64_t umma_desc_mn_sw128(uint32_t saddr, uint32_t block) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)(block >> 4) << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+
+// Instruction descriptor with both operands M (N) contiguous, M = 128, N = n.
+__device__ __forceinline__ uint32_t umma_idesc_bf16_mn(int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(n >> 3) << 17) |
+           ((uint32_t)(MM_BM >> 4) << 24);
+}
+
 // kind::f16 instruction descriptor: fp32 accumulator, bf16 A and B, both
 // K-major, M = 128, N = 128.
 __device__ __forceinline__ uint32_t umma_idesc_bf16_128x128() {
@@ -106,10 +125,26 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t *r) {
         : "memory");
 }
 
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// A bounded wait of a whole warp: one outcome for all lanes, which then go on
+// together (the TMEM accesses that follow are warp-wide).
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, MM_WAIT_NS));
+}
 
 // 64-wide K chunk c of a bf16 matrix's rows [0, n) into the K-major 128-byte-swizzle layout at
 // sdst (rows n .. 127 zeroed); every thread of the block takes part, cp.async.
@@ -121,6 +156,12 @@ __device__ __forceinline__ void load_weight_chunk(const __nv_bfloat16 *w, int64_
         if (R < n) cp_async16(dst, w + (int64_t)R * ldw + c * MM_BK + cc * 8);
         else asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "r"(0u) : "memory");
     }
+}
+
+__device__ __forceinline__ void ld8u(const void *p, uint32_t *d) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7])
+                 : "l"(p));
 }
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {

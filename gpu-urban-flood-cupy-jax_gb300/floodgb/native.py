@@ -148,6 +148,31 @@ class FlMpnnForwardDesc(C.Structure):
     ]
 
 
+class FlDenseGrad(C.Structure):
+    _fields_ = [("wt", C.c_void_p), ("ldwt", C.c_int64), ("gw", C.c_void_p), ("gb", C.c_void_p)]
+
+
+class FlMpnnBackwardDesc(C.Structure):
+    _fields_ = [
+        ("cells", C.c_int32), ("edges", C.c_int32), ("layers", C.c_int32),
+        ("src", C.c_void_p), ("dst", C.c_void_p), ("recv_start", C.c_void_p), ("send_start", C.c_void_p),
+        ("send_order", C.c_void_p), ("x", C.c_void_p), ("ef", C.c_void_p), ("ldx", C.c_int64), ("lde", C.c_int64),
+        ("enc_n", FlDenseGrad * 2), ("enc_e", FlDenseGrad * 2), ("dec", FlDenseGrad * 2),
+        ("edge", C.POINTER(FlDenseGrad)), ("node", C.POINTER(FlDenseGrad)),
+        ("zn", C.c_void_p), ("ze", C.c_void_p), ("e", C.c_void_p), ("zd", C.c_void_p),
+        ("h_bf", C.POINTER(C.c_void_p)), ("agg", C.POINTER(C.c_void_p)), ("z1e", C.POINTER(C.c_void_p)),
+        ("z1n", C.POINTER(C.c_void_p)), ("dy", C.c_void_p), ("ldy", C.c_int64), ("dh", C.c_void_p * 2),
+        ("dz2c", C.c_void_p), ("dz1c", C.c_void_p), ("dagg", C.c_void_p), ("dyb", C.c_void_p),
+        ("dze", C.POINTER(C.c_void_p)), ("dz2e", C.c_void_p), ("scratch", C.c_void_p), ("scratch_floats", C.c_int64),
+    ]
+
+
+class FlAdamTensor(C.Structure):
+    _fields_ = [("w", C.c_void_p), ("m1", C.c_void_p), ("m2", C.c_void_p), ("g", C.c_void_p),
+                ("w_bf16", C.c_void_p), ("wt_bf16", C.c_void_p), ("rows", C.c_int32), ("cols", C.c_int32),
+                ("ldt", C.c_int32), ("reserved", C.c_int32)]
+
+
 _lib = None
 
 # symbol -> (restype, argtypes)
@@ -181,6 +206,10 @@ _SIGNATURES = {
     "fl_launch_count": (C.c_int64, []),
     "fl_gemm_bf16": (C.c_int, [C.POINTER(FlGemmDesc), C.c_void_p]),
     "fl_mpnn_forward": (C.c_int, [C.POINTER(FlMpnnForwardDesc), C.c_void_p]),
+    "fl_mpnn_backward_scratch": (C.c_int, [C.POINTER(C.c_int64)]),
+    "fl_mpnn_backward": (C.c_int, [C.POINTER(FlMpnnBackwardDesc), C.c_void_p]),
+    "fl_adam_all": (C.c_int, [C.POINTER(FlAdamTensor), C.c_int32, C.c_float, C.c_float, C.c_float, C.c_float, C.c_int32,
+                              C.c_float, C.c_void_p]),
     "fl_gemm_status": (C.c_int, [C.c_void_p]),
     "fl_wait_selftest": (C.c_int, [C.c_double, i32p, f64p]),
     "fl_transpose_bf16": (C.c_int, [C.POINTER(FlGemmSegment), C.c_int32, C.c_int32, C.c_void_p, C.c_int64,

@@ -34,7 +34,8 @@ FIN = 64
 FOUT = 64
 N_NODE_FEATURES = 12
 N_EDGE_FEATURES = 4
-MAX_IN = 3  # incoming dual edges per cell that the fused blocks take (a triangle has three edges)
+MAX_IN = 3  # incoming (outgoing) dual edges per cell that the fused blocks take (a triangle has three edges)
+MAX_LAYERS = 32  # processor layers that the fused backward pass takes
 
 
 def round64(x: int) -> int:
@@ -91,6 +92,7 @@ class DualGraph:
         self.row_start = t(np.arange(self.E + 1, dtype=np.int32), torch.int32)  # identity segments (row copies)
         self.indeg = t(self.indeg_h, torch.float32)
         self.max_in = int(self.indeg_h.max()) if self.C else 0
+        self.max_out = int(np.diff(send_start).max()) if self.C else 0
         self.ef_bf = t(ef, torch.float32).to(torch.bfloat16).contiguous()
 
     def replicate(self, copies: int) -> "DualGraph":
@@ -104,7 +106,7 @@ class DualGraph:
         off_c = (np.arange(k, dtype=np.int64) * C)[:, None]
         off_e = (np.arange(k, dtype=np.int64) * E)[:, None]
         g.C, g.E = C * k, E * k
-        g.max_in = self.max_in
+        g.max_in, g.max_out = self.max_in, self.max_out
         g.src_h = (self.src_h[None, :] + off_c).reshape(-1).astype(np.int32)
         g.dst_h = (self.dst_h[None, :] + off_c).reshape(-1).astype(np.int32)
         rs = self.recv_start.cpu().numpy().astype(np.int64)
@@ -188,21 +190,38 @@ class Workspace:
         if not train:
             return
         self.hidden()
-        # backward scratch
-        self.dz_bf_e = bf(E, H)
-        self.dzf_e = f32(E, H)
-        self.dcat = f32(E, 3 * H)
-        self.de = f32(E, H)
         self.dh = [f32(C, H), f32(C, H)]
-        self.dx_c = f32(C, 2 * H)
-        self.dz_bf_c, self.dzf_c = bf(C, H), f32(C, H)
         self.dagg_bf = bf(C, H)
         self.dy_bf = bf(C, FOUT)
-        Mp = round64(max(C, E))
-        self.tA = bf(H, Mp)          # dZ^T
-        self.tB = bf(3 * H, Mp)      # X^T
-        self.cs_scratch = f32(256 * 3 * H * H)
-        self.part = f32(512 * H * 3 * H)
+        self.dze = self.scratch = self.part = None
+
+    def fused(self):
+        """Buffers of the fused backward pass."""
+
+        if self.dze is None:
+            self.dz2_c, self.dz1_c, self.dz2_e = self._bf(self.C, H), self._bf(self.C, H), self._bf(self.E, H)
+            self.dy_f32 = self._f32(self.C, FOUT)
+            self.scratch = self._f32(ops.backward_scratch())
+            self.dze = [self._bf(self.E, H) for _ in range(self.n_layers)]
+        return self
+
+    def products(self):
+        """Buffers of the backward pass run product by product."""
+
+        if self.part is None:
+            C, E, bf, f32 = self.C, self.E, self._bf, self._f32
+            self.dz_bf_e = bf(E, H)
+            self.dzf_e = f32(E, H)
+            self.dcat = f32(E, 3 * H)
+            self.de = f32(E, H)
+            self.dx_c = f32(C, 2 * H)
+            self.dz_bf_c, self.dzf_c = bf(C, H), f32(C, H)
+            Mp = round64(max(C, E))
+            self.tA = bf(H, Mp)          # dZ^T
+            self.tB = bf(3 * H, Mp)      # X^T
+            self.cs_scratch = f32(256 * 3 * H * H)
+            self.part = f32(512 * H * 3 * H)
+        return self
 
     def hidden(self, messages: bool = False):
         """The MLPs' hidden activations (training; the blocks of the forward
@@ -320,6 +339,10 @@ class MPNN:
 
         ws = self.ws
         C, E, L = g.C, g.E, self.n_layers
+        if max(getattr(g, "max_in", MAX_IN + 1), getattr(g, "max_out", MAX_IN + 1)) <= MAX_IN and L <= MAX_LAYERS:
+            ops.mpnn_backward(self, g, x_bf, dy, ws.fused())
+            return
+        ws.products()
         # decoder
         a, b = self.dec
         ops.cast_bf16(dy, ws.dy_bf)
@@ -384,13 +407,13 @@ class MPNN:
         self._bgrad(a, ws.dzf_e, E)
 
     def zero_grad(self):
-        for d in self.layers():
-            d.zero_grad()
+        import torch
+
+        torch._foreach_zero_([g for d in self.layers() for g in (d.gw, d.gb)])
 
     def step(self, lr: float, weight_decay: float = 0.0):
         self.t += 1
-        for d in self.layers():
-            d.step(lr, self.t, weight_decay)
+        ops.adam_all(self.layers(), lr, self.t, weight_decay)
 
     def state(self) -> list:
         return [d.state() for d in self.layers()]

@@ -111,6 +111,74 @@ def mpnn_forward(net, g, x, ws):
     N.check(N.load().fl_mpnn_forward(C.byref(d), _stream()), "fl_mpnn_forward")
 
 
+def backward_scratch() -> int:
+    """Floats of scratch that mpnn_backward needs on the current device."""
+
+    n = C.c_int64()
+    N.check(N.load().fl_mpnn_backward_scratch(C.byref(n)), "fl_mpnn_backward_scratch")
+    return n.value
+
+
+def _dense_grads(layers):
+    arr = (N.FlDenseGrad * max(len(layers), 1))()
+    for r, d in zip(arr, layers):
+        r.wt, r.ldwt = d.wt_bf.data_ptr(), d.wt_bf.stride(0)
+        r.gw, r.gb = d.gw.data_ptr(), d.gb.data_ptr()
+    return arr
+
+
+def mpnn_backward(net, g, x, dy, ws):
+    """Add the parameter gradients for the output gradient dy (fp32 [C, 64])
+    of the forward pass whose activations ws holds."""
+
+    if dy.stride(1) != 1 or dy.stride(0) % 8 or dy.data_ptr() % 32:
+        ws.dy_f32.copy_(dy)
+        dy = ws.dy_f32
+    L = net.n_layers
+    d = N.FlMpnnBackwardDesc()
+    d.cells, d.edges, d.layers = g.C, g.E, L
+    d.src, d.dst, d.recv_start = _ptr(g.src), _ptr(g.dst), _ptr(g.recv_start)
+    d.send_start, d.send_order = _ptr(g.send_start), _ptr(g.send_order)
+    d.x, d.ldx = _ptr(x), x.stride(0)
+    d.ef, d.lde = _ptr(g.ef_bf), g.ef_bf.stride(0)
+    d.enc_n, d.enc_e, d.dec = _dense_grads(net.enc_n), _dense_grads(net.enc_e), _dense_grads(net.dec)
+    d.edge = _dense_grads([m for pair in net.edge for m in pair])
+    d.node = _dense_grads([m for pair in net.node for m in pair])
+    d.zn, d.ze, d.e, d.zd = _ptr(ws.zn), _ptr(ws.ze), _ptr(ws.e_bf), _ptr(ws.zd)
+    d.h_bf, d.agg = _pointers(ws.h_bf, L + 1), _pointers(ws.agg_bf, L)
+    d.z1e, d.z1n, d.dze = _pointers(ws.z1e, L), _pointers(ws.z1n, L), _pointers(ws.dze, L)
+    d.dy, d.ldy = _ptr(dy), dy.stride(0)
+    d.dh[0], d.dh[1] = ws.dh[0].data_ptr(), ws.dh[1].data_ptr()
+    d.dz2c, d.dz1c, d.dagg, d.dyb = _ptr(ws.dz2_c), _ptr(ws.dz1_c), _ptr(ws.dagg_bf), _ptr(ws.dy_bf)
+    d.dz2e = _ptr(ws.dz2_e)
+    d.scratch, d.scratch_floats = _ptr(ws.scratch), ws.scratch.numel()
+    N.check(N.load().fl_mpnn_backward(C.byref(d), _stream()), "fl_mpnn_backward")
+
+
+def adam_all(layers, lr, step, weight_decay=0.0, b1=0.9, b2=0.999, eps=1e-8):
+    """One Adam step on every layer's weights (decayed) and biases."""
+
+    n = len(layers)
+    # biases are not decayed: their tensors go in a second call where the weights are
+    for decay, part in (((weight_decay, "w"), (0.0, "b")) if weight_decay else ((0.0, "wb"),)):
+        arr = (N.FlAdamTensor * (n * len(part)))()
+        k = 0
+        for d in layers:
+            if "w" in part:
+                a = arr[k]
+                a.w, a.m1, a.m2, a.g = d.w.data_ptr(), d.m1w.data_ptr(), d.m2w.data_ptr(), d.gw.data_ptr()
+                a.w_bf16, a.wt_bf16 = d.w_bf.data_ptr(), d.wt_bf.data_ptr()
+                a.rows, a.cols, a.ldt = d.n_out, d.n_in, d.wt_bf.stride(0)
+                k += 1
+            if "b" in part:
+                a = arr[k]
+                a.w, a.m1, a.m2, a.g = d.b.data_ptr(), d.m1b.data_ptr(), d.m2b.data_ptr(), d.gb.data_ptr()
+                a.rows, a.cols = 1, d.n_out
+                k += 1
+        N.check(N.load().fl_adam_all(arr, k, float(lr), float(b1), float(b2), float(eps), int(step), float(decay),
+                                     _stream()), "fl_adam_all")
+
+
 def status():
     N.check(N.load().fl_gemm_status(_stream()), "fl_gemm_status")
 

@@ -465,6 +465,55 @@ typedef struct {
 
 FL_API int fl_mpnn_forward(const FlMpnnForwardDesc *desc, void *stream);
 
+/* Its backward pass: adds the gradients of every weight and bias for the
+ * output gradient dy [cells, ldy] (fp32, 64 columns) of the forward pass whose
+ * activations the pointers name (zn .. z1n as in FlMpnnForwardDesc, all kept;
+ * h_bf: layers + 1 different buffers).  At most three outgoing edges per cell
+ * too (send_order: edges by sending cell, send_start its CSR), at most 32
+ * layers.  wt: bf16 transposed weights [n_in, ldwt].  Buffers: dh two fp32
+ * [cells, 128]; dz2c, dz1c, dagg bf16 [cells, 128]; dyb bf16 [cells, 64];
+ * dze: layers x bf16 [edges, 128]; dz2e bf16 [edges, 128]; scratch of
+ * fl_mpnn_backward_scratch floats.  Gradients equal those of one launch per
+ * product up to the order of the fp32 sums over rows. */
+typedef struct {
+    const void *wt;
+    int64_t ldwt;
+    float *gw, *gb; /* [n_out, n_in], [n_out] */
+} FlDenseGrad;
+
+typedef struct {
+    int32_t cells, edges, layers;
+    const int32_t *src, *dst, *recv_start, *send_start, *send_order;
+    const void *x, *ef;
+    int64_t ldx, lde;
+    FlDenseGrad enc_n[2], enc_e[2], dec[2];
+    const FlDenseGrad *edge, *node;
+    const void *zn, *ze, *e, *zd;
+    void *const *h_bf, *const *agg, *const *z1e, *const *z1n;
+    const float *dy;
+    int64_t ldy;
+    float *dh[2];
+    void *dz2c, *dz1c, *dagg, *dyb;
+    void *const *dze;
+    void *dz2e;
+    float *scratch;
+    int64_t scratch_floats;
+} FlMpnnBackwardDesc;
+
+FL_API int fl_mpnn_backward_scratch(int64_t *floats);
+FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *desc, void *stream);
+
+/* fl_adam over n tensors of a network in one launch (same arithmetic). */
+typedef struct {
+    float *w, *m1, *m2;
+    const float *g;
+    void *w_bf16, *wt_bf16; /* or NULL */
+    int32_t rows, cols, ldt, reserved;
+} FlAdamTensor;
+
+FL_API int fl_adam_all(const FlAdamTensor *tensors, int32_t n, float lr, float b1, float b2, float eps, int32_t step,
+                       float weight_decay, void *stream);
+
 /* Self-test of the bounded device waits (no reference counterpart): one
  * warp waits on an mbarrier that nothing arrives on; *status receives
  * FL_E_TIMEOUT once the wait gives up after limit_s (at most 5 s), and the

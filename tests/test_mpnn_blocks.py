@@ -28,6 +28,7 @@ def _case(n, layers, copies=1):
         g = g.replicate(copies)
     assert g.max_in <= 3
     plain = copy.copy(g)
+    assert g.max_out <= 3
     plain.max_in = 99  # product by product
     net, ref = MPNN(n_layers=layers, seed=3), MPNN(n_layers=layers, seed=3)
     rng = np.random.default_rng(n)
@@ -55,6 +56,39 @@ def test_forward_blocks_give_the_products_bits(n, train):
         for k in ("z1e", "agg_bf", "z1n", "h_bf"):
             for p, q in zip(getattr(a, k), getattr(b, k)):
                 assert torch.equal(p, q), k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", GRIDS)
+@pytest.mark.parametrize("layers", [0, 1, 3])
+def test_backward_blocks_give_the_products_gradients(n, layers):
+    """Activation gradients have the same bits; a weight or bias gradient is a
+    sum over up to 61,000 rows whose fp32 partial sums are grouped otherwise:
+    2e-5 of the largest entry is ~170 rounding units (sqrt(rows) of them is
+    the size of such a sum's random rounding error)."""
+
+    torch, g, plain, net, ref, x = _case(n, layers)
+    rng = np.random.default_rng(n + 50)
+    dy = torch.as_tensor(rng.normal(size=(g.C, 64)).astype(np.float32), device="cuda")
+    wide = torch.zeros(g.C, 68, device="cuda")
+    wide[:, 3:67] = dy
+    for model, graph, grad in ((net, g, wide[:, 3:67] if n == 9 else dy), (ref, plain, dy)):
+        model.forward(graph, x)
+        model.zero_grad()
+        for d in model.layers():
+            d.gb.add_(1.0)  # gradients are added to
+        model.backward(graph, x, grad)
+    for k, (d, r) in enumerate(zip(net.layers(), ref.layers())):
+        for a, b in ((d.gw, r.gw), (d.gb, r.gb)):
+            assert float((a - b).abs().max()) <= 2e-5 * max(float(b.abs().max()), 1.0), (k, tuple(a.shape))
+    net.step(1e-3, weight_decay=0.01)
+    for d in ref.layers():
+        d.gw.copy_(net.layers()[ref.layers().index(d)].gw)
+        d.gb.copy_(net.layers()[ref.layers().index(d)].gb)
+        d.step(1e-3, 1, 0.01)
+    for d, r in zip(net.layers(), ref.layers()):  # the same arithmetic tensor by tensor
+        for a in ("w", "b", "m1w", "m2w", "m1b", "m2b", "w_bf", "wt_bf"):
+            assert torch.equal(getattr(d, a), getattr(r, a)), a
 
 
 @pytest.mark.gpu
