@@ -227,70 +227,19 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_gemm_bf16(const __grid_consta
 // k_gemm_bf16_pers: the same product for K <= 512 as a persistent,
 // warp-specialised kernel.  Each CTA keeps its 128 x K slice of B resident in
 // shared memory and walks M tiles:
-//   warps 0-1   producers: gather the A chunks of its tiles (64 rows each)
+//   warps 0-3   producers: gather the A chunks of its tiles (32 rows each)
 //               into a ring of as many 16 KB stages as shared memory holds
 //               next to B (cp.async, completion tracked by the stage's
-//               mbarrier)
-//   warp 2      MMA: one lane issues tcgen05.mma per chunk into one of two
+//               mbarrier); a tile's row maps are read one tile ahead
+//   warp 4      MMA: one lane issues tcgen05.mma per chunk into one of two
 //               TMEM accumulators and commits to the stage's "empty" and
 //               the accumulator's "full" barriers
-//   warps 3-10  epilogue: drain the other accumulator (tcgen05.ld; two
+//   warps 5-12  epilogue: drain the other accumulator (tcgen05.ld; two
 //               warps per TMEM lane quarter, 64 columns each), release it,
 //               and store with bias / ReLU / residual
 // so loads, tensor-core work and the epilogue of consecutive tiles overlap.
-constexpr int PG_PROD_WARPS = 2, PG_EPI_WARPS = 8, PG_THREADS = 32 * (PG_PROD_WARPS + 1 + PG_EPI_WARPS);
+constexpr int PG_PROD_WARPS = 4, PG_EPI_WARPS = 8, PG_THREADS = 32 * (PG_PROD_WARPS + 1 + PG_EPI_WARPS);
 constexpr int PG_MAX_STAGES = 8, PG_MAX_K = 512, PG_SMEM_LIMIT = 227 * 1024;
-
-// Source rows of the four tile rows (lane, lane + 32, ...) a producer lane
-// copies, per segment; -1 past the end.  Loaded once per tile so the chunk
-// copies do not wait on index loads.
-struct TileRows {
-    int64_t r[3][2];
-};
-
-// Producer warp pw copies tile rows 64 * pw + lane and 64 * pw + 32 + lane.
-__device__ __forceinline__ TileRows tile_rows(const GemmArgs &g, int m0, int pw, int lane) {
-    TileRows t;
-#pragma unroll
-    for (int s = 0; s < 3; ++s) {
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int r = m0 + 64 * pw + lane + 32 * j;
-            int64_t v = -1;
-            if (s < g.n_seg && r < g.M) v = g.a[s].idx ? (int64_t)g.a[s].idx[r] : (int64_t)r;
-            t.r[s][j] = v;
-        }
-    }
-    return t;
-}
-
-// Copy one 64-wide A chunk of a tile with the 32 threads of one warp: each
-// copy instruction moves four whole 128-byte row pieces (lane l: row
-// 4 i + l / 8, 16-byte piece l % 8), so every L2 sector is fetched once and
-// whole; a row's source index comes from the lane that loaded it.
-__device__ __forceinline__ void warp_load_chunk_a(const GemmArgs &g, const TileRows &tr, int chunk, uint32_t sdst,
-                                                  int pw, int lane) {
-    int seg = 0, kin = chunk * MM_BK;
-    while (seg + 1 < g.n_seg && kin >= g.a[seg].width) {
-        kin -= g.a[seg].width;
-        ++seg;
-    }
-    const GemmSeg s = g.a[seg];
-    const int64_t own0 = seg == 0 ? tr.r[0][0] : (seg == 1 ? tr.r[1][0] : tr.r[2][0]);
-    const int64_t own1 = seg == 0 ? tr.r[0][1] : (seg == 1 ? tr.r[1][1] : tr.r[2][1]);
-    const int c = lane & 7;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const int rr = 4 * i + (lane >> 3);  // row within this warp's 64 (rows rr < 32 are owned as j = 0)
-        const int64_t row = __shfl_sync(0xffffffffu, i < 8 ? own0 : own1, rr & 31);
-        const int R = 64 * pw + rr;
-        const uint32_t dst = sdst + (uint32_t)(R * 128) + (uint32_t)((c ^ (R & 7)) << 4);
-        if (row >= 0)
-            cp_async16(dst, s.base + row * s.ld + kin + c * 8);
-        else
-            asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "r"(0u) : "memory");
-    }
-}
 
 // The epilogue of one row's 32 columns [nb, nb + 32).  With g.wide, 16
 // columns at a time through 32-byte loads and stores (a bf16 row piece of 16
@@ -435,63 +384,88 @@ __global__ void __launch_bounds__(PG_THREADS, 1) k_gemm_bf16_pers(const __grid_c
     bool bad = false;
 
     if (warp < PG_PROD_WARPS) {
-        // producers
-        int q = 0;
+        // producers: lane = tile row 32 * warp + lane; its source row in each
+        // segment (nullptr: past M, the row stays stale and is not stored).
+        // The segments are walked by unrolled code over registers: picking
+        // them from the parameters per chunk cost more than the copies
+        const __nv_bfloat16 *base[3] = {g.a[0].base, g.a[1].base, g.a[2].base};
+        const int32_t *idx[3] = {g.a[0].idx, g.a[1].idx, g.a[2].idx};
+        const int n_seg = g.n_seg;
+        int row[3], nrow[3];
+        auto load_rows = [&](int t, int (&o)[3]) {
+            const int r = t * MM_BM + 32 * warp + lane;
+#pragma unroll
+            for (int x = 0; x < 3; ++x) o[x] = t < tiles && r < g.M && x < n_seg ? (idx[x] ? idx[x][r] : r) : -1;
+        };
+        load_rows(blockIdx.x, row);
+        int s = 0, u = 0;
         for (int t = blockIdx.x; t < tiles && !bad; t += gridDim.x) {
-            const TileRows tr = tile_rows(g, t * MM_BM, warp, lane);
-            for (int c = 0; c < nK && !bad; ++c, ++q) {
-                const int s = q % S, u = q / S;
-                if (u > 0 && !mbar_wait_bounded(smem_addr(&empty[s]), (u - 1) & 1, MM_WAIT_NS)) {
-                    bad = true;
-                    break;
-                }
-                warp_load_chunk_a(g, tr, c, sA + s * MM_CHUNK_BYTES, warp, lane);
-                cp_async_arrive_noinc(smem_addr(&full[s]));
-            }
-        }
-        cp_async_wait_all();
-    } else if (warp == PG_PROD_WARPS) {
-        // MMA issue (one lane)
-        if (lane == 0) {
-            const uint32_t idesc = umma_idesc_bf16_128x128();
-            int q = 0, i = 0;
-            for (int t = blockIdx.x; t < tiles && !bad; t += gridDim.x, ++i) {
-                const int b = i & 1, v = i >> 1;
-                if (v > 0 && !mbar_wait_bounded(smem_addr(&acce[b]), (v - 1) & 1, MM_WAIT_NS)) {
-                    bad = true;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int c = 0; c < nK; ++c, ++q) {
-                    const int s = q % S;
-                    if (!mbar_wait_bounded(smem_addr(&full[s]), (q / S) & 1, MM_WAIT_NS)) {
+            load_rows(t + gridDim.x, nrow);
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                if (x >= n_seg || bad) continue;
+                const __nv_bfloat16 *p = row[x] >= 0 ? base[x] + (int64_t)row[x] * g.a[x].ld : nullptr;
+                for (int k = 0; k < g.a[x].width; k += MM_BK) {
+                    if (u > 0 && !warp_wait(smem_addr(&empty[s]), (u - 1) & 1)) {
                         bad = true;
                         break;
                     }
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    warp_copy_rows(p ? p + k : nullptr, sA + s * MM_CHUNK_BYTES, warp, lane);
+                    cp_async_arrive_noinc(smem_addr(&full[s]));
+                    if (++s == S) {
+                        s = 0;
+                        ++u;
+                    }
+                }
+            }
+#pragma unroll
+            for (int x = 0; x < 3; ++x) row[x] = nrow[x];
+        }
+        cp_async_wait_all();
+    } else if (warp == PG_PROD_WARPS) {
+        // MMA issue: the whole warp runs the loop, one elected lane issues
+        const bool issuer = elect_one();
+        const uint32_t idesc = umma_idesc_bf16_128x128();
+        int s = 0, ph = 0, i = 0;
+        for (int t = blockIdx.x; t < tiles && !bad; t += gridDim.x, ++i) {
+            const int b = i & 1, v = i >> 1;
+            if (v > 0 && !warp_wait(smem_addr(&acce[b]), (v - 1) & 1)) {
+                bad = true;
+                break;
+            }
+            tmem_fence_after();
+            for (int c = 0; c < nK; ++c) {
+                if (!warp_wait(smem_addr(&full[s]), ph)) {
+                    bad = true;
+                    break;
+                }
+                fence_async_smem();
+                if (issuer) {
                     const uint32_t a0 = sA + s * MM_CHUNK_BYTES, b0 = sB + c * MM_CHUNK_BYTES;
 #pragma unroll
                     for (int k = 0; k < MM_BK / 16; ++k)
-                        umma_bf16(tmem + (uint32_t)(b * MM_BN), umma_desc_sw128(a0 + k * 32),
-                                  umma_desc_sw128(b0 + k * 32), idesc, (c > 0 || k > 0) ? 1u : 0u);
+                        umma_bf16(tmem + (uint32_t)(b * MM_BN), umma_desc_sw128(a0 + k * 32), umma_desc_sw128(b0 + k * 32),
+                                  idesc, (c > 0 || k > 0) ? 1u : 0u);
                     umma_commit(smem_addr(&empty[s]));
                 }
-                if (bad) break;
-                umma_commit(smem_addr(&accf[b]));
+                if (++s == S) {
+                    s = 0;
+                    ph ^= 1;
+                }
             }
-            // every MMA issued so far has completed before TMEM is released
-            umma_commit(smem_addr(drain));
-            (void)mbar_wait_bounded(smem_addr(drain), 0, MM_WAIT_NS);
+            if (bad) break;
+            if (issuer) umma_commit(smem_addr(&accf[b]));
         }
-        __syncwarp();
+        // every MMA issued so far has completed before TMEM is released
+        if (issuer) umma_commit(smem_addr(drain));
+        (void)warp_wait(smem_addr(drain), 0);
     } else {
         // epilogue: warp w reads TMEM lanes 32 * (w % 4) .., columns 64 * ((w - 3) / 4) ..
         const int quad = warp & 3, half = (warp - PG_PROD_WARPS - 1) >> 2;
         int i = 0;
         for (int t = blockIdx.x; t < tiles && !bad; t += gridDim.x, ++i) {
             const int b = i & 1, v = i >> 1;
-            if (!mbar_wait_bounded(smem_addr(&accf[b]), v & 1, MM_WAIT_NS)) {
+            if (!warp_wait(smem_addr(&accf[b]), v & 1)) {
                 bad = true;
                 break;
             }

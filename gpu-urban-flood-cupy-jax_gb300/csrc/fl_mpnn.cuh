@@ -14,21 +14,6 @@ int gemm_error_flag(int32_t **out);
 
 constexpr int MF_H = 128;  // hidden width
 
-// Producer warp's part of a 128-row chunk: its 32 rows, four whole 128-byte
-// row pieces per instruction.  `own`: this lane's row pointer (nullptr: the
-// row is left as it is), at the chunk's first column.
-__device__ __forceinline__ void warp_copy_rows(const __nv_bfloat16 *own, uint32_t sdst, int pw, int lane) {
-    const int c = lane & 7;
-    const uint64_t p = (uint64_t)own;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int rr = 4 * i + (lane >> 3);
-        const uint64_t row = __shfl_sync(0xffffffffu, p, rr);
-        const int R = 32 * pw + rr;
-        if (row) cp_async16(sdst + (uint32_t)(R * 128 + ((c ^ (R & 7)) << 4)), (const __nv_bfloat16 *)row + c * 8);
-    }
-}
-
 // Raise a kernel's dynamic shared memory limit once per device.
 inline cudaError_t allow_smem(const void *fn, int bytes, int dev, std::atomic<uint64_t> &done) {
     if (dev < 64 && (done.load(std::memory_order_acquire) >> dev & 1u)) return cudaSuccess;

@@ -785,7 +785,7 @@ __global__ void __launch_bounds__(ES_THREADS, 1) k_edge_dsum(const __grid_consta
 }
 
 // ------------------------------------------------------------- weight gradients
-constexpr int WG_PROD = 4, WG_THREADS = 32 * (WG_PROD + 1), WG_JOBS = 4;
+constexpr int WG_PROD = 8, WG_THREADS = 32 * (WG_PROD + 1), WG_JOBS = 4;
 constexpr int WG_BLOCK = 64 * 128;                  // 64 rows x 64 columns of bf16
 constexpr int WG_RING_BYTES = 224 * 1024, WG_MAX_RING = 7;
 constexpr int WG_SMEM = WG_RING_BYTES + 256 + 1024;
@@ -854,56 +854,73 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad(const __grid_constant__
     pdl_launch_dependents();
 
     if (warp < WG_PROD) {
-        // producers: 16 rows of each 64-row chunk; row maps one chunk ahead
-        int64_t row[4], nrow[4];  // dZ, X0, X1, X2 (lanes 0..15)
-        auto load_rows = [&](int c, int64_t (&o)[4]) {
-            const int r = c * 64 + 16 * warp + (lane & 15);
-            const bool in = c < c1 && r < J.M;
-            o[0] = in ? (J.a.rows ? (int64_t)J.a.rows[r] : (int64_t)r) : -1;
+        // producers: 8 rows of each 64-row chunk (lanes 0..7 own one each);
+        // row maps are read one chunk ahead.  The job's fields are held in
+        // registers: read from the parameters in the copy loop they made it
+        // 230 cycles an instruction
+        const WgSeg G[4] = {J.a, J.x[0], J.x[1], J.x[2]};
+        const int nx = J.nx, M = J.M, own = 8 * warp + (lane & 7), piece = lane & 7;
+        uint32_t off[4];
+        off[0] = 0;
+        off[1] = 2 * WG_BLOCK;
+        off[2] = off[1] + (G[1].width / 64) * WG_BLOCK;
+        off[3] = off[2] + (G[2].width / 64) * WG_BLOCK;
+        auto load_rows = [&](int c, const __nv_bfloat16 *(&o)[4]) {
+            const int r = c * 64 + own;
+            const bool in = c < c1 && r < M;
 #pragma unroll
-            for (int x = 0; x < 3; ++x) o[1 + x] = in && x < J.nx ? (J.x[x].rows ? (int64_t)J.x[x].rows[r] : (int64_t)r) : -1;
+            for (int x = 0; x < 4; ++x) {
+                o[x] = nullptr;
+                if (in && x <= nx) o[x] = G[x].base + (G[x].rows ? (int64_t)G[x].rows[r] : (int64_t)r) * G[x].ld;
+            }
         };
+        const __nv_bfloat16 *row[4], *nrow[4];
         load_rows(c0, row);
-        int q = 0;
-        for (int c = c0; c < c1 && !bad; ++c, ++q) {
+        int s = 0, u = 0;
+        for (int c = c0; c < c1 && !bad; ++c) {
             load_rows(c + 1, nrow);
-            const int s = q % S, u = q / S;
             if (u > 0 && !warp_wait(ringe + 8 * s, (u - 1) & 1)) {
                 bad = true;
                 break;
             }
-            uint32_t dst = sR + s * stage;
+            const uint32_t dst = sR + s * stage;
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
-                if (x > J.nx) break;
-                const WgSeg &G = x == 0 ? J.a : J.x[x == 0 ? 0 : x - 1];
-                const int piece = lane & 7;
+                if (x <= nx) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int rr = 4 * i + (lane >> 3), R = 16 * warp + rr;
-                    const int64_t src = __shfl_sync(0xffffffffu, row[x], rr);
-                    const uint32_t d = dst + (uint32_t)(R * 128 + ((piece ^ (R & 7)) << 4));
-                    for (int b = 0; b < G.width / 64; ++b) {
-                        if (src >= 0) cp_async16(d + b * WG_BLOCK, G.base + src * G.ld + b * 64 + piece * 8);
-                        else asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(d + b * WG_BLOCK), "r"(0u) : "memory");
+                    for (int i = 0; i < 2; ++i) {
+                        const int rr = 4 * i + (lane >> 3), R = 8 * warp + rr;
+                        const __nv_bfloat16 *src = (const __nv_bfloat16 *)__shfl_sync(0xffffffffu, (uint64_t)row[x], rr);
+                        const uint32_t d = dst + off[x] + (uint32_t)(R * 128 + ((piece ^ (R & 7)) << 4));
+                        if (src) {
+                            cp_async16(d, src + piece * 8);
+                            if (G[x].width == 128) cp_async16(d + WG_BLOCK, src + 64 + piece * 8);
+                        } else {
+                            asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(d), "r"(0u) : "memory");
+                            if (G[x].width == 128)
+                                asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(d + WG_BLOCK), "r"(0u) : "memory");
+                        }
                     }
                 }
-                dst += (x == 0 ? 2 : G.width / 64) * WG_BLOCK;
             }
             cp_async_arrive_noinc(ringf + 8 * s);
 #pragma unroll
             for (int x = 0; x < 4; ++x) row[x] = nrow[x];
+            if (++s == S) {
+                s = 0;
+                ++u;
+            }
         }
         cp_async_wait_all();
         // the partial product: thread = one output row
         if (!bad && !warp_wait(done, 0)) bad = true;
         if (!bad) {
             tmem_fence_after();
-            const int r = warp * 32 + lane;
+            const int r = (warp & 3) * 32 + lane;
             float *out = J.part + ((int64_t)li * J.a.width + r) * J.n_in;
-            for (int cb = 0; cb < J.n_in; cb += 32) {
+            for (int cb = (warp >> 2) * 32; cb < J.n_in; cb += 64) {
                 uint32_t v[32];
-                tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)cb, v);
+                tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cb, v);
                 if (r < J.a.width) {
 #pragma unroll
                     for (int u = 0; u < 32; u += 8) st8u(out + cb + u, v + u);
@@ -913,10 +930,13 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad(const __grid_constant__
         }
     } else {
         const bool issuer = elect_one();
-        int q = 0;
-        for (int c = c0; c < c1 && !bad; ++c, ++q) {
-            const int s = q % S;
-            if (!warp_wait(ringf + 8 * s, (q / S) & 1)) {
+        // at most 256 columns an instruction: columns [0, w0) and [256, n_in)
+        const int n_in = J.n_in, w0 = min(256, n_in);
+        const uint32_t i0 = umma_idesc_bf16_mn(w0), i1 = umma_idesc_bf16_mn(n_in > 256 ? n_in - 256 : 64);
+        int s = 0, ph = 0;
+        uint32_t acc = 0u;
+        for (int c = c0; c < c1 && !bad; ++c) {
+            if (!warp_wait(ringf + 8 * s, ph)) {
                 bad = true;
                 break;
             }
@@ -926,13 +946,15 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad(const __grid_constant__
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {  // 16 rows each
                     const uint64_t da = umma_desc_mn_sw128(a0 + k * 2048, WG_BLOCK);
-                    for (int n = 0; n < J.n_in; n += 256) {  // at most 256 columns an instruction
-                        const int w = min(256, J.n_in - n);
-                        umma_bf16(tmem + (uint32_t)n, da, umma_desc_mn_sw128(x0 + (n / 64) * WG_BLOCK + k * 2048, WG_BLOCK),
-                                  umma_idesc_bf16_mn(w), (q > 0 || k > 0) ? 1u : 0u);
-                    }
+                    umma_bf16(tmem, da, umma_desc_mn_sw128(x0 + k * 2048, WG_BLOCK), i0, acc);
+                    if (n_in > 256) umma_bf16(tmem + 256u, da, umma_desc_mn_sw128(x0 + 4 * WG_BLOCK + k * 2048, WG_BLOCK), i1, acc);
+                    acc = 1u;
                 }
                 umma_commit(ringe + 8 * s);
+            }
+            if (++s == S) {
+                s = 0;
+                ph ^= 1;
             }
         }
         if (issuer) umma_commit(done);

@@ -146,6 +146,21 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
     return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, MM_WAIT_NS));
 }
 
+// Producer warp's part of a 128-row chunk: its 32 rows, four whole 128-byte
+// row pieces per instruction.  `own`: this lane's row pointer (nullptr: the
+// row is left as it is), at the chunk's first column.
+__device__ __forceinline__ void warp_copy_rows(const __nv_bfloat16 *own, uint32_t sdst, int pw, int lane) {
+    const int c = lane & 7;
+    const uint64_t p = (uint64_t)own;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int rr = 4 * i + (lane >> 3);
+        const uint64_t row = __shfl_sync(0xffffffffu, p, rr);
+        const int R = 32 * pw + rr;
+        if (row) cp_async16(sdst + (uint32_t)(R * 128 + ((c ^ (R & 7)) << 4)), (const __nv_bfloat16 *)row + c * 8);
+    }
+}
+
 // 64-wide K chunk c of a bf16 matrix's rows [0, n) into the K-major 128-byte-swizzle layout at
 // sdst (rows n .. 127 zeroed); every thread of the block takes part, cp.async.
 __device__ __forceinline__ void load_weight_chunk(const __nv_bfloat16 *w, int64_t ldw, int n, int c, uint32_t sdst,
