@@ -98,3 +98,31 @@ def test_forward_rejects_inputs_of_another_shape():
         net.forward(g, x[:-1], train=False)
     with pytest.raises(ValueError):
         net.forward(g, x.float(), train=False)
+
+
+def test_union_of_copies_on_the_device_matches_the_shifted_host_arrays():
+    """The union's index arrays and its host copies (no GPU needed: torch on the CPU)."""
+
+    pytest.importorskip("torch")
+    from floodgb.surrogate.model import DualGraph
+    from floodgb.synthetic import make_grid_city
+
+    g = DualGraph(make_grid_city(n=5, size_m=50.0, seed=2).city.topologies.surface_topology, device="cpu")
+    k = 3
+    u = g.replicate(k)
+    assert (u.C, u.E, u.max_in, u.max_out) == (k * g.C, k * g.E, g.max_in, g.max_out)
+    for name, step in (("src", g.C), ("dst", g.C), ("send_order", g.E)):
+        want = np.concatenate([getattr(g, name).numpy() + j * step for j in range(k)])
+        np.testing.assert_array_equal(getattr(u, name).numpy(), want)
+    for name in ("recv_start", "send_start"):
+        a = getattr(g, name).numpy()
+        want = np.concatenate([a[:-1] + j * g.E for j in range(k)] + [[k * g.E]])
+        np.testing.assert_array_equal(getattr(u, name).numpy(), want)
+    np.testing.assert_array_equal(u.row_start.numpy(), np.arange(k * g.E + 1))
+    np.testing.assert_array_equal(u.src_h, u.src.numpy())
+    np.testing.assert_array_equal(u.dst_h, u.dst.numpy())
+    np.testing.assert_array_equal(u.indeg_h, u.indeg.numpy())
+    np.testing.assert_array_equal(u.edge_features_h, np.tile(g.edge_features_h, (k, 1)))
+    assert u.ef_bf.shape == (k * g.E, 64) and all(t.is_contiguous() for t in (u.src, u.ef_bf, u.recv_start))
+    with pytest.raises(AttributeError):
+        u.no_such_array
