@@ -396,7 +396,11 @@ static const void *surface_batch_fn(int kind, int tile) {
 
 cudaError_t batch_configure(int kind, int tile, int smem_bytes, int *per_sm) {
     const void *fn = surface_batch_fn(kind, tile);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+    // the device's own limit: the attribute is the function's, shared by every batch
+    int dev = 0, most = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, tile, (size_t)smem_bytes);
 }

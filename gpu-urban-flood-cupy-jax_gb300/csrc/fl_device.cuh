@@ -410,6 +410,7 @@ __device__ __forceinline__ void warp_add_ledger_at(const float (&v)[NT], float2 
 // one start; wait blocks until every prerequisite grid has completed and its
 // writes are visible (a no-op in a grid launched without the attribute).
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // --------------------------------------------------------------- async copies

@@ -93,13 +93,13 @@ __device__ __forceinline__ float node_depth(float2 V, float A) {
 // record arrives, so its latency overlaps theirs instead of adding to the
 // dependent-load chain.
 //
-// k_links, k_donor and k_network are launched as programmatic dependents of
-// the kernel before them: each kernel lets its dependent launch as soon as
+// All four are launched as programmatic dependents of the kernel before them: each kernel lets its dependent launch as soon as
 // its own blocks run (griddepcontrol.launch_dependents), and the dependent
 // loads its static tables, then waits for the whole previous grid to finish
 // and its writes to be visible (griddepcontrol.wait) before it reads them.
 // The launch latency and the static loads of each kernel overlap the
-// previous one.  k_nodes follows the surface kernel with an ordinary launch.
+// previous one.  (A surface grid that fills the device lets k_nodes start only
+// at its end.)
 
 
 // Capture limit factor of an inlet cell at depth h: its volume over the
@@ -366,8 +366,14 @@ __global__ void __launch_bounds__(128) k_nodes(const __grid_constant__ NodeArgs 
     pdl_launch_dependents();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = n < a.N;
-    const float2 V = in ? ff_clamp0(a.Va[n]) : make_float2(0.0f, 0.0f);
     const int j0 = in ? a.node_in_start[n] : 0, j1 = in ? a.node_in_start[n + 1] : 0;
+    if (j0 < j1) {  // the first inlet's static records, on their way to L1 during the wait
+        const int4 qk = a.in_qk[j0];
+        prefetch_l1(&a.inl.in_par[qk.x]);
+        prefetch_l1(&a.cinfo[qk.y]);
+    }
+    pdl_wait();  // the surface kernel's depths
+    const float2 V = in ? ff_clamp0(a.Va[n]) : make_float2(0.0f, 0.0f);
     const StepCtrl s = a.ctrl[slot];
     if (!s.active || !(s.phases & FL_PHASE_DRAINAGE)) return;
     float led[D1_TERMS] = {0.0f, 0.0f};
@@ -583,13 +589,6 @@ cudaError_t launch_recharge(const RechargeArgs &a, int slot, cudaStream_t stream
 int node_blocks(int32_t N) { return (N + 127) / 128 > 0 ? (N + 127) / 128 : 1; }
 int network_blocks(int32_t G) { return (G + 127) / 128 > 0 ? (G + 127) / 128 : 1; }
 
-cudaError_t launch_nodes(const NodeArgs &a, int slot, cudaStream_t stream) {
-    const dim3 grid((unsigned)node_blocks(a.N), (unsigned)std::max(a.ms.n, 1));
-    if (a.ms.n > 1) k_nodes<true><<<grid, 128, 0, stream>>>(a, slot);
-    else k_nodes<false><<<grid, 128, 0, stream>>>(a, slot);
-    return cudaGetLastError();
-}
-
 int link_blocks(int32_t L) { return (L + 127) / 128 > 0 ? (L + 127) / 128 : 1; }
 
 // Launch as a programmatic dependent of the previous kernel in the stream.
@@ -607,6 +606,10 @@ static cudaError_t launch_dependent(void (*kernel)(Args, int), int blocks, const
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, a, slot);
+}
+
+cudaError_t launch_nodes(const NodeArgs &a, int slot, cudaStream_t stream) {
+    return launch_dependent(a.ms.n > 1 ? k_nodes<true> : k_nodes<false>, node_blocks(a.N), a, slot, stream);
 }
 
 cudaError_t launch_links(const LinkArgs &a, int slot, cudaStream_t stream) {

@@ -176,6 +176,11 @@ struct SurfArgs {
     float g, half_g, md, vmax, stage;
     int32_t has_stage;
     const float *ext_add;         // [Cp] external inflow depth of receiver cells this step
+    int32_t early;                // the dependent kernel may start beside this grid
+    // ensemble members (members > 1: gridDim.y): strides of the per-member arrays
+    int32_t members, max_snaps;
+    int64_t m_cells, m_led, m_snap;
+    const HyetoView *hys;         // [members]
 };
 
 // Local-inertial surface step (two launches: edge discharge, cell update with

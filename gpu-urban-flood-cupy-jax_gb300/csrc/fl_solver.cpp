@@ -146,7 +146,7 @@ struct FlSolver {
     bool has_table() const { return sur.U > 0; }
     bool has_recharge() const { return rch.U > 0; }
     int launches_per_step() const {
-        return (li_mode ? 2 : 1) * members + (has_drain() ? 4 : 0) + (has_table() ? 1 : 0) + (has_inflow() ? 1 : 0) +
+        return (li_mode ? 2 : 1) + (has_drain() ? 4 : 0) + (has_table() ? 1 : 0) + (has_inflow() ? 1 : 0) +
                (has_recharge() ? 1 : 0);
     }
 
@@ -241,22 +241,6 @@ static int push_run(FlSolver *s, cudaStream_t st) {
 
 // The surface / CFL kernel arguments of member m: the solver's arguments
 // (the shared tables and settings) with that member's arrays.
-static SurfArgs surf_args(const FlSolver *s, int m) {
-    SurfArgs a = s->sa;
-    a.state0 = s->mb.state[0] + (size_t)m * s->Cp;
-    a.state1 = s->mb.state[1] + (size_t)m * s->Cp;
-    a.wet = s->mb.wet + (size_t)m * s->Cp;
-    a.ctrl = s->mb.ctrl + 2 * (size_t)m;
-    a.run = s->mb.run + m;
-    a.hy = s->hys[m];
-    a.ledger = s->mb.led_s + (size_t)m * s->n_led_s;
-    a.snap_h = s->mb.snap_h + m * s->snap_stride_h();
-    a.snap_hu = s->mb.snap_hu + m * s->snap_stride_h();
-    a.snap_hv = s->mb.snap_hv + m * s->snap_stride_h();
-    a.snap_t = s->mb.snap_t + (size_t)m * s->params.max_snapshots;
-    return a;
-}
-
 static DtArgs dt_args(const FlSolver *s, int m) {
     DtArgs d = s->da;
     d.state0 = s->mb.state[0] + (size_t)m * s->Cp;
@@ -284,9 +268,9 @@ static int launch_step(FlSolver *s, int slot, bool eval, bool plan_next, cudaStr
         FL_CUDA(launch_li(s->li, s->kind, slot, plan_next ? 1 : 0, s->sms, st));
         g_launches += 2;
     } else {
-        for (int m = 0; m < s->members; ++m)
-            FL_CUDA(launch_surface(surf_args(s, m), s->kind, slot, plan_next ? 1 : 0, s->surf_grid, s->surf_smem, st));
-        g_launches += s->members;
+        // (several members: s->sa addresses member 0 and one launch runs all)
+        FL_CUDA(launch_surface(s->sa, s->kind, slot, plan_next ? 1 : 0, s->surf_grid, s->surf_smem, st));
+        g_launches++;
     }
     if (s->has_drain()) {
         FL_CUDA(launch_nodes(s->nd, slot, st));
@@ -596,6 +580,7 @@ static int create_impl(const FlMeshDesc *mesh, const FlDrainDesc *drain, const F
     s->sa.n_tiles = (int32_t)L.tile_info.size();
     s->sa.e_cap = L.e_cap;
     s->sa.h_cap = L.h_cap;
+    s->sa.members = M;
     FL_CUDA(plan_surface_launch(s->sa, s->kind, device, &s->surf_grid, &s->surf_smem));
     int sms = 0;
     FL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
@@ -832,6 +817,13 @@ static int create_impl(const FlMeshDesc *mesh, const FlDrainDesc *drain, const F
     a.vmax = (float)p.max_speed_mps;
     a.stage = mesh->has_stage_boundary ? mesh->boundary_stage_m : 0.0f;
     a.has_stage = mesh->has_stage_boundary;
+    a.max_snaps = p.max_snapshots;
+    a.m_cells = Cp;
+    a.m_led = (int64_t)s->n_led_s;
+    a.m_snap = (int64_t)s->snap_stride_h();
+    HyetoView *hys = nullptr;
+    if ((rc = s->upload(&hys, s->hys))) return rc;
+    a.hys = hys;
     DtArgs &d = s->da;
     d.state0 = s->state[0];
     d.state1 = s->state[1];

@@ -63,27 +63,35 @@ __device__ __forceinline__ TileStage stage_at(const SurfArgs &a, unsigned char *
     return t;
 }
 
-// Issue the bulk copies of tile t into a stage (one thread).  The byte count
-// the barrier expects is the sum of exactly the copies issued here.
+// Issue the bulk copies of tile t into a stage (one thread): the static part
+// (cell info, Horton fields, entries, halo list) and the part that a step
+// writes (states, wet time).  The byte count a barrier expects is the sum of
+// exactly the copies issued for it.
 template <int KIND>
-__device__ __forceinline__ void issue_tile(const SurfArgs &a, const float4 *in, const TileStage &S, int4 *info_slot,
-                                           uint32_t bar, int t) {
-    const int4 ti = a.tile_info[t];
-    *info_slot = ti;
+__device__ __forceinline__ uint32_t static_bytes(const int4 ti) {
+    return TILE * 16u + (KIND == 1 ? TILE * 16u : 0u) + (uint32_t)ti.y * 16u + (uint32_t)((ti.w + 3) & ~3) * 4u;
+}
+template <int KIND>
+__device__ __forceinline__ uint32_t step_bytes() {
+    return TILE * 16u + (KIND == 1 ? TILE * 4u : 0u);
+}
+
+template <int KIND>
+__device__ __forceinline__ void issue_static(const SurfArgs &a, const TileStage &S, const int4 ti, uint32_t bar, int t) {
     const uint32_t ent_bytes = (uint32_t)ti.y * 16u;
     const uint32_t halo_bytes = (uint32_t)((ti.w + 3) & ~3) * 4u;
-    uint32_t bytes = TILE * 16u * 2u + ent_bytes + halo_bytes;
-    if (KIND == 1) bytes += TILE * 16u + TILE * 4u;
-    mbar_arrive_expect_tx(bar, bytes);
     const size_t c0 = (size_t)t * TILE;
-    bulk_copy_g2s(smem_addr(S.st), in + c0, TILE * 16u, bar);
     bulk_copy_g2s(smem_addr(S.ci), a.cinfo + c0, TILE * 16u, bar);
-    if (KIND == 1) {
-        bulk_copy_g2s(smem_addr(S.hz), a.horton + c0, TILE * 16u, bar);
-        bulk_copy_g2s(smem_addr(S.wt), a.wet + c0, TILE * 4u, bar);
-    }
+    if (KIND == 1) bulk_copy_g2s(smem_addr(S.hz), a.horton + c0, TILE * 16u, bar);
     if (ent_bytes) bulk_copy_g2s(smem_addr(S.en), a.ent + ti.x, ent_bytes, bar);
     if (halo_bytes) bulk_copy_g2s(smem_addr(S.hs), a.halo_src + ti.z, halo_bytes, bar);
+}
+
+template <int KIND>
+__device__ __forceinline__ void issue_step(const float4 *in, const float *wet, const TileStage &S, uint32_t bar, int t) {
+    const size_t c0 = (size_t)t * TILE;
+    bulk_copy_g2s(smem_addr(S.st), in + c0, TILE * 16u, bar);
+    if (KIND == 1) bulk_copy_g2s(smem_addr(S.wt), wet + c0, TILE * 4u, bar);
 }
 
 // Named barrier and barrier-reduction among the compute warps only (id 1).
@@ -115,20 +123,34 @@ __device__ __forceinline__ bool compute_all(bool p) {
 // the next tile therefore overlap both compute phases of the current one.
 // Every wait is bounded (1 s): a timeout records FL_E_TIMEOUT and the CTA
 // leaves after its copies in flight have landed (or a second bounded wait).
-template <int KIND>
+//
+// The static part of a CTA's first tile is fetched before the wait for the
+// step's previous kernel (barrier pre).  A grid that leaves CTA slots free
+// (a.early) also lets its dependent start once its own wait is over: the next
+// kernel's CTAs are then set up, with that fetch done, when this one ends.
+// (A grid that fills the device does not: CTAs waiting next to it cost more
+// than the launch latency they hide.)  Ensemble members (MEM): one launch,
+// blockIdx.y = member, each with the grid of a single run.
+template <int KIND, bool MEM>
 __global__ void __launch_bounds__(SURF_THREADS, 4) k_surface(const __grid_constant__ SurfArgs a, int slot, int plan_next) {
     extern __shared__ __align__(128) unsigned char smem[];
     float4 *s_flux = (float4 *)smem;  // [TILE * 3] per (cell, slot): {mass, x-mom, y-mom} x len
-    uint64_t *s_bar = (uint64_t *)(smem + a.off_bar);  // full[2], halo[2], empty[2]
-    int4 *s_info = (int4 *)(smem + a.off_bar + 48);
+    uint64_t *s_bar = (uint64_t *)(smem + a.off_bar);  // full[2], halo[2], empty[2], pre
+    int4 *s_info = (int4 *)(smem + a.off_bar + 64);
     const int tid = threadIdx.x;
     const int ncta = (int)gridDim.x - 1;  // the last CTA plans
+    const size_t mem = MEM ? blockIdx.y : 0;
+    RunCtrl *run = a.run + mem;
+    const StepCtrl *ctrl = a.ctrl + 2 * mem;
     if ((int)blockIdx.x == ncta) {
         pdl_wait();
-        if (plan_next && tid == 0) plan_step(a.run, a.snap_t, a.hy, &a.ctrl[slot ^ 1], false, 0.0f, FL_PHASE_ALL);
+        if (a.early) pdl_launch_dependents();
+        if (plan_next && tid == 0)
+            plan_step(run, a.snap_t + mem * (size_t)a.max_snaps, MEM ? a.hys[mem] : a.hy, &a.ctrl[2 * mem + (slot ^ 1)],
+                      false, 0.0f, FL_PHASE_ALL);
         return;
     }
-    // barrier addresses: full(s) = base + 8 s, halo(s) = base + 16 + 8 s, empty(s) = base + 32 + 8 s
+    // barrier addresses: full(s) = base + 8 s, halo(s) = base + 16 + 8 s, empty(s) = base + 32 + 8 s, pre = base + 48
     const uint32_t bar_base = smem_addr(s_bar);
     const TileStage S0 = stage_at(a, smem, 0), S1 = stage_at(a, smem, 1);
     if (tid < TILE) {
@@ -141,17 +163,31 @@ __global__ void __launch_bounds__(SURF_THREADS, 4) k_surface(const __grid_consta
             mbar_init(bar_base + 16u + 8u * k, 32);
             mbar_init(bar_base + 32u + 8u * k, TILE / 32);  // one arrival per compute warp
         }
+        mbar_init(bar_base + 48u, 1);
         mbar_fence_init();
     }
     __syncthreads();  // the last block-wide barrier: the roles split here
+    if (tid == TILE) {  // (every CTA has a tile)
+        const int4 ti = a.tile_info[blockIdx.x];
+        s_info[0] = ti;
+        mbar_arrive_expect_tx(bar_base + 48u, static_bytes<KIND>(ti));
+        issue_static<KIND>(a, S0, ti, bar_base + 48u, blockIdx.x);
+    }
     // launched as a programmatic dependent of the step's previous kernel: the
     // set-up above overlaps its end; the step record, the states and the wet
     // time it (or an earlier kernel) wrote are read after this wait
     pdl_wait();
-    const StepCtrl s = a.ctrl[slot];
-    if (!s.active) return;  // (uniform over the grid)
-    const float4 *__restrict__ in = s.parity ? a.state1 : a.state0;
-    float4 *__restrict__ out = s.parity ? a.state0 : a.state1;
+    if (a.early) pdl_launch_dependents();
+    const StepCtrl s = ctrl[slot];
+    if (!s.active) {  // (uniform over the member's grid; no copy may land after the CTA leaves)
+        if (tid == TILE && !mbar_wait_bounded(bar_base + 48u, 0, COPY_WAIT_NS))
+            (void)mbar_wait_bounded(bar_base + 48u, 0, COPY_WAIT_NS);
+        return;
+    }
+    const size_t mc = MEM ? mem * (size_t)a.m_cells : 0;
+    const float4 *__restrict__ in = (s.parity ? a.state1 : a.state0) + mc;
+    float4 *__restrict__ out = (s.parity ? a.state0 : a.state1) + mc;
+    float *__restrict__ wet = a.wet + mc;
 
     if (tid >= TILE) {
         // ---------------------------------------------------------- producer
@@ -169,12 +205,27 @@ __global__ void __launch_bounds__(SURF_THREADS, 4) k_surface(const __grid_consta
                     break;
                 }
             }
-            if (lane == 0) issue_tile<KIND>(a, in, S, &s_info[st], (bar_base + 8u * st), t);
+            if (lane == 0) {
+                const uint32_t bar = bar_base + 8u * st;
+                if (i == 0) {
+                    mbar_arrive_expect_tx(bar, step_bytes<KIND>());
+                } else {
+                    const int4 ti = a.tile_info[t];
+                    s_info[st] = ti;
+                    mbar_arrive_expect_tx(bar, static_bytes<KIND>(ti) + step_bytes<KIND>());
+                    issue_static<KIND>(a, S, ti, bar, t);
+                }
+                issue_step<KIND>(in, wet, S, bar, t);
+            }
             // every lane waits: each then reads the landed halo list itself
-            const bool ok = mbar_wait_bounded((bar_base + 8u * st), (i >> 1) & 1u, COPY_WAIT_NS);
+            // (the first tile's landed on pre; its gathers go out before its states are in)
+            const uint32_t lbar = i == 0 ? bar_base + 48u : bar_base + 8u * st;
+            const uint32_t lpar = i == 0 ? 0u : (uint32_t)((i >> 1) & 1);
+            const bool ok = mbar_wait_bounded(lbar, lpar, COPY_WAIT_NS);
             if (!__all_sync(0xffffffffu, ok)) {
                 // a copy is late: one more bounded wait so none lands after the CTA leaves
-                (void)mbar_wait_bounded((bar_base + 8u * st), (i >> 1) & 1u, COPY_WAIT_NS);
+                (void)mbar_wait_bounded(lbar, lpar, COPY_WAIT_NS);
+                if (i == 0) (void)mbar_wait_bounded(bar_base + 8u * st, 0u, COPY_WAIT_NS);
                 failed = true;
                 break;
             }
@@ -184,7 +235,7 @@ __global__ void __launch_bounds__(SURF_THREADS, 4) k_surface(const __grid_consta
         }
         cp_async_wait_all();
         if (failed && lane == 0) {
-            if (atomicCAS(&a.run->error, 0, FL_E_TIMEOUT) == 0) a.run->error_step = s.step;
+            if (atomicCAS(&run->error, 0, FL_E_TIMEOUT) == 0) run->error_step = s.step;
         }
         return;
     }
@@ -204,10 +255,11 @@ __global__ void __launch_bounds__(SURF_THREADS, 4) k_surface(const __grid_consta
         // reduction hands them to the other compute threads
         bool ok = true;
         if (tid == 0)
-            ok = mbar_wait_bounded((bar_base + 8u * st_i), (i >> 1) & 1u, COPY_WAIT_NS) &&
+            ok = (i > 0 || mbar_wait_bounded(bar_base + 48u, 0u, COPY_WAIT_NS)) &&
+                 mbar_wait_bounded((bar_base + 8u * st_i), (i >> 1) & 1u, COPY_WAIT_NS) &&
                  mbar_wait_bounded((bar_base + 16u + 8u * st_i), (i >> 1) & 1u, COPY_WAIT_NS);
         if (!compute_all(ok)) {
-            if (tid == 0 && atomicCAS(&a.run->error, 0, FL_E_TIMEOUT) == 0) a.run->error_step = s.step;
+            if (tid == 0 && atomicCAS(&run->error, 0, FL_E_TIMEOUT) == 0) run->error_step = s.step;
             break;  // the producer waits out its own copies
         }
 
@@ -228,7 +280,7 @@ __global__ void __launch_bounds__(SURF_THREADS, 4) k_surface(const __grid_consta
             const float4 ci = S.ci[tid];
             const uint32_t info = __float_as_uint(ci.z);
             if (s.check_finite && !isfinite(st.x)) {
-                if (atomicCAS(&a.run->error, 0, FL_E_NONFINITE) == 0) a.run->error_step = s.step;
+                if (atomicCAS(&run->error, 0, FL_E_NONFINITE) == 0) run->error_step = s.step;
             }
             float wt = 0.0f;
             float4 hz = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
@@ -255,9 +307,9 @@ __global__ void __launch_bounds__(SURF_THREADS, 4) k_surface(const __grid_consta
             out[c] = make_float4(hn, hun, hvn, st.w);
             const bool final_here = !(drain_finishes && (info & CELL_COUPLED)) &&
                                     !(recharge_finishes && (info & CELL_RECHARGE));
-            if (KIND == 1 && do_surface && final_here) a.wet[c] = wt + dt * (float)(hn > md);
+            if (KIND == 1 && do_surface && final_here) wet[c] = wt + dt * (float)(hn > md);
             if (s.snap_slot >= 0) {
-                const size_t o = (size_t)s.snap_slot * (size_t)a.C + (size_t)c;
+                const size_t o = (MEM ? mem * (size_t)a.m_snap : 0) + (size_t)s.snap_slot * (size_t)a.C + (size_t)c;
                 if (final_here) a.snap_h[o] = hn;
                 a.snap_hu[o] = hun;
                 a.snap_hv[o] = hvn;
@@ -270,11 +322,9 @@ __global__ void __launch_bounds__(SURF_THREADS, 4) k_surface(const __grid_consta
         __syncwarp();
         if ((tid & 31) == 0) mbar_arrive((bar_base + 32u + 8u * st_i));
     }
-    warp_add_ledger_at<SURF_TERMS>(led, a.ledger, (int)blockIdx.x * (TILE / 32) + (tid >> 5));
+    warp_add_ledger_at<SURF_TERMS>(led, a.ledger + (MEM ? mem * (size_t)a.m_led : 0), (int)blockIdx.x * (TILE / 32) + (tid >> 5));
 }
 
-template __global__ void k_surface<0>(const __grid_constant__ SurfArgs, int, int);
-template __global__ void k_surface<1>(const __grid_constant__ SurfArgs, int, int);
 
 // Global CFL minimum over all cells; the last block plans the step.
 __global__ void __launch_bounds__(256) k_dt(const __grid_constant__ DtArgs a, int slot, int plan) {
@@ -452,7 +502,7 @@ namespace fl {
 cudaError_t launch_surface(const SurfArgs &a, int kind, int slot, int plan_next, int grid, int smem_bytes,
                            cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
+    cfg.gridDim = dim3((unsigned)grid, (unsigned)std::max(a.members, 1));
     cfg.blockDim = dim3(SURF_THREADS);
     cfg.dynamicSmemBytes = (size_t)smem_bytes;
     cfg.stream = stream;
@@ -461,8 +511,9 @@ cudaError_t launch_surface(const SurfArgs &a, int kind, int slot, int plan_next,
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return kind ? cudaLaunchKernelEx(&cfg, k_surface<1>, a, slot, plan_next)
-                : cudaLaunchKernelEx(&cfg, k_surface<0>, a, slot, plan_next);
+    void (*fn)(SurfArgs, int, int) = a.members > 1 ? (kind ? k_surface<1, true> : k_surface<0, true>)
+                                                   : (kind ? k_surface<1, false> : k_surface<0, false>);
+    return cudaLaunchKernelEx(&cfg, fn, a, slot, plan_next);
 }
 
 // The persistent grid of k_surface: every CTA slot of the device (never more
@@ -475,10 +526,16 @@ cudaError_t launch_surface(const SurfArgs &a, int kind, int slot, int plan_next,
 // ledger slot sums the same values in the same order.
 cudaError_t plan_surface_launch(SurfArgs &a, int kind, int device, int *grid, int *smem_bytes) {
     *smem_bytes = surface_smem_layout(a, kind);
-    const void *fn = kind ? (const void *)k_surface<1> : (const void *)k_surface<0>;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, *smem_bytes);
+    const void *fn = kind ? (const void *)k_surface<1, false> : (const void *)k_surface<0, false>;
+    const void *fm = kind ? (const void *)k_surface<1, true> : (const void *)k_surface<0, true>;
+    // the limit belongs to the function, not to this solver: always the
+    // device's own, or a later solver with smaller tiles would lower it below
+    // what an earlier one launches with
+    int per_sm = 0, sms = 0, most = 0;
+    cudaError_t e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fm, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     if (e != cudaSuccess) return e;
-    int per_sm = 0, sms = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, SURF_THREADS, (size_t)*smem_bytes);
     if (e != cudaSuccess) return e;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -487,6 +544,8 @@ cudaError_t plan_surface_launch(SurfArgs &a, int kind, int device, int *grid, in
     const int slots = std::max(1, per_sm * sms - 1);
     const int ctas = std::max(1, std::min(slots, a.n_tiles));
     *grid = ctas + 1;
+    // the dependent may wait beside this grid while both fit twice over
+    a.early = 2ll * *grid * std::max(a.members, 1) <= per_sm * sms ? 1 : 0;
     return cudaSuccess;
 }
 
