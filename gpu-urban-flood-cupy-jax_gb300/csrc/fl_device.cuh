@@ -255,8 +255,8 @@ __device__ __forceinline__ float cfl_local_li(float h, float char_len, float cfl
 // inlet_exchange_request_kernel, triangular_inlet_exchange_cuda_kernels.py:52-131).
 // The head difference is (bed - invert) + h - V/A: a static datum offset plus
 // two small depths, exact in float32 at any elevation.
-__device__ __forceinline__ float2 inlet_request(const InletReqView &v, int i, float h_cell, float2 Vn, float dt) {
-    const float4 p = v.in_par[i];
+// p: the inlet's parameters (v.in_par[i]).
+__device__ __forceinline__ float2 inlet_request(const InletReqView &v, const float4 p, float h_cell, float2 Vn, float dt) {
     const float dn = fmax32(ff_val(Vn), 0.0f) / fmax32(p.w, 1.0e-12f);
     const float dh = p.x + h_cell - dn;
     const float capc = p.y * dt;

@@ -102,6 +102,21 @@ __device__ __forceinline__ float node_depth(float2 V, float A) {
 // at its end.)
 
 
+//
+// An item's static records (list ranges, the first four list entries, their
+// parameters) are loaded into registers before the wait; after it, everything
+// the item reads that a step writes is then one level of independent loads.
+// (Each level costs an L2 round trip, ~750 cycles, and a pass is little else:
+// read one inlet or link after the other, the node and network passes of a
+// 960-node network took 10,000 cycles each.)  k_nodes and k_network keep to 72
+// registers (seven blocks an SM): the records then cost no residency, which a
+// network of 118,768 nodes needs to hide its scattered sectors.  us per launch
+// before -> after, 960 nodes: k_nodes 5.0 -> 3.8, k_donor 2.0 -> 1.6, k_network
+// 5.2 -> 4.2; 118,768 nodes: 7.0 -> 6.6, 3.0 -> 2.2, 8.8 -> 8.5 (7.9 and 10.7
+// for the first and last at 78 and 96 registers).
+
+constexpr int DR_PRE = 4;  // list entries held in registers; the rest are read as they come
+
 // Capture limit factor of an inlet cell at depth h: its volume over the
 // summed capture requests of its inlets [q0, q1), in their order (reference
 // :133-177).  `own` is the capture request of the calling inlet: a cell whose
@@ -114,7 +129,14 @@ __device__ __forceinline__ float cell_capture_factor(const InletReqView &v, int 
     if (q1 - q0 == 1) {
         sum = sum + own;
     } else {
-        for (int q = q0; q < q1; ++q) sum += inlet_request(v, q, h, ff_clamp0(v.Va[v.in_node[q]]), dt).x;
+        for (int q = q0; q < q1; q += 2) {  // two at a time: most shared cells have two
+            const bool two = q + 1 < q1;
+            const int n0 = v.in_node[q], n1 = two ? v.in_node[q + 1] : n0;
+            const float4 p0 = v.in_par[q], p1 = two ? v.in_par[q + 1] : p0;
+            const float2 V0 = v.Va[n0], V1 = v.Va[n1];
+            sum += inlet_request(v, p0, h, ff_clamp0(V0), dt).x;
+            if (two) sum += inlet_request(v, p1, h, ff_clamp0(V1), dt).x;
+        }
     }
     return fmin32(1.0f, (fmax32(h, 0.0f) * area) / fmax32(sum, 1.0e-12f));
 }
@@ -123,79 +145,191 @@ __device__ __forceinline__ float cell_capture_factor(const InletReqView &v, int 
 // their cells (reference inlet_exchange_request_kernel :52-131), captures
 // limited by each cell's volume, surcharges by the node's, and the node
 // volume after the exchange.
-// V = the clamped start volume Va[n]; [j0, j1) = the node's inlets.
-__device__ __forceinline__ void node_item(const NodeArgs &a, const StepCtrl &s, int n, float2 V, int j0, int j1,
+struct NodeStatic {
+    int j0, j1;              // the node's inlets (node order)
+    int4 qk[DR_PRE];
+    float4 par[DR_PRE];
+    float area[DR_PRE];
+};
+
+__device__ __forceinline__ NodeStatic node_static(const NodeArgs &a, int n) {
+    NodeStatic t;
+    t.j0 = t.j1 = 0;
+    if (n < a.N) {
+        t.j0 = a.node_in_start[n];
+        t.j1 = a.node_in_start[n + 1];
+    }
+#pragma unroll
+    for (int u = 0; u < DR_PRE; ++u) t.qk[u] = t.j0 + u < t.j1 ? a.in_qk[t.j0 + u] : make_int4(0, 0, 0, 0);
+#pragma unroll
+    for (int u = 0; u < DR_PRE; ++u) {
+        t.par[u] = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+        t.area[u] = 1.0f;
+        if (t.j0 + u < t.j1) {
+            t.par[u] = a.inl.in_par[t.qk[u].x];
+            t.area[u] = a.cinfo[t.qk[u].y].x;
+            if (t.qk[u].w - t.qk[u].z > 1) {  // shared with another node's inlet
+                prefetch_l1(&a.inl.in_node[t.qk[u].z]);
+                prefetch_l1(&a.inl.in_par[t.qk[u].z]);
+            }
+        }
+    }
+    return t;
+}
+
+__device__ __forceinline__ void node_item(const NodeArgs &a, const StepCtrl &s, int n, const NodeStatic &t,
                                           float (&led)[D1_TERMS]) {
-    if (j0 == j1) {
+    const float4 *hs = s.parity ? a.state0 : a.state1;  // written by the surface step
+    const float2 Vr = a.Va[n];
+    float h[DR_PRE];
+#pragma unroll
+    for (int u = 0; u < DR_PRE; ++u) h[u] = t.j0 + u < t.j1 ? hs[t.qk[u].y].x : 0.0f;
+    const float2 V = ff_clamp0(Vr);
+    if (t.j0 == t.j1) {
         a.Vb[n] = V;
         return;
     }
-    const float4 *hs = s.parity ? a.state0 : a.state1;  // written by the surface step
     const float dt = s.dt_f;
     float sum = 0.0f;
-    for (int j = j0; j < j1; ++j) {
+    float2 r[DR_PRE];
+#pragma unroll
+    for (int u = 0; u < DR_PRE; ++u) {
+        r[u] = make_float2(0.0f, 0.0f);
+        if (t.j0 + u < t.j1) {
+            r[u] = inlet_request(a.inl, t.par[u], h[u], V, dt);
+            sum += r[u].y;
+        }
+    }
+    for (int j = t.j0 + DR_PRE; j < t.j1; ++j) {
         const int4 qk = a.in_qk[j];
-        sum += inlet_request(a.inl, qk.x, hs[qk.y].x, V, dt).y;
+        sum += inlet_request(a.inl, a.inl.in_par[qk.x], hs[qk.y].x, V, dt).y;
     }
     const float sf = fmin32(1.0f, fmax32(ff_val(V), 0.0f) / fmax32(sum, 1.0e-12f));
     float dv = 0.0f;
-    for (int j = j0; j < j1; ++j) {
-        const int4 qk = a.in_qk[j];
-        const int c = qk.y;
-        const float h = hs[c].x;
-        const float2 r = inlet_request(a.inl, qk.x, h, V, dt);
-        const float cap = r.x * cell_capture_factor(a.inl, qk.z, qk.w, r.x, h, a.cinfo[c].x, dt);
-        const float sur = r.y * sf;
+    auto grant = [&](const int4 qk, const float2 rq, float hc, float area) {
+        const float cap = rq.x * cell_capture_factor(a.inl, qk.z, qk.w, rq.x, hc, area, dt);
+        const float sur = rq.y * sf;
         a.capsur[qk.x] = make_float2(cap, sur);
         dv += cap - sur;
         led[0] += cap;
         led[1] += sur;
+    };
+#pragma unroll
+    for (int u = 0; u < DR_PRE; ++u)
+        if (t.j0 + u < t.j1) grant(t.qk[u], r[u], h[u], t.area[u]);
+    for (int j = t.j0 + DR_PRE; j < t.j1; ++j) {
+        const int4 qk = a.in_qk[j];
+        const float hc = hs[qk.y].x;
+        grant(qk, inlet_request(a.inl, a.inl.in_par[qk.x], hc, V, dt), hc, a.cinfo[qk.y].x);
     }
     a.Vb[n] = ff_add(V, dv);
 }
 
+// A node's link slots [js, je), the first ones in registers.
+struct SlotStatic {
+    int js, je;
+    int2 e[DR_PRE];
+};
+
+__device__ __forceinline__ SlotStatic slot_static(const int32_t *start, const int2 *nl, int n, bool in) {
+    SlotStatic t;
+    t.js = in ? start[n] : 0;
+    t.je = in ? start[n + 1] : 0;
+#pragma unroll
+    for (int u = 0; u < DR_PRE; ++u) t.e[u] = t.js + u < t.je ? nl[t.js + u] : make_int2(-1, 0);
+    return t;
+}
+
 // Node n: its donor factor min(1, V / sum of the transfers it gives), summed
 // in ascending link order.
-// [js, je) = the node's link slots.
-__device__ __forceinline__ float donor_item(const DonorArgs &a, int n, int js, int je) {
+__device__ __forceinline__ float donor_item(const DonorArgs &a, int n, const SlotStatic &st) {
+    const float2 Vr = __ldcg(&a.Vb[n]);
     float given = 0.0f;
-    for (int j0 = js; j0 < je; j0 += 4) {
-        int2 e[4];
+    for (int j0 = st.js; j0 < st.je; j0 += DR_PRE) {
+        int2 e[DR_PRE];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) e[u] = (j0 + u < je) ? a.nl[j0 + u] : make_int2(-1, 0);
-        float t[4];
+        for (int u = 0; u < DR_PRE; ++u)
+            e[u] = j0 == st.js ? st.e[u] : (j0 + u < st.je ? a.nl[j0 + u] : make_int2(-1, 0));
+        float t[DR_PRE];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) t[u] = e[u].x >= 0 ? __ldcg(&a.T[e[u].x]) : 0.0f;
+        for (int u = 0; u < DR_PRE; ++u) t[u] = e[u].x >= 0 ? __ldcg(&a.T[e[u].x]) : 0.0f;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < DR_PRE; ++u) {
             if (e[u].x < 0) continue;
             const uint32_t meta = (uint32_t)e[u].y;
             if (t[u] >= 0.0f ? (meta & NL_FROM) : (meta & NL_TO)) given += fabsf(t[u]);
         }
     }
-    return fmin32(1.0f, fmax32(ff_val(ff_clamp0(__ldcg(&a.Vb[n]))), 0.0f) / fmax32(given, 1.0e-12f));
+    return fmin32(1.0f, fmax32(ff_val(ff_clamp0(Vr)), 0.0f) / fmax32(given, 1.0e-12f));
 }
 
 // Group g: limited transfers, node continuity, outfall, overflow return and
 // the group cell's final depth.
-// gr = the group record grp[g]; ci = the cell info of its cell (if any).
-__device__ __forceinline__ void group_item(const NetArgs &a, const StepCtrl &s, int4 gr, float4 ci,
+struct GroupStatic {
+    int4 gr;                 // the group record
+    float4 ci;               // the cell info of its cell (if any)
+    int q0, q1;              // the cell's inlets
+    SlotStatic st;           // the first node's link slots and parameters
+    float4 nd;
+    float capv;
+};
+
+__device__ __forceinline__ GroupStatic group_static(const NetArgs &a, int g) {
+    GroupStatic t;
+    t.gr = g < a.G ? a.grp[g] : make_int4(-1, -1, 0, 0);
+    t.ci = t.gr.x >= 0 ? a.cinfo[t.gr.x] : make_float4(1.0f, 0.0f, 0.0f, 0.0f);
+    t.q0 = t.q1 = 0;
+    if (t.gr.x >= 0 && t.gr.y >= 0) {
+        t.q0 = a.kcell_start[t.gr.y];
+        t.q1 = a.kcell_start[t.gr.y + 1];
+    }
+    const bool node = t.gr.z < t.gr.w;
+    t.st = slot_static(a.node_link_start, a.nl, t.gr.z, node);
+    t.nd = node ? a.nd0[t.gr.z] : make_float4(1.0f, 0.0f, 0.0f, 0.0f);
+    t.capv = node ? a.nd_capv[t.gr.z] : 0.0f;
+    return t;
+}
+
+__device__ __forceinline__ void group_item(const NetArgs &a, const StepCtrl &s, const GroupStatic &gs,
                                            float (&led)[D2_TERMS]) {
     float4 *hs = s.parity ? a.state0 : a.state1;  // written by k_surface this step
     float *Qout = s.parity ? a.Q0 : a.Q1;
     const float dt = s.dt_f;
-    const int c = gr.x, k = gr.y;
-    float h = 0.0f, area = 1.0f;
+    const int4 gr = gs.gr;
+    const int c = gr.x;
+    // one level of loads: the cell's depth, its inlets' exchange, the first
+    // node's volume and factor, its transfers and their other ends' factors
+    float h = c >= 0 ? hs[c].x : 0.0f;
+    float2 cs[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) cs[u] = gs.q0 + u < gs.q1 ? __ldcg(&a.capsur[gs.q0 + u]) : make_float2(0.0f, 0.0f);
+    float2 V1 = make_float2(0.0f, 0.0f);
+    float f1 = 0.0f, t1[DR_PRE], o1[DR_PRE];
+    if (gr.z < gr.w) {
+        V1 = __ldcg(&a.Vb[gr.z]);
+        f1 = __ldcg(&a.fac[gr.z]);
+    }
+#pragma unroll
+    for (int u = 0; u < DR_PRE; ++u) {
+        t1[u] = o1[u] = 0.0f;
+        if (gs.st.e[u].x >= 0) {
+            t1[u] = __ldcg(&a.T[gs.st.e[u].x]);
+            o1[u] = __ldcg(&a.fac[(uint32_t)gs.st.e[u].y & NL_NODE_MASK]);
+        }
+    }
+    float area = 1.0f;
     uint32_t cflags = 0u;
     if (c >= 0) {
-        h = hs[c].x;
-        area = ci.x;
-        cflags = __float_as_uint(ci.z);
-        if (k >= 0) {  // the cell's inlet exchange, in its inlets' order
+        area = gs.ci.x;
+        cflags = __float_as_uint(gs.ci.z);
+        if (gr.y >= 0) {  // the cell's inlet exchange, in its inlets' order
             float dh = 0.0f;
-            for (int q = a.kcell_start[k]; q < a.kcell_start[k + 1]; ++q) {
-                const float2 cs = __ldcg(&a.capsur[q]);
-                dh += (cs.y - cs.x) / area;
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                if (gs.q0 + u < gs.q1) dh += (cs[u].y - cs[u].x) / area;
+            for (int q = gs.q0 + 2; q < gs.q1; ++q) {
+                const float2 x = __ldcg(&a.capsur[q]);
+                dh += (x.y - x.x) / area;
             }
             h = h + dh;
         }
@@ -203,24 +337,34 @@ __device__ __forceinline__ void group_item(const NetArgs &a, const StepCtrl &s, 
     float hd = 0.0f;
     double hd64 = 0.0;  // table mode: the fallback return depth in float64
     for (int n = gr.z; n < gr.w; ++n) {
-        const float2 Vp = ff_clamp0(__ldcg(&a.Vb[n]));
-        const float fn = __ldcg(&a.fac[n]);
-        const int js = a.node_link_start[n], je = a.node_link_start[n + 1];
+        const bool first = n == gr.z;
+        const float2 Vp = ff_clamp0(first ? V1 : __ldcg(&a.Vb[n]));
+        const float fn = first ? f1 : __ldcg(&a.fac[n]);
+        const int js = first ? gs.st.js : a.node_link_start[n], je = first ? gs.st.je : a.node_link_start[n + 1];
         float dv = 0.0f;
-        for (int j0 = js; j0 < je; j0 += 4) {
-            int2 e[4];
+        for (int j0 = js; j0 < je; j0 += DR_PRE) {
+            const bool held = first && j0 == js;
+            int2 e[DR_PRE];
+            float t[DR_PRE], fo[DR_PRE];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) e[u] = (j0 + u < je) ? a.nl[j0 + u] : make_int2(-1, 0);
-            float t[4], fo[4];
+            for (int u = 0; u < DR_PRE; ++u) {
+                e[u] = gs.st.e[u];
+                t[u] = t1[u];
+                fo[u] = o1[u];
+            }
+            if (!held) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (e[u].x >= 0) {
-                    t[u] = __ldcg(&a.T[e[u].x]);
-                    fo[u] = __ldcg(&a.fac[(uint32_t)e[u].y & NL_NODE_MASK]);
+                for (int u = 0; u < DR_PRE; ++u) e[u] = (j0 + u < je) ? a.nl[j0 + u] : make_int2(-1, 0);
+#pragma unroll
+                for (int u = 0; u < DR_PRE; ++u) {
+                    if (e[u].x >= 0) {
+                        t[u] = __ldcg(&a.T[e[u].x]);
+                        fo[u] = __ldcg(&a.fac[(uint32_t)e[u].y & NL_NODE_MASK]);
+                    }
                 }
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < DR_PRE; ++u) {
                 if (e[u].x < 0) continue;
                 const uint32_t meta = (uint32_t)e[u].y;
                 const bool is_from = (meta & NL_FROM) != 0, is_to = (meta & NL_TO) != 0;
@@ -239,7 +383,7 @@ __device__ __forceinline__ void group_item(const NetArgs &a, const StepCtrl &s, 
         }
         float2 V = ff_clamp0(ff_add(Vp, dv));
         // outfall (reference pipe_outfall_kernel :176-211)
-        const float4 nd = a.nd0[n];
+        const float4 nd = first ? gs.nd : a.nd0[n];
         const float vol = fmax32(ff_val(V), 0.0f);
         if (nd.z > 0.0f) {
             const float dh = nd.y + vol / fmax32(nd.x, 1.0e-12f);
@@ -250,7 +394,7 @@ __device__ __forceinline__ void group_item(const NetArgs &a, const StepCtrl &s, 
             V = ff_add(V, -out);
             led[0] += out;
         }
-        const float capv = a.nd_capv[n];
+        const float capv = first ? gs.capv : a.nd_capv[n];
         if (a.table) {
             // weighted return (reference triangular_backend.py:1424-1474) in
             // float64: a node with table entries returns overflow x weight
@@ -361,23 +505,16 @@ __device__ __forceinline__ NetArgs member_args(NetArgs a, int m) {
 }
 
 template <bool MEM>
-__global__ void __launch_bounds__(128) k_nodes(const __grid_constant__ NodeArgs a0, int slot) {
+__global__ void __launch_bounds__(128, 7) k_nodes(const __grid_constant__ NodeArgs a0, int slot) {
     const NodeArgs a = MEM ? member_args(a0, (int)blockIdx.y) : a0;
     pdl_launch_dependents();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool in = n < a.N;
-    const int j0 = in ? a.node_in_start[n] : 0, j1 = in ? a.node_in_start[n + 1] : 0;
-    if (j0 < j1) {  // the first inlet's static records, on their way to L1 during the wait
-        const int4 qk = a.in_qk[j0];
-        prefetch_l1(&a.inl.in_par[qk.x]);
-        prefetch_l1(&a.cinfo[qk.y]);
-    }
+    const NodeStatic t = node_static(a, n);
     pdl_wait();  // the surface kernel's depths
-    const float2 V = in ? ff_clamp0(a.Va[n]) : make_float2(0.0f, 0.0f);
     const StepCtrl s = a.ctrl[slot];
     if (!s.active || !(s.phases & FL_PHASE_DRAINAGE)) return;
     float led[D1_TERMS] = {0.0f, 0.0f};
-    if (in) node_item(a, s, n, V, j0, j1, led);
+    if (n < a.N) node_item(a, s, n, t, led);
     warp_add_ledger<D1_TERMS>(led, a.ledger);
 }
 
@@ -420,26 +557,25 @@ __global__ void __launch_bounds__(128) k_donor(const __grid_constant__ DonorArgs
     pdl_launch_dependents();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const StepCtrl s = a.ctrl[slot];
-    const int js = n < a.N ? a.node_link_start[n] : 0, je = n < a.N ? a.node_link_start[n + 1] : 0;
+    const SlotStatic t = slot_static(a.node_link_start, a.nl, n, n < a.N);
     pdl_wait();  // k_links' transfers
     if (n >= a.N) return;
-    const float fac = donor_item(a, n, js, je);
+    const float fac = donor_item(a, n, t);
     if (!s.active || !(s.phases & FL_PHASE_DRAINAGE)) return;
     a.fac[n] = fac;
 }
 
 template <bool MEM>
-__global__ void __launch_bounds__(128) k_network(const __grid_constant__ NetArgs a0, int slot) {
+__global__ void __launch_bounds__(128, 7) k_network(const __grid_constant__ NetArgs a0, int slot) {
     const NetArgs a = MEM ? member_args(a0, (int)blockIdx.y) : a0;
     pdl_launch_dependents();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    const int4 gr = g < a.G ? a.grp[g] : make_int4(-1, -1, 0, 0);
-    const float4 ci = gr.x >= 0 ? a.cinfo[gr.x] : make_float4(1.0f, 0.0f, 0.0f, 0.0f);
+    const GroupStatic t = group_static(a, g);
     const StepCtrl s = a.ctrl[slot];
     pdl_wait();  // k_donor's factors (and, through it, every earlier kernel's writes)
     if (!s.active || !(s.phases & FL_PHASE_DRAINAGE)) return;
     float led[D2_TERMS] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (g < a.G) group_item(a, s, gr, ci, led);
+    if (g < a.G) group_item(a, s, t, led);
     warp_add_ledger<D2_TERMS>(led, a.ledger);
 }
 

@@ -255,6 +255,16 @@ static DtArgs dt_args(const FlSolver *s, int m) {
 // One step: [CFL reduction + plan] surface [inlets network], the CFL and
 // surface launches once per member, each drainage kernel once for all
 // members.
+// The drainage passes of one step.
+static int launch_drainage(FlSolver *s, int slot, cudaStream_t st) {
+    FL_CUDA(launch_nodes(s->nd, slot, st));
+    FL_CUDA(launch_links(s->lk, slot, st));
+    FL_CUDA(launch_donor(s->dn, slot, st));
+    FL_CUDA(launch_network(s->nw, slot, st));
+    g_launches += 4;
+    return FL_OK;
+}
+
 static int launch_step(FlSolver *s, int slot, bool eval, bool plan_next, cudaStream_t st) {
     if (eval) {
         for (int m = 0; m < s->members; ++m) FL_CUDA(launch_dt(dt_args(s, m), s->dt_blocks, slot, 1, st));
@@ -273,11 +283,8 @@ static int launch_step(FlSolver *s, int slot, bool eval, bool plan_next, cudaStr
         g_launches++;
     }
     if (s->has_drain()) {
-        FL_CUDA(launch_nodes(s->nd, slot, st));
-        FL_CUDA(launch_links(s->lk, slot, st));
-        FL_CUDA(launch_donor(s->dn, slot, st));
-        FL_CUDA(launch_network(s->nw, slot, st));
-        g_launches += 4;
+        const int rc = launch_drainage(s, slot, st);
+        if (rc) return rc;
     }
     if (s->has_table()) {
         FL_CUDA(launch_surcharge(s->sur, slot, st));
@@ -1354,11 +1361,7 @@ FL_API int fl_step(FlSolver *s, double dt_s, int32_t phases, double rain_rate_mp
         g_launches++;
     }
     if (s->has_drain() && (phases & FL_PHASE_DRAINAGE)) {
-        FL_CUDA(launch_nodes(s->nd, s->slot, st));
-        FL_CUDA(launch_links(s->lk, s->slot, st));
-        FL_CUDA(launch_donor(s->dn, s->slot, st));
-        FL_CUDA(launch_network(s->nw, s->slot, st));
-        g_launches += 4;
+        if ((rc = launch_drainage(s, s->slot, st))) return rc;
         if (s->has_table()) {
             FL_CUDA(launch_surcharge(s->sur, s->slot, st));
             g_launches++;
