@@ -68,7 +68,7 @@ struct FlBatch {
     BatchArgs ba{};
     PlanArgs pa{};
     // host
-    BatchList *poll_h = nullptr;  // pinned, 2 slots (header only is read)
+    BatchList *poll_h = nullptr;  // pinned, 2 slots (the tile counts are read)
     cudaStream_t cap_stream = nullptr;
     cudaGraphExec_t graph = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -98,7 +98,7 @@ static int batch_smem_layout(BatchArgs &a, int kind, int S) {
     auto up = [](int x, int m) { return (x + m - 1) / m * m; };
     const int T = a.tile;
     a.off_bar = T * 3 * 16;
-    a.off_list = up(a.off_bar + 64 + (T / 32) * 5 * 4, 128);
+    a.off_list = up(a.off_bar + 96 + (T / 32) * 5 * 4, 128);
     a.off_stage = up(a.off_list + MAX_SCEN * 4 + 16 + S * (int)sizeof(BatchEntry), 128);
     int o = (T + a.h_cap) * 16;
     a.so_ci = o;
@@ -283,9 +283,6 @@ static int batch_create_impl(int32_t n, const FlMeshDesc *meshes, const FlForcin
     }
     HyetoView *d_hy;
     if ((rc = b->upload(&d_hy, hv))) return rc;
-    unsigned int *counter = nullptr;
-    if ((rc = b->alloc(&counter, 1))) return rc;
-    FB_CUDA(cudaMemset(counter, 0, sizeof(unsigned int)));
 
     // kernel arguments and launch shape
     BatchArgs &a = b->ba;
@@ -308,6 +305,7 @@ static int batch_create_impl(int32_t n, const FlMeshDesc *meshes, const FlForcin
     a.snap_hv = snap_hv;
     a.snap_base = d_snap_base;
     a.run = b->run;
+    a.n_scen = n;
     a.n_tiles = b->tiles;
     a.tile = b->tile;
     a.e_cap = e_cap;
@@ -338,7 +336,6 @@ static int batch_create_impl(int32_t n, const FlMeshDesc *meshes, const FlForcin
     pa.tile_led = tile_led;
     pa.ledger = b->ledger;
     pa.list = b->list;
-    pa.counter = counter;
     pa.n = n;
     pa.max_snaps = b->max_snaps;
 
@@ -476,12 +473,14 @@ FL_API int fl_batch_run(FlBatch *b, int64_t max_steps, void *stream) {
     while (true) {
         FB_CUDA(cudaGraphLaunch(b->graph, st));
         add_launches(2 * (int64_t)b->chunk);
-        FB_CUDA(cudaMemcpyAsync(&b->poll_h[launched & 1], b->list, 16, cudaMemcpyDeviceToHost, st));
+        FB_CUDA(cudaMemcpyAsync(b->poll_h[launched & 1].tiles, b->list->tiles, sizeof(int32_t) * b->S, cudaMemcpyDeviceToHost,
+                                st));
         FB_CUDA(cudaEventRecord(b->ev[launched & 1], st));
         ++launched;
         if (launched >= 2) {
             FB_CUDA(cudaEventSynchronize(b->ev[launched & 1]));
-            if (b->poll_h[launched & 1].n == 0) break;
+            const int32_t *left = b->poll_h[launched & 1].tiles;
+            if (std::all_of(left, left + b->S, [](int32_t t) { return t == 0; })) break;
         }
     }
     FB_CUDA(cudaStreamSynchronize(st));

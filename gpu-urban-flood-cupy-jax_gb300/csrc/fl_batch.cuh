@@ -21,13 +21,11 @@ struct BatchEntry {
     int32_t scen, flags, tile0, cells;
 };
 
-// The step's active scenarios; tiles of entry k are virtual tiles
-// [prefix[k], prefix[k + 1]).
+// The step's scenarios: entry s and its tile count (0: not active in this
+// step).  Each surface CTA forms the running sums of the counts itself; the
+// tiles of scenario s are virtual tiles [sum before s, sum before s + 1).
 struct BatchList {
-    int32_t n;
-    int32_t pad[3];
-    int32_t prefix[MAX_SCEN + 1];
-    int32_t pad2[3];
+    int32_t tiles[MAX_SCEN];
     BatchEntry e[MAX_SCEN];
 };
 
@@ -48,7 +46,7 @@ struct BatchArgs {
     float *snap_hu, *snap_hv;     // momentum at each snapshot (same layout)
     const int64_t *snap_base;     // [n] first snapshot element of each scenario
     RunCtrl *run;                 // [n]
-    int32_t n_tiles, tile, e_cap, h_cap;
+    int32_t n_scen, n_tiles, tile, e_cap, h_cap;
     int32_t off_bar, off_list, off_stage, stage_bytes;
     int32_t so_ci, so_hz, so_wt, so_hm, so_en, so_hs;
     int32_t forcing_kind;
@@ -67,7 +65,6 @@ struct PlanArgs {
     const float *tile_led;
     float2 *ledger;               // [n * SURF_TERMS] float-float running sums
     BatchList *list;
-    unsigned int *counter;
     int32_t n, max_snaps;
 };
 

@@ -1,20 +1,26 @@
 // Batched-ensemble kernels for sm_103a.
 //
-// k_surface_batch: the persistent surface kernel of k_surface (fl_surface.cu)
-// over the tiles of every active scenario of a batch.  The planner's list
-// maps a virtual tile index to (scenario, tile); each CTA walks virtual tiles
-// through the same two-stage pipeline (bulk async copies of the tile's states,
-// cell info, Horton fields, wet time, running maximum depth, edge entries and
-// halo list; cp.async gathers of the halo states) and evaluates them with the
-// same tile_entry / cell_update / clamp code as the single-scenario kernel,
-// with the scenario's own dt, rain and flags.  Per tile it stores the step's
-// ledger terms and, when the scenario's next step evaluates the CFL dt, the
-// minimum local dt of the tile's output state -- plain stores, reduced per
-// scenario by the planner.
+// k_surface_batch: the persistent, warp-specialised surface kernel of
+// k_surface (fl_surface.cu) over the tiles of every active scenario of a
+// batch.  The planner's list maps a virtual tile index to (scenario, tile); a
+// CTA's producer warp brings its virtual tiles into two stages (bulk async
+// copies of the tile's states, cell info, Horton fields, wet time, running
+// maximum depth, edge entries and halo list; then cp.async gathers of the halo
+// states) and its compute warps evaluate them with the same tile_entry /
+// cell_update / clamp code as the single-scenario kernel, with the scenario's
+// own dt, rain and flags.  Per tile it stores the step's ledger terms and,
+// when the scenario's next step evaluates the CFL dt, the minimum local dt of
+// the tile's output state -- plain stores, reduced per scenario by the planner.
+// A tile's warp partials are added up after the next tile's opening barrier,
+// so a tile costs two barriers of the compute warps and none of the CTA.
 //
 // k_plan_batch: one CTA per scenario reduces its tiles' ledger terms and CFL
-// minima and plans its next step with plan_step (the single-scenario
-// planner); the last CTA to finish rebuilds the list of active scenarios.
+// minima, plans its next step with plan_step (the single-scenario planner) and
+// writes the scenario's entry of the step's list.  It sits between two surface
+// launches, so its length counts in full: the run record and the hyetograph
+// are brought to shared memory in one level of loads (read field by field by
+// the one planning thread they made it 12 us a step), and no CTA waits for the
+// others -- the surface CTAs add up the tile counts.
 //
 // k_cfl_batch: the CFL minima of every tile's initial state (before step 0).
 #include "fl_batch.cuh"
@@ -58,18 +64,11 @@ __device__ __forceinline__ BStage<T> bstage_at(const BatchArgs &a, unsigned char
     return t;
 }
 
-// Issue the bulk copies of virtual tile v into a stage (one thread); the
-// expected byte count is the sum of exactly the copies issued.
+// Issue the bulk copies of tile t (scenario entry E) into a stage (one
+// thread); the expected byte count is the sum of exactly the copies issued.
 template <int KIND, int T>
-__device__ __forceinline__ void issue_btile(const BatchArgs &a, const int32_t *prefix, const BatchEntry *ent, int n,
-                                            int v, const BStage<T> &S, int4 *info_slot, int *kt_slot, uint32_t bar) {
-    const int k = find_entry(prefix, n, v);
-    const BatchEntry &E = ent[k];
-    const int t = E.tile0 + (v - prefix[k]);
-    kt_slot[0] = k;
-    kt_slot[1] = t;
-    const int4 ti = a.tile_info[t];
-    *info_slot = ti;
+__device__ __forceinline__ void issue_btile(const BatchArgs &a, const BatchEntry &E, int t, const int4 ti,
+                                            const BStage<T> &S, uint32_t bar) {
     const float4 *in = (E.flags & BF_PARITY) ? a.state1 : a.state0;
     const uint32_t ent_bytes = (uint32_t)ti.y * 16u;
     const uint32_t halo_bytes = (uint32_t)((ti.w + 3) & ~3) * 4u;
@@ -88,86 +87,177 @@ __device__ __forceinline__ void issue_btile(const BatchArgs &a, const int32_t *p
     if (halo_bytes) bulk_copy_g2s(smem_addr(S.hs), a.halo_src + ti.z, halo_bytes, bar);
 }
 
+// Named barrier and barrier-reduction among the T compute threads (id 1).
 template <int T>
-__device__ __forceinline__ void gather_bhalo(const BatchArgs &a, const BatchEntry &E, const BStage<T> &S, int count) {
-    const float4 *in = (E.flags & BF_PARITY) ? a.state1 : a.state0;
-    for (int j = threadIdx.x; j < count; j += T) cp_async16(smem_addr(&S.st[T + j]), in + S.hs[j]);
-    cp_async_commit();
+__device__ __forceinline__ void batch_sync() {
+    asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory");
 }
 
+template <int T>
+__device__ __forceinline__ bool batch_all(bool p) {
+    uint32_t r;
+    asm volatile(
+        "{\n"
+        ".reg .pred pi, po;\n"
+        "setp.ne.u32 pi, %1, 0;\n"
+        "bar.red.and.pred po, 1, %2, pi;\n"
+        "selp.u32 %0, 1, 0, po;\n"
+        "}\n"
+        : "=r"(r)
+        : "r"((uint32_t)p), "n"(T)
+        : "memory");
+    return r != 0;
+}
+
+// Four CTAs of 256-cell tiles an SM (seven of 128): 56 registers.
 template <int KIND, int T>
-__global__ void __launch_bounds__(T, 1024 / T) k_surface_batch(const __grid_constant__ BatchArgs a) {
+__global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(const __grid_constant__ BatchArgs a) {
     constexpr int W = T / 32;
     extern __shared__ __align__(128) unsigned char smem[];
     float4 *s_flux = (float4 *)smem;  // [T * 3]
-    uint64_t *s_bar = (uint64_t *)(smem + a.off_bar);
-    int4 *s_info = (int4 *)(smem + a.off_bar + 16);
-    int *s_kt = (int *)(smem + a.off_bar + 48);         // [2][2] list entry and tile of each stage
-    float *s_red = (float *)(smem + a.off_bar + 64);    // [W][5] warp partials
+    uint64_t *s_bar = (uint64_t *)(smem + a.off_bar);   // full[2], halo[2], empty[2]
+    int4 *s_info = (int4 *)(smem + a.off_bar + 48);
+    int *s_kt = (int *)(smem + a.off_bar + 80);         // [2][2] list entry and tile of each stage
+    float *s_red = (float *)(smem + a.off_bar + 96);    // [W][5] warp partials
     int32_t *s_prefix = (int32_t *)(smem + a.off_list);
-    const int tid = threadIdx.x;
-    const int n = a.list->n;
     BatchEntry *s_ent = (BatchEntry *)(smem + a.off_list + MAX_SCEN * 4 + 16);
-    for (int i = tid; i <= n; i += T) s_prefix[i] = a.list->prefix[i];
-    for (int i = tid; i < n; i += T) s_ent[i] = a.list->e[i];
+    const int tid = threadIdx.x;
+    const uint32_t bar_base = smem_addr(s_bar);
+    if (tid < T) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) s_flux[tid * 3 + k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    const uint32_t bar0 = smem_addr(&s_bar[0]), bar1 = smem_addr(&s_bar[1]);
+        for (int k = 0; k < 3; ++k) s_flux[tid * 3 + k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
     if (tid == 0) {
-        mbar_init(bar0, 1);
-        mbar_init(bar1, 1);
+        for (int k = 0; k < 2; ++k) {
+            mbar_init(bar_base + 8u * k, 1);
+            mbar_init(bar_base + 16u + 8u * k, 32);
+            mbar_init(bar_base + 32u + 8u * k, W);
+        }
         mbar_fence_init();
     }
-    __syncthreads();
-    const int total = n > 0 ? s_prefix[n] : 0;
-    int v = blockIdx.x;
-    if (v >= total) return;
-    const BStage<T> S0 = bstage_at<T>(a, smem, 0), S1 = bstage_at<T>(a, smem, 1);
-    const int G = gridDim.x;
-    const float md = a.md;
-    uint32_t wpar = 0u, pending = 0u;
-    if (tid == 0) {
-        issue_btile<KIND, T>(a, s_prefix, s_ent, n, v, S0, &s_info[0], &s_kt[0], bar0);
-        pending = 1u;
+    pdl_wait();  // the planner's list (its launch overlaps the set-up above)
+    const int n = a.n_scen;
+    for (int i = tid; i < n; i += T + 32) s_ent[i] = a.list->e[i];
+    if (tid < 32) {  // running sums of the tile counts (an inactive scenario's range is empty)
+        constexpr int PER = MAX_SCEN / 32;
+        int c[PER], sum = 0;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) c[j] = tid * PER + j < n ? a.list->tiles[tid * PER + j] : 0;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) sum += c[j];
+        int before = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, before, o);
+            if (tid >= o) before += x;
+        }
+        before -= sum;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            if (tid * PER + j <= n) s_prefix[tid * PER + j] = before;
+            before += c[j];
+        }
+        if (tid == 31 && n == MAX_SCEN) s_prefix[n] = before;
     }
-    bool timed_out = !mbar_wait_bounded(bar0, 0, BATCH_WAIT_NS);
-    wpar ^= 1u;
-    if (__syncthreads_or(timed_out)) goto abort;
-    pending = 0u;
-    gather_bhalo<T>(a, s_ent[s_kt[0]], S0, s_info[0].w);
+    __syncthreads();  // the last block-wide barrier: the roles split here
+    const int total = s_prefix[n];
+    const int G = gridDim.x;
+    const BStage<T> S0 = bstage_at<T>(a, smem, 0), S1 = bstage_at<T>(a, smem, 1);
+    auto fail = [&]() {  // (one thread)
+        for (int k = 0; k < n; ++k)
+            if (atomicCAS(&a.run[s_ent[k].scen].error, 0, FL_E_TIMEOUT) == 0)
+                a.run[s_ent[k].scen].error_step = a.run[s_ent[k].scen].step - 1;
+    };
 
-    for (int i = 0; v < total; ++i, v += G) {
-        const int si = i & 1;
-        const BStage<T> &S = si ? S1 : S0;
-        const BStage<T> &SN = si ? S0 : S1;
-        const uint32_t barN = si ? bar0 : bar1;
-        const int vn = v + G;
-        if (tid == 0 && vn < total) {
-            issue_btile<KIND, T>(a, s_prefix, s_ent, n, vn, SN, &s_info[si ^ 1], &s_kt[(si ^ 1) * 2], barN);
-            pending |= 1u << (si ^ 1);
+    if (tid >= T) {
+        // ---------------------------------------------------------- producer
+        const int lane = tid - T;
+        bool failed = false;
+        int i = 0;
+        for (int v = blockIdx.x; v < total; v += G, ++i) {
+            const int st = i & 1;
+            const BStage<T> &S = st ? S1 : S0;
+            const uint32_t full = bar_base + 8u * st;
+            if (i >= 2) {  // the compute warps released this stage's previous tile
+                bool ok = true;
+                if (lane == 0) ok = mbar_wait_bounded(bar_base + 32u + 8u * st, ((i >> 1) - 1) & 1u, BATCH_WAIT_NS);
+                if (!__shfl_sync(0xffffffffu, ok, 0)) {
+                    failed = true;
+                    break;
+                }
+            }
+            if (lane == 0) {
+                const int k = find_entry(s_prefix, n, v);
+                const int t = s_ent[k].tile0 + (v - s_prefix[k]);
+                const int4 ti = a.tile_info[t];
+                s_kt[2 * st] = k;
+                s_kt[2 * st + 1] = t;
+                s_info[st] = ti;
+                issue_btile<KIND, T>(a, s_ent[k], t, ti, S, full);
+            }
+            // every lane waits: each then reads the landed halo list itself
+            const bool ok = mbar_wait_bounded(full, (i >> 1) & 1u, BATCH_WAIT_NS);
+            if (!__all_sync(0xffffffffu, ok)) {
+                // a copy is late: one more bounded wait so none lands after the CTA leaves
+                (void)mbar_wait_bounded(full, (i >> 1) & 1u, BATCH_WAIT_NS);
+                failed = true;
+                break;
+            }
+            const float4 *in = (s_ent[s_kt[2 * st]].flags & BF_PARITY) ? a.state1 : a.state0;
+            const int hc = s_info[st].w;
+            for (int j = lane; j < hc; j += 32) cp_async16(smem_addr(&S.st[T + j]), in + S.hs[j]);
+            cp_async_arrive_noinc(bar_base + 16u + 8u * st);
         }
         cp_async_wait_all();
-        __syncthreads();  // this tile's halo states are in place
+        if (failed && lane == 0) fail();
+        return;
+    }
 
-        const BatchEntry E = s_ent[s_kt[si * 2]];
-        const int t = s_kt[si * 2 + 1];
+    // ------------------------------------------------------------- compute
+    const float md = a.md;
+    // the tile's ledger terms and CFL minimum from its warp partials (one thread)
+    auto finish_tile = [&](int t, bool cfl) {
+#pragma unroll
+        for (int j = 0; j < SURF_TERMS; ++j) {
+            float sum = 0.0f;
+#pragma unroll
+            for (int w = 0; w < W; ++w) sum += s_red[w * 5 + j];
+            a.tile_led[(size_t)t * SURF_TERMS + j] = sum;
+        }
+        if (cfl) {
+            float m = CUDART_INF_F;
+#pragma unroll
+            for (int w = 0; w < W; ++w) m = fminf(m, s_red[w * 5 + 4]);
+            a.tile_min[t] = m;
+        }
+    };
+    int i = 0, done_t = -1;
+    bool done_cfl = false;
+    for (int v = blockIdx.x; v < total; v += G, ++i) {
+        const int st_i = i & 1;
+        const BStage<T> &S = st_i ? S1 : S0;
+        bool ok = true;
+        if (tid == 0)
+            ok = mbar_wait_bounded(bar_base + 8u * st_i, (i >> 1) & 1u, BATCH_WAIT_NS) &&
+                 mbar_wait_bounded(bar_base + 16u + 8u * st_i, (i >> 1) & 1u, BATCH_WAIT_NS);
+        if (!batch_all<T>(ok)) {  // also: every warp's partials of the previous tile are in place
+            if (tid == 0) fail();
+            return;  // the producer waits out its own copies
+        }
+        if (tid == 0 && done_t >= 0) finish_tile(done_t, done_cfl);
+        const BatchEntry &E = s_ent[s_kt[2 * st_i]];
+        const int t = s_kt[2 * st_i + 1];
+        const int flags = E.flags;
         const float dt = E.dt;
-        const int phases = (E.flags >> BF_PHASE_SHIFT) & 7;
+        const int phases = (flags >> BF_PHASE_SHIFT) & 7;
         const bool do_surface = (phases & FL_PHASE_SURFACE) != 0;
         float led[SURF_TERMS] = {0.0f, 0.0f, 0.0f, 0.0f};
         if (do_surface) {
-            const int n_e = s_info[si].y;
+            const int n_e = s_info[st_i].y;
 #pragma unroll 1
             for (int e = tid; e < n_e; e += T) tile_entry(S.en[e], S.st, s_flux, a.g, a.half_g, md, a.stage, dt, led[2], led[3]);
         }
-        bool bad = false;
-        if (vn < total) {
-            bad = !mbar_wait_bounded(barN, (wpar >> (si ^ 1)) & 1u, BATCH_WAIT_NS);
-            wpar ^= 1u << (si ^ 1);
-        }
-        if (__syncthreads_or(bad)) goto abort;  // also: phase 2's slots are complete
-        pending = 0u;
-        if (vn < total) gather_bhalo<T>(a, s_ent[s_kt[(si ^ 1) * 2]], SN, s_info[si ^ 1].w);
+        batch_sync<T>();  // phase 2's slots are complete
 
         // phase 3: the cell update
         const int c_local = (t - E.tile0) * T + tid;
@@ -177,7 +267,7 @@ __global__ void __launch_bounds__(T, 1024 / T) k_surface_batch(const __grid_cons
             const float4 st = S.st[tid];
             const float4 ci = S.ci[tid];
             const uint32_t info = __float_as_uint(ci.z);
-            if ((E.flags & BF_FINITE) && !isfinite(st.x)) {
+            if ((flags & BF_FINITE) && !isfinite(st.x)) {
                 if (atomicCAS(&a.run[E.scen].error, 0, FL_E_NONFINITE) == 0) a.run[E.scen].error_step = a.run[E.scen].step - 1;
             }
             float wt = 0.0f;
@@ -202,10 +292,10 @@ __global__ void __launch_bounds__(T, 1024 / T) k_surface_batch(const __grid_cons
 #pragma unroll
             for (int k = 0; k < 3; ++k) s_flux[tid * 3 + k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (phases & FL_PHASE_CLAMP) clamp_velocity_exact(hn, hun, hvn, a.vmax);
-            (E.flags & BF_PARITY ? a.state0 : a.state1)[c] = make_float4(hn, hun, hvn, st.w);
+            (flags & BF_PARITY ? a.state0 : a.state1)[c] = make_float4(hn, hun, hvn, st.w);
             if (KIND == 1 && do_surface) a.wet[c] = wt + dt * (float)(hn > md);
             const float hm = fmax32(S.hm[tid], hn);
-            const int snap = (E.flags >> BF_SNAP_SHIFT) - 1;
+            const int snap = (flags >> BF_SNAP_SHIFT) - 1;
             if (snap >= 0) {
                 const size_t o = (size_t)a.snap_base[E.scen] + (size_t)snap * (size_t)E.cells + (size_t)c_local;
                 a.snap_h[o] = hn;
@@ -216,52 +306,35 @@ __global__ void __launch_bounds__(T, 1024 / T) k_surface_batch(const __grid_cons
             } else {
                 a.hmax[c] = hm;
             }
-            if (E.flags & BF_CFL) {
+            if (flags & BF_CFL) {
                 const float local = cfl_local(hn, hun, hvn, a.char_len[c], a.cfl, a.g, md);
                 if (isfinite(local)) cmin = local;
             }
         }
-        // the tile's ledger terms and CFL minimum: warp partials, then thread 0
+        // the warp's partials; its lanes are done with the stage
+        __syncwarp();
+        if ((tid & 31) == 0) mbar_arrive(bar_base + 32u + 8u * st_i);
 #pragma unroll
         for (int j = 0; j < SURF_TERMS; ++j) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) led[j] += __shfl_down_sync(0xffffffffu, led[j], o);
         }
+        if (flags & BF_CFL) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) cmin = fminf(cmin, __shfl_down_sync(0xffffffffu, cmin, o));
+            for (int o = 16; o > 0; o >>= 1) cmin = fminf(cmin, __shfl_down_sync(0xffffffffu, cmin, o));
+        }
         if ((tid & 31) == 0) {
 #pragma unroll
             for (int j = 0; j < SURF_TERMS; ++j) s_red[(tid >> 5) * 5 + j] = led[j];
             s_red[(tid >> 5) * 5 + 4] = cmin;
         }
-        __syncthreads();  // this stage, the flux slots and the partials are complete
-        if (tid == 0) {
-#pragma unroll
-            for (int j = 0; j < SURF_TERMS; ++j) {
-                float sum = 0.0f;
-#pragma unroll
-                for (int w = 0; w < W; ++w) sum += s_red[w * 5 + j];
-                a.tile_led[(size_t)t * SURF_TERMS + j] = sum;
-            }
-            if (E.flags & BF_CFL) {
-                float m = CUDART_INF_F;
-#pragma unroll
-                for (int w = 0; w < W; ++w) m = fminf(m, s_red[w * 5 + 4]);
-                a.tile_min[t] = m;
-            }
-        }
+        done_t = t;
+        done_cfl = (flags & BF_CFL) != 0;
     }
-    return;
-
-abort:
-    if (tid == 0) {
-        for (int k = 0; k < n; ++k)
-            if (atomicCAS(&a.run[s_ent[k].scen].error, 0, FL_E_TIMEOUT) == 0) a.run[s_ent[k].scen].error_step = a.run[s_ent[k].scen].step - 1;
-        if (pending & 1u) (void)mbar_wait_bounded(bar0, (wpar & 1u) ^ 1u, BATCH_WAIT_NS);
-        if (pending & 2u) (void)mbar_wait_bounded(bar1, ((wpar >> 1) & 1u) ^ 1u, BATCH_WAIT_NS);
+    if (done_t >= 0) {
+        batch_sync<T>();
+        if (tid == 0) finish_tile(done_t, done_cfl);
     }
-    cp_async_wait_all();
-    __syncthreads();
 }
 
 // CFL minima of every tile's state before the first step (all scenarios'
@@ -292,26 +365,63 @@ __global__ void __launch_bounds__(T) k_cfl_batch(const float4 *state0, const flo
 }
 
 // One CTA per scenario: fold the step's tile terms into the scenario's
-// ledger, plan its next step, and (last CTA) rebuild the active list.
+// ledger, plan its next step and write its entry of the list.
+constexpr int PLAN_HYETO = 128;  // hyetograph blocks held in shared memory
+
 __global__ void __launch_bounds__(128) k_plan_batch(const __grid_constant__ PlanArgs a, int slot, int init) {
+    __shared__ RunCtrl s_run;
+    __shared__ StepCtrl s_next;
+    __shared__ double s_hy[3][PLAN_HYETO];
+    __shared__ float red[4][SURF_TERMS + 1];
     const int b = blockIdx.x;
     const int tid = threadIdx.x;
-    RunCtrl *run = &a.run[b];
-    const StepCtrl cur = a.ctrl[2 * b + slot];
-    const int cfl_interval = run->cfl_interval;
-    const bool had_step = !init && cur.active;
-    const bool cfl_done = init || (had_step && ((cur.step + 1) % cfl_interval == 0));
     const int t0 = a.scen_tile0[b], t1 = a.scen_tile0[b + 1];
+    HyetoView hy = a.hy[b];
+    if (hy.n <= PLAN_HYETO) {  // (inputs: not written by the step)
+        if (tid < hy.n) {
+            s_hy[0][tid] = hy.start_s[tid];
+            s_hy[1][tid] = hy.end_s[tid];
+            s_hy[2][tid] = hy.rate[tid];
+        }
+        hy.start_s = s_hy[0];
+        hy.end_s = s_hy[1];
+        hy.rate = s_hy[2];
+    }
+    pdl_wait();               // the step's surface kernel
+    pdl_launch_dependents();  // the next one may set up meanwhile
+    RunCtrl *run = &a.run[b];
+    static_assert(sizeof(RunCtrl) % 4 == 0 && sizeof(RunCtrl) <= 128 * 4 && sizeof(StepCtrl) % 4 == 0 && sizeof(StepCtrl) <= 128 * 4,
+                  "records are copied a word per thread");
+    if (tid < (int)(sizeof(RunCtrl) / 4)) ((uint32_t *)&s_run)[tid] = ((const uint32_t *)run)[tid];
+    const int cfl_interval = run->cfl_interval;
+    const int cur_active = a.ctrl[2 * b + slot].active;
+    const int64_t cur_step = a.ctrl[2 * b + slot].step;
     float m = CUDART_INF_F;
     float l[SURF_TERMS] = {0.0f, 0.0f, 0.0f, 0.0f};
-    for (int t = t0 + tid; t < t1; t += 128) {
-        if (cfl_done) m = fminf(m, a.tile_min[t]);
-        if (had_step) {
+    static_assert(SURF_TERMS == 4, "a tile's ledger terms are one float4");
+    const float4 *led = (const float4 *)a.tile_led;
+    for (int t = t0 + tid; t < t1; t += 128 * 4) {  // four tiles' loads in flight (whether or not the step uses them), added in order
+        float4 v[4];
+        float q[4];
 #pragma unroll
-            for (int j = 0; j < SURF_TERMS; ++j) l[j] += a.tile_led[(size_t)t * SURF_TERMS + j];
+        for (int u = 0; u < 4; ++u) {
+            const bool in = t + u * 128 < t1;
+            v[u] = in ? led[t + u * 128] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            q[u] = in ? a.tile_min[t + u * 128] : CUDART_INF_F;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (t + u * 128 >= t1) break;
+            m = fminf(m, q[u]);
+            l[0] += v[u].x;
+            l[1] += v[u].y;
+            l[2] += v[u].z;
+            l[3] += v[u].w;
         }
     }
-    __shared__ float red[4][SURF_TERMS + 1];
+    const bool had_step = !init && cur_active;
+    const bool cfl_done = init || (had_step && step_mod(cur_step + 1, cfl_interval) == 0);
+    if (!cfl_done) m = CUDART_INF_F;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -324,64 +434,33 @@ __global__ void __launch_bounds__(128) k_plan_batch(const __grid_constant__ Plan
         red[tid >> 5][SURF_TERMS] = m;
     }
     __syncthreads();
-    __shared__ bool last;
-    if (tid == 0) {
+    if (tid < SURF_TERMS && had_step)
+        ff_accumulate(&a.ledger[b * SURF_TERMS + tid], red[0][tid] + red[1][tid] + red[2][tid] + red[3][tid]);
+    if (tid == 32) {  // (a warp of its own: the ledger's round trip does not delay it)
         float mm = red[0][SURF_TERMS];
         for (int w = 1; w < 4; ++w) mm = fminf(mm, red[w][SURF_TERMS]);
-        if (had_step) {
-            for (int j = 0; j < SURF_TERMS; ++j)
-                ff_accumulate(&a.ledger[b * SURF_TERMS + j], red[0][j] + red[1][j] + red[2][j] + red[3][j]);
+        const bool eval = step_mod(s_run.step, cfl_interval) == 0;
+        plan_step(&s_run, a.snap_t + (size_t)b * a.max_snaps, hy, &s_next, eval, mm, FL_PHASE_SURFACE | FL_PHASE_CLAMP);
+        const StepCtrl &nx = s_next;
+        a.list->tiles[b] = nx.active ? t1 - t0 : 0;
+        if (nx.active) {
+            BatchEntry e;
+            e.dt = nx.dt_f;
+            e.dtg = nx.dtg_f;
+            e.rain = nx.rain_f;
+            e.infil = a.scen_infil[b];
+            e.scen = b;
+            const bool cfl_next = step_mod(nx.step + 1, cfl_interval) == 0;
+            e.flags = (nx.parity ? BF_PARITY : 0) | (cfl_next ? BF_CFL : 0) | (nx.check_finite ? BF_FINITE : 0) |
+                      (nx.phases << BF_PHASE_SHIFT) | ((nx.snap_slot + 1) << BF_SNAP_SHIFT);
+            e.tile0 = t0;
+            e.cells = a.scen_cells[b];
+            a.list->e[b] = e;
         }
-        const bool eval = (run->step % cfl_interval) == 0;
-        plan_step(run, a.snap_t + (size_t)b * a.max_snaps, a.hy[b], &a.ctrl[2 * b + (slot ^ 1)], eval, mm,
-                  FL_PHASE_SURFACE | FL_PHASE_CLAMP);
-        __threadfence();
-        last = atomicAdd(a.counter, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (!last) return;
-    __threadfence();
-    // the last CTA: list of the scenarios active in the next step, in order
-    __shared__ int32_t cnt[MAX_SCEN];
-    __shared__ int32_t pos[MAX_SCEN + 1];
-    for (int s = tid; s < a.n; s += 128) {
-        const volatile StepCtrl *nx = &a.ctrl[2 * s + (slot ^ 1)];
-        cnt[s] = nx->active ? (a.scen_tile0[s + 1] - a.scen_tile0[s]) : -1;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        int k = 0, acc = 0;
-        for (int s = 0; s < a.n; ++s) {
-            if (cnt[s] >= 0) {
-                pos[s] = k;
-                a.list->prefix[k] = acc;
-                acc += cnt[s];
-                ++k;
-            } else {
-                pos[s] = -1;
-            }
-        }
-        a.list->prefix[k] = acc;
-        a.list->n = k;
-        *a.counter = 0u;
-    }
-    __syncthreads();
-    for (int s = tid; s < a.n; s += 128) {
-        if (pos[s] < 0) continue;
-        const volatile StepCtrl *nx = &a.ctrl[2 * s + (slot ^ 1)];
-        BatchEntry e;
-        e.dt = nx->dt_f;
-        e.dtg = nx->dtg_f;
-        e.rain = nx->rain_f;
-        e.infil = a.scen_infil[s];
-        e.scen = s;
-        const bool cfl_next = ((nx->step + 1) % a.run[s].cfl_interval) == 0;
-        e.flags = (nx->parity ? BF_PARITY : 0) | (cfl_next ? BF_CFL : 0) | (nx->check_finite ? BF_FINITE : 0) |
-                  (nx->phases << BF_PHASE_SHIFT) | ((nx->snap_slot + 1) << BF_SNAP_SHIFT);
-        e.tile0 = a.scen_tile0[s];
-        e.cells = a.scen_cells[s];
-        a.list->e[pos[s]] = e;
-    }
+    if (tid < (int)(sizeof(RunCtrl) / 4)) ((uint32_t *)run)[tid] = ((const uint32_t *)&s_run)[tid];
+    if (tid < (int)(sizeof(StepCtrl) / 4)) ((uint32_t *)&a.ctrl[2 * b + (slot ^ 1)])[tid] = ((const uint32_t *)&s_next)[tid];
 }
 
 template __global__ void k_surface_batch<0, 128>(const __grid_constant__ BatchArgs);
@@ -402,18 +481,30 @@ cudaError_t batch_configure(int kind, int tile, int smem_bytes, int *per_sm) {
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, tile, (size_t)smem_bytes);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, tile + 32, (size_t)smem_bytes);
+}
+
+// Launch as a programmatic dependent of the previous kernel in the stream.
+template <class Args, class... Rest>
+static cudaError_t launch_dependent(void (*kernel)(Args, Rest...), int grid, int threads, int smem_bytes, cudaStream_t stream,
+                                    const Args &a, Rest... rest) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem_bytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, a, rest...);
 }
 
 cudaError_t launch_surface_batch(const BatchArgs &a, int kind, int grid, int smem_bytes, cudaStream_t stream) {
-    if (a.tile == 128) {
-        if (kind) k_surface_batch<1, 128><<<grid, 128, (size_t)smem_bytes, stream>>>(a);
-        else k_surface_batch<0, 128><<<grid, 128, (size_t)smem_bytes, stream>>>(a);
-    } else {
-        if (kind) k_surface_batch<1, 256><<<grid, 256, (size_t)smem_bytes, stream>>>(a);
-        else k_surface_batch<0, 256><<<grid, 256, (size_t)smem_bytes, stream>>>(a);
-    }
-    return cudaGetLastError();
+    void (*fn)(BatchArgs) = a.tile == 128 ? (kind ? k_surface_batch<1, 128> : k_surface_batch<0, 128>)
+                                          : (kind ? k_surface_batch<1, 256> : k_surface_batch<0, 256>);
+    return launch_dependent(fn, grid, a.tile + 32, smem_bytes, stream, a);
 }
 
 cudaError_t launch_cfl_batch(const float4 *state0, const float *char_len, const int32_t *tile_valid, float *tile_min,
@@ -424,8 +515,7 @@ cudaError_t launch_cfl_batch(const float4 *state0, const float *char_len, const 
 }
 
 cudaError_t launch_plan_batch(const PlanArgs &a, int slot, int init, cudaStream_t stream) {
-    k_plan_batch<<<a.n, 128, 0, stream>>>(a, slot, init);
-    return cudaGetLastError();
+    return launch_dependent(k_plan_batch, a.n, 128, 0, stream, a, slot, init);
 }
 
 }  // namespace fl

@@ -294,6 +294,12 @@ __device__ __forceinline__ double hyeto_rate(const HyetoView &hy, double t) {
     return hy.rate[lo];
 }
 
+// a % b for a step count a >= 0 and an interval b > 0: 32-bit while it fits (a
+// 64-bit remainder is a call of some hundred instructions, in a single thread).
+__device__ __forceinline__ int64_t step_mod(int64_t a, int32_t b) {
+    return a >> 31 ? a % b : (int64_t)((uint32_t)a % (uint32_t)b);
+}
+
 // Plan the next step from the run state (single thread).  This is the
 // host-side control of the reference loop (engine.py:220-232, 306-313):
 // CFL dt evaluated every cfl_interval steps and reused x safety otherwise,
@@ -357,7 +363,7 @@ static __device__ __noinline__ void plan_step(RunCtrl *run, double *snap_t, cons
     s.dt_f = (float)dt;
     s.dtg_f = (float)(dt * run->g);
     s.rain_f = (float)hyeto_rate(hy, t);
-    s.check_finite = (run->finite_interval > 0 && run->step > 0 && run->step % run->finite_interval == 0);
+    s.check_finite = (run->finite_interval > 0 && run->step > 0 && step_mod(run->step, run->finite_interval) == 0);
     run->t = te;
     run->step += 1;
     run->parity ^= 1;
