@@ -15,6 +15,8 @@
 // All sums run in a fixed order, so training is reproducible.
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "fl_device.cuh"
 
 namespace fl {
@@ -132,24 +134,63 @@ __global__ void k_colsum_final(const float *__restrict__ partial, int32_t nb, in
 }
 
 // Adam (Kingma & Ba 2015) with bias correction; w is [rows, cols] (row = output feature).
+__device__ __forceinline__ float adam_step(float *w, float *m1, float *m2, const float *__restrict__ g, int64_t i, float lr,
+                                           float b1, float b2, float eps, float c1, float c2, float wd) {
+    const float gi = g[i] + wd * w[i];
+    const float a = b1 * m1[i] + (1.0f - b1) * gi;
+    const float b = b2 * m2[i] + (1.0f - b2) * gi * gi;
+    m1[i] = a;
+    m2[i] = b;
+    const float wi = w[i] - lr * (a / c1) / (sqrtf(b / c2) + eps);
+    w[i] = wi;
+    return wi;
+}
+
 __global__ void k_adam(float *w, float *m1, float *m2, const float *__restrict__ g, int32_t rows, int32_t cols, float lr,
                        float b1, float b2, float eps, float c1, float c2, float wd, __nv_bfloat16 *w_bf16,
                        __nv_bfloat16 *wt_bf16, int64_t ldt) {
     const int64_t n = (int64_t)rows * cols;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float gi = g[i] + wd * w[i];
-        const float a = b1 * m1[i] + (1.0f - b1) * gi;
-        const float b = b2 * m2[i] + (1.0f - b2) * gi * gi;
-        m1[i] = a;
-        m2[i] = b;
-        const float wi = w[i] - lr * (a / c1) / (sqrtf(b / c2) + eps);
-        w[i] = wi;
-        const __nv_bfloat16 h = __float2bfloat16(wi);
+        const __nv_bfloat16 h = __float2bfloat16(adam_step(w, m1, m2, g, i, lr, b1, b2, eps, c1, c2, wd));
         if (w_bf16) w_bf16[i] = h;
         if (wt_bf16) {
             const int64_t r = i / cols, c = i - r * cols;
             wt_bf16[c * ldt + r] = h;
         }
+    }
+}
+
+constexpr int AD_JOBS = 128;
+
+struct AdJob {
+    float *w, *m1, *m2;
+    const float *g;
+    __nv_bfloat16 *wb, *wt;
+    int32_t rows, cols, ldt, block0;
+};
+
+struct AdArgs {
+    AdJob job[AD_JOBS];
+    float lr, b1, b2, eps, c1, c2, wd;
+    int32_t jobs;
+};
+
+// One Adam step over all of a network's tensors: one launch instead of one per
+// tensor (76 of the eight-layer network, most of them of 128 values).
+__global__ void __launch_bounds__(256) k_adam_all(const __grid_constant__ AdArgs g) {
+    int lo = 0, hi = g.jobs;  // job[lo].block0 <= blockIdx.x < job[hi].block0
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (g.job[mid].block0 <= (int)blockIdx.x) lo = mid; else hi = mid;
+    }
+    const AdJob &J = g.job[lo];
+    const int i = ((int)blockIdx.x - J.block0) * 256 + (int)threadIdx.x;
+    if (i >= J.rows * J.cols) return;
+    const __nv_bfloat16 h = __float2bfloat16(adam_step(J.w, J.m1, J.m2, J.g, i, g.lr, g.b1, g.b2, g.eps, g.c1, g.c2, g.wd));
+    if (J.wb) J.wb[i] = h;
+    if (J.wt) {
+        const int r = i / J.cols, c = i - r * J.cols;
+        J.wt[(int64_t)c * J.ldt + r] = h;
     }
 }
 
@@ -251,6 +292,38 @@ FL_API int fl_adam(float *w, float *m1, float *m2, const float *g, int32_t rows,
         w, m1, m2, g, rows, cols, lr, b1, b2, eps, c1, c2, weight_decay, (__nv_bfloat16 *)w_bf16,
         (__nv_bfloat16 *)wt_bf16, ldt);
     FM_LAUNCHED("k_adam");
+}
+
+FL_API int fl_adam_all(const FlAdamTensor *t, int32_t n, float lr, float b1, float b2, float eps, int32_t step,
+                       float weight_decay, void *stream) {
+    if (!t || n < 1 || step < 1) return set_error(FL_E_INVALID, "fl_adam_all: bad arguments");
+    for (int k = 0; k < n; ++k)
+        if (!t[k].w || !t[k].m1 || !t[k].m2 || !t[k].g || t[k].rows < 1 || t[k].cols < 1 ||
+            (int64_t)t[k].rows * t[k].cols > (1 << 30) || (t[k].wt_bf16 && t[k].ldt < t[k].rows))
+            return set_error(FL_E_INVALID, "fl_adam_all: tensor %d: bad arguments", k);
+    AdArgs a;
+    a.lr = lr;
+    a.b1 = b1;
+    a.b2 = b2;
+    a.eps = eps;
+    a.c1 = 1.0f - powf(b1, (float)step);
+    a.c2 = 1.0f - powf(b2, (float)step);
+    a.wd = weight_decay;
+    for (int k0 = 0; k0 < n; k0 += AD_JOBS) {
+        int blocks = 0;
+        a.jobs = std::min(AD_JOBS, n - k0);
+        for (int k = 0; k < a.jobs; ++k) {
+            const FlAdamTensor &s = t[k0 + k];
+            a.job[k] = AdJob{s.w, s.m1, s.m2, s.g, (__nv_bfloat16 *)s.w_bf16, (__nv_bfloat16 *)s.wt_bf16,
+                             s.rows, s.cols, s.ldt, blocks};
+            blocks += (int)(((int64_t)s.rows * s.cols + 255) / 256);
+        }
+        k_adam_all<<<blocks, 256, 0, (cudaStream_t)stream>>>(a);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return set_error(FL_E_CUDA, "k_adam_all launch: %s", cudaGetErrorString(e));
+        add_launches(1);
+    }
+    return FL_OK;
 }
 
 FL_API int fl_cast_bf16(const float *src, int64_t lds, int32_t m, int32_t n, void *dst, int64_t ldd, void *stream) {

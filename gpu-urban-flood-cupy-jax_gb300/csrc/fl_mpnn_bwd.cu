@@ -1,8 +1,6 @@
 // The surrogate network's backward pass as fused blocks on the tensor cores:
 //   k_mlp_bwd    a two-layer MLP's backward over rows: dz2 = bf16(dy), dz1 =
-//                relu'(z) (dz2 W2), dx = dz1 W1, with the bias gradients
-//                (column sums of the fp32 values) on the way; for a processor
-//                layer also dh = dy + dx, the message gradient
+//                relu'(z) (dz2 W2), dx = dz1 W1; for a processor layer also dh = dy + dx, the message gradient
 //                dagg = dz1 W1[:, 128:], and per incoming edge of a cell
 //                dz_e = relu'(z1_e) (dagg W_e2) -- one product per cell, as
 //                all of a cell's messages have the same gradient
@@ -16,36 +14,26 @@
 //   k_wgrad      the weight gradients dZ^T X of a layer's products in one
 //                launch: rows are the reduction index, so both operands are
 //                read as they lie in memory (M / N contiguous descriptors);
-//                no transposed copies.  Each CTA reduces a fixed range of rows
-//   k_reduce     the CTAs' partial sums, in CTA order, into the gradients
-// Activation gradients keep the rounding points and orders of sums of the
-// separate products (same bits); weight and bias gradients are fp32 sums over
-// rows in a fixed order.
+//                no transposed copies.  Rows are split into short partial
+//                sums, the splits shared out over the CTAs
+//   k_reduce     the partial sums, in order, into the gradients, and the fp32
+//                column sums of the bias gradients by row class (mod 256)
+//   k_bias_final the class sums, in order, into the bias gradients
+// Everything keeps the rounding points and the orders of sums of the separate
+// products (same bits): a bias that differs in its last bit moves some
+// activation across a bf16 boundary every few steps, and a training run then
+// goes its own way.  The message layers' second bias is the caller's.
 //
 // Measured: one optimizer step on 100,352 cells and 299,712 dual edges, 8
 // layers: see the figures at fl_mpnn_backward.
 //
 // Every mbarrier wait is bounded; one that gives up sets the error flag.
+#include <utility>
+#include <vector>
+
 #include "fl_mpnn.cuh"
 
 namespace fl {
-
-// ------------------------------------------------------------- column sums
-// x[u] of lane l: row l, column u of a 32 x 32 block; returns the sum of
-// column l over the rows, in a fixed tree order.
-__device__ __forceinline__ float column_sums32(float (&x)[32], int lane) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const bool hi = (lane & o) != 0;
-#pragma unroll
-        for (int j = 0; j < o; ++j) {
-            const float send = hi ? x[j] : x[j + o];
-            const float keep = hi ? x[j + o] : x[j];
-            x[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-    }
-    return x[0];
-}
 
 __device__ __forceinline__ uint32_t positive_mask(uint32_t z) {  // 0xffff where a bf16 half is > 0
     const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
@@ -60,7 +48,7 @@ constexpr int MB_SMEM = MB_CHUNKS * MM_CHUNK_BYTES + 256 + 1024;
 struct MlpBwdArgs {
     const float *dy;               // [M, ldy >= n2] fp32, or nullptr with dyb
     int64_t ldy;
-    const __nv_bfloat16 *dyb;      // [M, 128] bf16 (n2 = 128): already rounded, its column sums already taken
+    const __nv_bfloat16 *dyb;      // [M, 128] bf16 (n2 = 128): already rounded
     const __nv_bfloat16 *z;        // [M, 128] hidden activations
     const __nv_bfloat16 *w2t;      // [128, n2]
     const __nv_bfloat16 *w1t;      // [128 (decoder) or 256 (layer), 128]
@@ -73,7 +61,9 @@ struct MlpBwdArgs {
     const int32_t *start;          // [M + 1] incoming edges (layer)
     const __nv_bfloat16 *z1e;      // [E, 128] (layer)
     __nv_bfloat16 *dze;            // [E, 128] (layer)
-    float *cs_b2, *cs_b1, *cs_e2, *cs_e1;  // column sums, [4 x grid, n2 or 128] each
+    // the fp32 values that the bias gradients sum, [M, 128] each
+    float *dz1f;                   // masked dz1
+    float *daggf, *gf;             // message gradient; dagg W_e2 before the masks (layer)
     int32_t n2, M;
     int32_t *error;
 };
@@ -173,7 +163,6 @@ __global__ void __launch_bounds__(MB_THREADS, 1) k_mlp_bwd(const __grid_constant
         const int quad = warp & 3, half = warp >> 2;
         const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
         const int col = half * 64;
-        float s_b2[2] = {0.0f, 0.0f}, s_b1[2] = {0.0f, 0.0f}, s_e2[2] = {0.0f, 0.0f}, s_e1[2] = {0.0f, 0.0f};
         auto hand_over = [&](uint32_t bar) {  // this warp's operand columns are written
             tmem_wait_st();
             tmem_fence_before();
@@ -211,7 +200,6 @@ __global__ void __launch_bounds__(MB_THREADS, 1) k_mlp_bwd(const __grid_constant
                         }
                         __syncwarp();
                         tmem_st16(lanes + 384u + (uint32_t)(half * 32 + hh * 16), w);
-                        s_b2[hh] += column_sums32(x, lane);
                     }
                 }
             } else {
@@ -257,13 +245,14 @@ __global__ void __launch_bounds__(MB_THREADS, 1) k_mlp_bwd(const __grid_constant
                         w[u] = pack_bf16x2(x[2 * u], x[2 * u + 1]);
                     }
                     if (in) {
-                        __nv_bfloat16 *p = g.dz1 + (int64_t)r * MF_H + col + hh * 32;
-                        st8u(p, w);
-                        st8u(p + 16, w + 8);
+                        const int64_t at = (int64_t)r * MF_H + col + hh * 32;
+                        st8u(g.dz1 + at, w);
+                        st8u(g.dz1 + at + 16, w + 8);
+#pragma unroll
+                        for (int u = 0; u < 32; u += 8) st8f(g.dz1f + at + u, x + u);
                     }
                     __syncwarp();
                     if (MODE > 0) tmem_st16(lanes + 384u + (uint32_t)(half * 32 + hh * 16), w);
-                    s_b1[hh] += column_sums32(x, lane);
                 }
             }
             if (MODE == 0) {
@@ -272,7 +261,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1) k_mlp_bwd(const __grid_constant
             }
             hand_over(in2);
             if (MODE == 2) {
-                // the message gradient, rounded; its sum over the cell's edges for the bias
+                // the message gradient, rounded
                 if (!warp_wait(d2a, i & 1)) {
                     bad = true;
                     break;
@@ -282,22 +271,17 @@ __global__ void __launch_bounds__(MB_THREADS, 1) k_mlp_bwd(const __grid_constant
                 for (int hh = 0; hh < 2; ++hh) {
                     uint32_t v[32], w[16];
                     tmem_ld32(lanes + 128u + (uint32_t)(col + hh * 32), v);
-                    float x[32];
 #pragma unroll
-                    for (int u = 0; u < 16; ++u) {
-                        const float a = __uint_as_float(v[2 * u]), b = __uint_as_float(v[2 * u + 1]);
-                        w[u] = pack_bf16x2(a, b);
-                        x[2 * u] = in ? a * (float)deg : 0.0f;
-                        x[2 * u + 1] = in ? b * (float)deg : 0.0f;
-                    }
+                    for (int u = 0; u < 16; ++u) w[u] = pack_bf16x2(__uint_as_float(v[2 * u]), __uint_as_float(v[2 * u + 1]));
                     if (in) {
-                        __nv_bfloat16 *p = g.dagg + (int64_t)r * MF_H + col + hh * 32;
-                        st8u(p, w);
-                        st8u(p + 16, w + 8);
+                        const int64_t at = (int64_t)r * MF_H + col + hh * 32;
+                        st8u(g.dagg + at, w);
+                        st8u(g.dagg + at + 16, w + 8);
+#pragma unroll
+                        for (int u = 0; u < 32; u += 8) st8u(g.daggf + at + u, v + u);
                     }
                     __syncwarp();
                     tmem_st16(lanes + 448u + (uint32_t)(half * 32 + hh * 16), w);
-                    s_e2[hh] += column_sums32(x, lane);
                 }
                 hand_over(in3);
             }
@@ -340,45 +324,35 @@ __global__ void __launch_bounds__(MB_THREADS, 1) k_mlp_bwd(const __grid_constant
                 for (int hh = 0; hh < 2; ++hh) {
                     uint32_t v[32], w[16];
                     tmem_ld32(lanes + (uint32_t)(col + hh * 32), v);
-                    float x[32];
-#pragma unroll
-                    for (int u = 0; u < 32; ++u) x[u] = 0.0f;
 #pragma unroll
                     for (int u = 0; u < 16; ++u) w[u] = pack_bf16x2(__uint_as_float(v[2 * u]), __uint_as_float(v[2 * u + 1]));
-#pragma unroll 1
+                    if (in) {
+#pragma unroll
+                        for (int u = 0; u < 32; u += 8) st8u(g.gf + (int64_t)r * MF_H + col + hh * 32 + u, v + u);
+                    }
+                    uint32_t m[3][16];
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {  // all three edges' hidden activations in flight
+                        if (k < deg) {
+                            const int64_t at = (int64_t)(rs + k) * MF_H + col + hh * 32;
+                            ld8u(g.z1e + at, m[k]);
+                            ld8u(g.z1e + at + 16, m[k] + 8);
+                        }
+                    }
+#pragma unroll
                     for (int k = 0; k < 3; ++k) {
                         if (k < deg) {
                             const int64_t at = (int64_t)(rs + k) * MF_H + col + hh * 32;
-                            uint32_t m[16];
-                            ld8u(g.z1e + at, m);
-                            ld8u(g.z1e + at + 16, m + 8);
 #pragma unroll
-                            for (int u = 0; u < 16; ++u) {
-                                m[u] = positive_mask(m[u]);
-                                if (m[u] & 0xffffu) x[2 * u] += __uint_as_float(v[2 * u]);
-                                if (m[u] >> 16) x[2 * u + 1] += __uint_as_float(v[2 * u + 1]);
-                                m[u] &= w[u];
-                            }
-                            st8u(g.dze + at, m);
-                            st8u(g.dze + at + 16, m + 8);
+                            for (int u = 0; u < 16; ++u) m[k][u] = positive_mask(m[k][u]) & w[u];
+                            st8u(g.dze + at, m[k]);
+                            st8u(g.dze + at + 16, m[k] + 8);
                         }
                     }
                     __syncwarp();
-                    s_e1[hh] += column_sums32(x, lane);
                 }
             }
             tmem_fence_before();
-        }
-        const int64_t row = (int64_t)blockIdx.x * 4 + quad;
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            const int c = col + hh * 32 + lane;
-            if (g.dy && col < g.n2) g.cs_b2[row * g.n2 + c] = s_b2[hh];
-            g.cs_b1[row * MF_H + c] = s_b1[hh];
-            if (MODE == 2) {
-                g.cs_e2[row * MF_H + c] = s_e2[hh];
-                g.cs_e1[row * MF_H + c] = s_e1[hh];
-            }
         }
     }
     if (bad) atomicCAS(g.error, 0, FL_E_TIMEOUT);
@@ -402,21 +376,6 @@ struct EdgeBwdArgs {
     int32_t C;
     int32_t *error;
 };
-
-// A producer warp's 64 rows of a 128-row chunk; own0 / own1: this lane's rows
-// (lane, lane + 32), nullptr: left as it is.
-__device__ __forceinline__ void warp_copy_rows64(const __nv_bfloat16 *own0, const __nv_bfloat16 *own1, uint32_t sdst, int pw,
-                                                 int lane) {
-    const int c = lane & 7;
-    const uint64_t p0 = (uint64_t)own0, p1 = (uint64_t)own1;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const int rr = 4 * i + (lane >> 3);
-        const uint64_t row = __shfl_sync(0xffffffffu, i < 8 ? p0 : p1, rr & 31);
-        const int R = 64 * pw + rr;
-        if (row) cp_async16(sdst + (uint32_t)(R * 128 + ((c ^ (R & 7)) << 4)), (const __nv_bfloat16 *)row + c * 8);
-    }
-}
 
 // Products p = 0..2: incoming slots, 3..5: outgoing slots of 128 cells; four
 // 128-column TMEM regions in turn.
@@ -621,7 +580,7 @@ struct EdgeSumArgs {
     const __nv_bfloat16 *wt[ES_MAX_LAYERS];   // [128, ldwt]: rows = the edge features' columns of the weight
     int64_t ldwt[ES_MAX_LAYERS];
     __nv_bfloat16 *out;                        // [E, 128] bf16
-    float *cs;                                 // column sums of the fp32 values, [8 x grid, 128]
+    float *outf;                               // the same before rounding (for the bias gradient)
     int32_t layers, E;
     int32_t *error;
 };
@@ -727,7 +686,6 @@ __global__ void __launch_bounds__(ES_THREADS, 1) k_edge_dsum(const __grid_consta
         // thread = one row of one of the two tiles, 64 of its 128 columns
         const int quad = warp & 3, half = ((warp - ES_PROD - 1) >> 2) & 1, j = (warp - ES_PROD - 1) >> 3;
         const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(j * 128 + half * 64);
-        float sum[2] = {0.0f, 0.0f};
         int n = 0;
         for (int t = blockIdx.x; t < steps && !bad; t += gridDim.x) {
             const int r = t * 2 * MM_BM + j * MM_BM + quad * 32 + lane;
@@ -769,14 +727,13 @@ __global__ void __launch_bounds__(ES_THREADS, 1) k_edge_dsum(const __grid_consta
                         for (int y = 0; y < 8; ++y) w[y] = pack_bf16x2(acc[hh][u + 2 * y], acc[hh][u + 2 * y + 1]);
                         st8u(p + u, w);
                     }
+                    float *f = g.outf + (int64_t)r * MF_H + half * 64 + hh * 32;
+#pragma unroll
+                    for (int u = 0; u < 32; u += 8) st8f(f + u, acc[hh] + u);
                 }
                 __syncwarp();
-                sum[hh] += column_sums32(acc[hh], lane);
             }
         }
-        const int64_t row = (int64_t)blockIdx.x * 8 + j * 4 + quad;
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) g.cs[row * MF_H + half * 64 + hh * 32 + lane] = sum[hh];
     }
     if (bad) atomicCAS(g.error, 0, FL_E_TIMEOUT);
     tmem_fence_before();
@@ -785,10 +742,11 @@ __global__ void __launch_bounds__(ES_THREADS, 1) k_edge_dsum(const __grid_consta
 }
 
 // ------------------------------------------------------------- weight gradients
-constexpr int WG_PROD = 8, WG_THREADS = 32 * (WG_PROD + 1), WG_JOBS = 4;
+constexpr int WG_PROD = 8, WG_EPI = 4, WG_THREADS = 32 * (WG_PROD + 1 + WG_EPI), WG_JOBS = 4;
 constexpr int WG_BLOCK = 64 * 128;                  // 64 rows x 64 columns of bf16
 constexpr int WG_RING_BYTES = 224 * 1024, WG_MAX_RING = 7;
 constexpr int WG_SMEM = WG_RING_BYTES + 256 + 1024;
+constexpr int WG_SPLITS = 512, WG_CTAS = 256;
 
 struct WgSeg {
     const __nv_bfloat16 *base;
@@ -800,38 +758,52 @@ struct WgSeg {
 struct WgJob {
     WgSeg a, x[3];                                  // dZ (64 or 128 columns) and the segments of X
     int32_t nx, n_in, M;
-    int32_t cta0, ctas;
-    float *part;                                    // [ctas, a.width, n_in]
+    int32_t per, splits;                            // 64-row chunks per split, splits
+    float *part;                                    // [splits, a.width, n_in]
 };
 
+// CTA b takes items first[b] .. first[b + 1] - 1: job << 14 | split.
 struct WgArgs {
     WgJob job[WG_JOBS];
-    int32_t jobs;
     int32_t *error;
+    uint16_t first[WG_CTAS + 1];
+    uint16_t item[WG_JOBS * WG_SPLITS];
 };
 
-// Stage: 64 rows of dZ (two 64-column blocks of 8 KB) then of X's segments.
+// Splits of a product over M rows with n_in input features: partial sums of a
+// few chunks each, because a tensor-core accumulator that runs over many
+// hundred steps loses low bits that an fp32 sum of short partials keeps.
+static void wg_split(int M, int n_in, int *per, int *splits) {
+    const int chunks = (M + 63) / 64, tiles = (n_in + 127) / 128;
+    const int want = std::max(1, std::min(std::min(chunks, WG_SPLITS), 4 * 152 / tiles));
+    *per = (chunks + want - 1) / want;
+    *splits = (chunks + *per - 1) / *per;
+}
+
+// Stage: 64 rows of dZ (two 64-column blocks of 8 KB) then of X's segments; as
+// many as fit, so the ring is laid out anew where a CTA goes on to another job.
+// Accumulators: columns 0 and 256 in turn for n_in <= 256, else both at once.
+// Each split's accumulator is drained by the epilogue warps to its own slot.
 __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad(const __grid_constant__ WgArgs g) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t sR = smem_addr(smem);
     uint64_t *bars = (uint64_t *)(smem + WG_RING_BYTES);
-    const uint32_t ringf = smem_addr(bars), ringe = ringf + 8 * WG_MAX_RING, done = ringe + 8 * WG_MAX_RING;
-    uint32_t *tmem_slot = (uint32_t *)(bars + 2 * WG_MAX_RING + 1);
+    const uint32_t ringf = smem_addr(bars), ringe = ringf + 8 * WG_MAX_RING, accf = ringe + 8 * WG_MAX_RING, acce = accf + 16,
+                   drain = acce + 16;
+    uint32_t *tmem_slot = (uint32_t *)(bars + 2 * WG_MAX_RING + 5);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    int jn = 0;
-    while (jn + 1 < g.jobs && (int)blockIdx.x >= g.job[jn + 1].cta0) ++jn;
-    const WgJob &J = g.job[jn];
-    const int li = (int)blockIdx.x - J.cta0;
-    const int stage = (2 + J.n_in / 64) * WG_BLOCK, S = min(WG_MAX_RING, WG_RING_BYTES / stage);
-    const int64_t chunks = (J.M + 63) / 64;
-    const int c0 = (int)(chunks * li / J.ctas), c1 = (int)(chunks * (li + 1) / J.ctas);
+    const int it0 = g.first[blockIdx.x], it1 = g.first[blockIdx.x + 1];
     if (tid == 0) {
         for (int s = 0; s < WG_MAX_RING; ++s) {
             mbar_init(ringf + 8 * s, 32 * WG_PROD);
             mbar_init(ringe + 8 * s, 1);
         }
-        mbar_init(done, 1);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(accf + 8 * b, 1);
+            mbar_init(acce + 8 * b, WG_EPI);
+        }
+        mbar_init(drain, 1);
         mbar_fence_init();
     }
     if (warp == WG_PROD) {
@@ -839,12 +811,6 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad(const __grid_constant__
                      "r"(512u));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    if (J.a.width == 64) {  // the upper 64 output rows do not exist: zero operand columns
-        for (int s = 0; s < S; ++s)
-            for (int p = tid; p < WG_BLOCK / 16; p += WG_THREADS)
-                asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(sR + s * stage + WG_BLOCK + p * 16), "r"(0u) : "memory");
-    }
-    fence_async_smem();
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
@@ -858,107 +824,170 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad(const __grid_constant__
         // row maps are read one chunk ahead.  The job's fields are held in
         // registers: read from the parameters in the copy loop they made it
         // 230 cycles an instruction
-        const WgSeg G[4] = {J.a, J.x[0], J.x[1], J.x[2]};
-        const int nx = J.nx, M = J.M, own = 8 * warp + (lane & 7), piece = lane & 7;
-        uint32_t off[4];
-        off[0] = 0;
-        off[1] = 2 * WG_BLOCK;
-        off[2] = off[1] + (G[1].width / 64) * WG_BLOCK;
-        off[3] = off[2] + (G[2].width / 64) * WG_BLOCK;
-        auto load_rows = [&](int c, const __nv_bfloat16 *(&o)[4]) {
-            const int r = c * 64 + own;
-            const bool in = c < c1 && r < M;
-#pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                o[x] = nullptr;
-                if (in && x <= nx) o[x] = G[x].base + (G[x].rows ? (int64_t)G[x].rows[r] : (int64_t)r) * G[x].ld;
+        uint32_t busy = 0u, par = 0u;  // per stage: filled and not known empty; parity of its next "empty"
+        const int piece = lane & 7, own = 8 * warp + piece;
+        int s = 0, last = -1;
+        for (int it = it0; it < it1 && !bad; ++it) {
+            const int jn = g.item[it] >> 14, sp = g.item[it] & 0x3fff;
+            const WgJob &J = g.job[jn];
+            const int n_in = J.n_in, nx = J.nx, M = J.M, stage = (2 + n_in / 64) * WG_BLOCK;
+            const int S = min(WG_MAX_RING, WG_RING_BYTES / stage);
+            const WgSeg G[4] = {J.a, J.x[0], J.x[1], J.x[2]};
+            if (jn != last) {  // another layout: every stage of the old one must be empty
+                for (int k = 0; k < WG_MAX_RING && !bad; ++k) {
+                    if (!(busy >> k & 1u)) continue;
+                    if (!warp_wait(ringe + 8 * k, par >> k & 1u)) bad = true;
+                    par ^= 1u << k;
+                }
+                if (bad) break;
+                busy = 0u;
+                s = 0;
+                last = jn;
             }
-        };
-        const __nv_bfloat16 *row[4], *nrow[4];
-        load_rows(c0, row);
-        int s = 0, u = 0;
-        for (int c = c0; c < c1 && !bad; ++c) {
-            load_rows(c + 1, nrow);
-            if (u > 0 && !warp_wait(ringe + 8 * s, (u - 1) & 1)) {
-                bad = true;
-                break;
-            }
-            const uint32_t dst = sR + s * stage;
+            uint32_t off[4];
+            off[0] = 0;
+            off[1] = 2 * WG_BLOCK;
+            off[2] = off[1] + (G[1].width / 64) * WG_BLOCK;
+            off[3] = off[2] + (G[2].width / 64) * WG_BLOCK;
+            const int c0 = sp * J.per, c1 = min((M + 63) / 64, c0 + J.per);
+            auto load_rows = [&](int c, const __nv_bfloat16 *(&o)[4]) {
+                const int r = c * 64 + own;
+                const bool in = c < c1 && r < M;
 #pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                if (x <= nx) {
+                for (int x = 0; x < 4; ++x) {
+                    o[x] = nullptr;
+                    if (in && x <= nx) o[x] = G[x].base + (G[x].rows ? (int64_t)G[x].rows[r] : (int64_t)r) * G[x].ld;
+                }
+            };
+            const __nv_bfloat16 *row[4], *nrow[4];
+            load_rows(c0, row);
+            for (int c = c0; c < c1; ++c) {
+                load_rows(c + 1, nrow);
+                if (busy >> s & 1u) {
+                    if (!warp_wait(ringe + 8 * s, par >> s & 1u)) {
+                        bad = true;
+                        break;
+                    }
+                    par ^= 1u << s;
+                }
+                busy |= 1u << s;
+                const uint32_t dst = sR + s * stage;
 #pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        const int rr = 4 * i + (lane >> 3), R = 8 * warp + rr;
-                        const __nv_bfloat16 *src = (const __nv_bfloat16 *)__shfl_sync(0xffffffffu, (uint64_t)row[x], rr);
-                        const uint32_t d = dst + off[x] + (uint32_t)(R * 128 + ((piece ^ (R & 7)) << 4));
-                        if (src) {
-                            cp_async16(d, src + piece * 8);
-                            if (G[x].width == 128) cp_async16(d + WG_BLOCK, src + 64 + piece * 8);
-                        } else {
-                            asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(d), "r"(0u) : "memory");
-                            if (G[x].width == 128)
+                for (int x = 0; x < 4; ++x) {
+                    if (x <= nx) {
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const int rr = 4 * i + (lane >> 3), R = 8 * warp + rr;
+                            const __nv_bfloat16 *src = (const __nv_bfloat16 *)__shfl_sync(0xffffffffu, (uint64_t)row[x], rr);
+                            const uint32_t d = dst + off[x] + (uint32_t)(R * 128 + ((piece ^ (R & 7)) << 4));
+                            if (src) cp_async16(d, src + piece * 8);
+                            else asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(d), "r"(0u) : "memory");
+                            // the upper 64 columns; dZ of 64: zero operand columns
+                            if (src && G[x].width == 128) cp_async16(d + WG_BLOCK, src + 64 + piece * 8);
+                            else if (x == 0 || G[x].width == 128)
                                 asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(d + WG_BLOCK), "r"(0u) : "memory");
                         }
                     }
                 }
-            }
-            cp_async_arrive_noinc(ringf + 8 * s);
+                cp_async_arrive_noinc(ringf + 8 * s);
 #pragma unroll
-            for (int x = 0; x < 4; ++x) row[x] = nrow[x];
-            if (++s == S) {
-                s = 0;
-                ++u;
+                for (int x = 0; x < 4; ++x) row[x] = nrow[x];
+                if (++s == S) s = 0;
             }
         }
         cp_async_wait_all();
-        // the partial product: thread = one output row
-        if (!bad && !warp_wait(done, 0)) bad = true;
-        if (!bad) {
+    } else if (warp == WG_PROD) {
+        const bool issuer = elect_one();
+        uint32_t par = 0u, used = 0u, upar = 0u;  // stages' next "full" parity; accumulators in use and their parity
+        int s = 0, last = -1, turn = 0;
+        bool wide = false;
+        auto free_acc = [&](int b) {
+            if (!(used >> b & 1u)) return;
+            if (!warp_wait(acce + 8 * b, upar >> b & 1u)) bad = true;
+            upar ^= 1u << b;
+            used &= ~(1u << b);
+        };
+        for (int it = it0; it < it1 && !bad; ++it) {
+            const int jn = g.item[it] >> 14, sp = g.item[it] & 0x3fff;
+            const WgJob &J = g.job[jn];
+            const int n_in = J.n_in, stage = (2 + n_in / 64) * WG_BLOCK, S = min(WG_MAX_RING, WG_RING_BYTES / stage);
+            const int chunks = min((J.M + 63) / 64, (sp + 1) * J.per) - sp * J.per;
+            if (jn != last) {
+                s = 0;
+                last = jn;
+            }
+            // at most 256 columns an instruction: columns [0, w0) and [256, n_in)
+            const int w0 = min(256, n_in);
+            const uint32_t i0 = umma_idesc_bf16_mn(w0), i1 = umma_idesc_bf16_mn(n_in > 256 ? n_in - 256 : 64);
+            if (wide || n_in > 256) free_acc(0);
+            if (n_in > 256) free_acc(1);
+            wide = n_in > 256;
+            const int b = wide ? 0 : turn;
+            turn = b ^ 1;
+            free_acc(b);
+            if (bad) break;
+            used |= 1u << b;
             tmem_fence_after();
-            const int r = (warp & 3) * 32 + lane;
-            float *out = J.part + ((int64_t)li * J.a.width + r) * J.n_in;
-            for (int cb = (warp >> 2) * 32; cb < J.n_in; cb += 64) {
+            const uint32_t d = tmem + 256u * b;
+            uint32_t acc = 0u;
+            for (int c = 0; c < chunks; ++c) {
+                if (!warp_wait(ringf + 8 * s, par >> s & 1u)) {
+                    bad = true;
+                    break;
+                }
+                par ^= 1u << s;
+                fence_async_smem();
+                if (issuer) {
+                    const uint32_t a0 = sR + s * stage, x0 = a0 + 2 * WG_BLOCK;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {  // 16 rows each
+                        const uint64_t da = umma_desc_mn_sw128(a0 + k * 2048, WG_BLOCK);
+                        umma_bf16(d, da, umma_desc_mn_sw128(x0 + k * 2048, WG_BLOCK), i0, acc);
+                        if (n_in > 256) umma_bf16(d + 256u, da, umma_desc_mn_sw128(x0 + 4 * WG_BLOCK + k * 2048, WG_BLOCK), i1, acc);
+                        acc = 1u;
+                    }
+                    umma_commit(ringe + 8 * s);
+                }
+                if (++s == S) s = 0;
+            }
+            if (bad) break;
+            if (issuer) umma_commit(accf + 8 * b);
+        }
+        if (issuer) umma_commit(drain);
+        (void)warp_wait(drain, 0);
+    } else {
+        // epilogue: thread = one output row
+        const int quad = warp & 3, r = quad * 32 + lane;
+        const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
+        uint32_t par = 0u;
+        int turn = 0;
+        for (int it = it0; it < it1 && !bad; ++it) {
+            const WgJob &J = g.job[g.item[it] >> 14];
+            const int sp = g.item[it] & 0x3fff, n_in = J.n_in, rows = J.a.width;
+            const int b = n_in > 256 ? 0 : turn;
+            turn = b ^ 1;
+            if (!warp_wait(accf + 8 * b, par >> b & 1u)) {
+                bad = true;
+                break;
+            }
+            par ^= 1u << b;
+            tmem_fence_after();
+            float *out = J.part + ((int64_t)sp * rows + r) * n_in;
+            for (int cb = 0; cb < n_in; cb += 32) {
                 uint32_t v[32];
-                tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cb, v);
-                if (r < J.a.width) {
+                tmem_ld32(lanes + 256u * b + (uint32_t)cb, v);
+                if (cb + 32 >= n_in) {
+                    tmem_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(acce + 8 * b);
+                }
+                if (r < rows) {
 #pragma unroll
                     for (int u = 0; u < 32; u += 8) st8u(out + cb + u, v + u);
                 }
                 __syncwarp();
             }
         }
-    } else {
-        const bool issuer = elect_one();
-        // at most 256 columns an instruction: columns [0, w0) and [256, n_in)
-        const int n_in = J.n_in, w0 = min(256, n_in);
-        const uint32_t i0 = umma_idesc_bf16_mn(w0), i1 = umma_idesc_bf16_mn(n_in > 256 ? n_in - 256 : 64);
-        int s = 0, ph = 0;
-        uint32_t acc = 0u;
-        for (int c = c0; c < c1 && !bad; ++c) {
-            if (!warp_wait(ringf + 8 * s, ph)) {
-                bad = true;
-                break;
-            }
-            fence_async_smem();
-            if (issuer) {
-                const uint32_t a0 = sR + s * stage, x0 = a0 + 2 * WG_BLOCK;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {  // 16 rows each
-                    const uint64_t da = umma_desc_mn_sw128(a0 + k * 2048, WG_BLOCK);
-                    umma_bf16(tmem, da, umma_desc_mn_sw128(x0 + k * 2048, WG_BLOCK), i0, acc);
-                    if (n_in > 256) umma_bf16(tmem + 256u, da, umma_desc_mn_sw128(x0 + 4 * WG_BLOCK + k * 2048, WG_BLOCK), i1, acc);
-                    acc = 1u;
-                }
-                umma_commit(ringe + 8 * s);
-            }
-            if (++s == S) {
-                s = 0;
-                ph ^= 1;
-            }
-        }
-        if (issuer) umma_commit(done);
-        (void)warp_wait(done, 0);
     }
     if (bad) atomicCAS(g.error, 0, FL_E_TIMEOUT);
     tmem_fence_before();
@@ -966,8 +995,8 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad(const __grid_constant__
     if (warp == WG_PROD) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
 }
 
-// ------------------------------------------------------------- partial sums
-constexpr int RD_JOBS = 12;
+// ------------------------------------------------------------- sums over rows
+constexpr int RD_JOBS = 4, RD_STRIDE = 256, CS_JOBS = 3, BF_JOBS = 112;
 
 struct RdJob {
     const float *part;  // [count, n]
@@ -975,84 +1004,162 @@ struct RdJob {
     int32_t count, n;   // n a multiple of 4
 };
 
-struct RdArgs {
-    RdJob job[RD_JOBS];
+// Column sums of x over M rows by row class (r mod 256): part[class][n].  With
+// z: row r counts x[map[r]] where z[r] > 0 (a cell's message gradient over its edges).
+struct CsJob {
+    const float *x;
+    const __nv_bfloat16 *z;  // [M, 128] or nullptr
+    const int32_t *map;
+    float *part;             // [256, n]
+    int64_t ld;
+    int32_t M, n;
 };
 
-// Block (32, 8): 32 groups of four columns, each over eight interleaved
-// subsets of the partials, combined in subset order.
+struct RdArgs {
+    RdJob job[RD_JOBS];
+    CsJob cs[CS_JOBS];
+    int32_t jobs;            // blockIdx.y < jobs: partial products; else column sums
+};
+
+struct BfJob {
+    const float *part;       // [256, n]
+    float *out;              // [n], added to
+    int32_t n;
+};
+
+struct BfArgs {
+    BfJob job[BF_JOBS];
+};
+
+__device__ __forceinline__ void add4(float4 &s, const float4 v) {
+    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+}
+
+// Partial weight gradients: part[p] and part[p + 256], then over p in order.
+// Column sums for the bias gradients: a warp per row class walks its rows in
+// order, 16 rows' loads in flight (the order of a sum is kept, so many classes
+// of rows, not many adders, are what hides the latency).  Both in one launch:
+// either alone leaves the device half idle.
 __global__ void __launch_bounds__(256) k_reduce(const __grid_constant__ RdArgs g) {
     pdl_wait();
     pdl_launch_dependents();
-    const RdJob &J = g.job[blockIdx.y];
-    const int i = ((int)blockIdx.x * 32 + (int)threadIdx.x) * 4;
-    __shared__ float4 red[8][32];
+    if ((int)blockIdx.y < g.jobs) {
+        const RdJob &J = g.job[blockIdx.y];
+        const int n = J.n, count = J.count;
+        const int i = ((int)blockIdx.x * 256 + (int)threadIdx.x) * 4;
+        if (i >= n) return;
+        float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float *p = J.part + i;
+        const int lim = min(count, RD_STRIDE);
+        for (int b = 0; b < lim; b += 8) {
+            float4 v[8], w[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                v[u] = w[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (b + u < lim) v[u] = *(const float4 *)(p + (int64_t)(b + u) * n);
+                if (b + u + RD_STRIDE < count) w[u] = *(const float4 *)(p + (int64_t)(b + u + RD_STRIDE) * n);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                if (b + u + RD_STRIDE < count) add4(v[u], w[u]);
+                if (b + u < lim) add4(s, v[u]);
+            }
+        }
+        float4 *o = (float4 *)(J.out + i);
+        float4 v = *o;
+        add4(v, s);
+        *o = v;
+        return;
+    }
+    const CsJob &J = g.cs[blockIdx.y - g.jobs];
+    const int cls = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int c = lane * 4, M = J.M;
+    if (cls >= RD_STRIDE) return;
+    const bool in = c < J.n;
+    const float *x = J.x + c;
+    const int64_t ld = J.ld;
     float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (i < J.n) {
-#pragma unroll 4
-        for (int p = threadIdx.y; p < J.count; p += 8) {
-            const float4 v = *(const float4 *)(J.part + (int64_t)p * J.n + i);
-            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    if (!J.z) {
+        for (int r = cls; r < M; r += 16 * RD_STRIDE) {
+            float4 v[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) {
+                v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (in && r + u * RD_STRIDE < M) v[u] = *(const float4 *)(x + (int64_t)(r + u * RD_STRIDE) * ld);
+            }
+#pragma unroll
+            for (int u = 0; u < 16; ++u)
+                if (r + u * RD_STRIDE < M) add4(s, v[u]);
+        }
+    } else {
+        const __nv_bfloat16 *z = J.z + c;
+        for (int r0 = cls; r0 < M; r0 += 32 * RD_STRIDE) {
+            const int mine = r0 + lane * RD_STRIDE, at = mine < M ? J.map[mine] : 0;  // 32 rows' map entries at once
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float4 v[16];
+                uint2 m[16];
+#pragma unroll
+                for (int u = 0; u < 16; ++u) {
+                    const int r = r0 + (16 * h + u) * RD_STRIDE, row = __shfl_sync(0xffffffffu, at, 16 * h + u);
+                    v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    m[u] = make_uint2(0u, 0u);
+                    if (r < M) {
+                        v[u] = *(const float4 *)(x + (int64_t)row * ld);
+                        m[u] = *(const uint2 *)(z + (int64_t)r * MF_H);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 16; ++u) {
+                    if (r0 + (16 * h + u) * RD_STRIDE >= M) break;
+                    const uint32_t a = positive_mask(m[u].x), b = positive_mask(m[u].y);
+                    s.x += (a & 0xffffu) ? v[u].x : 0.0f;
+                    s.y += (a >> 16) ? v[u].y : 0.0f;
+                    s.z += (b & 0xffffu) ? v[u].z : 0.0f;
+                    s.w += (b >> 16) ? v[u].w : 0.0f;
+                }
+            }
         }
     }
-    red[threadIdx.y][threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.y || i >= J.n) return;
+    if (in) *(float4 *)(J.part + (int64_t)cls * J.n + c) = s;
+}
+
+// Bias gradients: the 256 class sums in order, added.
+__global__ void __launch_bounds__(128) k_bias_final(const __grid_constant__ BfArgs g) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const BfJob &J = g.job[blockIdx.x];
+    const int c = threadIdx.x;
+    if (c >= J.n) return;
+    float s = 0.0f;
+    for (int b = 0; b < RD_STRIDE; b += 32) {
+        float v[32];
 #pragma unroll
-    for (int p = 1; p < 8; ++p) {
-        const float4 v = red[p][threadIdx.x];
-        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        for (int u = 0; u < 32; ++u) v[u] = J.part[(b + u) * J.n + c];
+#pragma unroll
+        for (int u = 0; u < 32; ++u) s += v[u];
     }
-    float4 *o = (float4 *)(J.out + i);
-    const float4 v = *o;
-    *o = make_float4(v.x + s.x, v.y + s.y, v.z + s.z, v.w + s.w);
+    J.out[c] += s;
 }
 
-// ------------------------------------------------------------- optimizer
-constexpr int AD_JOBS = 128;
-
-struct AdJob {
-    float *w, *m1, *m2;
-    const float *g;
-    __nv_bfloat16 *wb, *wt;
-    int32_t rows, cols, ldt, block0;
-};
-
-struct AdArgs {
-    AdJob job[AD_JOBS];
-    float lr, b1, b2, eps, c1, c2, wd;
-    int32_t jobs;
-};
-
-// One Adam step over all of a network's tensors (k_adam's arithmetic).
-__global__ void __launch_bounds__(256) k_adam_all(const __grid_constant__ AdArgs g) {
-    int lo = 0, hi = g.jobs;  // job[lo].block0 <= blockIdx.x < job[hi].block0
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (g.job[mid].block0 <= (int)blockIdx.x) lo = mid; else hi = mid;
-    }
-    const AdJob &J = g.job[lo];
-    const int i = ((int)blockIdx.x - J.block0) * 256 + (int)threadIdx.x;
-    if (i >= J.rows * J.cols) return;
-    const float w0 = J.w[i], gi = J.g[i] + g.wd * w0;
-    const float a = g.b1 * J.m1[i] + (1.0f - g.b1) * gi;
-    const float b = g.b2 * J.m2[i] + (1.0f - g.b2) * gi * gi;
-    J.m1[i] = a;
-    J.m2[i] = b;
-    const float wi = w0 - g.lr * (a / g.c1) / (sqrtf(b / g.c2) + g.eps);
-    J.w[i] = wi;
-    const __nv_bfloat16 h = __float2bfloat16(wi);
-    if (J.wb) J.wb[i] = h;
-    if (J.wt) {
-        const int r = i / J.cols, c = i - r * J.cols;
-        J.wt[(int64_t)c * J.ldt + r] = h;
-    }
+// floats of scratch that fl_mpnn_backward needs: the weight gradients' partials
+// of the launch that has most, and every bias gradient's 256 class sums.
+static int64_t wg_floats(int M, int n_out, int n_in) {
+    int per = 0, splits = 0;
+    if (M < 1) return 0;
+    wg_split(M, n_in, &per, &splits);
+    return (int64_t)splits * n_out * n_in;
 }
 
-// floats of scratch that fl_mpnn_backward needs on a device of `sms` SMs: the
-// weight gradients' partials (at most 128 x 384 per CTA) and eight sets of
-// column sums (four rows of 128 per CTA).
-static int64_t backward_scratch(int sms) { return (int64_t)sms * (MF_H * 3 * MF_H + 8 * 4 * MF_H); }
+static int64_t partial_floats(int C, int E, int L) {
+    const int H = MF_H;
+    const int64_t layer = wg_floats(E, H, 3 * H) + wg_floats(E, H, H) + wg_floats(C, H, 2 * H) + wg_floats(C, H, H);
+    const int64_t enc = wg_floats(C, H, H) + wg_floats(C, H, 64) + wg_floats(E, H, H) + wg_floats(E, H, 64);
+    const int64_t dec = wg_floats(C, 64, H) + wg_floats(C, H, H);
+    return std::max(std::max(L > 0 ? layer : 0, enc), dec);
+}
+
+static int64_t backward_scratch(int C, int E, int L) { return partial_floats(C, E, L) + (int64_t)(3 * L + 6) * RD_STRIDE * MF_H; }
 
 static cudaError_t current_sms(int *dev, int *sms) {
     cudaError_t e = cudaGetDevice(dev);
@@ -1065,12 +1172,10 @@ using namespace fl;
 
 extern "C" {
 
-FL_API int fl_mpnn_backward_scratch(int64_t *floats) {
-    if (!floats) return set_error(FL_E_INVALID, "fl_mpnn_backward_scratch: NULL output");
-    int dev = 0, sms = 0;
-    const cudaError_t e = current_sms(&dev, &sms);
-    if (e != cudaSuccess) return set_error(FL_E_NO_DEVICE, "no usable CUDA device: %s", cudaGetErrorString(e));
-    *floats = backward_scratch(sms);
+FL_API int fl_mpnn_backward_scratch(int32_t cells, int32_t edges, int32_t layers, int64_t *floats) {
+    if (!floats || cells < 1 || edges < 0 || layers < 0)
+        return set_error(FL_E_INVALID, "fl_mpnn_backward_scratch: bad sizes or NULL output");
+    *floats = backward_scratch(cells, edges, layers);
     return FL_OK;
 }
 
@@ -1079,16 +1184,17 @@ FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *d, void *stream) {
         return set_error(FL_E_INVALID, "fl_mpnn_backward: bad sizes (at most %d layers)", ES_MAX_LAYERS);
     const int C = d->cells, E = d->edges, L = d->layers;
     if (!d->x || !d->dy || !d->recv_start || !d->zn || !d->zd || !d->h_bf || !d->dh[0] || !d->dh[1] || !d->dz2c || !d->dz1c ||
-        !d->dyb || !d->scratch ||
-        (L > 0 && (!d->edge || !d->node || !d->agg || !d->z1n || !d->z1e || !d->dze || !d->dagg || !d->send_start)) ||
-        (E > 0 && (!d->src || !d->dst || !d->send_order || !d->ef || !d->ze || !d->e || !d->dz2e)))
+        !d->dyb || !d->dz1f || !d->scratch ||
+        (L > 0 && (!d->edge || !d->node || !d->agg || !d->z1n || !d->z1e || !d->dze || !d->dagg || !d->daggf || !d->gf || !d->send_start)) ||
+        (E > 0 && (!d->src || !d->dst || !d->send_order || !d->ef || !d->ze || !d->e || !d->dz2e || !d->ef32)))
         return set_error(FL_E_INVALID, "fl_mpnn_backward: NULL pointer");
     if (d->ldx < 64 || d->ldx % 8 || d->lde < 64 || d->lde % 8 || d->ldy < 64 || d->ldy % 8)
         return set_error(FL_E_INVALID, "fl_mpnn_backward: leading dimensions must be multiples of 8 and at least 64");
     uintptr_t a16 = (uintptr_t)d->x | (uintptr_t)d->ef;
     uintptr_t a32 = (uintptr_t)d->dy | (uintptr_t)d->zn | (uintptr_t)d->ze | (uintptr_t)d->e | (uintptr_t)d->zd |
                     (uintptr_t)d->dh[0] | (uintptr_t)d->dh[1] | (uintptr_t)d->dz2c | (uintptr_t)d->dz1c | (uintptr_t)d->dagg |
-                    (uintptr_t)d->dyb | (uintptr_t)d->dz2e | (uintptr_t)d->scratch;
+                    (uintptr_t)d->dyb | (uintptr_t)d->dz2e | (uintptr_t)d->dz1f | (uintptr_t)d->gf | (uintptr_t)d->ef32 |
+                    (uintptr_t)d->scratch;
     bool ok = true;
     auto dense = [&](const FlDenseGrad &r, int n_out) {
         a16 |= (uintptr_t)r.wt | (uintptr_t)r.gw | (uintptr_t)r.gb;
@@ -1101,8 +1207,9 @@ FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *d, void *stream) {
             dense(d->edge[2 * l + j], 128);
             dense(d->node[2 * l + j], 128);
         }
-        ok = ok && d->h_bf[l] && d->agg[l] && d->z1n[l] && (E == 0 || (d->z1e[l] && d->dze[l]));
-        a32 |= (uintptr_t)d->h_bf[l] | (uintptr_t)d->agg[l] | (uintptr_t)d->z1n[l] | (uintptr_t)d->z1e[l] | (uintptr_t)d->dze[l];
+        ok = ok && d->h_bf[l] && d->agg[l] && d->z1n[l] && d->daggf[l] && (E == 0 || (d->z1e[l] && d->dze[l]));
+        a32 |= (uintptr_t)d->h_bf[l] | (uintptr_t)d->agg[l] | (uintptr_t)d->z1n[l] | (uintptr_t)d->z1e[l] | (uintptr_t)d->dze[l] |
+               (uintptr_t)d->daggf[l];
     }
     if (!ok || !d->h_bf[L]) return set_error(FL_E_INVALID, "fl_mpnn_backward: bad layer");
     a32 |= (uintptr_t)d->h_bf[L];
@@ -1113,9 +1220,9 @@ FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *d, void *stream) {
     if (rc) return rc;
     int dev = 0, sms = 0;
     cudaError_t e = current_sms(&dev, &sms);
-    if (e == cudaSuccess && d->scratch_floats < backward_scratch(sms))
+    if (e == cudaSuccess && d->scratch_floats < backward_scratch(C, E, L))
         return set_error(FL_E_INVALID, "fl_mpnn_backward: scratch of %lld floats, %lld needed", (long long)d->scratch_floats,
-                         (long long)backward_scratch(sms));
+                         (long long)backward_scratch(C, E, L));
     static std::atomic<uint64_t> done[6];
     if (e == cudaSuccess) e = allow_smem((const void *)k_mlp_bwd<0>, MB_SMEM, dev, done[0]);
     if (e == cudaSuccess) e = allow_smem((const void *)k_mlp_bwd<1>, MB_SMEM, dev, done[1]);
@@ -1126,27 +1233,48 @@ FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *d, void *stream) {
     cudaStream_t st = (cudaStream_t)stream;
     using bf = __nv_bfloat16;
     int64_t launched = 0;
-    float *part = d->scratch, *cs[8];
-    for (int k = 0; k < 8; ++k) cs[k] = part + (int64_t)sms * (MF_H * 3 * MF_H + k * 4 * MF_H);
+    float *part = d->scratch, *classes = part + partial_floats(C, E, L);
     const int c_tiles = (C + MM_BM - 1) / MM_BM, e_tiles = (E + MM_BM - 1) / MM_BM;
-    const int c_grid = std::min(c_tiles, sms), e_grid = std::max(1, std::min(e_tiles, sms));
 
-    // the weight gradients of up to four products in one launch, the CTAs
-    // shared out by the bytes each product stages; then every partial sum
+    // the weight gradients of up to four products in one launch, then every
+    // partial sum.  The items (splits) go to the CTAs largest first, each to
+    // the CTA with least to stage so far; a launch's jobs have the same sizes
+    // in every layer, so the assignment is made once per kind of launch
     RdArgs rd;
-    int n_rd = 0, rd_cols = 0;
-    auto sums = [&](const float *p, int count, int n, float *out) {
-        rd.job[n_rd++] = RdJob{p, out, count, n};
-        rd_cols = std::max(rd_cols, n);
+    BfArgs bf_args;
+    int n_rd = 0, n_cs = 0, n_bf = 0, rd_blocks = 0;
+    auto sums = [&](const float *x, int64_t ld, int M, int n, float *gb, const void *z = nullptr, const int32_t *map = nullptr) {
+        if (M < 1) return;
+        rd.cs[n_cs++] = CsJob{x, (const bf *)z, map, classes, ld, M, n};
+        bf_args.job[n_bf++] = BfJob{classes, gb, n};
+        classes += RD_STRIDE * MF_H;
+        rd_blocks = std::max(rd_blocks, RD_STRIDE / 8);
+    };
+    auto reduce = [&]() {
+        if (e != cudaSuccess) return;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)rd_blocks, (unsigned)(n_rd + n_cs));
+        cfg.blockDim = dim3(256);
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        rd.jobs = n_rd;
+        e = cudaLaunchKernelEx(&cfg, k_reduce, rd);
+        ++launched;
+        n_rd = n_cs = rd_blocks = 0;
     };
     WgArgs wg;
-    wg.jobs = 0;
     wg.error = err;
+    int n_wg = 0, ctas = 0;
+    bool planned = false;
     float *wg_out[WG_JOBS];
     auto seg = [](const void *p, const int32_t *rows, int64_t ld, int width) { return WgSeg{(const bf *)p, rows, ld, width}; };
     auto product = [&](int M, WgSeg a, std::initializer_list<WgSeg> xs, float *gw) {
         if (M < 1) return;
-        WgJob &J = wg.job[wg.jobs];
+        WgJob &J = wg.job[n_wg];
         J = WgJob{};
         J.a = a;
         J.M = M;
@@ -1154,43 +1282,53 @@ FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *d, void *stream) {
             J.x[J.nx++] = x;
             J.n_in += x.width;
         }
-        wg_out[wg.jobs++] = gw;
+        wg_split(M, J.n_in, &J.per, &J.splits);
+        wg_out[n_wg++] = gw;
+    };
+    auto plan = [&]() {
+        ctas = std::min(sms, WG_CTAS);
+        std::vector<std::vector<uint16_t>> list(ctas);
+        std::vector<std::pair<int64_t, int>> load(ctas);  // heap: least loaded first, then the lower CTA
+        for (int b = 0; b < ctas; ++b) load[b] = {0, b};
+        int order[WG_JOBS];
+        auto cost = [&](int j) { return (int64_t)wg.job[j].per * (wg.job[j].a.width + wg.job[j].n_in) + wg.job[j].n_in; };
+        for (int j = 0; j < n_wg; ++j) order[j] = j;
+        std::sort(order, order + n_wg, [&](int x, int y) { return cost(x) != cost(y) ? cost(x) > cost(y) : x < y; });
+        auto more = [](const std::pair<int64_t, int> &x, const std::pair<int64_t, int> &y) { return x > y; };
+        for (int k = 0; k < n_wg; ++k) {
+            const int j = order[k];
+            for (int sp = 0; sp < wg.job[j].splits; ++sp) {
+                std::pop_heap(load.begin(), load.end(), more);
+                list[load.back().second].push_back((uint16_t)(j << 14 | sp));
+                load.back().first += cost(j);
+                std::push_heap(load.begin(), load.end(), more);
+            }
+        }
+        int n = 0, used = 0;
+        for (int b = 0; b < ctas; ++b) {
+            if (list[b].empty()) continue;
+            wg.first[used++] = (uint16_t)n;
+            for (uint16_t x : list[b]) wg.item[n++] = x;
+        }
+        wg.first[used] = (uint16_t)n;
+        ctas = used;
     };
     auto flush = [&]() {
         if (e != cudaSuccess) return;
-        double total = 0.0;
-        for (int j = 0; j < wg.jobs; ++j) total += (double)wg.job[j].M * (wg.job[j].a.width + wg.job[j].n_in);
-        int cta = 0;
         float *p = part;
-        for (int j = 0; j < wg.jobs; ++j) {
+        for (int j = 0; j < n_wg; ++j) {
             WgJob &J = wg.job[j];
-            const int left = wg.jobs - 1 - j, chunks = (J.M + 63) / 64;
-            const double cost = (double)J.M * (J.a.width + J.n_in);
-            int n = (int)(sms * cost / total + 0.5);
-            n = std::max(1, std::min(std::min(n, chunks), sms - cta - left));
-            J.cta0 = cta;
-            J.ctas = n;
             J.part = p;
-            cta += n;
-            p += (int64_t)n * J.a.width * J.n_in;
-            sums(J.part, n, J.a.width * J.n_in, wg_out[j]);
+            p += (int64_t)J.splits * J.a.width * J.n_in;
+            rd.job[n_rd++] = RdJob{J.part, wg_out[j], J.splits, J.a.width * J.n_in};
+            rd_blocks = std::max(rd_blocks, (J.a.width * J.n_in + 1023) / 1024);
         }
-        e = launch_blocks(k_wgrad, wg, cta, sms, WG_THREADS, WG_SMEM, launched > 0, st);
+        if (!planned) plan();
+        planned = true;
+        e = launch_blocks(k_wgrad, wg, ctas, sms, WG_THREADS, WG_SMEM, launched > 0, st);
         ++launched;
-        if (e == cudaSuccess) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)((rd_cols + 127) / 128), (unsigned)n_rd);
-            cfg.blockDim = dim3(32, 8);
-            cfg.stream = st;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[0].val.programmaticStreamSerializationAllowed = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            e = cudaLaunchKernelEx(&cfg, k_reduce, rd);
-            ++launched;
-        }
-        wg.jobs = n_rd = rd_cols = 0;
+        n_wg = 0;
+        reduce();
     };
     auto mlp = [&](auto kernel, MlpBwdArgs a, int blocks) {
         if (e != cudaSuccess) return;
@@ -1212,18 +1350,18 @@ FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *d, void *stream) {
         a.dz2 = (bf *)d->dyb;
         a.dz1 = (bf *)d->dz1c;
         a.dx = d->dh[0];
-        a.cs_b2 = cs[0];
-        a.cs_b1 = cs[1];
+        a.dz1f = d->dz1f;
         a.n2 = 64;
         a.M = C;
         mlp(k_mlp_bwd<1>, a, c_tiles);
-        sums(cs[0], 4 * c_grid, 64, d->dec[1].gb);
-        sums(cs[1], 4 * c_grid, MF_H, d->dec[0].gb);
+        sums(d->dy, d->ldy, C, 64, d->dec[1].gb);
+        sums(d->dz1f, MF_H, C, MF_H, d->dec[0].gb);
         product(C, seg(d->dyb, nullptr, 64, 64), {seg(d->zd, nullptr, MF_H, MF_H)}, d->dec[1].gw);
         product(C, seg(d->dz1c, nullptr, MF_H, MF_H), {seg(d->h_bf[L], nullptr, MF_H, MF_H)}, d->dec[0].gw);
         flush();
     }
     int cur = 0;
+    planned = false;
     for (int l = L - 1; l >= 0 && e == cudaSuccess; --l, cur ^= 1) {
         const FlDenseGrad &e1 = d->edge[2 * l], &e2 = d->edge[2 * l + 1], &n1 = d->node[2 * l], &n2 = d->node[2 * l + 1];
         MlpBwdArgs a{};
@@ -1243,10 +1381,9 @@ FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *d, void *stream) {
         a.start = d->recv_start;
         a.z1e = (const bf *)d->z1e[l];
         a.dze = (bf *)d->dze[l];
-        a.cs_b2 = cs[0];
-        a.cs_b1 = cs[1];
-        a.cs_e2 = cs[2];
-        a.cs_e1 = cs[3];
+        a.dz1f = d->dz1f;
+        a.daggf = d->daggf[l];
+        a.gf = d->gf;
         a.n2 = MF_H;
         a.M = C;
         mlp(k_mlp_bwd<2>, a, c_tiles);
@@ -1264,10 +1401,9 @@ FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *d, void *stream) {
             e = launch_blocks(k_edge_bwd, b, c_tiles, sms, EB_THREADS, EB_SMEM, true, st);
             ++launched;
         }
-        sums(cs[0], 4 * c_grid, MF_H, n2.gb);
-        sums(cs[1], 4 * c_grid, MF_H, n1.gb);
-        sums(cs[2], 4 * c_grid, MF_H, e2.gb);
-        sums(cs[3], 4 * c_grid, MF_H, e1.gb);
+        sums(d->dh[cur], MF_H, C, MF_H, n2.gb);
+        sums(d->dz1f, MF_H, C, MF_H, n1.gb);
+        sums(d->gf, MF_H, E, MF_H, e1.gb, d->z1e[l], d->dst);
         product(E, seg(d->dze[l], nullptr, MF_H, MF_H),
                 {seg(d->h_bf[l], d->dst, MF_H, MF_H), seg(d->h_bf[l], d->src, MF_H, MF_H), seg(d->e, nullptr, MF_H, MF_H)}, e1.gw);
         product(E, seg(d->dagg, d->dst, MF_H, MF_H), {seg(d->z1e[l], nullptr, MF_H, MF_H)}, e2.gw);
@@ -1277,6 +1413,7 @@ FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *d, void *stream) {
         flush();
     }
     // encoders
+    planned = false;
     {
         MlpBwdArgs a{};
         a.dy = d->dh[cur];
@@ -1286,13 +1423,12 @@ FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *d, void *stream) {
         a.ldw2t = d->enc_n[1].ldwt;
         a.dz2 = (bf *)d->dz2c;
         a.dz1 = (bf *)d->dz1c;
-        a.cs_b2 = cs[0];
-        a.cs_b1 = cs[1];
+        a.dz1f = d->dz1f;
         a.n2 = MF_H;
         a.M = C;
         mlp(k_mlp_bwd<0>, a, c_tiles);
-        sums(cs[0], 4 * c_grid, MF_H, d->enc_n[1].gb);
-        sums(cs[1], 4 * c_grid, MF_H, d->enc_n[0].gb);
+        sums(d->dh[cur], MF_H, C, MF_H, d->enc_n[1].gb);
+        sums(d->dz1f, MF_H, C, MF_H, d->enc_n[0].gb);
         product(C, seg(d->dz2c, nullptr, MF_H, MF_H), {seg(d->zn, nullptr, MF_H, MF_H)}, d->enc_n[1].gw);
         product(C, seg(d->dz1c, nullptr, MF_H, MF_H), {seg(d->x, nullptr, d->ldx, 64)}, d->enc_n[0].gw);
     }
@@ -1306,63 +1442,45 @@ FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *d, void *stream) {
                 b.ldwt[k] = d->edge[2 * l].ldwt;
             }
             b.out = (bf *)d->dz2e;
-            b.cs = cs[4];
+            b.outf = d->ef32;
             b.layers = L;
             b.E = E;
             b.error = err;
             e = launch_blocks(k_edge_dsum, b, (E + 2 * MM_BM - 1) / (2 * MM_BM), sms, ES_THREADS, ES_SMEM, true, st);
             ++launched;
         }
+        sums(d->ef32, MF_H, E, MF_H, d->enc_e[1].gb);
+        reduce();  // (the fp32 buffer is used again)
         MlpBwdArgs a{};
         a.dyb = (const bf *)d->dz2e;
         a.z = (const bf *)d->ze;
         a.w2t = (const bf *)d->enc_e[1].wt;
         a.ldw2t = d->enc_e[1].ldwt;
         a.dz1 = (bf *)d->dze[0];  // (no longer needed)
-        a.cs_b1 = cs[6];
+        a.dz1f = d->ef32;
         a.n2 = MF_H;
         a.M = E;
         mlp(k_mlp_bwd<0>, a, e_tiles);
-        sums(cs[4], 8 * std::min((E + 2 * MM_BM - 1) / (2 * MM_BM), sms), MF_H, d->enc_e[1].gb);  // (sets 4 and 5)
-        sums(cs[6], 4 * e_grid, MF_H, d->enc_e[0].gb);
+        sums(d->ef32, MF_H, E, MF_H, d->enc_e[0].gb);
         product(E, seg(d->dz2e, nullptr, MF_H, MF_H), {seg(d->ze, nullptr, MF_H, MF_H)}, d->enc_e[1].gw);
         product(E, seg(d->dze[0], nullptr, MF_H, MF_H), {seg(d->ef, nullptr, d->lde, 64)}, d->enc_e[0].gw);
     }
     flush();
+    if (e == cudaSuccess) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)n_bf);
+        cfg.blockDim = dim3(128);
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        e = cudaLaunchKernelEx(&cfg, k_bias_final, bf_args);
+        ++launched;
+    }
     if (e != cudaSuccess) return set_error(FL_E_CUDA, "fl_mpnn_backward: %s", cudaGetErrorString(e));
     add_launches(launched);
-    return FL_OK;
-}
-
-FL_API int fl_adam_all(const FlAdamTensor *t, int32_t n, float lr, float b1, float b2, float eps, int32_t step,
-                       float weight_decay, void *stream) {
-    if (!t || n < 1 || step < 1) return set_error(FL_E_INVALID, "fl_adam_all: bad arguments");
-    for (int k = 0; k < n; ++k)
-        if (!t[k].w || !t[k].m1 || !t[k].m2 || !t[k].g || t[k].rows < 1 || t[k].cols < 1 ||
-            (int64_t)t[k].rows * t[k].cols > (1 << 30) || (t[k].wt_bf16 && t[k].ldt < t[k].rows))
-            return set_error(FL_E_INVALID, "fl_adam_all: tensor %d: bad arguments", k);
-    AdArgs a;
-    a.lr = lr;
-    a.b1 = b1;
-    a.b2 = b2;
-    a.eps = eps;
-    a.c1 = 1.0f - powf(b1, (float)step);
-    a.c2 = 1.0f - powf(b2, (float)step);
-    a.wd = weight_decay;
-    for (int k0 = 0; k0 < n; k0 += AD_JOBS) {
-        int blocks = 0;
-        a.jobs = std::min(AD_JOBS, n - k0);
-        for (int k = 0; k < a.jobs; ++k) {
-            const FlAdamTensor &s = t[k0 + k];
-            a.job[k] = AdJob{s.w, s.m1, s.m2, s.g, (__nv_bfloat16 *)s.w_bf16, (__nv_bfloat16 *)s.wt_bf16,
-                             s.rows, s.cols, s.ldt, blocks};
-            blocks += (int)(((int64_t)s.rows * s.cols + 255) / 256);
-        }
-        k_adam_all<<<blocks, 256, 0, (cudaStream_t)stream>>>(a);
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return set_error(FL_E_CUDA, "k_adam_all launch: %s", cudaGetErrorString(e));
-        add_launches(1);
-    }
     return FL_OK;
 }
 

@@ -34,9 +34,9 @@
 
 namespace fl {
 
-constexpr int MF_PROD_WARPS = 4, MF_EPI_WARPS = 8, MF_THREADS = 32 * (MF_PROD_WARPS + 1 + MF_EPI_WARPS);
+constexpr int MF_PROD_WARPS = 2, MF_EPI_WARPS = 16, MF_THREADS = 32 * (MF_PROD_WARPS + 1 + MF_EPI_WARPS);
 constexpr int MF_CHUNKS = 14;  // 16 KB chunks of shared memory
-constexpr int MF_SMEM = MF_CHUNKS * MM_CHUNK_BYTES + 1024 /* biases */ + 256 /* barriers */ + 1024 /* alignment */;
+constexpr int MF_SMEM = MF_CHUNKS * MM_CHUNK_BYTES + 256 /* barriers */ + 1024 /* alignment */;
 constexpr int EF_RING = 4;
 constexpr int M2_MAX_RING = 8;
 
@@ -67,14 +67,39 @@ struct Mlp2Args {
     int32_t *error;
 };
 
-// relu(v + bias) of 32 columns as 16 bf16 pairs; bias in shared memory.
-__device__ __forceinline__ void relu_pack32(const uint32_t (&v)[32], const float *bias, uint32_t *out) {
+// Epilogue: warp = 32 rows (its TMEM lanes) x 32 columns in the fragment shape,
+// so a lane needs only eight of a layer's biases and holds them for the whole
+// kernel (read per row and column from shared memory, a four-wavefront
+// broadcast each, they took a third of the shared-memory pipe that the MMA
+// operands and the gathers need).  Four lanes hold a row's 32 columns; a 4 x 4
+// transpose gives each eight consecutive ones for full 128-byte lines.
+struct FragBias {
+    float2 b[4];  // columns 8 j + 2 q, + 1
+};
+
+__device__ __forceinline__ FragBias frag_bias(const float *p, int q, bool in) {
+    FragBias f;
 #pragma unroll
-    for (int q = 0; q < 32; q += 4) {
-        const float4 b = *(const float4 *)(bias + q);
-        out[q / 2] = pack_bf16x2(fmaxf(__uint_as_float(v[q]) + b.x, 0.0f), fmaxf(__uint_as_float(v[q + 1]) + b.y, 0.0f));
-        out[q / 2 + 1] = pack_bf16x2(fmaxf(__uint_as_float(v[q + 2]) + b.z, 0.0f), fmaxf(__uint_as_float(v[q + 3]) + b.w, 0.0f));
+    for (int j = 0; j < 4; ++j) f.b[j] = in ? make_float2(p[8 * j + 2 * q], p[8 * j + 2 * q + 1]) : make_float2(0.0f, 0.0f);
+    return f;
+}
+
+// relu(v + bias) of 16 rows as bf16 pairs.
+__device__ __forceinline__ void relu_pack_frag(const uint32_t (&v)[16], const FragBias &f, uint32_t (&w)[8]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+            w[2 * j + r] = pack_bf16x2(fmaxf(__uint_as_float(v[4 * j + 2 * r]) + f.b[j].x, 0.0f),
+                                       fmaxf(__uint_as_float(v[4 * j + 2 * r + 1]) + f.b[j].y, 0.0f));
     }
+}
+
+// Row r (0: g, 1: g + 8) of packed pairs to global memory: 16 bytes a lane.
+__device__ __forceinline__ void store_pairs(const uint32_t (&w)[8], int r, int q, __nv_bfloat16 *row, bool in) {
+    uint32_t x0 = w[r], x1 = w[2 + r], x2 = w[4 + r], x3 = w[6 + r];
+    transpose4(x0, x1, x2, x3, q);
+    if (in) *(uint4 *)(row + 8 * q) = make_uint4(x0, x1, x2, x3);
 }
 
 // One 128-deep second product: A = the z buffer in TMEM, B = w2 in shared memory.
@@ -90,8 +115,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_edge_fwd(const __grid_constan
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t sW1 = smem_addr(smem), sW2 = sW1 + 6 * MM_CHUNK_BYTES, sD = sW2 + 2 * MM_CHUNK_BYTES;
     const uint32_t sR = sD + 2 * MM_CHUNK_BYTES;
-    float *bias = (float *)(smem + MF_CHUNKS * MM_CHUNK_BYTES);  // b1, b2
-    uint64_t *bars = (uint64_t *)(bias + 256);
+    uint64_t *bars = (uint64_t *)(smem + MF_CHUNKS * MM_CHUNK_BYTES);
     const uint32_t dstf = smem_addr(bars), dste = dstf + 8, ringf = dstf + 16, ringe = ringf + 8 * EF_RING;
     const uint32_t d1f = ringe + 8 * EF_RING, zf = d1f + 24, d2f = zf + 16, de = d2f + 24, drain = de + 24;
     uint32_t *tmem_slot = (uint32_t *)(bars + 2 + 2 * EF_RING + 3 + 2 + 3 + 3 + 1);
@@ -123,7 +147,6 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_edge_fwd(const __grid_constan
     // weights: not written by the kernel before this one (they change between passes only)
     for (int c = 0; c < 6; ++c) load_weight_chunk(g.w1, g.ldw1, MF_H, c, sW1 + c * MM_CHUNK_BYTES, tid, MF_THREADS);
     for (int c = 0; c < 2; ++c) load_weight_chunk(g.w2, g.ldw2, MF_H, c, sW2 + c * MM_CHUNK_BYTES, tid, MF_THREADS);
-    if (tid < 256) bias[tid] = tid < 128 ? g.b1[tid] : g.b2[tid - 128];
     cp_async_commit();
     cp_async_wait_all();
     fence_async_smem();
@@ -136,46 +159,51 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_edge_fwd(const __grid_constan
     pdl_launch_dependents();
 
     if (warp < MF_PROD_WARPS) {
-        // producers: lane = tile row 32 * warp + lane
-        int t = blockIdx.x;
-        int c = t * MM_BM + 32 * warp + lane;
-        int rs = 0, re = 0, s0 = 0, s1 = 0, s2 = 0;
-        if (t < tiles && c < g.C) {
-            rs = g.start[c];
-            re = g.start[c + 1];
-            if (rs < re) s0 = g.src[rs];
-            if (rs + 1 < re) s1 = g.src[rs + 1];
-            if (rs + 2 < re) s2 = g.src[rs + 2];
-        }
-        int q = 0;
-        for (int i = 0; t < tiles && !bad; ++i) {
-            // the next tile's index loads are issued here and used in the next round
-            const int tn = t + gridDim.x, cn = tn * MM_BM + 32 * warp + lane;
-            int rsn = 0, ren = 0, n0 = 0, n1 = 0, n2 = 0;
-            const bool more = tn < tiles && cn < g.C;
-            if (more) {
-                rsn = g.start[cn];
-                ren = g.start[cn + 1];
+        // producers: a lane's tile rows are 64 * warp + lane and + 32; first
+        // edge, edge count and senders, the next tile's read one tile ahead
+        int t = blockIdx.x, q = 0;
+        int rs[2], deg[2], snd[2][3];
+        auto load_starts = [&](int tt, int (&a)[2], int (&b)[2]) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int c = tt * MM_BM + 64 * warp + lane + 32 * j;
+                a[j] = b[j] = 0;
+                if (tt < tiles && c < g.C) {
+                    a[j] = g.start[c];
+                    b[j] = g.start[c + 1] - a[j];
+                }
             }
+        };
+        auto load_senders = [&](const int (&a)[2], const int (&b)[2], int (&o)[2][3]) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int k = 0; k < 3; ++k) o[j][k] = k < b[j] ? g.src[a[j] + k] : -1;
+        };
+        load_starts(t, rs, deg);
+        load_senders(rs, deg, snd);
+        for (int i = 0; t < tiles && !bad; ++i) {
+            const int tn = t + gridDim.x, c0 = t * MM_BM + 64 * warp + lane, c1 = c0 + 32;
+            int nrs[2], ndeg[2], nsnd[2][3];
+            load_starts(tn, nrs, ndeg);
             if (i > 0 && !warp_wait(dste, (i - 1) & 1)) {
                 bad = true;
                 break;
             }
-            const __nv_bfloat16 *own = c < g.C ? g.h + (int64_t)c * MF_H : nullptr;
-            warp_copy_rows(own, sD, warp, lane);
-            warp_copy_rows(own ? own + 64 : nullptr, sD + MM_CHUNK_BYTES, warp, lane);
+            const __nv_bfloat16 *h0 = c0 < g.C ? g.h + (int64_t)c0 * MF_H : nullptr;
+            const __nv_bfloat16 *h1 = c1 < g.C ? g.h + (int64_t)c1 * MF_H : nullptr;
+            warp_copy_rows64(h0, h1, sD, warp, lane);
+            warp_copy_rows64(h0 ? h0 + 64 : nullptr, h1 ? h1 + 64 : nullptr, sD + MM_CHUNK_BYTES, warp, lane);
             cp_async_arrive_noinc(dstf);
-            if (more) {
-                if (rsn < ren) n0 = g.src[rsn];
-                if (rsn + 1 < ren) n1 = g.src[rsn + 1];
-                if (rsn + 2 < ren) n2 = g.src[rsn + 2];
-            }
-#pragma unroll 1
-            for (int k = 0; k < 3 && !bad; ++k) {
-                const bool valid = rs + k < re;
-                const int sk = k == 0 ? s0 : (k == 1 ? s1 : s2);
-                const __nv_bfloat16 *ph = valid ? g.h + (int64_t)sk * MF_H : nullptr;
-                const __nv_bfloat16 *pe = valid ? g.e + (int64_t)(rs + k) * MF_H : nullptr;
+            load_senders(nrs, ndeg, nsnd);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const __nv_bfloat16 *ph[2], *pe[2];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    ph[j] = snd[j][k] >= 0 ? g.h + (int64_t)snd[j][k] * MF_H : nullptr;
+                    pe[j] = k < deg[j] ? g.e + (int64_t)(rs[j] + k) * MF_H : nullptr;
+                }
 #pragma unroll
                 for (int j = 0; j < 4; ++j, ++q) {
                     const int s = q % EF_RING, u = q / EF_RING;
@@ -183,12 +211,21 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_edge_fwd(const __grid_constan
                         bad = true;
                         break;
                     }
-                    const __nv_bfloat16 *p = j < 2 ? ph : pe;
-                    warp_copy_rows(p ? p + (j & 1) * 64 : nullptr, sR + s * MM_CHUNK_BYTES, warp, lane);
+                    const __nv_bfloat16 *p0 = j < 2 ? ph[0] : pe[0], *p1 = j < 2 ? ph[1] : pe[1];
+                    warp_copy_rows64(p0 ? p0 + (j & 1) * 64 : nullptr, p1 ? p1 + (j & 1) * 64 : nullptr,
+                                     sR + s * MM_CHUNK_BYTES, warp, lane);
                     cp_async_arrive_noinc(ringf + 8 * s);
                 }
+                if (bad) break;
             }
-            t = tn; c = cn; rs = rsn; re = ren; s0 = n0; s1 = n1; s2 = n2;
+            t = tn;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                rs[j] = nrs[j];
+                deg[j] = ndeg[j];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) snd[j][k] = nsnd[j][k];
+            }
         }
         cp_async_wait_all();
     } else if (warp == MF_PROD_WARPS) {
@@ -258,59 +295,71 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_edge_fwd(const __grid_constan
             (void)warp_wait(drain, 0);
         }
     } else {
-        // epilogue: thread = one cell, 64 of its 128 columns
-        const int quad = warp & 3, half = (warp - MF_PROD_WARPS - 1) >> 2;
-        const uint32_t lanes = (uint32_t)(quad * 32) << 16;
-        const float *b1 = bias + half * 64, *b2 = bias + 128 + half * 64;
-        float acc[64];
-        int n = 0, pc = 0, pdeg = 0;
-        // the messages of slot m (region k) of cell cc: summed, and stored after the last
-        auto sum_slot = [&](int m, int k, int cc, int deg) {
+        // epilogue: lane = rows g + 8 i (i < 4) of its warp's 32, 32 of the 128 columns
+        const int quad = warp & 3, col = ((warp - MF_PROD_WARPS - 1) >> 2) * 32, gq = lane >> 2, fq = lane & 3;
+        const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
+        const FragBias f1 = frag_bias(g.b1 + col, fq, true), f2 = frag_bias(g.b2 + col, fq, true);
+        float acc[32];  // [i][j][2]
+        int n = 0, pt = 0, pdeg[4];
+        // the messages of slot m (region k) of tile tt: summed, and stored after the last
+        auto sum_slot = [&](int m, int k, int tt, const int (&deg)[4]) {
             if (!warp_wait(d2f + 8 * k, (m / 3) & 1)) {
                 bad = true;
                 return;
             }
             tmem_fence_after();
-            const bool valid = k < deg;
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
-                uint32_t v[32];
-                tmem_ld32(tmem + lanes + (uint32_t)(k * 128 + half * 64 + hh * 32), v);
+                uint32_t v[16];
+                tmem_ld_frag32(lanes + ((uint32_t)(hh * 16) << 16) + (uint32_t)(k * 128 + col), v);
                 if (hh == 1) {
                     tmem_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(de + 8 * k);
                 }
 #pragma unroll
-                for (int u = 0; u < 32; u += 4) {
-                    const float4 b = *(const float4 *)(b2 + hh * 32 + u);
-                    const float x[4] = {__uint_as_float(v[u]) + b.x, __uint_as_float(v[u + 1]) + b.y,
-                                        __uint_as_float(v[u + 2]) + b.z, __uint_as_float(v[u + 3]) + b.w};
+                for (int r = 0; r < 2; ++r) {
+                    const int i = 2 * hh + r;
+                    const bool valid = k < deg[i];
 #pragma unroll
-                    for (int w = 0; w < 4; ++w) {
-                        const float a = k == 0 ? 0.0f : acc[hh * 32 + u + w];
-                        acc[hh * 32 + u + w] = valid ? a + x[w] : a;
+                    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                        for (int x = 0; x < 2; ++x) {
+                            const float msg = __uint_as_float(v[4 * j + 2 * r + x]) + (x ? f2.b[j].y : f2.b[j].x);
+                            const float a = k == 0 ? 0.0f : acc[8 * i + 2 * j + x];
+                            acc[8 * i + 2 * j + x] = valid ? a + msg : a;
+                        }
                     }
                 }
             }
-            if (k == 2 && cc < g.C) {
-                __nv_bfloat16 *p = g.agg + (int64_t)cc * MF_H + half * 64;
+            if (k == 2) {
 #pragma unroll
-                for (int u = 0; u < 64; u += 16) {
+                for (int hh = 0; hh < 2; ++hh) {
                     uint32_t w[8];
 #pragma unroll
-                    for (int x = 0; x < 8; ++x) w[x] = pack_bf16x2(acc[u + 2 * x], acc[u + 2 * x + 1]);
-                    st8u(p + u, w);
+                    for (int j = 0; j < 4; ++j)
+#pragma unroll
+                        for (int r = 0; r < 2; ++r)
+                            w[2 * j + r] = pack_bf16x2(acc[8 * (2 * hh + r) + 2 * j], acc[8 * (2 * hh + r) + 2 * j + 1]);
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        const int c = tt * MM_BM + quad * 32 + gq + 8 * (2 * hh + r);
+                        store_pairs(w, r, fq, g.agg + (int64_t)c * MF_H + col, c < g.C);
+                    }
                 }
+                __syncwarp();
             }
-            __syncwarp();
         };
         for (int t = blockIdx.x, i = 0; t < tiles && !bad; t += gridDim.x, ++i) {
-            const int c = t * MM_BM + quad * 32 + lane;
-            int rs = 0, deg = 0;
-            if (c < g.C) {
-                rs = g.start[c];
-                deg = g.start[c + 1] - rs;
+            int rs[4], deg[4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const int c = t * MM_BM + quad * 32 + gq + 8 * x;
+                rs[x] = deg[x] = 0;
+                if (c < g.C) {
+                    rs[x] = g.start[c];
+                    deg[x] = g.start[c + 1] - rs[x];
+                }
             }
 #pragma unroll
             for (int k = 0; k < 3; ++k, ++n) {
@@ -319,31 +368,36 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_edge_fwd(const __grid_constan
                     break;
                 }
                 tmem_fence_after();
-                const uint32_t z = tmem + lanes + 384u + 64u * (n & 1) + (uint32_t)(half * 32);
+                const uint32_t z = lanes + 384u + 64u * (n & 1) + (uint32_t)(col / 2);
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
-                    uint32_t v[32], w[16];
-                    tmem_ld32(tmem + lanes + (uint32_t)(k * 128 + half * 64 + hh * 32), v);
-                    relu_pack32(v, b1 + hh * 32, w);
-                    tmem_st16(z + (uint32_t)(hh * 16), w);
-                    if (g.z1 && k < deg) {
-                        __nv_bfloat16 *p = g.z1 + (int64_t)(rs + k) * MF_H + half * 64 + hh * 32;
-                        st8u(p, w);
-                        st8u(p + 16, w + 8);
+                    uint32_t v[16], w[8];
+                    const uint32_t half = (uint32_t)(hh * 16) << 16;
+                    tmem_ld_frag32(lanes + half + (uint32_t)(k * 128 + col), v);
+                    relu_pack_frag(v, f1, w);
+                    tmem_st_frag_pairs(z + half, w);
+                    if (g.z1) {
+#pragma unroll
+                        for (int r = 0; r < 2; ++r)
+                            store_pairs(w, r, fq, g.z1 + (int64_t)(rs[2 * hh + r] + k) * MF_H + col, k < deg[2 * hh + r]);
+                        __syncwarp();
                     }
-                    __syncwarp();
                 }
                 tmem_wait_st();
                 tmem_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(zf + 8 * (n & 1));
-                if (n > 0) sum_slot(n - 1, k == 0 ? 2 : k - 1, k == 0 ? pc : c, k == 0 ? pdeg : deg);
+                if (n > 0) {
+                    if (k == 0) sum_slot(n - 1, 2, pt, pdeg);
+                    else sum_slot(n - 1, k - 1, t, deg);
+                }
                 if (bad) break;
             }
-            pc = c;
-            pdeg = deg;
+            pt = t;
+#pragma unroll
+            for (int x = 0; x < 4; ++x) pdeg[x] = deg[x];
         }
-        if (n > 0 && !bad) sum_slot(n - 1, 2, pc, pdeg);
+        if (n > 0 && !bad) sum_slot(n - 1, 2, pt, pdeg);
     }
     if (bad) atomicCAS(g.error, 0, FL_E_TIMEOUT);
     tmem_fence_before();
@@ -356,8 +410,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_mlp2(const __grid_constant__ 
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const int nK = g.nk[0] + g.nk[1], S = g.ring;
     const uint32_t sW1 = smem_addr(smem), sW2 = sW1 + nK * MM_CHUNK_BYTES, sR = sW2 + 2 * MM_CHUNK_BYTES;
-    float *bias = (float *)(smem + MF_CHUNKS * MM_CHUNK_BYTES);
-    uint64_t *bars = (uint64_t *)(bias + 256);
+    uint64_t *bars = (uint64_t *)(smem + MF_CHUNKS * MM_CHUNK_BYTES);
     const uint32_t ringf = smem_addr(bars), ringe = ringf + 8 * M2_MAX_RING;
     const uint32_t d1f = ringe + 8 * M2_MAX_RING, zf = d1f + 24, d2f = zf + 16, de = d2f + 24, drain = de + 24;
     uint32_t *tmem_slot = (uint32_t *)(bars + 2 * M2_MAX_RING + 3 + 2 + 3 + 3 + 1);
@@ -386,7 +439,6 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_mlp2(const __grid_constant__ 
     }
     for (int c = 0; c < nK; ++c) load_weight_chunk(g.w1, g.ldw1, MF_H, c, sW1 + c * MM_CHUNK_BYTES, tid, MF_THREADS);
     for (int c = 0; c < 2; ++c) load_weight_chunk(g.w2, g.ldw2, g.n2, c, sW2 + c * MM_CHUNK_BYTES, tid, MF_THREADS);
-    if (tid < 256) bias[tid] = tid < 128 ? g.b1[tid] : (tid - 128 < g.n2 ? g.b2[tid - 128] : 0.0f);
     cp_async_commit();
     cp_async_wait_all();
     fence_async_smem();
@@ -399,21 +451,25 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_mlp2(const __grid_constant__ 
     pdl_launch_dependents();
 
     if (warp < MF_PROD_WARPS) {
-        int q = 0;
+        int s = 0, u = 0;
         for (int t = blockIdx.x; t < tiles && !bad; t += gridDim.x) {
-            const int r = t * MM_BM + 32 * warp + lane;
-            const __nv_bfloat16 *p0 = r < g.M ? g.a[0] + (int64_t)r * g.lda[0] : nullptr;
-            const __nv_bfloat16 *p1 = r < g.M && g.nk[1] ? g.a[1] + (int64_t)r * g.lda[1] : nullptr;
-            for (int c = 0; c < nK; ++c, ++q) {
-                const int s = q % S, u = q / S;
-                if (u > 0 && !warp_wait(ringe + 8 * s, (u - 1) & 1)) {
-                    bad = true;
-                    break;
+            const int r0 = t * MM_BM + 64 * warp + lane, r1 = r0 + 32;
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const __nv_bfloat16 *p0 = r0 < g.M ? g.a[x] + (int64_t)r0 * g.lda[x] : nullptr;
+                const __nv_bfloat16 *p1 = r1 < g.M ? g.a[x] + (int64_t)r1 * g.lda[x] : nullptr;
+                for (int c = 0; c < g.nk[x] && !bad; ++c) {
+                    if (u > 0 && !warp_wait(ringe + 8 * s, (u - 1) & 1)) {
+                        bad = true;
+                        break;
+                    }
+                    warp_copy_rows64(p0 ? p0 + c * 64 : nullptr, p1 ? p1 + c * 64 : nullptr, sR + s * MM_CHUNK_BYTES, warp, lane);
+                    cp_async_arrive_noinc(ringf + 8 * s);
+                    if (++s == S) {
+                        s = 0;
+                        ++u;
+                    }
                 }
-                const __nv_bfloat16 *p = c < g.nk[0] ? p0 : p1;
-                const int col = (c < g.nk[0] ? c : c - g.nk[0]) * 64;
-                warp_copy_rows(p ? p + col : nullptr, sR + s * MM_CHUNK_BYTES, warp, lane);
-                cp_async_arrive_noinc(ringf + 8 * s);
             }
         }
         cp_async_wait_all();
@@ -469,96 +525,100 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_mlp2(const __grid_constant__ 
             (void)warp_wait(drain, 0);
         }
     } else {
-        const int quad = warp & 3, half = (warp - MF_PROD_WARPS - 1) >> 2;
-        const uint32_t lanes = (uint32_t)(quad * 32) << 16;
-        const float *b1 = bias + half * 64, *b2 = bias + 128 + half * 64;
-        const bool has_out = half * 64 < g.n2;  // (n2 = 64: the upper columns do not exist)
-        int n = 0, pr = 0;
-        auto finish = [&](int m, int r) {
+        // epilogue: lane = rows g + 8 i (i < 4) of its warp's 32, 32 of the 128 columns
+        const int quad = warp & 3, col = ((warp - MF_PROD_WARPS - 1) >> 2) * 32, gq = lane >> 2, fq = lane & 3;
+        const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
+        const bool has_out = col < g.n2;  // (n2 = 64: the upper columns do not exist)
+        const FragBias f1 = frag_bias(g.b1 + col, fq, true), f2 = frag_bias(g.b2 + col, fq, has_out);
+        int n = 0, pt = 0;
+        auto finish = [&](int m, int tt) {
             const int k = m % 3;
-            float res[32];
-            const float *rp = g.residual && r < g.M ? g.residual + (int64_t)r * MF_H + half * 64 : nullptr;
+            // the residual's rows, eight consecutive columns a lane, on their way during the wait
+            float res[4][8];
+            const int64_t r0 = (int64_t)tt * MM_BM + quad * 32 + gq;
+            if (g.residual && has_out) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (r0 + 8 * i < g.M) ld8f(g.residual + (r0 + 8 * i) * MF_H + col + 8 * fq, res[i]);
+                __syncwarp();
+            }
+            if (!warp_wait(d2f + 8 * k, (m / 3) & 1)) {
+                bad = true;
+                return;
+            }
+            tmem_fence_after();
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
-                if (rp) {
-#pragma unroll
-                    for (int u = 0; u < 32; u += 8) ld8f(rp + hh * 32 + u, res + u);
-                }
-                if (hh == 0) {
-                    if (!warp_wait(d2f + 8 * k, (m / 3) & 1)) {
-                        bad = true;
-                        return;
-                    }
-                    tmem_fence_after();
-                }
-                uint32_t v[32];
-                tmem_ld32(tmem + lanes + (uint32_t)(k * 128 + half * 64 + hh * 32), v);
+                uint32_t v[16];
+                tmem_ld_frag32(lanes + ((uint32_t)(hh * 16) << 16) + (uint32_t)(k * 128 + col), v);
                 if (hh == 1) {
                     tmem_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(de + 8 * k);
                 }
-                if (has_out && r < g.M) {
-                    float x[32];
+                if (!has_out) continue;  // (uniform over the warp)
 #pragma unroll
-                    for (int u = 0; u < 32; u += 4) {
-                        const float4 b = *(const float4 *)(b2 + hh * 32 + u);
-                        x[u] = __uint_as_float(v[u]) + b.x;
-                        x[u + 1] = __uint_as_float(v[u + 1]) + b.y;
-                        x[u + 2] = __uint_as_float(v[u + 2]) + b.z;
-                        x[u + 3] = __uint_as_float(v[u + 3]) + b.w;
+                for (int r = 0; r < 2; ++r) {
+                    const int i = 2 * hh + r;
+                    uint32_t x[8];  // columns 8 fq .. + 7 of the row after the transposes
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        x[2 * j] = __float_as_uint(__uint_as_float(v[4 * j + 2 * r]) + f2.b[j].x);
+                        x[2 * j + 1] = __float_as_uint(__uint_as_float(v[4 * j + 2 * r + 1]) + f2.b[j].y);
                     }
-                    if (rp) {
+                    transpose4(x[0], x[2], x[4], x[6], fq);
+                    transpose4(x[1], x[3], x[5], x[7], fq);
+                    const int64_t row = r0 + 8 * i;
+                    if (row < g.M) {
+                        float y[8];
 #pragma unroll
-                        for (int u = 0; u < 32; ++u) x[u] += res[u];
-                    }
-                    const int64_t o = (int64_t)r * g.n2 + half * 64 + hh * 32;
-                    if (g.out_f32) {
+                        for (int u = 0; u < 8; ++u) y[u] = __uint_as_float(x[u]);
+                        if (g.residual) {
 #pragma unroll
-                        for (int u = 0; u < 32; u += 8) st8f(g.out_f32 + o + u, x + u);
-                    }
-                    if (g.out_bf16) {
-#pragma unroll
-                        for (int u = 0; u < 32; u += 16) {
-                            uint32_t w[8];
-#pragma unroll
-                            for (int y = 0; y < 8; ++y) w[y] = pack_bf16x2(x[u + 2 * y], x[u + 2 * y + 1]);
-                            st8u(g.out_bf16 + o + u, w);
+                            for (int u = 0; u < 8; ++u) y[u] += res[i][u];
                         }
+                        const int64_t o = row * g.n2 + col + 8 * fq;
+                        if (g.out_f32) st8f(g.out_f32 + o, y);
+                        if (g.out_bf16)
+                            *(uint4 *)(g.out_bf16 + o) = make_uint4(pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]),
+                                                                    pack_bf16x2(y[4], y[5]), pack_bf16x2(y[6], y[7]));
                     }
+                    __syncwarp();
                 }
-                __syncwarp();
             }
         };
         for (int t = blockIdx.x; t < tiles && !bad; t += gridDim.x, ++n) {
-            const int r = t * MM_BM + quad * 32 + lane, k = n % 3;
+            const int k = n % 3;
             if (!warp_wait(d1f + 8 * k, (n / 3) & 1)) {
                 bad = true;
                 break;
             }
             tmem_fence_after();
-            const uint32_t z = tmem + lanes + 384u + 64u * (n & 1) + (uint32_t)(half * 32);
+            const uint32_t z = lanes + 384u + 64u * (n & 1) + (uint32_t)(col / 2);
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
-                uint32_t v[32], w[16];
-                tmem_ld32(tmem + lanes + (uint32_t)(k * 128 + half * 64 + hh * 32), v);
-                relu_pack32(v, b1 + hh * 32, w);
-                tmem_st16(z + (uint32_t)(hh * 16), w);
-                if (g.z1 && r < g.M) {
-                    __nv_bfloat16 *p = g.z1 + (int64_t)r * MF_H + half * 64 + hh * 32;
-                    st8u(p, w);
-                    st8u(p + 16, w + 8);
+                uint32_t v[16], w[8];
+                const uint32_t half = (uint32_t)(hh * 16) << 16;
+                tmem_ld_frag32(lanes + half + (uint32_t)(k * 128 + col), v);
+                relu_pack_frag(v, f1, w);
+                tmem_st_frag_pairs(z + half, w);
+                if (g.z1) {
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        const int64_t row = (int64_t)t * MM_BM + quad * 32 + gq + 8 * (2 * hh + r);
+                        store_pairs(w, r, fq, g.z1 + row * MF_H + col, row < g.M);
+                    }
+                    __syncwarp();
                 }
-                __syncwarp();
             }
             tmem_wait_st();
             tmem_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(zf + 8 * (n & 1));
-            if (n > 0) finish(n - 1, pr);
-            pr = r;
+            if (n > 0) finish(n - 1, pt);
+            pt = t;
         }
-        if (n > 0 && !bad) finish(n - 1, pr);
+        if (n > 0 && !bad) finish(n - 1, pt);
     }
     if (bad) atomicCAS(g.error, 0, FL_E_TIMEOUT);
     tmem_fence_before();

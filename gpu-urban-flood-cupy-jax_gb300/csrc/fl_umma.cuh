@@ -135,6 +135,49 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// The mma-fragment shapes: 16 lanes (rows) from taddr's, 32 columns.  Lane
+// l = 4 g + q of the warp holds rows g and g + 8; of each 8-column block j the
+// columns 8 j + 2 q and + 1: r[4 j + 0, 1] of row g, r[4 j + 2, 3] of row g + 8.
+__device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// The same columns as packed pairs (16 words a row): r[2 j] of row g, r[2 j + 1] of row g + 8.
+__device__ __forceinline__ void tmem_st_frag_pairs(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]),
+                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+
+// 4 x 4 transpose over the lanes q = 0..3 of a group of four: afterwards word p
+// of lane q is what word q of lane p was.
+__device__ __forceinline__ void transpose4(uint32_t &w0, uint32_t &w1, uint32_t &w2, uint32_t &w3, int q) {
+    const bool o1 = (q & 1) != 0, o2 = (q & 2) != 0;
+    uint32_t a = __shfl_xor_sync(0xffffffffu, o1 ? w0 : w1, 1), b = __shfl_xor_sync(0xffffffffu, o1 ? w2 : w3, 1);
+    if (o1) {
+        w0 = a;
+        w2 = b;
+    } else {
+        w1 = a;
+        w3 = b;
+    }
+    a = __shfl_xor_sync(0xffffffffu, o2 ? w0 : w2, 2);
+    b = __shfl_xor_sync(0xffffffffu, o2 ? w1 : w3, 2);
+    if (o2) {
+        w0 = a;
+        w1 = b;
+    } else {
+        w2 = a;
+        w3 = b;
+    }
+}
+
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -157,6 +200,21 @@ __device__ __forceinline__ void warp_copy_rows(const __nv_bfloat16 *own, uint32_
         const int rr = 4 * i + (lane >> 3);
         const uint64_t row = __shfl_sync(0xffffffffu, p, rr);
         const int R = 32 * pw + rr;
+        if (row) cp_async16(sdst + (uint32_t)(R * 128 + ((c ^ (R & 7)) << 4)), (const __nv_bfloat16 *)row + c * 8);
+    }
+}
+
+// A producer warp's 64 rows of a 128-row chunk; own0 / own1: this lane's rows
+// (lane, lane + 32), nullptr: left as it is.
+__device__ __forceinline__ void warp_copy_rows64(const __nv_bfloat16 *own0, const __nv_bfloat16 *own1, uint32_t sdst, int pw,
+                                                 int lane) {
+    const int c = lane & 7;
+    const uint64_t p0 = (uint64_t)own0, p1 = (uint64_t)own1;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const int rr = 4 * i + (lane >> 3);
+        const uint64_t row = __shfl_sync(0xffffffffu, i < 8 ? p0 : p1, rr & 31);
+        const int R = 64 * pw + rr;
         if (row) cp_async16(sdst + (uint32_t)(R * 128 + ((c ^ (R & 7)) << 4)), (const __nv_bfloat16 *)row + c * 8);
     }
 }

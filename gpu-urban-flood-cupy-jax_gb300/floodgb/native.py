@@ -163,7 +163,9 @@ class FlMpnnBackwardDesc(C.Structure):
         ("h_bf", C.POINTER(C.c_void_p)), ("agg", C.POINTER(C.c_void_p)), ("z1e", C.POINTER(C.c_void_p)),
         ("z1n", C.POINTER(C.c_void_p)), ("dy", C.c_void_p), ("ldy", C.c_int64), ("dh", C.c_void_p * 2),
         ("dz2c", C.c_void_p), ("dz1c", C.c_void_p), ("dagg", C.c_void_p), ("dyb", C.c_void_p),
-        ("dze", C.POINTER(C.c_void_p)), ("dz2e", C.c_void_p), ("scratch", C.c_void_p), ("scratch_floats", C.c_int64),
+        ("dze", C.POINTER(C.c_void_p)), ("dz2e", C.c_void_p),
+        ("dz1f", C.c_void_p), ("gf", C.c_void_p), ("ef32", C.c_void_p), ("daggf", C.POINTER(C.c_void_p)),
+        ("scratch", C.c_void_p), ("scratch_floats", C.c_int64),
     ]
 
 
@@ -206,7 +208,7 @@ _SIGNATURES = {
     "fl_launch_count": (C.c_int64, []),
     "fl_gemm_bf16": (C.c_int, [C.POINTER(FlGemmDesc), C.c_void_p]),
     "fl_mpnn_forward": (C.c_int, [C.POINTER(FlMpnnForwardDesc), C.c_void_p]),
-    "fl_mpnn_backward_scratch": (C.c_int, [C.POINTER(C.c_int64)]),
+    "fl_mpnn_backward_scratch": (C.c_int, [C.c_int32, C.c_int32, C.c_int32, C.POINTER(C.c_int64)]),
     "fl_mpnn_backward": (C.c_int, [C.POINTER(FlMpnnBackwardDesc), C.c_void_p]),
     "fl_adam_all": (C.c_int, [C.POINTER(FlAdamTensor), C.c_int32, C.c_float, C.c_float, C.c_float, C.c_float, C.c_int32,
                               C.c_float, C.c_void_p]),

@@ -471,10 +471,13 @@ FL_API int fl_mpnn_forward(const FlMpnnForwardDesc *desc, void *stream);
  * h_bf: layers + 1 different buffers).  At most three outgoing edges per cell
  * too (send_order: edges by sending cell, send_start its CSR), at most 32
  * layers.  wt: bf16 transposed weights [n_in, ldwt].  Buffers: dh two fp32
- * [cells, 128]; dz2c, dz1c, dagg bf16 [cells, 128]; dyb bf16 [cells, 64];
- * dze: layers x bf16 [edges, 128]; dz2e bf16 [edges, 128]; scratch of
- * fl_mpnn_backward_scratch floats.  Gradients equal those of one launch per
- * product up to the order of the fp32 sums over rows. */
+ * [cells, 128]; dz2c, dz1c, dagg bf16, dz1f, gf fp32 [cells, 128]; dyb bf16
+ * [cells, 64]; dze: layers x bf16 [edges, 128]; dz2e bf16, ef32 fp32 [edges,
+ * 128]; scratch of fl_mpnn_backward_scratch floats.  daggf: layers x fp32
+ * [cells, 128], the gradients of the summed messages: the gradient of a message
+ * MLP's second bias (edge[2 l + 1].gb, left to the caller) is their sum over
+ * cells, each times the cell's incoming edges.  The other gradients are those
+ * of one launch per product, bit for bit. */
 typedef struct {
     const void *wt;
     int64_t ldwt;
@@ -496,11 +499,13 @@ typedef struct {
     void *dz2c, *dz1c, *dagg, *dyb;
     void *const *dze;
     void *dz2e;
+    float *dz1f, *gf, *ef32;
+    float *const *daggf;
     float *scratch;
     int64_t scratch_floats;
 } FlMpnnBackwardDesc;
 
-FL_API int fl_mpnn_backward_scratch(int64_t *floats);
+FL_API int fl_mpnn_backward_scratch(int32_t cells, int32_t edges, int32_t layers, int64_t *floats);
 FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *desc, void *stream);
 
 /* fl_adam over n tensors of a network in one launch (same arithmetic). */
