@@ -63,7 +63,8 @@ struct MlpBwdArgs {
     __nv_bfloat16 *dze;            // [E, 128] (layer)
     // the fp32 values that the bias gradients sum, [M, 128] each
     float *dz1f;                   // masked dz1
-    float *daggf, *gf;             // message gradient; dagg W_e2 before the masks (layer)
+    float *daggf, *gf;             // message gradient x incoming edges; dagg W_e2 before the masks (layer)
+    uint32_t *bits;                // [E, 4] which of an edge's 128 hidden activations are positive (layer)
     int32_t n2, M;
     int32_t *error;
 };
@@ -277,8 +278,11 @@ __global__ void __launch_bounds__(MB_THREADS, 1) k_mlp_bwd(const __grid_constant
                         const int64_t at = (int64_t)r * MF_H + col + hh * 32;
                         st8u(g.dagg + at, w);
                         st8u(g.dagg + at + 16, w + 8);
+                        float x[32];
 #pragma unroll
-                        for (int u = 0; u < 32; u += 8) st8u(g.daggf + at + u, v + u);
+                        for (int u = 0; u < 32; ++u) x[u] = __uint_as_float(v[u]) * (float)deg;
+#pragma unroll
+                        for (int u = 0; u < 32; u += 8) st8f(g.daggf + at + u, x + u);
                     }
                     __syncwarp();
                     tmem_st16(lanes + 448u + (uint32_t)(half * 32 + hh * 16), w);
@@ -343,8 +347,14 @@ __global__ void __launch_bounds__(MB_THREADS, 1) k_mlp_bwd(const __grid_constant
                     for (int k = 0; k < 3; ++k) {
                         if (k < deg) {
                             const int64_t at = (int64_t)(rs + k) * MF_H + col + hh * 32;
+                            uint32_t bits = 0u;
 #pragma unroll
-                            for (int u = 0; u < 16; ++u) m[k][u] = positive_mask(m[k][u]) & w[u];
+                            for (int u = 0; u < 16; ++u) {
+                                const uint32_t p = positive_mask(m[k][u]);
+                                bits |= (p & 1u) << (2 * u) | (p >> 31) << (2 * u + 1);
+                                m[k][u] = p & w[u];
+                            }
+                            g.bits[(int64_t)(rs + k) * 4 + (col + hh * 32) / 32] = bits;
                             st8u(g.dze + at, m[k]);
                             st8u(g.dze + at + 16, m[k] + 8);
                         }
@@ -956,8 +966,11 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad(const __grid_constant__
         if (issuer) umma_commit(drain);
         (void)warp_wait(drain, 0);
     } else {
-        // epilogue: thread = one output row
-        const int quad = warp & 3, r = quad * 32 + lane;
+        // epilogue: a warp's 32 output rows, 32 columns at a time in the fragment
+        // shape; after the transposes a row's 32 columns are one 128-byte line
+        // (a row a lane wrote 32-byte pieces, and the next split's accumulator
+        // waited for them)
+        const int quad = warp & 3, gq = lane >> 2, fq = lane & 3;
         const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
         uint32_t par = 0u;
         int turn = 0;
@@ -972,20 +985,32 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad(const __grid_constant__
             }
             par ^= 1u << b;
             tmem_fence_after();
-            float *out = J.part + ((int64_t)sp * rows + r) * n_in;
+            float *out = J.part + (int64_t)sp * rows * n_in + 8 * fq;
             for (int cb = 0; cb < n_in; cb += 32) {
-                uint32_t v[32];
-                tmem_ld32(lanes + 256u * b + (uint32_t)cb, v);
-                if (cb + 32 >= n_in) {
-                    tmem_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(acce + 8 * b);
-                }
-                if (r < rows) {
 #pragma unroll
-                    for (int u = 0; u < 32; u += 8) st8u(out + cb + u, v + u);
+                for (int hh = 0; hh < 2; ++hh) {
+                    uint32_t v[16];
+                    tmem_ld_frag32(lanes + ((uint32_t)(hh * 16) << 16) + 256u * b + (uint32_t)cb, v);
+                    if (hh == 1 && cb + 32 >= n_in) {
+                        tmem_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(acce + 8 * b);
+                    }
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        uint32_t x[8];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            x[2 * j] = v[4 * j + 2 * r];
+                            x[2 * j + 1] = v[4 * j + 2 * r + 1];
+                        }
+                        transpose4(x[0], x[2], x[4], x[6], fq);
+                        transpose4(x[1], x[3], x[5], x[7], fq);
+                        const int row = quad * 32 + gq + 8 * (2 * hh + r);
+                        if (row < rows) st8u(out + (int64_t)row * n_in + cb, x);
+                        __syncwarp();
+                    }
                 }
-                __syncwarp();
             }
         }
     }
@@ -1005,10 +1030,11 @@ struct RdJob {
 };
 
 // Column sums of x over M rows by row class (r mod 256): part[class][n].  With
-// z: row r counts x[map[r]] where z[r] > 0 (a cell's message gradient over its edges).
+// bits: row r counts x[map[r]] in the columns whose bit is set (a cell's
+// message gradient over its edges).
 struct CsJob {
     const float *x;
-    const __nv_bfloat16 *z;  // [M, 128] or nullptr
+    const uint32_t *bits;    // [M, 4] or nullptr
     const int32_t *map;
     float *part;             // [256, n]
     int64_t ld;
@@ -1036,10 +1062,11 @@ __device__ __forceinline__ void add4(float4 &s, const float4 v) {
 }
 
 // Partial weight gradients: part[p] and part[p + 256], then over p in order.
-// Column sums for the bias gradients: a warp per row class walks its rows in
-// order, 16 rows' loads in flight (the order of a sum is kept, so many classes
-// of rows, not many adders, are what hides the latency).  Both in one launch:
-// either alone leaves the device half idle.
+// Column sums for the bias gradients: a thread per row class and column walks
+// its rows in order (a sum's order is kept, so loads in flight, not adders,
+// hide the latency: 16 rows by four columns a thread took 300 us a layer on
+// 299,712 rows, 32 rows by one 80).  Both in one launch: either alone leaves
+// the device half idle.
 __global__ void __launch_bounds__(256) k_reduce(const __grid_constant__ RdArgs g) {
     pdl_wait();
     pdl_launch_dependents();
@@ -1071,57 +1098,56 @@ __global__ void __launch_bounds__(256) k_reduce(const __grid_constant__ RdArgs g
         *o = v;
         return;
     }
+    // a thread per (row class, column): 32 columns a warp, 32 rows' loads in flight
     const CsJob &J = g.cs[blockIdx.y - g.jobs];
-    const int cls = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const int c = lane * 4, M = J.M;
-    if (cls >= RD_STRIDE) return;
-    const bool in = c < J.n;
+    const int id = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int cls = id >> 2, c = (id & 3) * 32 + lane, M = J.M;
+    if (cls >= RD_STRIDE || (id & 3) * 32 >= J.n) return;  // (uniform over the warp)
     const float *x = J.x + c;
     const int64_t ld = J.ld;
-    float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (!J.z) {
-        for (int r = cls; r < M; r += 16 * RD_STRIDE) {
-            float4 v[16];
+    float s = 0.0f;
+    if (!J.bits) {
+        for (int r = cls; r < M; r += 32 * RD_STRIDE) {
+            float v[32];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (in && r + u * RD_STRIDE < M) v[u] = *(const float4 *)(x + (int64_t)(r + u * RD_STRIDE) * ld);
+            for (int u = 0; u < 32; ++u) {
+                v[u] = 0.0f;
+                if (r + u * RD_STRIDE < M) v[u] = x[(int64_t)(r + u * RD_STRIDE) * ld];
             }
 #pragma unroll
-            for (int u = 0; u < 16; ++u)
-                if (r + u * RD_STRIDE < M) add4(s, v[u]);
+            for (int u = 0; u < 32; ++u) s += v[u];
         }
     } else {
-        const __nv_bfloat16 *z = J.z + c;
-        for (int r0 = cls; r0 < M; r0 += 32 * RD_STRIDE) {
-            const int mine = r0 + lane * RD_STRIDE, at = mine < M ? J.map[mine] : 0;  // 32 rows' map entries at once
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                float4 v[16];
-                uint2 m[16];
-#pragma unroll
-                for (int u = 0; u < 16; ++u) {
-                    const int r = r0 + (16 * h + u) * RD_STRIDE, row = __shfl_sync(0xffffffffu, at, 16 * h + u);
-                    v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    m[u] = make_uint2(0u, 0u);
-                    if (r < M) {
-                        v[u] = *(const float4 *)(x + (int64_t)row * ld);
-                        m[u] = *(const uint2 *)(z + (int64_t)r * MF_H);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 16; ++u) {
-                    if (r0 + (16 * h + u) * RD_STRIDE >= M) break;
-                    const uint32_t a = positive_mask(m[u].x), b = positive_mask(m[u].y);
-                    s.x += (a & 0xffffu) ? v[u].x : 0.0f;
-                    s.y += (a >> 16) ? v[u].y : 0.0f;
-                    s.z += (b & 0xffffu) ? v[u].z : 0.0f;
-                    s.w += (b >> 16) ? v[u].w : 0.0f;
-                }
+        const uint32_t *bits = J.bits + (id & 3);
+        const int32_t *map = J.map;
+        // the map entries and bits of 32 rows at once, a row a lane
+        auto load = [&](int r, int &row, uint32_t &m) {
+            row = 0;
+            m = 0u;
+            if (r < M) {
+                row = map[r];
+                m = bits[(int64_t)r * 4];
             }
+        };
+        int at;
+        uint32_t mask;
+        load(cls + lane * RD_STRIDE, at, mask);
+        for (int r = cls; r < M; r += 32 * RD_STRIDE) {
+            int next;
+            uint32_t next_mask;
+            load(r + (32 + lane) * RD_STRIDE, next, next_mask);
+            // (rows past the end read row 0 and have no bits: branches around
+            // the loads made them wait for one another)
+            float v[32];
+#pragma unroll
+            for (int u = 0; u < 32; ++u) v[u] = x[(int64_t)__shfl_sync(0xffffffffu, at, u) * ld];
+#pragma unroll
+            for (int u = 0; u < 32; ++u) s += __shfl_sync(0xffffffffu, mask, u) >> lane & 1u ? v[u] : 0.0f;
+            at = next;
+            mask = next_mask;
         }
     }
-    if (in) *(float4 *)(J.part + (int64_t)cls * J.n + c) = s;
+    J.part[(int64_t)cls * J.n + c] = s;
 }
 
 // Bias gradients: the 256 class sums in order, added.
@@ -1186,7 +1212,7 @@ FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *d, void *stream) {
     if (!d->x || !d->dy || !d->recv_start || !d->zn || !d->zd || !d->h_bf || !d->dh[0] || !d->dh[1] || !d->dz2c || !d->dz1c ||
         !d->dyb || !d->dz1f || !d->scratch ||
         (L > 0 && (!d->edge || !d->node || !d->agg || !d->z1n || !d->z1e || !d->dze || !d->dagg || !d->daggf || !d->gf || !d->send_start)) ||
-        (E > 0 && (!d->src || !d->dst || !d->send_order || !d->ef || !d->ze || !d->e || !d->dz2e || !d->ef32)))
+        (E > 0 && (!d->src || !d->dst || !d->send_order || !d->ef || !d->ze || !d->e || !d->dz2e || !d->ef32 || !d->bits)))
         return set_error(FL_E_INVALID, "fl_mpnn_backward: NULL pointer");
     if (d->ldx < 64 || d->ldx % 8 || d->lde < 64 || d->lde % 8 || d->ldy < 64 || d->ldy % 8)
         return set_error(FL_E_INVALID, "fl_mpnn_backward: leading dimensions must be multiples of 8 and at least 64");
@@ -1243,12 +1269,13 @@ FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *d, void *stream) {
     RdArgs rd;
     BfArgs bf_args;
     int n_rd = 0, n_cs = 0, n_bf = 0, rd_blocks = 0;
-    auto sums = [&](const float *x, int64_t ld, int M, int n, float *gb, const void *z = nullptr, const int32_t *map = nullptr) {
+    auto sums = [&](const float *x, int64_t ld, int M, int n, float *gb, const uint32_t *bits = nullptr,
+                    const int32_t *map = nullptr) {
         if (M < 1) return;
-        rd.cs[n_cs++] = CsJob{x, (const bf *)z, map, classes, ld, M, n};
+        rd.cs[n_cs++] = CsJob{x, bits, map, classes, ld, M, n};
         bf_args.job[n_bf++] = BfJob{classes, gb, n};
         classes += RD_STRIDE * MF_H;
-        rd_blocks = std::max(rd_blocks, RD_STRIDE / 8);
+        rd_blocks = std::max(rd_blocks, RD_STRIDE * 4 / 8);
     };
     auto reduce = [&]() {
         if (e != cudaSuccess) return;
@@ -1384,6 +1411,7 @@ FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *d, void *stream) {
         a.dz1f = d->dz1f;
         a.daggf = d->daggf[l];
         a.gf = d->gf;
+        a.bits = (uint32_t *)d->bits;
         a.n2 = MF_H;
         a.M = C;
         mlp(k_mlp_bwd<2>, a, c_tiles);
@@ -1403,7 +1431,7 @@ FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *d, void *stream) {
         }
         sums(d->dh[cur], MF_H, C, MF_H, n2.gb);
         sums(d->dz1f, MF_H, C, MF_H, n1.gb);
-        sums(d->gf, MF_H, E, MF_H, e1.gb, d->z1e[l], d->dst);
+        sums(d->gf, MF_H, E, MF_H, e1.gb, (const uint32_t *)d->bits, d->dst);
         product(E, seg(d->dze[l], nullptr, MF_H, MF_H),
                 {seg(d->h_bf[l], d->dst, MF_H, MF_H), seg(d->h_bf[l], d->src, MF_H, MF_H), seg(d->e, nullptr, MF_H, MF_H)}, e1.gw);
         product(E, seg(d->dagg, d->dst, MF_H, MF_H), {seg(d->z1e[l], nullptr, MF_H, MF_H)}, e2.gw);

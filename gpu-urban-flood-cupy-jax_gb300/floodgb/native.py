@@ -164,7 +164,7 @@ class FlMpnnBackwardDesc(C.Structure):
         ("z1n", C.POINTER(C.c_void_p)), ("dy", C.c_void_p), ("ldy", C.c_int64), ("dh", C.c_void_p * 2),
         ("dz2c", C.c_void_p), ("dz1c", C.c_void_p), ("dagg", C.c_void_p), ("dyb", C.c_void_p),
         ("dze", C.POINTER(C.c_void_p)), ("dz2e", C.c_void_p),
-        ("dz1f", C.c_void_p), ("gf", C.c_void_p), ("ef32", C.c_void_p), ("daggf", C.POINTER(C.c_void_p)),
+        ("dz1f", C.c_void_p), ("gf", C.c_void_p), ("ef32", C.c_void_p), ("bits", C.c_void_p), ("daggf", C.POINTER(C.c_void_p)),
         ("scratch", C.c_void_p), ("scratch_floats", C.c_int64),
     ]
 

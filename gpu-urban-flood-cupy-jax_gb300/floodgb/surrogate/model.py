@@ -211,6 +211,7 @@ class Workspace:
             self.dz2_c, self.dz1_c, self.dz2_e = self._bf(self.C, H), self._bf(self.C, H), self._bf(self.E, H)
             self.dy_f32 = self._f32(self.C, FOUT)
             self.dz1_f32, self.g_f32, self.e_f32 = self._f32(self.C, H), self._f32(self.C, H), self._f32(self.E, H)
+            self.bits = self._f32(self.E, 4)  # (32-bit words)
             self.dagg_f32 = [self._f32(self.C, H) for _ in range(self.n_layers)]
             self.scratch = self._f32(ops.backward_scratch(self.C, self.E, self.n_layers))
             self.dze = [self._bf(self.E, H) for _ in range(self.n_layers)]
@@ -353,7 +354,7 @@ class MPNN:
         if max(getattr(g, "max_in", MAX_IN + 1), getattr(g, "max_out", MAX_IN + 1)) <= MAX_IN and L <= MAX_LAYERS:
             ops.mpnn_backward(self, g, x_bf, dy, ws.fused())
             for (_, e2), dagg in zip(self.edge, ws.dagg_f32):
-                e2.gb.add_((dagg * g.indeg[:, None]).sum(0))
+                e2.gb.add_(dagg.sum(0))
             return
         ws.products()
         # decoder

@@ -151,6 +151,7 @@ def mpnn_backward(net, g, x, dy, ws):
     d.dh[0], d.dh[1] = ws.dh[0].data_ptr(), ws.dh[1].data_ptr()
     d.dz2c, d.dz1c, d.dagg, d.dyb = _ptr(ws.dz2_c), _ptr(ws.dz1_c), _ptr(ws.dagg_bf), _ptr(ws.dy_bf)
     d.dz2e, d.dz1f, d.gf, d.ef32 = _ptr(ws.dz2_e), _ptr(ws.dz1_f32), _ptr(ws.g_f32), _ptr(ws.e_f32)
+    d.bits = _ptr(ws.bits)
     d.daggf = _pointers(ws.dagg_f32, L)
     d.scratch, d.scratch_floats = _ptr(ws.scratch), ws.scratch.numel()
     N.check(N.load().fl_mpnn_backward(C.byref(d), _stream()), "fl_mpnn_backward")

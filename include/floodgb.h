@@ -473,11 +473,11 @@ FL_API int fl_mpnn_forward(const FlMpnnForwardDesc *desc, void *stream);
  * layers.  wt: bf16 transposed weights [n_in, ldwt].  Buffers: dh two fp32
  * [cells, 128]; dz2c, dz1c, dagg bf16, dz1f, gf fp32 [cells, 128]; dyb bf16
  * [cells, 64]; dze: layers x bf16 [edges, 128]; dz2e bf16, ef32 fp32 [edges,
- * 128]; scratch of fl_mpnn_backward_scratch floats.  daggf: layers x fp32
- * [cells, 128], the gradients of the summed messages: the gradient of a message
- * MLP's second bias (edge[2 l + 1].gb, left to the caller) is their sum over
- * cells, each times the cell's incoming edges.  The other gradients are those
- * of one launch per product, bit for bit. */
+ * 128], bits 4 words per edge; scratch of fl_mpnn_backward_scratch floats.
+ * daggf: layers x fp32 [cells, 128], the gradients of the summed messages, each
+ * times its cell's incoming edges: the gradient of a message MLP's second bias
+ * (edge[2 l + 1].gb) is their sum over the cells and left to the caller.  The
+ * other gradients are those of one launch per product, bit for bit. */
 typedef struct {
     const void *wt;
     int64_t ldwt;
@@ -500,6 +500,7 @@ typedef struct {
     void *const *dze;
     void *dz2e;
     float *dz1f, *gf, *ef32;
+    void *bits;
     float *const *daggf;
     float *scratch;
     int64_t scratch_floats;
