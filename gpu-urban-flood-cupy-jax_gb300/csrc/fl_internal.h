@@ -226,6 +226,30 @@ struct LiArgs {
     float infil_scalar, g, md, vmax;
 };
 
+// The local-inertial step over surface tiles (one launch).  A tile's local
+// indices: its own cells 0 .. TILE - 1, then the cells across its active
+// interior edges (ring 1), then those across ring 1's other such edges (ring 2).
+// An entry is an active interior edge of an own or ring-1 cell, or a routable
+// boundary edge of an own cell; no other edge carries a discharge.
+constexpr int LT_LEFT_SHIFT = 0, LT_RIGHT_SHIFT = 10;   // local indices
+constexpr int LT_SLOTL_SHIFT = 20, LT_SLOTR_SHIFT = 22; // the edge's slot in each cell
+constexpr uint32_t LT_IDX_MASK = 1023u, LT_AI = 1u << 24;
+constexpr uint32_t LT_LKEEP = 1u << 25, LT_RKEEP = 1u << 26;  // the cell is own or ring 1
+
+struct LiTileArgs {
+    LiArgs c;                     // the shared fields (states, fields, control, outputs, settings)
+    const int4 *tile;             // [2 x tiles] {first entry, entries, first halo cell, halo cells}, {ring-1 cells, first area, -, -}
+    const float4 *ent;            // {nx, ny, length, bits}; a tile's count is even
+    const float2 *dm;             // {face distance, face Manning n}
+    const int32_t *halo_src;      // ring 1 then ring 2 cells (padded to 4 per tile)
+    const float *harea;           // ring 1 cells' areas (padded to 4 per tile)
+    const float *char_len;        // [whole tiles]
+    int32_t n_tiles, e_cap, h_cap, r1_cap;
+    int32_t off_scale, off_bar, off_stage, stage_bytes;
+    int32_t so_ci, so_hz, so_wt, so_cl, so_en, so_dm, so_hs, so_ha;
+    int32_t early;                // the dependent kernel may start beside this grid
+};
+
 struct DtArgs {
     const float4 *state0, *state1;
     const float *char_len;

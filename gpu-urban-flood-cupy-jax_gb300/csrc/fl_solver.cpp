@@ -68,6 +68,9 @@ cudaError_t launch_inflow(const InflowArgs &a, int slot, cudaStream_t stream);
 cudaError_t launch_surcharge(const SurchargeArgs &a, int slot, cudaStream_t stream);
 cudaError_t launch_li(const LiArgs &a, int kind, int slot, int plan_next, int sms, cudaStream_t stream);
 int li_cell_blocks(int32_t C);
+cudaError_t plan_li_tiles(LiTileArgs &a, int kind, int device, int *grid, int *smem_bytes);
+cudaError_t launch_li_tiles(const LiTileArgs &a, int kind, int slot, int plan_next, int grid, int smem_bytes,
+                            cudaStream_t stream);
 int node_blocks(int32_t N);
 int network_blocks(int32_t G);
 cudaError_t launch_f64_to_ff_perm(const double *src, float2 *dst, const int32_t *perm, int32_t n, cudaStream_t stream);
@@ -137,6 +140,9 @@ struct FlSolver {
     InflowArgs ext{};
     LiArgs li{};
     bool li_mode = false;     // surface_step_mode = local_inertial
+    LiTileArgs lt{};          // its tiles (lt_grid 0: the two launches over edges and cells)
+    int lt_grid = 0, lt_smem = 0;
+    int surface_launches() const { return li_mode && !lt_grid ? 2 : 1; }
     int sms = 1;
     SurchargeArgs sur{};
     RechargeArgs rch{};
@@ -146,7 +152,7 @@ struct FlSolver {
     bool has_table() const { return sur.U > 0; }
     bool has_recharge() const { return rch.U > 0; }
     int launches_per_step() const {
-        return (li_mode ? 2 : 1) + (has_drain() ? 4 : 0) + (has_table() ? 1 : 0) + (has_inflow() ? 1 : 0) +
+        return surface_launches() + (has_drain() ? 4 : 0) + (has_table() ? 1 : 0) + (has_inflow() ? 1 : 0) +
                (has_recharge() ? 1 : 0);
     }
 
@@ -265,6 +271,13 @@ static int launch_drainage(FlSolver *s, int slot, cudaStream_t st) {
     return FL_OK;
 }
 
+// The local-inertial surface step.
+static cudaError_t launch_inertial(FlSolver *s, int slot, int plan_next, cudaStream_t st) {
+    if (!s->lt_grid) return launch_li(s->li, s->kind, slot, plan_next, s->sms, st);
+    s->lt.c = s->li;  // (the fields that a caller may change between steps)
+    return launch_li_tiles(s->lt, s->kind, slot, plan_next, s->lt_grid, s->lt_smem, st);
+}
+
 static int launch_step(FlSolver *s, int slot, bool eval, bool plan_next, cudaStream_t st) {
     if (eval) {
         for (int m = 0; m < s->members; ++m) FL_CUDA(launch_dt(dt_args(s, m), s->dt_blocks, slot, 1, st));
@@ -275,8 +288,8 @@ static int launch_step(FlSolver *s, int slot, bool eval, bool plan_next, cudaStr
         g_launches++;
     }
     if (s->li_mode) {
-        FL_CUDA(launch_li(s->li, s->kind, slot, plan_next ? 1 : 0, s->sms, st));
-        g_launches += 2;
+        FL_CUDA(launch_inertial(s, slot, plan_next ? 1 : 0, st));
+        g_launches += s->surface_launches();
     } else {
         // (several members: s->sa addresses member 0 and one launch runs all)
         FL_CUDA(launch_surface(s->sa, s->kind, slot, plan_next ? 1 : 0, s->surf_grid, s->surf_smem, st));
@@ -466,6 +479,127 @@ FL_API void fl_destroy(FlSolver *s) {
     if (run_h) cudaFreeHost(run_h);
     if (s->poll_h) cudaFreeHost(s->poll_h);
     delete s;
+}
+
+// Tiles of the one-launch local-inertial step: entries, rings and areas per
+// tile of 256 cells (s->lt; s->lt_grid stays 0 where they do not fit).  lr, geo
+// (with the slots), edm: the edges in the order enew[reference edge].
+static int build_li_tiles(FlSolver *s, const HostLayout &L, const std::vector<int32_t> &enew, const std::vector<int2> &lr,
+                          const std::vector<float4> &geo, const std::vector<float2> &edm) {
+    const int32_t C = L.C, tiles = L.Cp / TILE;
+    std::vector<int4> info(2 * (size_t)tiles);
+    std::vector<float4> ent;
+    std::vector<float2> dm;
+    std::vector<int32_t> halo, local(C, -1), edge_tile(lr.size(), -1);
+    std::vector<float> harea;
+    LiTileArgs &a = s->lt;
+    a.e_cap = a.h_cap = a.r1_cap = 0;
+    auto bits_of = [&](int32_t k) {
+        uint32_t f;
+        memcpy(&f, &geo[k].w, 4);
+        return f;
+    };
+    std::vector<int32_t> ring;  // ring 1, then ring 2
+    for (int32_t t = 0; t < tiles; ++t) {
+        const int32_t c0 = t * TILE, c1 = std::min(C, c0 + TILE), ent0 = (int32_t)ent.size();
+        ring.clear();
+        for (int32_t c = c0; c < c1; ++c) local[c] = c - c0;
+        auto index_of = [&](int32_t c) {
+            if (local[c] < 0) {
+                local[c] = TILE + (int32_t)ring.size();
+                ring.push_back(c);
+            }
+            return local[c];
+        };
+        // the discharge-carrying edges of the cells [from, to) of a list, each edge once a tile
+        auto add_edges = [&](int32_t c) {
+            const int32_t cref = L.perm[c];
+            for (int j = 0; j < 3; ++j) {
+                const int32_t eo = L.inc[(size_t)cref * 3 + j];
+                if (eo < 0) continue;
+                const int32_t k = enew[eo];
+                const uint32_t f = bits_of(k);
+                const bool ai = (f & LI_AI) != 0, own = c >= c0 && c < c1;
+                if (edge_tile[k] == t || !(ai || ((f & LI_BEDGE) && own))) continue;
+                edge_tile[k] = t;
+                const int32_t l = index_of(lr[k].x), r = ai ? index_of(lr[k].y) : l;
+                uint32_t b = (uint32_t)l << LT_LEFT_SHIFT | (uint32_t)r << LT_RIGHT_SHIFT;
+                b |= ((f >> LI_SLOTL_SHIFT) & 3u) << LT_SLOTL_SHIFT | ((f >> LI_SLOTR_SHIFT) & 3u) << LT_SLOTR_SHIFT;
+                if (ai) b |= LT_AI;
+                float4 g = geo[k];
+                memcpy(&g.w, &b, 4);
+                ent.push_back(g);
+                dm.push_back(edm[k]);
+            }
+        };
+        for (int32_t c = c0; c < c1; ++c) add_edges(c);
+        const int32_t n1 = (int32_t)ring.size();
+        for (int32_t k = 0; k < n1; ++k) add_edges(ring[k]);
+        const int32_t keep = TILE + n1;
+        const bool fits = TILE + (int32_t)ring.size() <= (int32_t)LT_IDX_MASK + 1;
+        for (size_t k = ent0; k < ent.size() && fits; ++k) {  // own and ring-1 cells keep the edge's discharge
+            uint32_t b;
+            memcpy(&b, &ent[k].w, 4);
+            if ((int32_t)((b >> LT_LEFT_SHIFT) & LT_IDX_MASK) < keep) b |= LT_LKEEP;
+            if ((b & LT_AI) && (int32_t)((b >> LT_RIGHT_SHIFT) & LT_IDX_MASK) < keep) b |= LT_RKEEP;
+            memcpy(&ent[k].w, &b, 4);
+        }
+        if (ent.size() & 1) {  // an even count (16-byte copies of dm): an edge that nobody keeps
+            ent.push_back(make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+            dm.push_back(make_float2(1.0f, 0.0f));
+        }
+        const int32_t n_e = (int32_t)ent.size() - ent0;
+        info[2 * t] = make_int4(ent0, n_e, (int32_t)halo.size(), (int32_t)ring.size());
+        info[2 * t + 1] = make_int4(n1, (int32_t)harea.size(), 0, 0);
+        for (int32_t c : ring) halo.push_back(c);
+        for (int32_t k = 0; k < n1; ++k) harea.push_back(L.cinfo[ring[k]].x);
+        while (halo.size() % 4) halo.push_back(0);
+        while (harea.size() % 4) harea.push_back(0.0f);
+        a.e_cap = std::max(a.e_cap, n_e);
+        a.h_cap = std::max(a.h_cap, ((int32_t)ring.size() + 3) & ~3);
+        a.r1_cap = std::max(a.r1_cap, (n1 + 3) & ~3);
+        for (int32_t c = c0; c < c1; ++c) local[c] = -1;
+        for (int32_t c : ring) local[c] = -1;
+        if (!fits) return FL_OK;
+    }
+    a.n_tiles = tiles;
+    FL_CUDA(plan_li_tiles(a, s->kind, s->device, &s->lt_grid, &s->lt_smem));
+    if (!s->lt_grid) return FL_OK;
+    // every index against the buffers that the kernel reads
+    for (int32_t t = 0; t < tiles; ++t) {
+        const int4 i = info[2 * t], j = info[2 * t + 1];
+        bool ok = i.x >= 0 && i.x % 2 == 0 && (size_t)i.x + i.y <= ent.size() && i.z % 4 == 0 &&
+                  (size_t)i.z + ((i.w + 3) & ~3) <= halo.size() && j.x <= i.w && j.y % 4 == 0 &&
+                  (size_t)j.y + ((j.x + 3) & ~3) <= harea.size() && i.y <= a.e_cap && i.w <= a.h_cap && j.x <= a.r1_cap;
+        for (int32_t k = 0; ok && k < i.y; ++k) {
+            uint32_t b;
+            memcpy(&b, &ent[i.x + k].w, 4);
+            const int32_t l = (int32_t)((b >> LT_LEFT_SHIFT) & LT_IDX_MASK), r = (int32_t)((b >> LT_RIGHT_SHIFT) & LT_IDX_MASK);
+            ok = l < TILE + i.w && r < TILE + i.w && (!(b & LT_LKEEP) || l < TILE + j.x) && (!(b & LT_RKEEP) || r < TILE + j.x) &&
+                 ((b >> LT_SLOTL_SHIFT) & 3u) < 3u && ((b >> LT_SLOTR_SHIFT) & 3u) < 3u;
+        }
+        for (int32_t k = 0; ok && k < i.w; ++k) ok = halo[i.z + k] >= 0 && halo[i.z + k] < C;
+        if (!ok) return set_error(FL_E_INVALID, "local-inertial tile %d has an index out of range", t);
+    }
+    std::vector<float> len(L.char_len);
+    len.resize((size_t)L.Cp, 0.0f);  // whole tiles are copied
+    int4 *d_info = nullptr;
+    float4 *d_ent = nullptr;
+    float2 *d_dm = nullptr;
+    int32_t *d_halo = nullptr;
+    float *d_area = nullptr, *d_len = nullptr;
+    int rc;
+    if ((rc = s->upload(&d_len, len))) return rc;
+    if ((rc = s->upload(&d_info, info)) || (rc = s->upload(&d_ent, ent)) || (rc = s->upload(&d_dm, dm)) ||
+        (rc = s->upload(&d_halo, halo)) || (rc = s->upload(&d_area, harea)))
+        return rc;
+    a.tile = d_info;
+    a.ent = d_ent;
+    a.dm = d_dm;
+    a.halo_src = d_halo;
+    a.harea = d_area;
+    a.char_len = d_len;
+    return FL_OK;
 }
 
 // forcings: M entries (the members' rainfall); the per-cell fields come from
@@ -919,29 +1053,32 @@ static int create_impl(const FlMeshDesc *mesh, const FlDrainDesc *drain, const F
             const float mn = (f & LI_AI) ? 0.5f * (L.cinfo[l].y + L.cinfo[r].y) : L.cinfo[l].y;
             edm[k] = make_float2(dist, mn);
         }
-        int2 *d_lr;
-        float4 *d_geo, *d_qs;
-        float2 *d_dm, *d_nrm;
-        uint32_t *d_bits;
-        int4 *d_oth;
-        if ((rc = s->upload(&d_lr, lr)) || (rc = s->upload(&d_geo, geo)) || (rc = s->upload(&d_dm, edm)) ||
-            (rc = s->upload(&d_bits, cbits)) || (rc = s->upload(&d_oth, coth)) || (rc = s->upload(&d_nrm, cnrm)) ||
-            (rc = s->alloc(&d_qs, (size_t)Cp)))
-            return rc;
+        if ((rc = build_li_tiles(s, L, enew, lr, geo, edm))) return rc;
         LiArgs &q = s->li;
-        q.e_lr = d_lr;
-        q.e_geo = d_geo;
-        q.e_dm = d_dm;
-        q.c_bits = d_bits;
-        q.c_other = d_oth;
-        q.c_nrm = d_nrm;
+        if (!s->lt_grid) {
+            int2 *d_lr;
+            float4 *d_geo, *d_qs;
+            float2 *d_dm, *d_nrm;
+            uint32_t *d_bits;
+            int4 *d_oth;
+            if ((rc = s->upload(&d_lr, lr)) || (rc = s->upload(&d_geo, geo)) || (rc = s->upload(&d_dm, edm)) ||
+                (rc = s->upload(&d_bits, cbits)) || (rc = s->upload(&d_oth, coth)) || (rc = s->upload(&d_nrm, cnrm)) ||
+                (rc = s->alloc(&d_qs, (size_t)Cp)))
+                return rc;
+            q.e_lr = d_lr;
+            q.e_geo = d_geo;
+            q.e_dm = d_dm;
+            q.c_bits = d_bits;
+            q.c_other = d_oth;
+            q.c_nrm = d_nrm;
+            q.Qs = d_qs;
+        }
         q.cinfo = cinfo;
         q.char_len = char_len;
         q.horton = horton;
         q.wet = s->wet;
         q.state0 = s->state[0];
         q.state1 = s->state[1];
-        q.Qs = d_qs;
         q.ctrl = s->ctrl;
         q.run = s->run;
         q.hy = s->hy;
@@ -1354,8 +1491,8 @@ FL_API int fl_step(FlSolver *s, double dt_s, int32_t phases, double rain_rate_mp
         g_launches++;
     }
     if (s->li_mode) {
-        FL_CUDA(launch_li(s->li, s->kind, s->slot, 0, s->sms, st));
-        g_launches += 2;
+        FL_CUDA(launch_inertial(s, s->slot, 0, st));
+        g_launches += s->surface_launches();
     } else {
         FL_CUDA(launch_surface(s->sa, s->kind, s->slot, 0, s->surf_grid, s->surf_smem, st));
         g_launches++;
@@ -1408,7 +1545,7 @@ FL_API int fl_time_kernel(FlSolver *s, int32_t kernel, int32_t reps, void *strea
     auto launch = [&](cudaStream_t ls) -> cudaError_t {
         switch (kernel) {
             case 0:
-                return s->li_mode ? launch_li(s->li, s->kind, 0, 0, s->sms, ls)
+                return s->li_mode ? launch_inertial(s, 0, 0, ls)
                                   : launch_surface(s->sa, s->kind, 0, 0, s->surf_grid, s->surf_smem, ls);
             case 1: return launch_nodes(s->nd, 0, ls);
             case 2: return launch_network(s->nw, 0, ls);
@@ -1421,7 +1558,7 @@ FL_API int fl_time_kernel(FlSolver *s, int32_t kernel, int32_t reps, void *strea
             }
         }
     };
-    const int per = (kernel == 0 && s->li_mode) ? 2 : 1;  // kernels per launch
+    const int per = kernel == 0 ? s->surface_launches() : 1;  // kernels per launch
     // A chain of launches captured as one graph and replayed, as in the step
     // loop: the time is the kernels' own, not the host's launch rate or a
     // graph launch's.

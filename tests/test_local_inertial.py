@@ -176,3 +176,58 @@ def test_gpu_li_coupled_run_against_oracle_and_ledger_closes(gpu):
     rhs = (led["surface_volume_m3"] + led["node_volume_m3"] + led["infiltration_loss_m3"]
            + led["outfall_discharge_m3"] + led["unreturned_overflow_m3"] - led["boundary_net_flux_m3"])
     assert abs(lhs - rhs) <= 1e-5 * max(abs(lhs), 1.0), (lhs, rhs)
+
+
+def _random_grid(n: int):
+    """An n x n grid of squares in two triangles, with dry, wet and inactive
+    cells and open and closed boundary edges."""
+    from dataclasses import replace
+
+    from floodgb.synthetic import make_grid_city
+
+    sc = make_grid_city(n=n, size_m=10.0 * n, seed=n, duration_min=1.0)
+    rng = np.random.default_rng(n)
+    st = sc.city.topologies.surface_topology
+    C = st.cell_count
+    right, code = np.asarray(st.edge_right_cell), np.asarray(st.boundary_code).copy()
+    code[right < 0] = rng.choice([0, 1, 4], int((right < 0).sum()))
+    st = replace(st, boundary_code=code, active_mask=(rng.random(C) < 0.9).astype(np.float32))
+    h = np.where(rng.random(C) < 0.3, 0.0, rng.uniform(0.0, 0.3, C)).astype(np.float32)
+    hu, hv = (rng.uniform(-0.1, 0.1, (2, C)) * (h > 0)).astype(np.float32)
+    return st, h, hu, hv
+
+
+# 2 cells; a partial tile; one tile and 32 cells; two whole tiles; 13 tiles
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 11, 12, 16, 40])
+@pytest.mark.parametrize("phi", [0.0, 2.0e-6])
+def test_gpu_li_tiles_and_scattered_cells(gpu, n, phi):
+    """Neighbouring cells in one tile take the one launch over tiles; the same
+    mesh with its cells in a random order has rings too large for a tile (at 40:
+    about 2,000 cells around each) and takes the launches over edges and cells.
+    Both do the same arithmetic in the same order, so they agree bit for bit."""
+    from dataclasses import replace
+
+    from floodgb.backend import step_triangular_surface_local_inertial
+    from floodgb.topology import TriangularSurfaceForcing, TriangularSurfaceState
+
+    st, h, hu, hv = _random_grid(n)
+    rain, infil = np.full(h.size, 1.0e-5, np.float32), np.full(h.size, phi, np.float32)
+    out, _ = step_triangular_surface_local_inertial(
+        TriangularSurfaceState(h, hu, hv), st,
+        TriangularSurfaceForcing(rainfall_rate_mps=rain, infiltration_capacity_mps=infil), 0.2)
+    for a, b in zip((out.h_m, out.hu_m2ps, out.hv_m2ps), O.li_step(st, h, hu, hv, 0.2, rain, infil)):
+        within(a, b)
+    perm = np.random.default_rng(1).permutation(h.size)  # new cell i is cell perm[i]
+    inv = np.argsort(perm)
+    left, right = np.asarray(st.edge_left_cell), np.asarray(st.edge_right_cell)
+    cells = {k: np.asarray(getattr(st, k))[perm]
+             for k in ("bed_elevation_m", "manning_n", "cell_area_m2", "characteristic_length_m", "active_mask")}
+    sh = replace(st, edge_left_cell=inv[left].astype(left.dtype),
+                 edge_right_cell=np.where(right >= 0, inv[np.maximum(right, 0)], right).astype(right.dtype),
+                 cell_edge_indices=None, **cells)
+    sc, _ = step_triangular_surface_local_inertial(
+        TriangularSurfaceState(h[perm], hu[perm], hv[perm]), sh,
+        TriangularSurfaceForcing(rainfall_rate_mps=rain, infiltration_capacity_mps=infil), 0.2)
+    for a, b in zip((sc.h_m, sc.hu_m2ps, sc.hv_m2ps), (out.h_m, out.hu_m2ps, out.hv_m2ps)):
+        np.testing.assert_array_equal(np.asarray(a), np.asarray(b)[perm])
