@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) k_gemm_bf16_pers(const __grid_c
 
     if (warp < PG_PROD_WARPS) {
         // producers: lane = tile row 32 * warp + lane; its source row in each
-        // segment (nullptr: past M, the row stays stale and is not stored).
+        // segment (-1: past M, the row stays stale and is not stored).
         // The segments are walked by unrolled code over registers: picking
         // them from the parameters per chunk cost more than the copies
         const __nv_bfloat16 *base[3] = {g.a[0].base, g.a[1].base, g.a[2].base};
@@ -404,13 +404,14 @@ __global__ void __launch_bounds__(PG_THREADS, 1) k_gemm_bf16_pers(const __grid_c
 #pragma unroll
             for (int x = 0; x < 3; ++x) {
                 if (x >= n_seg || bad) continue;
-                const __nv_bfloat16 *p = row[x] >= 0 ? base[x] + (int64_t)row[x] * g.a[x].ld : nullptr;
+                int own[8];
+                rows_of_lane(row[x], own, lane);
                 for (int k = 0; k < g.a[x].width; k += MM_BK) {
                     if (u > 0 && !warp_wait(smem_addr(&empty[s]), (u - 1) & 1)) {
                         bad = true;
                         break;
                     }
-                    warp_copy_rows(p ? p + k : nullptr, sA + s * MM_CHUNK_BYTES, warp, lane);
+                    warp_copy_numbered(base[x] + k, g.a[x].ld, own, sA + s * MM_CHUNK_BYTES, warp, lane);
                     cp_async_arrive_noinc(smem_addr(&full[s]));
                     if (++s == S) {
                         s = 0;

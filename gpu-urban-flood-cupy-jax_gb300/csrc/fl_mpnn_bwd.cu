@@ -460,12 +460,10 @@ __global__ void __launch_bounds__(EB_THREADS, 1) k_edge_bwd(const __grid_constan
             load_starts(tn, nrs, ndeg, nso, nsd);  // the next tile's, used in the next round
 #pragma unroll
             for (int p = 0; p < 6; ++p) {
-                const __nv_bfloat16 *row[2];
+                int row[2][8];
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const int e = p < 3 ? (p < deg[j] ? rs[j] + p : -1) : ord[j][p - 3 < 0 ? 0 : p - 3];
-                    row[j] = e >= 0 ? g.dze + (int64_t)e * MF_H : nullptr;
-                }
+                for (int j = 0; j < 2; ++j)
+                    rows_of_lane(p < 3 ? (p < deg[j] ? rs[j] + p : -1) : ord[j][p < 3 ? 0 : p - 3], row[j], lane);
                 if (p == 3) load_orders(nso, nsd, nord);
 #pragma unroll 1
                 for (int c = 0; c < 2; ++c, ++q) {
@@ -474,8 +472,9 @@ __global__ void __launch_bounds__(EB_THREADS, 1) k_edge_bwd(const __grid_constan
                         bad = true;
                         break;
                     }
-                    warp_copy_rows64(row[0] ? row[0] + c * 64 : nullptr, row[1] ? row[1] + c * 64 : nullptr,
-                                     sR + s * MM_CHUNK_BYTES, warp, lane);
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+                        warp_copy_numbered(g.dze + c * 64, MF_H, row[j], sR + s * MM_CHUNK_BYTES, 2 * warp + j, lane);
                     cp_async_arrive_noinc(ringf + 8 * s);
                 }
                 if (bad) break;
@@ -634,7 +633,6 @@ __global__ void __launch_bounds__(ES_THREADS, 1) k_edge_dsum(const __grid_consta
 
     if (warp < ES_PROD) {
         int q = 0;
-        const int R0 = 64 * warp + lane, R1 = R0 + 32;
         for (int t = blockIdx.x; t < steps && !bad; t += gridDim.x) {
             for (int c = 0; c < 2 * g.layers; ++c, ++q) {
                 const int s = q % ES_RING, u = q / ES_RING;
@@ -646,12 +644,10 @@ __global__ void __launch_bounds__(ES_THREADS, 1) k_edge_dsum(const __grid_consta
                 const uint32_t dst = sR + s * ES_STAGE;
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
-                    const int r0 = t * 2 * MM_BM + j * MM_BM + R0, r1 = r0 + 32;
-                    warp_copy_rows64(r0 < g.E ? z + (int64_t)r0 * MF_H : nullptr, r1 < g.E ? z + (int64_t)r1 * MF_H : nullptr,
-                                     dst + j * MM_CHUNK_BYTES, warp, lane);
+                    const int r0 = t * 2 * MM_BM + j * MM_BM + 64 * warp;
+                    warp_copy_span<64>(z, MF_H, r0, g.E, dst + j * MM_CHUNK_BYTES, 64 * warp, lane);
                 }
-                warp_copy_rows64(w + (int64_t)R0 * g.ldwt[c >> 1], w + (int64_t)R1 * g.ldwt[c >> 1],
-                                 dst + 2 * MM_CHUNK_BYTES, warp, lane);
+                warp_copy_span<64>(w, g.ldwt[c >> 1], 64 * warp, MM_BN, dst + 2 * MM_CHUNK_BYTES, 64 * warp, lane);
                 cp_async_arrive_noinc(ringf + 8 * s);
             }
         }
@@ -830,12 +826,12 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad(const __grid_constant__
     pdl_launch_dependents();
 
     if (warp < WG_PROD) {
-        // producers: 8 rows of each 64-row chunk (lanes 0..7 own one each);
+        // producers: 8 rows of each 64-row chunk, a lane rows own and own + 4;
         // row maps are read one chunk ahead.  The job's fields are held in
         // registers: read from the parameters in the copy loop they made it
         // 230 cycles an instruction
         uint32_t busy = 0u, par = 0u;  // per stage: filled and not known empty; parity of its next "empty"
-        const int piece = lane & 7, own = 8 * warp + piece;
+        const int piece = lane & 7, own = 8 * warp + (lane >> 3);
         int s = 0, last = -1;
         for (int it = it0; it < it1 && !bad; ++it) {
             const int jn = g.item[it] >> 14, sp = g.item[it] & 0x3fff;
@@ -860,16 +856,16 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad(const __grid_constant__
             off[2] = off[1] + (G[1].width / 64) * WG_BLOCK;
             off[3] = off[2] + (G[2].width / 64) * WG_BLOCK;
             const int c0 = sp * J.per, c1 = min((M + 63) / 64, c0 + J.per);
-            auto load_rows = [&](int c, const __nv_bfloat16 *(&o)[4]) {
-                const int r = c * 64 + own;
-                const bool in = c < c1 && r < M;
+            auto load_rows = [&](int c, int (&o)[4][2]) {
 #pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                    o[x] = nullptr;
-                    if (in && x <= nx) o[x] = G[x].base + (G[x].rows ? (int64_t)G[x].rows[r] : (int64_t)r) * G[x].ld;
+                for (int i = 0; i < 2; ++i) {
+                    const int r = c * 64 + own + 4 * i;
+                    const bool in = c < c1 && r < M;
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) o[x][i] = in && x <= nx ? (G[x].rows ? G[x].rows[r] : r) : -1;
                 }
             };
-            const __nv_bfloat16 *row[4], *nrow[4];
+            int row[4][2], nrow[4][2];
             load_rows(c0, row);
             for (int c = c0; c < c1; ++c) {
                 load_rows(c + 1, nrow);
@@ -887,8 +883,8 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad(const __grid_constant__
                     if (x <= nx) {
 #pragma unroll
                         for (int i = 0; i < 2; ++i) {
-                            const int rr = 4 * i + (lane >> 3), R = 8 * warp + rr;
-                            const __nv_bfloat16 *src = (const __nv_bfloat16 *)__shfl_sync(0xffffffffu, (uint64_t)row[x], rr);
+                            const int R = own + 4 * i;
+                            const __nv_bfloat16 *src = row[x][i] >= 0 ? G[x].base + row[x][i] * G[x].ld : nullptr;
                             const uint32_t d = dst + off[x] + (uint32_t)(R * 128 + ((piece ^ (R & 7)) << 4));
                             if (src) cp_async16(d, src + piece * 8);
                             else asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(d), "r"(0u) : "memory");
@@ -901,7 +897,9 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad(const __grid_constant__
                 }
                 cp_async_arrive_noinc(ringf + 8 * s);
 #pragma unroll
-                for (int x = 0; x < 4; ++x) row[x] = nrow[x];
+                for (int x = 0; x < 4; ++x)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) row[x][i] = nrow[x][i];
                 if (++s == S) s = 0;
             }
         }
@@ -1044,7 +1042,7 @@ struct CsJob {
 struct RdArgs {
     RdJob job[RD_JOBS];
     CsJob cs[CS_JOBS];
-    int32_t jobs;            // blockIdx.y < jobs: partial products; else column sums
+    int32_t jobs, first;     // blockIdx.y: the first column sums, the partial products, the other column sums
 };
 
 struct BfJob {
@@ -1065,13 +1063,14 @@ __device__ __forceinline__ void add4(float4 &s, const float4 v) {
 // Column sums for the bias gradients: a thread per row class and column walks
 // its rows in order (a sum's order is kept, so loads in flight, not adders,
 // hide the latency: 16 rows by four columns a thread took 300 us a layer on
-// 299,712 rows, 32 rows by one 80).  Both in one launch: either alone leaves
-// the device half idle.
+// 299,712 rows, 32 rows by one 80, of which the next batch's loads now overlap
+// the adds).  Both in one launch: either alone leaves the device half idle.
 __global__ void __launch_bounds__(256) k_reduce(const __grid_constant__ RdArgs g) {
     pdl_wait();
     pdl_launch_dependents();
-    if ((int)blockIdx.y < g.jobs) {
-        const RdJob &J = g.job[blockIdx.y];
+    const int y = (int)blockIdx.y - g.first;
+    if (y >= 0 && y < g.jobs) {
+        const RdJob &J = g.job[y];
         const int n = J.n, count = J.count;
         const int i = ((int)blockIdx.x * 256 + (int)threadIdx.x) * 4;
         if (i >= n) return;
@@ -1099,29 +1098,42 @@ __global__ void __launch_bounds__(256) k_reduce(const __grid_constant__ RdArgs g
         return;
     }
     // a thread per (row class, column): 32 columns a warp, 32 rows' loads in flight
-    const CsJob &J = g.cs[blockIdx.y - g.jobs];
+    const CsJob &J = g.cs[y < 0 ? y + g.first : y - g.jobs + g.first];
     const int id = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int cls = id >> 2, c = (id & 3) * 32 + lane, M = J.M;
     if (cls >= RD_STRIDE || (id & 3) * 32 >= J.n) return;  // (uniform over the warp)
     const float *x = J.x + c;
     const int64_t ld = J.ld;
-    float s = 0.0f;
+    constexpr int N = 32, STEP = N * RD_STRIDE;  // rows of a batch; two batches' loads in flight
+    float s = 0.0f, v[N], w[N];
     if (!J.bits) {
-        for (int r = cls; r < M; r += 32 * RD_STRIDE) {
-            float v[32];
+        auto fetch = [&](int r, float (&o)[N]) {
 #pragma unroll
-            for (int u = 0; u < 32; ++u) {
-                v[u] = 0.0f;
-                if (r + u * RD_STRIDE < M) v[u] = x[(int64_t)(r + u * RD_STRIDE) * ld];
+            for (int u = 0; u < N; ++u) {
+                o[u] = 0.0f;
+                if (r + u * RD_STRIDE < M) o[u] = x[(int64_t)(r + u * RD_STRIDE) * ld];
             }
+        };
+        auto add = [&](const float (&o)[N]) {
 #pragma unroll
-            for (int u = 0; u < 32; ++u) s += v[u];
+            for (int u = 0; u < N; ++u) s += o[u];
+        };
+        fetch(cls, v);
+        for (int r = cls; r < M; r += 2 * STEP) {
+            fetch(r + STEP, w);
+            add(v);
+            if (r + STEP >= M) break;
+            fetch(r + 2 * STEP, v);
+            add(w);
         }
     } else {
         const uint32_t *bits = J.bits + (id & 3);
         const int32_t *map = J.map;
-        // the map entries and bits of 32 rows at once, a row a lane
+        // the map entries and bits of a batch at once, a row a lane; rows past
+        // the end read row 0 and have no bits (branches around the loads made
+        // them wait for one another)
         auto load = [&](int r, int &row, uint32_t &m) {
+            r += lane * RD_STRIDE;
             row = 0;
             m = 0u;
             if (r < M) {
@@ -1129,22 +1141,31 @@ __global__ void __launch_bounds__(256) k_reduce(const __grid_constant__ RdArgs g
                 m = bits[(int64_t)r * 4];
             }
         };
-        int at;
-        uint32_t mask;
-        load(cls + lane * RD_STRIDE, at, mask);
-        for (int r = cls; r < M; r += 32 * RD_STRIDE) {
-            int next;
-            uint32_t next_mask;
-            load(r + (32 + lane) * RD_STRIDE, next, next_mask);
-            // (rows past the end read row 0 and have no bits: branches around
-            // the loads made them wait for one another)
-            float v[32];
+        auto fetch = [&](int at, float (&o)[N]) {
 #pragma unroll
-            for (int u = 0; u < 32; ++u) v[u] = x[(int64_t)__shfl_sync(0xffffffffu, at, u) * ld];
+            for (int u = 0; u < N; ++u) o[u] = x[(int64_t)__shfl_sync(0xffffffffu, at, u) * ld];
+        };
+        auto add = [&](uint32_t mask, const float (&o)[N]) {
 #pragma unroll
-            for (int u = 0; u < 32; ++u) s += __shfl_sync(0xffffffffu, mask, u) >> lane & 1u ? v[u] : 0.0f;
-            at = next;
-            mask = next_mask;
+            for (int u = 0; u < N; ++u) s += __shfl_sync(0xffffffffu, mask, u) >> lane & 1u ? o[u] : 0.0f;
+        };
+        int a0, a1, a2;
+        uint32_t m0, m1, m2;
+        load(cls, a0, m0);
+        load(cls + STEP, a1, m1);
+        fetch(a0, v);
+        for (int r = cls; r < M; r += 2 * STEP) {
+            load(r + 2 * STEP, a2, m2);
+            fetch(a1, w);
+            add(m0, v);
+            if (r + STEP >= M) break;
+            a0 = a2;
+            m0 = m2;
+            load(r + 3 * STEP, a2, m2);
+            fetch(a0, v);
+            add(m1, w);
+            a1 = a2;
+            m1 = m2;
         }
     }
     J.part[(int64_t)cls * J.n + c] = s;
@@ -1289,6 +1310,13 @@ FL_API int fl_mpnn_backward(const FlMpnnBackwardDesc *d, void *stream) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         rd.jobs = n_rd;
+        // the longest chains start first: sums of more than 16 batches of rows,
+        // the partial products (up to 32 batches), then the short sums, which
+        // fill in (two blocks fit an SM; 99,904 cells: 70 us, with the products
+        // first 80, with them last 78)
+        std::sort(rd.cs, rd.cs + n_cs, [](const CsJob &a, const CsJob &b) { return a.M > b.M; });
+        rd.first = 0;
+        while (rd.first < n_cs && rd.cs[rd.first].M > 16 * 32 * RD_STRIDE) ++rd.first;
         e = cudaLaunchKernelEx(&cfg, k_reduce, rd);
         ++launched;
         n_rd = n_cs = rd_blocks = 0;

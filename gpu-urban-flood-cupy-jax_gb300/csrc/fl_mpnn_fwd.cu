@@ -19,14 +19,16 @@
 // stored or summed.
 //
 // Measured (8 layers, 1.9 M cells and 5.7 M edges): 34.7 ms a pass with one
-// launch per product, 12.0 ms here; per launch and 401,408 cells k_edge_fwd
-// 156 us (the SM's shared-memory pipe 91 % busy: MMA operands, gathers, bias
-// reads), k_mlp2 as node update 150 us (4.5 TB/s).
+// launch per product, 11.0 ms here (k_edge_fwd: the SM's shared-memory pipe, which
+// MMA operands and gathers share, is full); 20,402 cells 777 -> 230 us (a
+// launch's fill and drain, one or two tiles a CTA).
 //
-// Both kernels are persistent and warp-specialised like k_gemm_bf16_pers:
-// four producer warps (cp.async gathers into 16 KB stages), one MMA lane,
-// eight epilogue warps; weights stay in shared memory.  The rounding points
-// (bf16 activations, fp32 accumulation in K order, fp32 sums in edge order)
+// Both kernels are persistent and warp-specialised: four producer warps
+// (cp.async gathers into 16 KB stages; two warps, each copy's row pointer
+// shuffled to its lanes, took 11.9 ms and 297 us), one MMA lane, sixteen epilogue
+// warps; weights stay in shared memory, and only the MMA
+// warp waits for them.  The rounding points (bf16 activations, fp32
+// accumulation in K order, fp32 sums in edge order)
 // are those of the separate products, so both give the same bits.
 //
 // Every mbarrier wait is bounded; one that gives up sets the error flag.
@@ -34,7 +36,7 @@
 
 namespace fl {
 
-constexpr int MF_PROD_WARPS = 2, MF_EPI_WARPS = 16, MF_THREADS = 32 * (MF_PROD_WARPS + 1 + MF_EPI_WARPS);
+constexpr int MF_PROD_WARPS = 4, MF_EPI_WARPS = 16, MF_THREADS = 32 * (MF_PROD_WARPS + 1 + MF_EPI_WARPS);
 constexpr int MF_CHUNKS = 14;  // 16 KB chunks of shared memory
 constexpr int MF_SMEM = MF_CHUNKS * MM_CHUNK_BYTES + 256 /* barriers */ + 1024 /* alignment */;
 constexpr int EF_RING = 4;
@@ -117,8 +119,8 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_edge_fwd(const __grid_constan
     const uint32_t sR = sD + 2 * MM_CHUNK_BYTES;
     uint64_t *bars = (uint64_t *)(smem + MF_CHUNKS * MM_CHUNK_BYTES);
     const uint32_t dstf = smem_addr(bars), dste = dstf + 8, ringf = dstf + 16, ringe = ringf + 8 * EF_RING;
-    const uint32_t d1f = ringe + 8 * EF_RING, zf = d1f + 24, d2f = zf + 16, de = d2f + 24, drain = de + 24;
-    uint32_t *tmem_slot = (uint32_t *)(bars + 2 + 2 * EF_RING + 3 + 2 + 3 + 3 + 1);
+    const uint32_t d1f = ringe + 8 * EF_RING, zf = d1f + 24, d2f = zf + 16, de = d2f + 24, drain = de + 24, wbar = drain + 8;
+    uint32_t *tmem_slot = (uint32_t *)(bars + 2 + 2 * EF_RING + 3 + 2 + 3 + 3 + 2);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tiles = (g.C + MM_BM - 1) / MM_BM;
 
@@ -137,6 +139,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_edge_fwd(const __grid_constan
         mbar_init(zf, MF_EPI_WARPS);
         mbar_init(zf + 8, MF_EPI_WARPS);
         mbar_init(drain, 1);
+        mbar_init(wbar, MF_THREADS);
         mbar_fence_init();
     }
     if (warp == MF_PROD_WARPS) {
@@ -147,11 +150,10 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_edge_fwd(const __grid_constan
     // weights: not written by the kernel before this one (they change between passes only)
     for (int c = 0; c < 6; ++c) load_weight_chunk(g.w1, g.ldw1, MF_H, c, sW1 + c * MM_CHUNK_BYTES, tid, MF_THREADS);
     for (int c = 0; c < 2; ++c) load_weight_chunk(g.w2, g.ldw2, MF_H, c, sW2 + c * MM_CHUNK_BYTES, tid, MF_THREADS);
-    cp_async_commit();
-    cp_async_wait_all();
     fence_async_smem();
     tmem_fence_before();
     __syncthreads();
+    cp_async_arrive_noinc(wbar);  // only the MMA warp waits for the weights
     tmem_fence_after();
     const uint32_t tmem = *tmem_slot;
     bool bad = false;
@@ -159,51 +161,44 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_edge_fwd(const __grid_constan
     pdl_launch_dependents();
 
     if (warp < MF_PROD_WARPS) {
-        // producers: a lane's tile rows are 64 * warp + lane and + 32; first
-        // edge, edge count and senders, the next tile's read one tile ahead
+        // producers: lane = tile row 32 * warp + lane; first edge, edge count
+        // and senders, the next tile's read one tile ahead
         int t = blockIdx.x, q = 0;
-        int rs[2], deg[2], snd[2][3];
-        auto load_starts = [&](int tt, int (&a)[2], int (&b)[2]) {
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int c = tt * MM_BM + 64 * warp + lane + 32 * j;
-                a[j] = b[j] = 0;
-                if (tt < tiles && c < g.C) {
-                    a[j] = g.start[c];
-                    b[j] = g.start[c + 1] - a[j];
-                }
+        int rs, deg, snd[3];
+        auto load_starts = [&](int tt, int &a, int &b) {
+            const int c = tt * MM_BM + 32 * warp + lane;
+            a = b = 0;
+            if (tt < tiles && c < g.C) {
+                a = g.start[c];
+                b = g.start[c + 1] - a;
             }
         };
-        auto load_senders = [&](const int (&a)[2], const int (&b)[2], int (&o)[2][3]) {
+        auto load_senders = [&](int a, int b, int (&o)[3]) {
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
-#pragma unroll
-                for (int k = 0; k < 3; ++k) o[j][k] = k < b[j] ? g.src[a[j] + k] : -1;
+            for (int k = 0; k < 3; ++k) o[k] = k < b ? g.src[a + k] : -1;
         };
         load_starts(t, rs, deg);
         load_senders(rs, deg, snd);
         for (int i = 0; t < tiles && !bad; ++i) {
-            const int tn = t + gridDim.x, c0 = t * MM_BM + 64 * warp + lane, c1 = c0 + 32;
-            int nrs[2], ndeg[2], nsnd[2][3];
+            const int tn = t + gridDim.x;
+            int nrs, ndeg, nsnd[3];
             load_starts(tn, nrs, ndeg);
             if (i > 0 && !warp_wait(dste, (i - 1) & 1)) {
                 bad = true;
                 break;
             }
-            const __nv_bfloat16 *h0 = c0 < g.C ? g.h + (int64_t)c0 * MF_H : nullptr;
-            const __nv_bfloat16 *h1 = c1 < g.C ? g.h + (int64_t)c1 * MF_H : nullptr;
-            warp_copy_rows64(h0, h1, sD, warp, lane);
-            warp_copy_rows64(h0 ? h0 + 64 : nullptr, h1 ? h1 + 64 : nullptr, sD + MM_CHUNK_BYTES, warp, lane);
+            int row[8];
+#pragma unroll
+            for (int x = 0; x < 8; ++x) {
+                row[x] = t * MM_BM + 32 * warp + 4 * x + (lane >> 3);
+                if (row[x] >= g.C) row[x] = -1;
+            }
+            warp_copy_numbered(g.h, MF_H, row, sD, warp, lane);
+            warp_copy_numbered(g.h + 64, MF_H, row, sD + MM_CHUNK_BYTES, warp, lane);
             cp_async_arrive_noinc(dstf);
             load_senders(nrs, ndeg, nsnd);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                const __nv_bfloat16 *ph[2], *pe[2];
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    ph[j] = snd[j][k] >= 0 ? g.h + (int64_t)snd[j][k] * MF_H : nullptr;
-                    pe[j] = k < deg[j] ? g.e + (int64_t)(rs[j] + k) * MF_H : nullptr;
-                }
 #pragma unroll
                 for (int j = 0; j < 4; ++j, ++q) {
                     const int s = q % EF_RING, u = q / EF_RING;
@@ -211,21 +206,18 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_edge_fwd(const __grid_constan
                         bad = true;
                         break;
                     }
-                    const __nv_bfloat16 *p0 = j < 2 ? ph[0] : pe[0], *p1 = j < 2 ? ph[1] : pe[1];
-                    warp_copy_rows64(p0 ? p0 + (j & 1) * 64 : nullptr, p1 ? p1 + (j & 1) * 64 : nullptr,
-                                     sR + s * MM_CHUNK_BYTES, warp, lane);
+                    if (j == 0) rows_of_lane(snd[k], row, lane);
+                    if (j == 2) rows_of_lane(k < deg ? rs + k : -1, row, lane);
+                    warp_copy_numbered((j < 2 ? g.h : g.e) + (j & 1) * 64, MF_H, row, sR + s * MM_CHUNK_BYTES, warp, lane);
                     cp_async_arrive_noinc(ringf + 8 * s);
                 }
                 if (bad) break;
             }
             t = tn;
+            rs = nrs;
+            deg = ndeg;
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                rs[j] = nrs[j];
-                deg[j] = ndeg[j];
-#pragma unroll
-                for (int k = 0; k < 3; ++k) snd[j][k] = nsnd[j][k];
-            }
+            for (int k = 0; k < 3; ++k) snd[k] = nsnd[k];
         }
         cp_async_wait_all();
     } else if (warp == MF_PROD_WARPS) {
@@ -248,6 +240,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_edge_fwd(const __grid_constan
                     umma_commit(d2f + 8 * k);
                 }
             };
+            bad = !warp_wait(wbar, 0);
             for (int t = blockIdx.x; t < tiles && !bad; t += gridDim.x, ++i) {
                 if (!warp_wait(dstf, i & 1)) {
                     bad = true;
@@ -400,6 +393,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_edge_fwd(const __grid_constan
         if (n > 0 && !bad) sum_slot(n - 1, 2, pt, pdeg);
     }
     if (bad) atomicCAS(g.error, 0, FL_E_TIMEOUT);
+    cp_async_wait_all();
     tmem_fence_before();
     __syncthreads();
     if (warp == MF_PROD_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
@@ -412,8 +406,8 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_mlp2(const __grid_constant__ 
     const uint32_t sW1 = smem_addr(smem), sW2 = sW1 + nK * MM_CHUNK_BYTES, sR = sW2 + 2 * MM_CHUNK_BYTES;
     uint64_t *bars = (uint64_t *)(smem + MF_CHUNKS * MM_CHUNK_BYTES);
     const uint32_t ringf = smem_addr(bars), ringe = ringf + 8 * M2_MAX_RING;
-    const uint32_t d1f = ringe + 8 * M2_MAX_RING, zf = d1f + 24, d2f = zf + 16, de = d2f + 24, drain = de + 24;
-    uint32_t *tmem_slot = (uint32_t *)(bars + 2 * M2_MAX_RING + 3 + 2 + 3 + 3 + 1);
+    const uint32_t d1f = ringe + 8 * M2_MAX_RING, zf = d1f + 24, d2f = zf + 16, de = d2f + 24, drain = de + 24, wbar = drain + 8;
+    uint32_t *tmem_slot = (uint32_t *)(bars + 2 * M2_MAX_RING + 3 + 2 + 3 + 3 + 2);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tiles = (g.M + MM_BM - 1) / MM_BM;
 
@@ -430,6 +424,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_mlp2(const __grid_constant__ 
         mbar_init(zf, MF_EPI_WARPS);
         mbar_init(zf + 8, MF_EPI_WARPS);
         mbar_init(drain, 1);
+        mbar_init(wbar, MF_THREADS);
         mbar_fence_init();
     }
     if (warp == MF_PROD_WARPS) {
@@ -439,11 +434,10 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_mlp2(const __grid_constant__ 
     }
     for (int c = 0; c < nK; ++c) load_weight_chunk(g.w1, g.ldw1, MF_H, c, sW1 + c * MM_CHUNK_BYTES, tid, MF_THREADS);
     for (int c = 0; c < 2; ++c) load_weight_chunk(g.w2, g.ldw2, g.n2, c, sW2 + c * MM_CHUNK_BYTES, tid, MF_THREADS);
-    cp_async_commit();
-    cp_async_wait_all();
     fence_async_smem();
     tmem_fence_before();
     __syncthreads();
+    cp_async_arrive_noinc(wbar);  // only the MMA warp waits for the weights
     tmem_fence_after();
     const uint32_t tmem = *tmem_slot;
     bool bad = false;
@@ -453,17 +447,20 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_mlp2(const __grid_constant__ 
     if (warp < MF_PROD_WARPS) {
         int s = 0, u = 0;
         for (int t = blockIdx.x; t < tiles && !bad; t += gridDim.x) {
-            const int r0 = t * MM_BM + 64 * warp + lane, r1 = r0 + 32;
+            int row[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                row[i] = t * MM_BM + 32 * warp + 4 * i + (lane >> 3);
+                if (row[i] >= g.M) row[i] = -1;
+            }
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
-                const __nv_bfloat16 *p0 = r0 < g.M ? g.a[x] + (int64_t)r0 * g.lda[x] : nullptr;
-                const __nv_bfloat16 *p1 = r1 < g.M ? g.a[x] + (int64_t)r1 * g.lda[x] : nullptr;
                 for (int c = 0; c < g.nk[x] && !bad; ++c) {
                     if (u > 0 && !warp_wait(ringe + 8 * s, (u - 1) & 1)) {
                         bad = true;
                         break;
                     }
-                    warp_copy_rows64(p0 ? p0 + c * 64 : nullptr, p1 ? p1 + c * 64 : nullptr, sR + s * MM_CHUNK_BYTES, warp, lane);
+                    warp_copy_numbered(g.a[x] + c * 64, g.lda[x], row, sR + s * MM_CHUNK_BYTES, warp, lane);
                     cp_async_arrive_noinc(ringf + 8 * s);
                     if (++s == S) {
                         s = 0;
@@ -492,6 +489,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_mlp2(const __grid_constant__ 
                     umma_commit(d2f + 8 * k);
                 }
             };
+            bad = !warp_wait(wbar, 0);
             for (int t = blockIdx.x; t < tiles && !bad; t += gridDim.x, ++n) {
                 const int k = n % 3;
                 if (n >= 3 && !warp_wait(de + 8 * k, (n / 3 - 1) & 1)) {
@@ -621,6 +619,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1) k_mlp2(const __grid_constant__ 
         if (n > 0 && !bad) finish(n - 1, pt);
     }
     if (bad) atomicCAS(g.error, 0, FL_E_TIMEOUT);
+    cp_async_wait_all();
     tmem_fence_before();
     __syncthreads();
     if (warp == MF_PROD_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));

@@ -189,34 +189,39 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
     return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, MM_WAIT_NS));
 }
 
-// Producer warp's part of a 128-row chunk: its 32 rows, four whole 128-byte
-// row pieces per instruction.  `own`: this lane's row pointer (nullptr: the
-// row is left as it is), at the chunk's first column.
-__device__ __forceinline__ void warp_copy_rows(const __nv_bfloat16 *own, uint32_t sdst, int pw, int lane) {
+// 32 rows of a 128-row chunk (those from 32 pw), by one warp: four whole 128-byte
+// row pieces per instruction.  Lane l copies the rows 4 i + l / 8, whose numbers
+// it holds itself (row[i]; < 0: the row is left as it is), from `base`, the
+// matrix at the chunk's first column.  The numbers are exchanged once for all
+// chunks of a row (rows_of_lane): a shuffled pointer per copy instruction took
+// two of every six cycles of the pipe that also writes the copies.
+__device__ __forceinline__ void warp_copy_numbered(const __nv_bfloat16 *base, int64_t ld, const int (&row)[8], uint32_t sdst, int pw,
+                                                   int lane) {
     const int c = lane & 7;
-    const uint64_t p = (uint64_t)own;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const int rr = 4 * i + (lane >> 3);
-        const uint64_t row = __shfl_sync(0xffffffffu, p, rr);
-        const int R = 32 * pw + rr;
-        if (row) cp_async16(sdst + (uint32_t)(R * 128 + ((c ^ (R & 7)) << 4)), (const __nv_bfloat16 *)row + c * 8);
+        const int R = 32 * pw + 4 * i + (lane >> 3);
+        if (row[i] >= 0) cp_async16(sdst + (uint32_t)(R * 128 + ((c ^ (R & 7)) << 4)), base + row[i] * ld + c * 8);
     }
 }
 
-// A producer warp's 64 rows of a 128-row chunk; own0 / own1: this lane's rows
-// (lane, lane + 32), nullptr: left as it is.
-__device__ __forceinline__ void warp_copy_rows64(const __nv_bfloat16 *own0, const __nv_bfloat16 *own1, uint32_t sdst, int pw,
-                                                 int lane) {
+// ROWS consecutive rows of a matrix from `first` (those past `limit` are left
+// as they are) to the rows R0 .. of a chunk.
+template <int ROWS>
+__device__ __forceinline__ void warp_copy_span(const __nv_bfloat16 *base, int64_t ld, int64_t first, int64_t limit, uint32_t sdst,
+                                               int R0, int lane) {
     const int c = lane & 7;
-    const uint64_t p0 = (uint64_t)own0, p1 = (uint64_t)own1;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const int rr = 4 * i + (lane >> 3);
-        const uint64_t row = __shfl_sync(0xffffffffu, i < 8 ? p0 : p1, rr & 31);
-        const int R = 64 * pw + rr;
-        if (row) cp_async16(sdst + (uint32_t)(R * 128 + ((c ^ (R & 7)) << 4)), (const __nv_bfloat16 *)row + c * 8);
+    for (int i = 0; i < ROWS / 4; ++i) {
+        const int rr = 4 * i + (lane >> 3), R = R0 + rr;
+        if (first + rr < limit) cp_async16(sdst + (uint32_t)(R * 128 + ((c ^ (R & 7)) << 4)), base + (first + rr) * ld + c * 8);
     }
+}
+
+// own: a value per tile row of the warp (lane = row) to the lanes that copy them.
+__device__ __forceinline__ void rows_of_lane(int own, int (&row)[8], int lane) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) row[i] = __shfl_sync(0xffffffffu, own, 4 * i + (lane >> 3));
 }
 
 // 64-wide K chunk c of a bf16 matrix's rows [0, n) into the K-major 128-byte-swizzle layout at
