@@ -24,8 +24,11 @@
 // activation across a bf16 boundary every few steps, and a training run then
 // goes its own way.  The message layers' second bias is the caller's.
 //
-// Measured: one optimizer step on 100,352 cells and 299,712 dual edges, 8
-// layers: see the figures at fl_mpnn_backward.
+// Measured: one optimizer step on 99,904 cells and 299,712 dual edges, 8 layers:
+// 34.5 ms product by product, 5.48 ms here.  Per layer (cold L2): k_mlp_bwd 105 us
+// (510 MB: 4.9 TB/s; one row a lane, whose 32-byte pieces lie in 32 lines an
+// instruction, took 139), k_wgrad 94, k_reduce 70, k_edge_bwd 53 (4.8 TB/s),
+// k_edge_dsum 144 once.
 //
 // Every mbarrier wait is bounded; one that gives up sets the error flag.
 #include <utility>
@@ -40,8 +43,29 @@ __device__ __forceinline__ uint32_t positive_mask(uint32_t z) {  // 0xffff where
     return __hgt2_mask(*(const __nv_bfloat162 *)&z, zero);
 }
 
+// The 32 columns of row r (0: g, 1: g + 8) of a fragment (tmem_ld_frag32): the
+// lane's eight consecutive ones from 8 q.
+__device__ __forceinline__ void frag_to_row(const uint32_t (&v)[16], int r, int q, uint32_t (&x)[8]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        x[2 * j] = v[4 * j + 2 * r];
+        x[2 * j + 1] = v[4 * j + 2 * r + 1];
+    }
+    transpose4(x[0], x[2], x[4], x[6], q);
+    transpose4(x[1], x[3], x[5], x[7], q);
+}
+
+// Eight consecutive 16-bit values of row r to the packed fragment (tmem_st_frag_pairs).
+__device__ __forceinline__ void pairs_to_frag(uint4 y, int r, int q, uint32_t (&w)[8]) {
+    transpose4(y.x, y.y, y.z, y.w, q);
+    w[r] = y.x;
+    w[2 + r] = y.y;
+    w[4 + r] = y.z;
+    w[6 + r] = y.w;
+}
+
 // ------------------------------------------------------------- MLP backward
-constexpr int MB_WARPS = 8, MB_THREADS = 32 * (MB_WARPS + 1);
+constexpr int MB_WARPS = 16, MB_THREADS = 32 * (MB_WARPS + 1);
 constexpr int MB_CHUNKS = 8;
 constexpr int MB_SMEM = MB_CHUNKS * MM_CHUNK_BYTES + 256 + 1024;
 
@@ -78,8 +102,8 @@ __global__ void __launch_bounds__(MB_THREADS, 1) k_mlp_bwd(const __grid_constant
     const uint32_t sW2 = smem_addr(smem), sW1 = sW2 + 2 * MM_CHUNK_BYTES, sE2 = sW1 + 4 * MM_CHUNK_BYTES;
     uint64_t *bars = (uint64_t *)(smem + MB_CHUNKS * MM_CHUNK_BYTES);
     const uint32_t in1 = smem_addr(bars), in2 = in1 + 8, in3 = in1 + 16, d1 = in1 + 24, d2a = in1 + 32, d2b = in1 + 40,
-                   d3 = in1 + 48, drain = in1 + 56;
-    uint32_t *tmem_slot = (uint32_t *)(bars + 8);
+                   d3 = in1 + 48, drain = in1 + 56, wbar = in1 + 64;
+    uint32_t *tmem_slot = (uint32_t *)(bars + 9);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tiles = (g.M + MM_BM - 1) / MM_BM;
     const int k2 = g.n2 / 64;  // chunks of the first product
@@ -92,6 +116,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1) k_mlp_bwd(const __grid_constant
         mbar_init(d2b, 1);
         mbar_init(d3, 1);
         mbar_init(drain, 1);
+        mbar_init(wbar, MB_THREADS);
         mbar_fence_init();
     }
     if (warp == MB_WARPS) {
@@ -109,11 +134,10 @@ __global__ void __launch_bounds__(MB_THREADS, 1) k_mlp_bwd(const __grid_constant
             }
         }
     }
-    cp_async_commit();
-    cp_async_wait_all();
     fence_async_smem();
     tmem_fence_before();
     __syncthreads();
+    cp_async_arrive_noinc(wbar);  // only the MMA warp waits for the weights
     tmem_fence_after();
     const uint32_t tmem = *tmem_slot;
     bool bad = false;
@@ -130,6 +154,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1) k_mlp_bwd(const __grid_constant
             umma_commit(done);
         };
         int i = 0;
+        bad = !warp_wait(wbar, 0);
         for (int t = blockIdx.x; t < tiles && !bad; t += gridDim.x, ++i) {
             if (!warp_wait(in1, i & 1)) {
                 bad = true;
@@ -160,74 +185,82 @@ __global__ void __launch_bounds__(MB_THREADS, 1) k_mlp_bwd(const __grid_constant
         if (issuer) umma_commit(drain);
         (void)warp_wait(drain, 0);
     } else {
-        // thread = one row, 64 of its 128 columns
-        const int quad = warp & 3, half = warp >> 2;
-        const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
-        const int col = half * 64;
+        // lane = rows gq + 8 i (i < 4) of its warp's 32, 32 of the 128 columns;
+        // in memory eight consecutive ones from 8 fq, so that four lanes cover
+        // a row's whole 128-byte line
+        const int quad = warp & 3, col = (warp >> 2) * 32, gq = lane >> 2, fq = lane & 3, mine = col + 8 * fq;
+        const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16), operand = lanes + 384u + (uint32_t)(col / 2);
         auto hand_over = [&](uint32_t bar) {  // this warp's operand columns are written
             tmem_wait_st();
             tmem_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar);
         };
+        auto pack_row = [](const uint32_t (&x)[8]) {
+            return make_uint4(pack_bf16x2(__uint_as_float(x[0]), __uint_as_float(x[1])),
+                              pack_bf16x2(__uint_as_float(x[2]), __uint_as_float(x[3])),
+                              pack_bf16x2(__uint_as_float(x[4]), __uint_as_float(x[5])),
+                              pack_bf16x2(__uint_as_float(x[6]), __uint_as_float(x[7])));
+        };
         int i = 0;
         for (int t = blockIdx.x; t < tiles && !bad; t += gridDim.x, ++i) {
-            const int r = t * MM_BM + quad * 32 + lane;
-            const bool in = r < g.M;
-            int rs = 0, deg = 0;
-            if (MODE == 2 && in) {
-                rs = g.start[r];
-                deg = g.start[r + 1] - rs;
-            }
-            // dy -> bf16
-            if (g.dy) {
-                if (col < g.n2) {
+            const int r0 = t * MM_BM + quad * 32 + gq;
+            auto in = [&](int k) { return r0 + 8 * k < g.M; };
+            auto at = [&](int k) { return (int64_t)(r0 + 8 * k) * MF_H + mine; };
+            int rs[4], deg[4];
+            if (MODE == 2) {
 #pragma unroll
-                    for (int hh = 0; hh < 2; ++hh) {
-                        float x[32];
-                        uint32_t w[16];
-#pragma unroll
-                        for (int u = 0; u < 32; ++u) x[u] = 0.0f;
-                        if (in) {
-#pragma unroll
-                            for (int u = 0; u < 32; u += 8) ld8f(g.dy + (int64_t)r * g.ldy + col + hh * 32 + u, x + u);
-                        }
-#pragma unroll
-                        for (int u = 0; u < 16; ++u) w[u] = pack_bf16x2(x[2 * u], x[2 * u + 1]);
-                        if (in) {
-                            __nv_bfloat16 *p = g.dz2 + (int64_t)r * g.n2 + col + hh * 32;
-                            st8u(p, w);
-                            st8u(p + 16, w + 8);
-                        }
-                        __syncwarp();
-                        tmem_st16(lanes + 384u + (uint32_t)(half * 32 + hh * 16), w);
+                for (int k = 0; k < 4; ++k) {
+                    rs[k] = deg[k] = 0;
+                    if (in(k)) {
+                        rs[k] = g.start[r0 + 8 * k];
+                        deg[k] = g.start[r0 + 8 * k + 1] - rs[k];
                     }
                 }
-            } else {
+            }
+            // dy -> bf16
+            if (col < g.n2) {  // (uniform over the warp)
+                uint4 y[4];
+                if (g.dy) {
+                    float x[4][8];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) x[k][u] = 0.0f;
+                        if (in(k)) ld8f(g.dy + (int64_t)(r0 + 8 * k) * g.ldy + mine, x[k]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        y[k] = make_uint4(pack_bf16x2(x[k][0], x[k][1]), pack_bf16x2(x[k][2], x[k][3]),
+                                          pack_bf16x2(x[k][4], x[k][5]), pack_bf16x2(x[k][6], x[k][7]));
+                        if (in(k)) *(uint4 *)(g.dz2 + (int64_t)(r0 + 8 * k) * g.n2 + mine) = y[k];
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        y[k] = make_uint4(0u, 0u, 0u, 0u);
+                        if (in(k)) y[k] = *(const uint4 *)(g.dyb + at(k));
+                    }
+                }
+                __syncwarp();
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
-                    uint32_t w[16];
+                    uint32_t w[8];
 #pragma unroll
-                    for (int u = 0; u < 16; ++u) w[u] = 0u;
-                    if (in) {
-                        const __nv_bfloat16 *p = g.dyb + (int64_t)r * MF_H + col + hh * 32;
-                        ld8u(p, w);
-                        ld8u(p + 16, w + 8);
-                    }
-                    __syncwarp();
-                    tmem_st16(lanes + 384u + (uint32_t)(half * 32 + hh * 16), w);
+                    for (int r = 0; r < 2; ++r) pairs_to_frag(y[2 * hh + r], r, fq, w);
+                    tmem_st_frag_pairs(operand + ((uint32_t)(hh * 16) << 16), w);
                 }
             }
             hand_over(in1);
             // dz1 = relu'(z) (dz2 W2)
             {
-                uint32_t zz[32];
+                uint4 z[4];
 #pragma unroll
-                for (int u = 0; u < 32; ++u) zz[u] = 0u;
-                if (in) {
-#pragma unroll
-                    for (int u = 0; u < 32; u += 8) ld8u(g.z + (int64_t)r * MF_H + col + 2 * u, zz + u);
+                for (int k = 0; k < 4; ++k) {
+                    z[k] = make_uint4(0u, 0u, 0u, 0u);
+                    if (in(k)) z[k] = *(const uint4 *)(g.z + at(k));
                 }
+                __syncwarp();
                 if (!warp_wait(d1, i & 1)) {
                     bad = true;
                     break;
@@ -235,25 +268,33 @@ __global__ void __launch_bounds__(MB_THREADS, 1) k_mlp_bwd(const __grid_constant
                 tmem_fence_after();
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
-                    uint32_t v[32], w[16];
-                    tmem_ld32(lanes + (uint32_t)(col + hh * 32), v);
-                    float x[32];
+                    const uint32_t half = (uint32_t)(hh * 16) << 16;
+                    uint32_t v[16], m[8], w[8];
+                    tmem_ld_frag32(lanes + half + (uint32_t)col, v);
 #pragma unroll
-                    for (int u = 0; u < 16; ++u) {
-                        const uint32_t m = positive_mask(zz[hh * 16 + u]);
-                        x[2 * u] = (m & 0xffffu) ? __uint_as_float(v[2 * u]) : 0.0f;
-                        x[2 * u + 1] = (m >> 16) ? __uint_as_float(v[2 * u + 1]) : 0.0f;
-                        w[u] = pack_bf16x2(x[2 * u], x[2 * u + 1]);
+                    for (int r = 0; r < 2; ++r) {
+                        const uint4 zz = z[2 * hh + r];
+                        pairs_to_frag(make_uint4(positive_mask(zz.x), positive_mask(zz.y), positive_mask(zz.z), positive_mask(zz.w)),
+                                      r, fq, m);
                     }
-                    if (in) {
-                        const int64_t at = (int64_t)r * MF_H + col + hh * 32;
-                        st8u(g.dz1 + at, w);
-                        st8u(g.dz1 + at + 16, w + 8);
 #pragma unroll
-                        for (int u = 0; u < 32; u += 8) st8f(g.dz1f + at + u, x + u);
+                    for (int j = 0; j < 8; ++j) {  // word j: columns 8 (j / 2) + 2 fq, + 1 of row j & 1
+                        const int a = 4 * (j >> 1) + 2 * (j & 1);
+                        v[a] = (m[j] & 0xffffu) ? v[a] : 0u;
+                        v[a + 1] = (m[j] >> 16) ? v[a + 1] : 0u;
+                        w[j] = pack_bf16x2(__uint_as_float(v[a]), __uint_as_float(v[a + 1]));
                     }
-                    __syncwarp();
-                    if (MODE > 0) tmem_st16(lanes + 384u + (uint32_t)(half * 32 + hh * 16), w);
+                    if (MODE > 0) tmem_st_frag_pairs(operand + half, w);
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        uint32_t x[8];
+                        frag_to_row(v, r, fq, x);
+                        if (in(2 * hh + r)) {
+                            *(uint4 *)(g.dz1 + at(2 * hh + r)) = pack_row(x);
+                            st8u(g.dz1f + at(2 * hh + r), x);
+                        }
+                        __syncwarp();
+                    }
                 }
             }
             if (MODE == 0) {
@@ -270,55 +311,80 @@ __global__ void __launch_bounds__(MB_THREADS, 1) k_mlp_bwd(const __grid_constant
                 tmem_fence_after();
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
-                    uint32_t v[32], w[16];
-                    tmem_ld32(lanes + 128u + (uint32_t)(col + hh * 32), v);
+                    const uint32_t half = (uint32_t)(hh * 16) << 16;
+                    uint32_t v[16], w[8];
+                    tmem_ld_frag32(lanes + half + 128u + (uint32_t)col, v);
 #pragma unroll
-                    for (int u = 0; u < 16; ++u) w[u] = pack_bf16x2(__uint_as_float(v[2 * u]), __uint_as_float(v[2 * u + 1]));
-                    if (in) {
-                        const int64_t at = (int64_t)r * MF_H + col + hh * 32;
-                        st8u(g.dagg + at, w);
-                        st8u(g.dagg + at + 16, w + 8);
-                        float x[32];
-#pragma unroll
-                        for (int u = 0; u < 32; ++u) x[u] = __uint_as_float(v[u]) * (float)deg;
-#pragma unroll
-                        for (int u = 0; u < 32; u += 8) st8f(g.daggf + at + u, x + u);
+                    for (int j = 0; j < 8; ++j) {
+                        const int a = 4 * (j >> 1) + 2 * (j & 1);
+                        w[j] = pack_bf16x2(__uint_as_float(v[a]), __uint_as_float(v[a + 1]));
                     }
-                    __syncwarp();
-                    tmem_st16(lanes + 448u + (uint32_t)(half * 32 + hh * 16), w);
+                    tmem_st_frag_pairs(operand + 64u + half, w);
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        const int k = 2 * hh + r;
+                        uint32_t x[8];
+                        frag_to_row(v, r, fq, x);
+                        if (in(k)) {
+                            *(uint4 *)(g.dagg + at(k)) = pack_row(x);
+#pragma unroll
+                            for (int u = 0; u < 8; ++u) x[u] = __float_as_uint(__uint_as_float(x[u]) * (float)deg[k]);
+                            st8u(g.daggf + at(k), x);
+                        }
+                        __syncwarp();
+                    }
                 }
                 hand_over(in3);
             }
             // dx (a layer: on top of dy, the residual's share)
-            float o[32];
+            {
+                float o[4][8];
+                if (MODE == 2) {
 #pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                if (MODE == 2 && in) {
-#pragma unroll
-                    for (int u = 0; u < 32; u += 8) ld8f(g.dy + (int64_t)r * g.ldy + col + hh * 32 + u, o + u);
+                    for (int k = 0; k < 4; ++k)
+                        if (in(k)) ld8f(g.dy + (int64_t)(r0 + 8 * k) * g.ldy + mine, o[k]);
+                    __syncwarp();
                 }
-                if (hh == 0) {
-                    if (!warp_wait(d2b, i & 1)) {
-                        bad = true;
-                        break;
+                if (!warp_wait(d2b, i & 1)) {
+                    bad = true;
+                    break;
+                }
+                tmem_fence_after();
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    uint32_t v[16];
+                    tmem_ld_frag32(lanes + ((uint32_t)(hh * 16) << 16) + 256u + (uint32_t)col, v);
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        const int k = 2 * hh + r;
+                        uint32_t x[8];
+                        frag_to_row(v, r, fq, x);
+                        if (in(k)) {
+                            if (MODE == 2) {
+#pragma unroll
+                                for (int u = 0; u < 8; ++u) x[u] = __float_as_uint(o[k][u] + __uint_as_float(x[u]));
+                            }
+                            st8u(g.dx + at(k), x);
+                        }
+                        __syncwarp();
                     }
-                    tmem_fence_after();
                 }
-                __syncwarp();
-                uint32_t v[32];
-                tmem_ld32(lanes + 256u + (uint32_t)(col + hh * 32), v);
-                if (in) {
-                    float x[32];
-#pragma unroll
-                    for (int u = 0; u < 32; ++u) x[u] = MODE == 2 ? o[u] + __uint_as_float(v[u]) : __uint_as_float(v[u]);
-#pragma unroll
-                    for (int u = 0; u < 32; u += 8) st8f(g.dx + (int64_t)r * MF_H + col + hh * 32 + u, x + u);
-                }
-                __syncwarp();
             }
-            if (bad) break;
             if (MODE == 2) {
                 // dz_e of the cell's edges
+                uint4 z[2][3];  // all the hidden activations of two rows' edges in flight
+                auto fetch = [&](int hh) {
+#pragma unroll
+                    for (int r = 0; r < 2; ++r)
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) {
+                            z[r][k] = make_uint4(0u, 0u, 0u, 0u);
+                            if (k < deg[2 * hh + r])
+                                z[r][k] = *(const uint4 *)(g.z1e + (int64_t)(rs[2 * hh + r] + k) * MF_H + mine);
+                        }
+                    __syncwarp();
+                };
+                fetch(0);
                 if (!warp_wait(d3, i & 1)) {
                     bad = true;
                     break;
@@ -326,53 +392,47 @@ __global__ void __launch_bounds__(MB_THREADS, 1) k_mlp_bwd(const __grid_constant
                 tmem_fence_after();
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
-                    uint32_t v[32], w[16];
-                    tmem_ld32(lanes + (uint32_t)(col + hh * 32), v);
+                    uint32_t v[16];
+                    tmem_ld_frag32(lanes + ((uint32_t)(hh * 16) << 16) + (uint32_t)col, v);
+                    if (hh == 1) fetch(1);
 #pragma unroll
-                    for (int u = 0; u < 16; ++u) w[u] = pack_bf16x2(__uint_as_float(v[2 * u]), __uint_as_float(v[2 * u + 1]));
-                    if (in) {
+                    for (int r = 0; r < 2; ++r) {
+                        const int n = 2 * hh + r;
+                        uint32_t x[8];
+                        frag_to_row(v, r, fq, x);
+                        const uint4 w = pack_row(x);
+                        if (in(n)) st8u(g.gf + at(n), x);
 #pragma unroll
-                        for (int u = 0; u < 32; u += 8) st8u(g.gf + (int64_t)r * MF_H + col + hh * 32 + u, v + u);
-                    }
-                    uint32_t m[3][16];
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) {  // all three edges' hidden activations in flight
-                        if (k < deg) {
-                            const int64_t at = (int64_t)(rs + k) * MF_H + col + hh * 32;
-                            ld8u(g.z1e + at, m[k]);
-                            ld8u(g.z1e + at + 16, m[k] + 8);
-                        }
-                    }
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        if (k < deg) {
-                            const int64_t at = (int64_t)(rs + k) * MF_H + col + hh * 32;
-                            uint32_t bits = 0u;
-#pragma unroll
-                            for (int u = 0; u < 16; ++u) {
-                                const uint32_t p = positive_mask(m[k][u]);
-                                bits |= (p & 1u) << (2 * u) | (p >> 31) << (2 * u + 1);
-                                m[k][u] = p & w[u];
+                        for (int k = 0; k < 3; ++k) {
+                            const uint4 p = make_uint4(positive_mask(z[r][k].x), positive_mask(z[r][k].y),
+                                                       positive_mask(z[r][k].z), positive_mask(z[r][k].w));
+                            uint32_t bits = (p.x & 1u) | (p.x >> 31) << 1 | (p.y & 1u) << 2 | (p.y >> 31) << 3 |
+                                            (p.z & 1u) << 4 | (p.z >> 31) << 5 | (p.w & 1u) << 6 | (p.w >> 31) << 7;
+                            bits <<= 8 * fq;
+                            bits |= __shfl_xor_sync(0xffffffffu, bits, 1);
+                            bits |= __shfl_xor_sync(0xffffffffu, bits, 2);
+                            if (k < deg[n]) {
+                                const int64_t e = rs[n] + k;
+                                if (fq == 0) g.bits[e * 4 + col / 32] = bits;
+                                *(uint4 *)(g.dze + e * MF_H + mine) = make_uint4(p.x & w.x, p.y & w.y, p.z & w.z, p.w & w.w);
                             }
-                            g.bits[(int64_t)(rs + k) * 4 + (col + hh * 32) / 32] = bits;
-                            st8u(g.dze + at, m[k]);
-                            st8u(g.dze + at + 16, m[k] + 8);
                         }
+                        __syncwarp();
                     }
-                    __syncwarp();
                 }
             }
             tmem_fence_before();
         }
     }
     if (bad) atomicCAS(g.error, 0, FL_E_TIMEOUT);
+    cp_async_wait_all();
     tmem_fence_before();
     __syncthreads();
     if (warp == MB_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
 }
 
 // ------------------------------------------------------------- edge input gradients
-constexpr int EB_PROD = 2, EB_EPI = 8, EB_THREADS = 32 * (EB_PROD + 1 + EB_EPI);
+constexpr int EB_PROD = 2, EB_EPI = 16, EB_THREADS = 32 * (EB_PROD + 1 + EB_EPI);
 constexpr int EB_RING = 9;
 constexpr int EB_SMEM = (4 + EB_RING) * MM_CHUNK_BYTES + 512 + 1024;
 
@@ -394,8 +454,8 @@ __global__ void __launch_bounds__(EB_THREADS, 1) k_edge_bwd(const __grid_constan
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t sW = smem_addr(smem), sR = sW + 4 * MM_CHUNK_BYTES;
     uint64_t *bars = (uint64_t *)(smem + (4 + EB_RING) * MM_CHUNK_BYTES);
-    const uint32_t ringf = smem_addr(bars), ringe = ringf + 8 * EB_RING, df = ringe + 8 * EB_RING, de = df + 32, drain = de + 32;
-    uint32_t *tmem_slot = (uint32_t *)(bars + 2 * EB_RING + 4 + 4 + 1);
+    const uint32_t ringf = smem_addr(bars), ringe = ringf + 8 * EB_RING, df = ringe + 8 * EB_RING, de = df + 32, drain = de + 32, wbar = drain + 8;
+    uint32_t *tmem_slot = (uint32_t *)(bars + 2 * EB_RING + 4 + 4 + 2);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tiles = (g.C + MM_BM - 1) / MM_BM;
     if (tid == 0) {
@@ -408,6 +468,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1) k_edge_bwd(const __grid_constan
             mbar_init(de + 8 * k, EB_EPI);
         }
         mbar_init(drain, 1);
+        mbar_init(wbar, EB_THREADS);
         mbar_fence_init();
     }
     if (warp == EB_PROD) {
@@ -417,11 +478,10 @@ __global__ void __launch_bounds__(EB_THREADS, 1) k_edge_bwd(const __grid_constan
     }
     for (int c = 0; c < 4; ++c)  // chunk = 64 K columns of 128 rows: receiver part 0, 1, sender part 0, 1
         load_weight_chunk(g.w1t + (c >> 1) * MF_H * g.ldw1t, g.ldw1t, MF_H, c & 1, sW + c * MM_CHUNK_BYTES, tid, EB_THREADS);
-    cp_async_commit();
-    cp_async_wait_all();
     fence_async_smem();
     tmem_fence_before();
     __syncthreads();
+    cp_async_arrive_noinc(wbar);  // only the MMA warp waits for the weights
     tmem_fence_after();
     const uint32_t tmem = *tmem_slot;
     bool bad = false;
@@ -493,6 +553,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1) k_edge_bwd(const __grid_constan
         const bool issuer = elect_one();
         const uint32_t idesc = umma_idesc_bf16_128x128();
         int q = 0, m = 0;
+        bad = !warp_wait(wbar, 0);
         for (int t = blockIdx.x; t < tiles && !bad; t += gridDim.x) {
             for (int p = 0; p < 6 && !bad; ++p, ++m) {
                 const int reg = m & 3;
@@ -524,22 +585,26 @@ __global__ void __launch_bounds__(EB_THREADS, 1) k_edge_bwd(const __grid_constan
         if (issuer) umma_commit(drain);
         (void)warp_wait(drain, 0);
     } else {
-        // thread = one cell, 64 of its 128 columns
-        const int quad = warp & 3, half = (warp - EB_PROD - 1) >> 2;
-        const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * 64);
+        // lane = rows gq + 8 i of its warp's 32, 32 of the 128 columns
+        const int quad = warp & 3, col = ((warp - EB_PROD - 1) >> 2) * 32, gq = lane >> 2, fq = lane & 3;
+        const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)col;
         int m = 0;
         for (int t = blockIdx.x; t < tiles && !bad; t += gridDim.x) {
-            const int c = t * MM_BM + quad * 32 + lane;
-            const bool in = c < g.C;
-            int deg = 0, sdeg = 0;
-            float tot[64], acc[64];
-            float *row = g.dh + (int64_t)c * MF_H + half * 64;
-            if (in) {
-                deg = g.start[c + 1] - g.start[c];
-                sdeg = g.send_start[c + 1] - g.send_start[c];
+            const int c0 = t * MM_BM + quad * 32 + gq;
+            float *row = g.dh + (int64_t)c0 * MF_H + col + 8 * fq;
+            int deg[4];           // incoming edges, outgoing ones << 16
+            float acc[32];        // [i][j][2], fragment order
+            uint32_t tot[4][8];   // the rows' eight columns from 8 fq
 #pragma unroll
-                for (int u = 0; u < 64; u += 8) ld8f(row + u, tot + u);
+            for (int k = 0; k < 4; ++k) {
+                deg[k] = 0;
+                if (c0 + 8 * k < g.C) {
+                    const int c = c0 + 8 * k;
+                    deg[k] = (g.start[c + 1] - g.start[c]) | (g.send_start[c + 1] - g.send_start[c]) << 16;
+                    ld8u(row + 8 * k * MF_H, tot[k]);
+                }
             }
+            __syncwarp();
 #pragma unroll
             for (int p = 0; p < 6; ++p, ++m) {
                 if (!warp_wait(df + 8 * (m & 3), (m >> 2) & 1)) {
@@ -547,33 +612,46 @@ __global__ void __launch_bounds__(EB_THREADS, 1) k_edge_bwd(const __grid_constan
                     break;
                 }
                 tmem_fence_after();
-                const bool valid = p < 3 ? p < deg : p - 3 < sdeg;
 #pragma unroll
-                for (int b = 0; b < 4; ++b) {
+                for (int hh = 0; hh < 2; ++hh) {
                     uint32_t v[16];
-                    tmem_ld16(base + 128u * (m & 3) + 16u * b, v);
-                    if (b == 3) {
+                    tmem_ld_frag32(base + ((uint32_t)(hh * 16) << 16) + 128u * (m & 3), v);
+                    if (hh == 1) {
                         tmem_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(de + 8 * (m & 3));
                     }
 #pragma unroll
-                    for (int u = 0; u < 16; ++u) {
-                        const float a = (p == 0 || p == 3) ? 0.0f : acc[b * 16 + u];
-                        acc[b * 16 + u] = valid ? a + __uint_as_float(v[u]) : a;
-                        if (p == 2 || p == 5) tot[b * 16 + u] = acc[b * 16 + u] + tot[b * 16 + u];
+                    for (int r = 0; r < 2; ++r) {
+                        const int k = 2 * hh + r;
+                        const bool valid = p < 3 ? p < (deg[k] & 0xffff) : p - 3 < (deg[k] >> 16);
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            const float a = (p == 0 || p == 3) ? 0.0f : acc[8 * k + u];
+                            acc[8 * k + u] = valid ? a + __uint_as_float(v[4 * (u >> 1) + 2 * r + (u & 1)]) : a;
+                        }
+                        if (p == 2 || p == 5) {
+                            uint32_t x[8];
+#pragma unroll
+                            for (int u = 0; u < 8; ++u) x[u] = __float_as_uint(acc[8 * k + u]);
+                            transpose4(x[0], x[2], x[4], x[6], fq);
+                            transpose4(x[1], x[3], x[5], x[7], fq);
+#pragma unroll
+                            for (int u = 0; u < 8; ++u)
+                                tot[k][u] = __float_as_uint(__uint_as_float(x[u]) + __uint_as_float(tot[k][u]));
+                        }
                     }
                 }
             }
             if (bad) break;
-            if (in) {
 #pragma unroll
-                for (int u = 0; u < 64; u += 8) st8f(row + u, tot + u);
-            }
+            for (int k = 0; k < 4; ++k)
+                if (c0 + 8 * k < g.C) st8u(row + 8 * k * MF_H, tot[k]);
             __syncwarp();
         }
     }
     if (bad) atomicCAS(g.error, 0, FL_E_TIMEOUT);
+    cp_async_wait_all();
     tmem_fence_before();
     __syncthreads();
     if (warp == EB_PROD) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
@@ -997,13 +1075,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad(const __grid_constant__
 #pragma unroll
                     for (int r = 0; r < 2; ++r) {
                         uint32_t x[8];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            x[2 * j] = v[4 * j + 2 * r];
-                            x[2 * j + 1] = v[4 * j + 2 * r + 1];
-                        }
-                        transpose4(x[0], x[2], x[4], x[6], fq);
-                        transpose4(x[1], x[3], x[5], x[7], fq);
+                        frag_to_row(v, r, fq, x);
                         const int row = quad * 32 + gq + 8 * (2 * hh + r);
                         if (row < rows) st8u(out + (int64_t)row * n_in + cb, x);
                         __syncwarp();
