@@ -69,6 +69,9 @@ cudaError_t launch_surcharge(const SurchargeArgs &a, int slot, cudaStream_t stre
 cudaError_t launch_li(const LiArgs &a, int kind, int slot, int plan_next, int sms, cudaStream_t stream);
 int li_cell_blocks(int32_t C);
 cudaError_t plan_li_tiles(LiTileArgs &a, int kind, int device, int *grid, int *smem_bytes);
+cudaError_t plan_surface_run(const SurfArgs &a, int kind, int device, int *smem_bytes, size_t *sync_words);
+cudaError_t launch_surface_run(const SurfArgs &a, int kind, uint32_t *sync, int slot, int steps, int smem_bytes,
+                               cudaStream_t stream);
 cudaError_t launch_li_tiles(const LiTileArgs &a, int kind, int slot, int plan_next, int grid, int smem_bytes,
                             cudaStream_t stream);
 int node_blocks(int32_t N);
@@ -142,6 +145,16 @@ struct FlSolver {
     bool li_mode = false;     // surface_step_mode = local_inertial
     LiTileArgs lt{};          // its tiles (lt_grid 0: the two launches over edges and cells)
     int lt_grid = 0, lt_smem = 0;
+    int run_smem = 0;         // k_surface_run's (0: a launch a step)
+    uint32_t *run_sync = nullptr;
+    // a run's steps up to the next CFL evaluation in one launch: the surface alone, one member
+    bool run_kernel() const {
+        return run_smem > 0 && members == 1 && !li_mode && !has_inflow() && !has_drain() && !has_table() && !has_recharge();
+    }
+    int launches_per_chunk() const {
+        const int interval = params.cfl_update_interval_steps, evals = (chunk + interval - 1) / interval;
+        return run_kernel() ? 2 * evals : chunk * launches_per_step() + members * evals;
+    }
     int surface_launches() const { return li_mode && !lt_grid ? 2 : 1; }
     int sms = 1;
     SurchargeArgs sur{};
@@ -368,7 +381,13 @@ static int capture_graph(FlSolver *s) {
     FL_CUDA(cudaStreamBeginCapture(s->cap_stream, cudaStreamCaptureModeThreadLocal));
     const int interval = s->params.cfl_update_interval_steps;
     int rc = FL_OK;
-    for (int j = 0; j < s->chunk && rc == FL_OK; ++j) {
+    for (int j = 0; j < s->chunk && rc == FL_OK && s->run_kernel(); j += interval) {
+        cudaError_t e = launch_dt(dt_args(s, 0), s->dt_blocks, j & 1, 1, s->cap_stream);
+        if (e == cudaSuccess) e = launch_surface_run(s->sa, s->kind, s->run_sync, j & 1, interval, s->run_smem, s->cap_stream);
+        g_launches += 2;
+        if (e != cudaSuccess) rc = set_error(FL_E_CUDA, "launch_surface_run: %s", cudaGetErrorString(e));
+    }
+    for (int j = 0; j < s->chunk && rc == FL_OK && !s->run_kernel(); ++j) {
         const bool eval = (j % interval) == 0;
         const bool next_eval = ((j + 1) % interval) == 0;
         rc = launch_step(s, j & 1, eval, !next_eval, s->cap_stream);
@@ -384,7 +403,7 @@ static int capture_graph(FlSolver *s) {
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return set_error(FL_E_CUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(e));
     // the launches above were captured, not executed
-    g_launches -= (int64_t)s->chunk * s->launches_per_step() + (int64_t)s->members * ((s->chunk + interval - 1) / interval);
+    g_launches -= s->launches_per_chunk();
     return FL_OK;
 }
 
@@ -602,6 +621,19 @@ static int build_li_tiles(FlSolver *s, const HostLayout &L, const std::vector<in
     return FL_OK;
 }
 
+// Every tile whose cells a tile reads reads cells of that tile.
+static bool halos_mutual(const HostLayout &L) {
+    std::vector<std::pair<int32_t, int32_t>> reads;
+    for (size_t t = 0; t < L.tile_info.size(); ++t)
+        for (int32_t j = 0; j < L.tile_info[t].w; ++j)
+            reads.emplace_back((int32_t)t, L.halo_src[(size_t)L.tile_info[t].z + j] / TILE);
+    std::sort(reads.begin(), reads.end());
+    reads.erase(std::unique(reads.begin(), reads.end()), reads.end());
+    for (const auto &r : reads)
+        if (!std::binary_search(reads.begin(), reads.end(), std::make_pair(r.second, r.first))) return false;
+    return true;
+}
+
 // forcings: M entries (the members' rainfall); the per-cell fields come from
 // forcings[0].
 static int create_impl(const FlMeshDesc *mesh, const FlDrainDesc *drain, const FlForcingDesc *forcings, int32_t M,
@@ -731,6 +763,16 @@ static int create_impl(const FlMeshDesc *mesh, const FlDrainDesc *drain, const F
     s->li_mode = p.surface_step_mode == 1;
     // the surface ledger: per warp of the surface kernel (or of the local-inertial cell kernel)
     s->n_led_s = (size_t)std::max(surface_warps(s->surf_grid), s->li_mode ? li_cell_blocks(C) * 8 : 0) * SURF_TERMS;
+    // (a tile waits only for the tiles that it reads, so these have to read it too;
+    // with a few steps between CFL evaluations there is little to keep resident)
+    if (!s->li_mode && M == 1 && !drain && p.cfl_update_interval_steps >= 8 && halos_mutual(L)) {
+        size_t words = 0;
+        FL_CUDA(plan_surface_run(s->sa, s->kind, device, &s->run_smem, &words));
+        if (s->run_smem) {
+            if ((rc = s->alloc(&s->run_sync, words))) return rc;
+            FL_CUDA(cudaMemset(s->run_sync, 0, words * sizeof(uint32_t)));
+        }
+    }
     s->dt_blocks = std::max(1, std::min(sms * 4, (C + 255) / 256));
     float *dt_partial = nullptr;
     unsigned int *counter = nullptr;
@@ -1343,7 +1385,7 @@ static int run_members(FlSolver *s, double t_target_s, int64_t max_steps, cudaSt
     if (rc) return rc;
     int64_t launched = 0, last_total = -1;
     int stalled = 0;
-    const int per_chunk = s->chunk * s->launches_per_step() + M * ((s->chunk + interval - 1) / interval);
+    const int per_chunk = s->launches_per_chunk();
     while (true) {
         FL_CUDA(cudaGraphLaunch(s->graph, st));
         g_launches += per_chunk;
@@ -1424,7 +1466,7 @@ FL_API int fl_run(FlSolver *s, double t_target_s, int64_t max_steps, void *strea
     int64_t launched = 0;
     int64_t last_step = -1;
     int stalled = 0;
-    const int per_chunk = s->chunk * s->launches_per_step() + s->members * ((s->chunk + interval - 1) / interval);
+    const int per_chunk = s->launches_per_chunk();
     while (true) {
         FL_CUDA(cudaGraphLaunch(s->graph, st));
         g_launches += per_chunk;

@@ -325,6 +325,193 @@ __global__ void __launch_bounds__(SURF_THREADS, 4) k_surface(const __grid_consta
     warp_add_ledger_at<SURF_TERMS>(led, a.ledger + (MEM ? mem * (size_t)a.m_led : 0), (int)blockIdx.x * (TILE / 32) + (tid >> 5));
 }
 
+// Bounded poll: *p has reached v (serial numbers; they may wrap).
+__device__ __forceinline__ bool poll_reached(const uint32_t *p, uint32_t v) {
+    uint64_t t0 = 0;
+    for (int i = 0;; ++i) {
+        uint32_t x;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(p) : "memory");
+        if ((int32_t)(x - v) >= 0) return true;
+        if ((i & 63) == 63) {
+            if (t0 == 0) t0 = global_ns();
+            else if (global_ns() - t0 > COPY_WAIT_NS) return false;
+        }
+    }
+}
+
+__device__ __forceinline__ void publish(uint32_t *p, uint32_t v) {
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// `steps` steps of a run of the surface alone in one cooperative launch, a CTA a
+// tile: the tile's entries, halo list, cell data, wet time and own states stay in
+// shared memory and registers; per step a CTA waits for the steps of its
+// neighbours (a serial number per tile, release / acquire) and the step record,
+// reads the halo states through L2, and runs k_surface's two phases.  The last
+// CTA plans step k + 1 once every tile has finished step k - 1, as the planner of
+// k_surface does, and the ledger sums keep k_surface's slots and order: the same
+// bits, step by step.
+//
+// A launch a step costs a small mesh more than its work.  us a step with 32 (8)
+// steps between CFL evaluations, a launch a step -> here: 1,800 cells 5.4 -> 3.4
+// (6.0 -> 4.4), 20,000 cells 5.7 -> 4.8 (6.7 -> 5.5), 154,568 cells 8.7 -> 7.1
+// (9.6 -> 7.5); what is left is a chain of L2 round trips (serial numbers, halo
+// states, step record) and the two phases.
+//
+// sync: SYNC_STRIDE words a tile, then the planner's.  All of them hold the same
+// number between launches (each CTA ends at its first + steps, also when the run
+// ends early or a wait gives up), so nothing has to be reset.  Co-residency comes
+// from the cooperative launch; every wait is bounded.
+constexpr int SYNC_STRIDE = 8;      // words: a sector each
+constexpr int RUN_MAX_TILES = 1024;
+
+template <int KIND>
+__global__ void __launch_bounds__(TILE, 4) k_surface_run(const __grid_constant__ SurfArgs a, uint32_t *sync, int slot, int steps) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ StepCtrl s_ctrl;
+    __shared__ uint32_t s_near[RUN_MAX_TILES / 32];
+    float4 *s_flux = (float4 *)smem;
+    const uint32_t bar = smem_addr(smem + a.off_bar);
+    const int tid = threadIdx.x, tile = blockIdx.x, n_tiles = a.n_tiles;
+    uint32_t *mine = sync + (size_t)tile * SYNC_STRIDE;  // (the planner's: tile = n_tiles)
+    const uint32_t *planned = sync + (size_t)n_tiles * SYNC_STRIDE;
+    const uint32_t base = *mine;
+    if (tile == n_tiles) {
+        for (int k = 0; k < steps; ++k) {
+            bool ok = true;
+            if (k > 0)
+                for (int t = tid; t < n_tiles; t += TILE) ok = ok && poll_reached(sync + (size_t)t * SYNC_STRIDE, base + k);
+            if (!__syncthreads_and(ok)) {
+                if (tid == 0 && atomicCAS(&a.run->error, 0, FL_E_TIMEOUT) == 0) a.run->error_step = a.run->step;
+                break;
+            }
+            const int active = __ldcg(&a.ctrl[(slot + k) & 1].active);
+            if (tid == 0 && k + 1 < steps) {
+                plan_step(a.run, a.snap_t, a.hy, &a.ctrl[(slot + k + 1) & 1], false, 0.0f, FL_PHASE_ALL);
+                publish(mine, base + k + 1);
+            }
+            if (!active) break;  // (uniform; both records say so now)
+        }
+        __syncthreads();
+        if (tid == 0) publish(mine, base + steps);
+        return;
+    }
+    const StepCtrl first = a.ctrl[slot];
+    if (!first.active) {  // (uniform over the grid)
+        if (tid == 0) publish(mine, base + steps);
+        return;
+    }
+    const TileStage S = stage_at(a, smem, 0);
+    const int4 ti = a.tile_info[tile];
+    for (int i = tid; i < RUN_MAX_TILES / 32; i += TILE) s_near[i] = 0u;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) s_flux[tid * 3 + k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        mbar_fence_init();
+        mbar_arrive_expect_tx(bar, static_bytes<KIND>(ti) + step_bytes<KIND>());
+        issue_static<KIND>(a, S, ti, bar, tile);
+        issue_step<KIND>(first.parity ? a.state1 : a.state0, a.wet, S, bar, tile);
+    }
+    float2 total[SURF_TERMS];  // lane 0 of a warp: its ledger sums
+    float2 *ledger = a.ledger + (size_t)(tile * (TILE / 32) + (tid >> 5)) * SURF_TERMS;
+#pragma unroll
+    for (int j = 0; j < SURF_TERMS; ++j) total[j] = (tid & 31) == 0 ? ledger[j] : make_float2(0.0f, 0.0f);
+    __syncthreads();
+    bool ok = mbar_wait_bounded(bar, 0, COPY_WAIT_NS);
+    if (!ok) ok = mbar_wait_bounded(bar, 0, COPY_WAIT_NS);  // none may land after the CTA leaves
+    if (ok)
+        for (int j = tid; j < ti.w; j += TILE) {
+            const int t = S.hs[j] / TILE;
+            atomicOr(&s_near[t >> 5], 1u << (t & 31));
+        }
+    ok = __syncthreads_and(ok);
+    const int c = tile * TILE + tid;
+    const float4 ci = S.ci[tid];
+    const uint32_t info = __float_as_uint(ci.z);
+    float wt = 0.0f;
+    float4 hz = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+    if (KIND == 1) {
+        wt = S.wt[tid];
+        hz = S.hz[tid];
+    }
+    const float md = a.md;
+    for (int k = 0; k < steps; ++k) {
+        if (ok && k > 0) {
+            if (tid == TILE - 1) ok = poll_reached(planned, base + k);
+            for (int t = tid; t < n_tiles && ok; t += TILE)
+                if (s_near[t >> 5] >> (t & 31) & 1u) ok = poll_reached(sync + (size_t)t * SYNC_STRIDE, base + k);
+        }
+        if (!__syncthreads_and(ok)) {
+            if (tid == 0 && atomicCAS(&a.run->error, 0, FL_E_TIMEOUT) == 0) a.run->error_step = first.step + k;
+            break;
+        }
+        const bool odd = ((first.parity ^ k) & 1) != 0;
+        const float4 *in = odd ? a.state1 : a.state0;
+        float4 *out = odd ? a.state0 : a.state1;
+        for (int j = tid; j < ti.w; j += TILE) S.st[TILE + j] = __ldcg(in + S.hs[j]);
+        if (tid >= TILE - 32 && tid < TILE - 32 + (int)(sizeof(StepCtrl) / 16))
+            ((uint4 *)&s_ctrl)[tid - (TILE - 32)] = __ldcg((const uint4 *)&a.ctrl[(slot + k) & 1] + (tid - (TILE - 32)));
+        __syncthreads();
+        const StepCtrl s = s_ctrl;
+        if (!s.active) break;  // (uniform over the grid)
+        const float dt = s.dt_f;
+        const bool do_surface = (s.phases & FL_PHASE_SURFACE) != 0;
+        float led[SURF_TERMS] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (do_surface) {
+#pragma unroll 1
+            for (int e = tid; e < ti.y; e += TILE)
+                tile_entry(S.en[e], S.st, s_flux, a.g, a.half_g, md, a.stage, dt, led[2], led[3]);
+        }
+        __syncthreads();
+        if (c < a.C) {
+            const float4 st = S.st[tid];
+            if (s.check_finite && !isfinite(st.x)) {
+                if (atomicCAS(&a.run->error, 0, FL_E_NONFINITE) == 0) a.run->error_step = s.step;
+            }
+            float hn = 0.0f, hun = 0.0f, hvn = 0.0f;
+            if (!do_surface) {
+                hn = st.x; hun = st.y; hvn = st.z;
+            } else if (info & CELL_ACTIVE) {
+                const float rain = KIND == 1 ? s.rain_f * hz.w : s.rain_f;
+                const float infil = KIND == 1 ? hz.y + (hz.x - hz.y) * __expf(-hz.z * wt) : a.infil_scalar;
+                const CellNew u = cell_update(st, ci, &s_flux[tid * 3], dt, s.dtg_f, md, rain, infil);
+                hn = u.h; hun = u.hu; hvn = u.hv;
+                led[0] += u.rd * ci.x;
+                led[1] += u.id * ci.x;
+            }
+#pragma unroll
+            for (int j = 0; j < 3; ++j) s_flux[tid * 3 + j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (s.phases & FL_PHASE_CLAMP) clamp_velocity_exact(hn, hun, hvn, a.vmax);
+            const float4 u = make_float4(hn, hun, hvn, st.w);
+            out[c] = u;
+            S.st[tid] = u;
+            if (KIND == 1 && do_surface) wt = wt + dt * (float)(hn > md);
+            if (s.snap_slot >= 0) {
+                const size_t o = (size_t)s.snap_slot * (size_t)a.C + (size_t)c;
+                a.snap_h[o] = hn;
+                a.snap_hu[o] = hun;
+                a.snap_hv[o] = hvn;
+            }
+        }
+        __syncthreads();  // the tile's new states are stored
+        if (tid == 0) publish(mine, base + k + 1);
+#pragma unroll
+        for (int j = 0; j < SURF_TERMS; ++j) {
+            float x = led[j];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+            if ((tid & 31) == 0) ff_accumulate(&total[j], x);
+        }
+    }
+    if (KIND == 1 && c < a.C) a.wet[c] = wt;
+    if ((tid & 31) == 0) {
+#pragma unroll
+        for (int j = 0; j < SURF_TERMS; ++j) ledger[j] = total[j];
+    }
+    __syncthreads();
+    if (tid == 0) publish(mine, base + steps);
+}
 
 // Global CFL minimum over all cells; the last block plans the step.
 __global__ void __launch_bounds__(256) k_dt(const __grid_constant__ DtArgs a, int slot, int plan) {
@@ -547,6 +734,43 @@ cudaError_t plan_surface_launch(SurfArgs &a, int kind, int device, int *grid, in
     // the dependent may wait beside this grid while both fit twice over
     a.early = 2ll * *grid * std::max(a.members, 1) <= per_sm * sms ? 1 : 0;
     return cudaSuccess;
+}
+
+// Whether k_surface_run can run the mesh: every tile's CTA and the planner resident
+// at once (on 152 SMs up to 607 tiles, 155,000 cells).  *smem_bytes 0: it cannot.
+// sync_words: what it needs of zeroed memory.
+cudaError_t plan_surface_run(const SurfArgs &a, int kind, int device, int *smem_bytes, size_t *sync_words) {
+    const void *fn = kind ? (const void *)k_surface_run<1> : (const void *)k_surface_run<0>;
+    const int bytes = a.off_stage + a.stage_bytes;
+    *smem_bytes = 0;
+    *sync_words = (size_t)(a.n_tiles + 1) * SYNC_STRIDE;
+    int per_sm = 0, sms = 0, most = 0, coop = 0;
+    cudaError_t e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    cudaFuncAttributes at{};
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, fn);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)at.sharedSizeBytes);
+    if (e != cudaSuccess || !coop || bytes > most - (int)at.sharedSizeBytes) return e;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, TILE, (size_t)bytes);
+    if (e == cudaSuccess && a.n_tiles + 1 <= per_sm * sms && a.n_tiles <= RUN_MAX_TILES) *smem_bytes = bytes;
+    return e;
+}
+
+cudaError_t launch_surface_run(const SurfArgs &a, int kind, uint32_t *sync, int slot, int steps, int smem_bytes,
+                               cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)a.n_tiles + 1);
+    cfg.blockDim = dim3(TILE);
+    cfg.dynamicSmemBytes = (size_t)smem_bytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return kind ? cudaLaunchKernelEx(&cfg, k_surface_run<1>, a, sync, slot, steps)
+                : cudaLaunchKernelEx(&cfg, k_surface_run<0>, a, sync, slot, steps);
 }
 
 int surface_warps(int grid) { return grid * (TILE / 32); }
