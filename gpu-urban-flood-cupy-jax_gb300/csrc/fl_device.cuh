@@ -354,7 +354,7 @@ static __device__ __noinline__ void plan_step(RunCtrl *run, double *snap_t, cons
             return;
         }
         s.snap_slot = run->snap_count;
-        snap_t[run->snap_count] = te;
+        if (snap_t) snap_t[run->snap_count] = te;  // (nullptr: another block keeps the times)
         run->snap_count += 1;
         run->next_snap_t += run->snap_interval;
     }

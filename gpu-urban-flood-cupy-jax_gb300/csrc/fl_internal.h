@@ -226,6 +226,14 @@ struct LiArgs {
     float infil_scalar, g, md, vmax;
 };
 
+// What the tiles of a run in one launch exchange (k_surface_run).
+struct RunArgs {
+    uint32_t *serial;        // steps done: a word per tile, then the planner's (a sector each)
+    const uint32_t *sent;    // a bit per cell: another tile's halo cell
+    float4 *exchange;        // [2 x cells] {h, hu, hv, serial number}
+    int32_t cells;           // whole tiles
+};
+
 // The local-inertial step over surface tiles (one launch).  A tile's local
 // indices: its own cells 0 .. TILE - 1, then the cells across its active
 // interior edges (ring 1), then those across ring 1's other such edges (ring 2).

@@ -69,8 +69,8 @@ cudaError_t launch_surcharge(const SurchargeArgs &a, int slot, cudaStream_t stre
 cudaError_t launch_li(const LiArgs &a, int kind, int slot, int plan_next, int sms, cudaStream_t stream);
 int li_cell_blocks(int32_t C);
 cudaError_t plan_li_tiles(LiTileArgs &a, int kind, int device, int *grid, int *smem_bytes);
-cudaError_t plan_surface_run(const SurfArgs &a, int kind, int device, int *smem_bytes, size_t *sync_words);
-cudaError_t launch_surface_run(const SurfArgs &a, int kind, uint32_t *sync, int slot, int steps, int smem_bytes,
+cudaError_t plan_surface_run(const SurfArgs &a, int kind, int device, int *smem_bytes, size_t *serial_words);
+cudaError_t launch_surface_run(const SurfArgs &a, int kind, const RunArgs &x, int slot, int steps, int smem_bytes,
                                cudaStream_t stream);
 cudaError_t launch_li_tiles(const LiTileArgs &a, int kind, int slot, int plan_next, int grid, int smem_bytes,
                             cudaStream_t stream);
@@ -146,7 +146,7 @@ struct FlSolver {
     LiTileArgs lt{};          // its tiles (lt_grid 0: the two launches over edges and cells)
     int lt_grid = 0, lt_smem = 0;
     int run_smem = 0;         // k_surface_run's (0: a launch a step)
-    uint32_t *run_sync = nullptr;
+    RunArgs run_args{};
     // a run's steps up to the next CFL evaluation in one launch: the surface alone, one member
     bool run_kernel() const {
         return run_smem > 0 && members == 1 && !li_mode && !has_inflow() && !has_drain() && !has_table() && !has_recharge();
@@ -383,7 +383,7 @@ static int capture_graph(FlSolver *s) {
     int rc = FL_OK;
     for (int j = 0; j < s->chunk && rc == FL_OK && s->run_kernel(); j += interval) {
         cudaError_t e = launch_dt(dt_args(s, 0), s->dt_blocks, j & 1, 1, s->cap_stream);
-        if (e == cudaSuccess) e = launch_surface_run(s->sa, s->kind, s->run_sync, j & 1, interval, s->run_smem, s->cap_stream);
+        if (e == cudaSuccess) e = launch_surface_run(s->sa, s->kind, s->run_args, j & 1, interval, s->run_smem, s->cap_stream);
         g_launches += 2;
         if (e != cudaSuccess) rc = set_error(FL_E_CUDA, "launch_surface_run: %s", cudaGetErrorString(e));
     }
@@ -764,13 +764,28 @@ static int create_impl(const FlMeshDesc *mesh, const FlDrainDesc *drain, const F
     // the surface ledger: per warp of the surface kernel (or of the local-inertial cell kernel)
     s->n_led_s = (size_t)std::max(surface_warps(s->surf_grid), s->li_mode ? li_cell_blocks(C) * 8 : 0) * SURF_TERMS;
     // (a tile waits only for the tiles that it reads, so these have to read it too;
-    // with a few steps between CFL evaluations there is little to keep resident)
-    if (!s->li_mode && M == 1 && !drain && p.cfl_update_interval_steps >= 8 && halos_mutual(L)) {
+    // with a few steps between CFL evaluations there is little to keep resident, and
+    // a run that meets a non-finite depth goes on up to the next evaluation)
+    if (!s->li_mode && M == 1 && !drain && p.cfl_update_interval_steps >= 8 && p.cfl_update_interval_steps <= 256 &&
+        halos_mutual(L)) {
         size_t words = 0;
         FL_CUDA(plan_surface_run(s->sa, s->kind, device, &s->run_smem, &words));
         if (s->run_smem) {
-            if ((rc = s->alloc(&s->run_sync, words))) return rc;
-            FL_CUDA(cudaMemset(s->run_sync, 0, words * sizeof(uint32_t)));
+            std::vector<uint32_t> sent((size_t)L.Cp / 32, 0u);
+            for (const int4 &ti : L.tile_info)
+                for (int32_t j = 0; j < ti.w; ++j) {
+                    const int32_t c = L.halo_src[(size_t)ti.z + j];
+                    sent[c / 32] |= 1u << (c % 32);
+                }
+            uint32_t *d_sent = nullptr;
+            RunArgs &x = s->run_args;
+            x.cells = L.Cp;
+            if ((rc = s->alloc(&x.serial, words)) || (rc = s->upload(&d_sent, sent)) ||
+                (rc = s->alloc(&x.exchange, 2 * (size_t)L.Cp)))
+                return rc;
+            x.sent = d_sent;
+            FL_CUDA(cudaMemset(x.serial, 0, words * sizeof(uint32_t)));
+            FL_CUDA(cudaMemset(x.exchange, 0, 2 * (size_t)L.Cp * sizeof(float4)));
         }
     }
     s->dt_blocks = std::max(1, std::min(sms * 4, (C + 255) / 256));

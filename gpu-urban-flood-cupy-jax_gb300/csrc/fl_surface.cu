@@ -343,92 +343,167 @@ __device__ __forceinline__ void publish(uint32_t *p, uint32_t v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// A state and the serial number of its step, as one 16-byte access each way.
+__device__ __forceinline__ void send_state(float4 *p, float h, float hu, float hv, uint32_t serial) {
+    const uint64_t lo = (uint64_t)__float_as_uint(h) | (uint64_t)__float_as_uint(hu) << 32;
+    const uint64_t hi = (uint64_t)__float_as_uint(hv) | (uint64_t)serial << 32;
+    asm volatile(
+        "{\n"
+        ".reg .b128 t;\n"
+        "mov.b128 t, {%1, %2};\n"
+        "st.relaxed.gpu.global.b128 [%0], t;\n"
+        "}\n" ::"l"(p), "l"(lo), "l"(hi)
+        : "memory");
+}
+
+// Bounded poll for the state with this serial number.
+__device__ __forceinline__ bool receive_state(const float4 *p, uint32_t serial, float4 &v) {
+    uint64_t t0 = 0;
+    for (int i = 0;; ++i) {
+        uint64_t lo, hi;
+        asm volatile(
+            "{\n"
+            ".reg .b128 t;\n"
+            "ld.relaxed.gpu.global.b128 t, [%2];\n"
+            "mov.b128 {%0, %1}, t;\n"
+            "}\n"
+            : "=l"(lo), "=l"(hi)
+            : "l"(p)
+            : "memory");
+        if ((uint32_t)(hi >> 32) == serial) {
+            v.x = __uint_as_float((uint32_t)lo);
+            v.y = __uint_as_float((uint32_t)(lo >> 32));
+            v.z = __uint_as_float((uint32_t)hi);
+            return true;
+        }
+        if ((i & 63) == 63) {
+            if (t0 == 0) t0 = global_ns();
+            else if (global_ns() - t0 > COPY_WAIT_NS) return false;
+        }
+    }
+}
+
 // `steps` steps of a run of the surface alone in one cooperative launch, a CTA a
-// tile: the tile's entries, halo list, cell data, wet time and own states stay in
-// shared memory and registers; per step a CTA waits for the steps of its
-// neighbours (a serial number per tile, release / acquire) and the step record,
-// reads the halo states through L2, and runs k_surface's two phases.  The last
-// CTA plans step k + 1 once every tile has finished step k - 1, as the planner of
-// k_surface does, and the ledger sums keep k_surface's slots and order: the same
-// bits, step by step.
+// tile: the tile's entries, halo list, cell data, wet time and states stay in
+// shared memory and registers.  After a step a CTA sends the states of the cells
+// that other tiles read, each with its step's serial number in one 16-byte store,
+// and polls its halo cells for theirs: one L2 round trip, no fence.  The exchange
+// has two buffers in turn; a tile's step k + 2 overwrites what its step k sent, and
+// starts after its neighbours' step k + 1, which read that (halos are mutual).
+//
+// Every CTA plans for itself: its ninth warp advances a copy of the run control by
+// plan_step during the step before (the records depend on times alone, so all CTAs
+// get the same ones), and the last CTA, which has no tile, writes the run control's
+// end back when every other CTA has copied its start.  (One planner for all put two
+// more L2 round trips across the dies into every step: 4.9 instead of 3.0 us on
+// 20,000 cells.)  An error that a tile finds ends the run at the next CFL
+// evaluation.  The ledger sums keep k_surface's slots and order: the same bits,
+// step by step.
 //
 // A launch a step costs a small mesh more than its work.  us a step with 32 (8)
-// steps between CFL evaluations, a launch a step -> here: 1,800 cells 5.4 -> 3.4
-// (6.0 -> 4.4), 20,000 cells 5.7 -> 4.8 (6.7 -> 5.5), 154,568 cells 8.7 -> 7.1
-// (9.6 -> 7.5); what is left is a chain of L2 round trips (serial numbers, halo
-// states, step record) and the two phases.
+// steps between CFL evaluations, a launch a step -> here: 1,800 cells 5.4 -> 3.0
+// (6.0 -> 3.9), 20,000 cells 5.7 -> 3.0 (6.7 -> 3.8), 154,568 cells 8.7 -> 4.5
+// (9.6 -> 5.8); what is left is the halo states' round trip and the two phases.
 //
-// sync: SYNC_STRIDE words a tile, then the planner's.  All of them hold the same
-// number between launches (each CTA ends at its first + steps, also when the run
-// ends early or a wait gives up), so nothing has to be reset.  Co-residency comes
-// from the cooperative launch; every wait is bounded.
+// Serial numbers: SYNC_STRIDE words a tile, then the last CTA's.  All of them hold
+// the same number between launches (each CTA adds `steps`, also when the run ends
+// early or a wait gives up), so nothing has to be reset.  Co-residency comes from
+// the cooperative launch; every wait is bounded.
 constexpr int SYNC_STRIDE = 8;      // words: a sector each
-constexpr int RUN_MAX_TILES = 1024;
+constexpr int RUN_THREADS = TILE + 32;
+
+__device__ __forceinline__ bool run_all(bool p) {
+    uint32_t r;
+    asm volatile(
+        "{\n"
+        ".reg .pred pi, po;\n"
+        "setp.ne.u32 pi, %1, 0;\n"
+        "bar.red.and.pred po, 2, %2, pi;\n"
+        "selp.u32 %0, 1, 0, po;\n"
+        "}\n"
+        : "=r"(r)
+        : "r"((uint32_t)p), "n"(RUN_THREADS)
+        : "memory");
+    return r != 0;
+}
 
 template <int KIND>
-__global__ void __launch_bounds__(TILE, 4) k_surface_run(const __grid_constant__ SurfArgs a, uint32_t *sync, int slot, int steps) {
+__global__ void __launch_bounds__(RUN_THREADS, 4) k_surface_run(const __grid_constant__ SurfArgs a, const RunArgs x, int slot, int steps) {
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ StepCtrl s_ctrl;
-    __shared__ uint32_t s_near[RUN_MAX_TILES / 32];
+    __shared__ StepCtrl s_ctrl[2];
+    __shared__ RunCtrl s_run;
     float4 *s_flux = (float4 *)smem;
     const uint32_t bar = smem_addr(smem + a.off_bar);
     const int tid = threadIdx.x, tile = blockIdx.x, n_tiles = a.n_tiles;
-    uint32_t *mine = sync + (size_t)tile * SYNC_STRIDE;  // (the planner's: tile = n_tiles)
-    const uint32_t *planned = sync + (size_t)n_tiles * SYNC_STRIDE;
+    uint32_t *mine = x.serial + (size_t)tile * SYNC_STRIDE;
     const uint32_t base = *mine;
-    if (tile == n_tiles) {
-        for (int k = 0; k < steps; ++k) {
-            bool ok = true;
-            if (k > 0)
-                for (int t = tid; t < n_tiles; t += TILE) ok = ok && poll_reached(sync + (size_t)t * SYNC_STRIDE, base + k);
-            if (!__syncthreads_and(ok)) {
-                if (tid == 0 && atomicCAS(&a.run->error, 0, FL_E_TIMEOUT) == 0) a.run->error_step = a.run->step;
-                break;
-            }
-            const int active = __ldcg(&a.ctrl[(slot + k) & 1].active);
-            if (tid == 0 && k + 1 < steps) {
-                plan_step(a.run, a.snap_t, a.hy, &a.ctrl[(slot + k + 1) & 1], false, 0.0f, FL_PHASE_ALL);
-                publish(mine, base + k + 1);
-            }
-            if (!active) break;  // (uniform; both records say so now)
-        }
-        __syncthreads();
-        if (tid == 0) publish(mine, base + steps);
-        return;
-    }
     const StepCtrl first = a.ctrl[slot];
     if (!first.active) {  // (uniform over the grid)
         if (tid == 0) publish(mine, base + steps);
         return;
     }
+    if (tile == n_tiles) {  // the run control after the last step
+        if (tid == 0) {
+            s_run = *a.run;
+            s_run.error = 0;  // (first is active; a tile that is ahead may have set it since)
+            s_ctrl[1] = first;
+            for (int k = 1; k < steps && s_ctrl[1].active; ++k)
+                plan_step(&s_run, a.snap_t, a.hy, &s_ctrl[1], false, 0.0f, FL_PHASE_ALL);
+        }
+        bool ok = true;
+        for (int t = tid; t < n_tiles; t += RUN_THREADS) ok = ok && poll_reached(x.serial + (size_t)t * SYNC_STRIDE, base + steps);
+        ok = __syncthreads_and(ok);
+        if (tid == 0) {
+            const int err = ok ? s_run.error : FL_E_TIMEOUT;
+            if (err && atomicCAS(&a.run->error, 0, err) == 0) a.run->error_step = s_run.error ? s_run.error_step : first.step;
+            a.run->t = s_run.t;
+            a.run->next_snap_t = s_run.next_snap_t;
+            a.run->step = s_run.step;
+            a.run->last_dt = s_run.last_dt;
+            a.run->cfl_reused = s_run.cfl_reused;
+            a.run->parity = s_run.parity;
+            a.run->snap_count = s_run.snap_count;
+            if (!s_ctrl[1].active) a.ctrl[0] = a.ctrl[1] = s_ctrl[1];
+            publish(mine, base + steps);
+        }
+        return;
+    }
     const TileStage S = stage_at(a, smem, 0);
     const int4 ti = a.tile_info[tile];
-    for (int i = tid; i < RUN_MAX_TILES / 32; i += TILE) s_near[i] = 0u;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) s_flux[tid * 3 + k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int i = tid; i < TILE * 3; i += RUN_THREADS) s_flux[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (tid == 0) {
         mbar_init(bar, 1);
         mbar_fence_init();
         mbar_arrive_expect_tx(bar, static_bytes<KIND>(ti) + step_bytes<KIND>());
         issue_static<KIND>(a, S, ti, bar, tile);
         issue_step<KIND>(first.parity ? a.state1 : a.state0, a.wet, S, bar, tile);
+        s_ctrl[0] = first;
+        s_run = *a.run;
+        s_run.error = 0;  // (a tile that is ahead may have set it)
+        publish(mine, base + steps);  // the run control and the first record are read
     }
+    __syncthreads();
+    bool ok = mbar_wait_bounded(bar, 0, COPY_WAIT_NS);
+    if (!ok) ok = mbar_wait_bounded(bar, 0, COPY_WAIT_NS);  // none may land after the CTA leaves
+
+    if (tid >= TILE) {  // the ninth warp: the next step's record
+        for (int k = 0; k < steps; ++k) {
+            if (!run_all(ok) || !s_ctrl[k & 1].active) break;
+            if (tid == TILE && k + 1 < steps)
+                plan_step(&s_run, nullptr, a.hy, &s_ctrl[(k + 1) & 1], false, 0.0f, FL_PHASE_ALL);
+            __syncwarp();
+        }
+        return;
+    }
+
     float2 total[SURF_TERMS];  // lane 0 of a warp: its ledger sums
     float2 *ledger = a.ledger + (size_t)(tile * (TILE / 32) + (tid >> 5)) * SURF_TERMS;
 #pragma unroll
     for (int j = 0; j < SURF_TERMS; ++j) total[j] = (tid & 31) == 0 ? ledger[j] : make_float2(0.0f, 0.0f);
-    __syncthreads();
-    bool ok = mbar_wait_bounded(bar, 0, COPY_WAIT_NS);
-    if (!ok) ok = mbar_wait_bounded(bar, 0, COPY_WAIT_NS);  // none may land after the CTA leaves
-    if (ok)
-        for (int j = tid; j < ti.w; j += TILE) {
-            const int t = S.hs[j] / TILE;
-            atomicOr(&s_near[t >> 5], 1u << (t & 31));
-        }
-    ok = __syncthreads_and(ok);
     const int c = tile * TILE + tid;
     const float4 ci = S.ci[tid];
     const uint32_t info = __float_as_uint(ci.z);
+    const bool sent = (x.sent[c >> 5] >> (c & 31) & 1u) != 0;  // another tile reads the cell
     float wt = 0.0f;
     float4 hz = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
     if (KIND == 1) {
@@ -436,24 +511,26 @@ __global__ void __launch_bounds__(TILE, 4) k_surface_run(const __grid_constant__
         hz = S.hz[tid];
     }
     const float md = a.md;
-    for (int k = 0; k < steps; ++k) {
-        if (ok && k > 0) {
-            if (tid == TILE - 1) ok = poll_reached(planned, base + k);
-            for (int t = tid; t < n_tiles && ok; t += TILE)
-                if (s_near[t >> 5] >> (t & 31) & 1u) ok = poll_reached(sync + (size_t)t * SYNC_STRIDE, base + k);
+    int k = 0;
+    for (; k < steps; ++k) {
+        if (k == 0) {
+            const float4 *in = first.parity ? a.state1 : a.state0;
+            for (int j = tid; j < ti.w && ok; j += TILE) S.st[TILE + j] = in[S.hs[j]];
+        } else {  // (a halo cell's bed, the fourth word, stays)
+            const float4 *in = x.exchange + (size_t)((base + k) & 1u) * x.cells;
+            for (int j = tid; j < ti.w && ok; j += TILE) {
+                float4 v;
+                ok = receive_state(in + S.hs[j], base + k, v);
+                S.st[TILE + j].x = v.x;
+                S.st[TILE + j].y = v.y;
+                S.st[TILE + j].z = v.z;
+            }
         }
-        if (!__syncthreads_and(ok)) {
+        if (!run_all(ok)) {  // the halo states and the step record are in place
             if (tid == 0 && atomicCAS(&a.run->error, 0, FL_E_TIMEOUT) == 0) a.run->error_step = first.step + k;
             break;
         }
-        const bool odd = ((first.parity ^ k) & 1) != 0;
-        const float4 *in = odd ? a.state1 : a.state0;
-        float4 *out = odd ? a.state0 : a.state1;
-        for (int j = tid; j < ti.w; j += TILE) S.st[TILE + j] = __ldcg(in + S.hs[j]);
-        if (tid >= TILE - 32 && tid < TILE - 32 + (int)(sizeof(StepCtrl) / 16))
-            ((uint4 *)&s_ctrl)[tid - (TILE - 32)] = __ldcg((const uint4 *)&a.ctrl[(slot + k) & 1] + (tid - (TILE - 32)));
-        __syncthreads();
-        const StepCtrl s = s_ctrl;
+        const StepCtrl s = s_ctrl[k & 1];
         if (!s.active) break;  // (uniform over the grid)
         const float dt = s.dt_f;
         const bool do_surface = (s.phases & FL_PHASE_SURFACE) != 0;
@@ -463,7 +540,7 @@ __global__ void __launch_bounds__(TILE, 4) k_surface_run(const __grid_constant__
             for (int e = tid; e < ti.y; e += TILE)
                 tile_entry(S.en[e], S.st, s_flux, a.g, a.half_g, md, a.stage, dt, led[2], led[3]);
         }
-        __syncthreads();
+        compute_sync();
         if (c < a.C) {
             const float4 st = S.st[tid];
             if (s.check_finite && !isfinite(st.x)) {
@@ -480,12 +557,11 @@ __global__ void __launch_bounds__(TILE, 4) k_surface_run(const __grid_constant__
                 led[0] += u.rd * ci.x;
                 led[1] += u.id * ci.x;
             }
+            if (s.phases & FL_PHASE_CLAMP) clamp_velocity_exact(hn, hun, hvn, a.vmax);
+            if (sent) send_state(x.exchange + (size_t)((base + k + 1) & 1u) * x.cells + c, hn, hun, hvn, base + k + 1);
+            S.st[tid] = make_float4(hn, hun, hvn, st.w);
 #pragma unroll
             for (int j = 0; j < 3; ++j) s_flux[tid * 3 + j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (s.phases & FL_PHASE_CLAMP) clamp_velocity_exact(hn, hun, hvn, a.vmax);
-            const float4 u = make_float4(hn, hun, hvn, st.w);
-            out[c] = u;
-            S.st[tid] = u;
             if (KIND == 1 && do_surface) wt = wt + dt * (float)(hn > md);
             if (s.snap_slot >= 0) {
                 const size_t o = (size_t)s.snap_slot * (size_t)a.C + (size_t)c;
@@ -494,23 +570,23 @@ __global__ void __launch_bounds__(TILE, 4) k_surface_run(const __grid_constant__
                 a.snap_hv[o] = hvn;
             }
         }
-        __syncthreads();  // the tile's new states are stored
-        if (tid == 0) publish(mine, base + k + 1);
 #pragma unroll
         for (int j = 0; j < SURF_TERMS; ++j) {
-            float x = led[j];
+            float y = led[j];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-            if ((tid & 31) == 0) ff_accumulate(&total[j], x);
+            for (int o = 16; o > 0; o >>= 1) y += __shfl_down_sync(0xffffffffu, y, o);
+            if ((tid & 31) == 0) ff_accumulate(&total[j], y);
         }
     }
-    if (KIND == 1 && c < a.C) a.wet[c] = wt;
+    // k steps were run: the states go where the next launch reads them
+    if (c < a.C) {
+        if (k > 0) (((first.parity ^ k) & 1) ? a.state1 : a.state0)[c] = S.st[tid];
+        if (KIND == 1) a.wet[c] = wt;
+    }
     if ((tid & 31) == 0) {
 #pragma unroll
         for (int j = 0; j < SURF_TERMS; ++j) ledger[j] = total[j];
     }
-    __syncthreads();
-    if (tid == 0) publish(mine, base + steps);
 }
 
 // Global CFL minimum over all cells; the last block plans the step.
@@ -738,12 +814,12 @@ cudaError_t plan_surface_launch(SurfArgs &a, int kind, int device, int *grid, in
 
 // Whether k_surface_run can run the mesh: every tile's CTA and the planner resident
 // at once (on 152 SMs up to 607 tiles, 155,000 cells).  *smem_bytes 0: it cannot.
-// sync_words: what it needs of zeroed memory.
-cudaError_t plan_surface_run(const SurfArgs &a, int kind, int device, int *smem_bytes, size_t *sync_words) {
+// serial_words: the zeroed words of RunArgs::serial.
+cudaError_t plan_surface_run(const SurfArgs &a, int kind, int device, int *smem_bytes, size_t *serial_words) {
     const void *fn = kind ? (const void *)k_surface_run<1> : (const void *)k_surface_run<0>;
     const int bytes = a.off_stage + a.stage_bytes;
     *smem_bytes = 0;
-    *sync_words = (size_t)(a.n_tiles + 1) * SYNC_STRIDE;
+    *serial_words = (size_t)(a.n_tiles + 1) * SYNC_STRIDE;
     int per_sm = 0, sms = 0, most = 0, coop = 0;
     cudaError_t e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
@@ -752,16 +828,16 @@ cudaError_t plan_surface_run(const SurfArgs &a, int kind, int device, int *smem_
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, fn);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)at.sharedSizeBytes);
     if (e != cudaSuccess || !coop || bytes > most - (int)at.sharedSizeBytes) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, TILE, (size_t)bytes);
-    if (e == cudaSuccess && a.n_tiles + 1 <= per_sm * sms && a.n_tiles <= RUN_MAX_TILES) *smem_bytes = bytes;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, RUN_THREADS, (size_t)bytes);
+    if (e == cudaSuccess && a.n_tiles + 1 <= per_sm * sms) *smem_bytes = bytes;
     return e;
 }
 
-cudaError_t launch_surface_run(const SurfArgs &a, int kind, uint32_t *sync, int slot, int steps, int smem_bytes,
+cudaError_t launch_surface_run(const SurfArgs &a, int kind, const RunArgs &x, int slot, int steps, int smem_bytes,
                                cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)a.n_tiles + 1);
-    cfg.blockDim = dim3(TILE);
+    cfg.blockDim = dim3(RUN_THREADS);
     cfg.dynamicSmemBytes = (size_t)smem_bytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -769,8 +845,8 @@ cudaError_t launch_surface_run(const SurfArgs &a, int kind, uint32_t *sync, int 
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return kind ? cudaLaunchKernelEx(&cfg, k_surface_run<1>, a, sync, slot, steps)
-                : cudaLaunchKernelEx(&cfg, k_surface_run<0>, a, sync, slot, steps);
+    return kind ? cudaLaunchKernelEx(&cfg, k_surface_run<1>, a, x, slot, steps)
+                : cudaLaunchKernelEx(&cfg, k_surface_run<0>, a, x, slot, steps);
 }
 
 int surface_warps(int grid) { return grid * (TILE / 32); }

@@ -11,13 +11,15 @@ from floodgb import native
 from floodgb.config import load_config
 from floodgb.domain import ProductionInfiltrationFields
 from floodgb.exceptions import SimulationError
+from floodgb.rainfall import rainfall_event
 from floodgb.solver import FloodSolver
 from floodgb.synthetic import make_grid_city
 
 
-def _solver(n, per_cell, max_snapshots=None):
+def _solver(n, per_cell, max_snapshots=None, rain=None):
     sc = make_grid_city(n=n, size_m=10.0 * n, seed=n, duration_min=3.0)
-    cfg = load_config(None, dict(sc.overrides, **{"solver.snapshot_interval_min": 1.0}))
+    cfg = load_config(None, dict(sc.overrides, **{"solver.snapshot_interval_min": 1.0,
+                                               "solver.finite_check_interval_steps": 20}))
     topo = sc.city.topologies.surface_topology
     rng = np.random.default_rng(n)
     C = topo.cell_count
@@ -27,7 +29,7 @@ def _solver(n, per_cell, max_snapshots=None):
         fields = ProductionInfiltrationFields(
             rainfall_multiplier=f[0], horton_f0_mps=f[1], horton_fc_mps=f[2], horton_k_per_s=f[3],
             open_fraction=np.ones_like(f[0]), active_mask=np.ones(C, bool))
-    s = FloodSolver(topo, rainfall=sc.rainfall, cfg=cfg, infiltration_fields=fields, infiltration_mps=1.0e-6,
+    s = FloodSolver(topo, rainfall=rain or sc.rainfall, cfg=cfg, infiltration_fields=fields, infiltration_mps=1.0e-6,
                     centroids=sc.city.mesh.centroids_xy, duration_s=150.0, max_snapshots=max_snapshots)
     h = rng.uniform(0.0, 0.5, C).astype(np.float32)
     s.set_state(h, np.zeros_like(h), np.zeros_like(h))
@@ -93,3 +95,28 @@ def test_an_error_of_the_planner_stops_the_long_launch():
     finally:
         a.close()
         b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("single", [False, True])
+def test_a_non_finite_depth_is_reported_at_its_step(single):
+    from floodgb.build import build_library
+
+    build_library()
+    native.load()
+    if native.device_count() < 1:
+        pytest.skip("no CUDA device")
+    # beyond float32: an infinite rain depth from the first step, checked at step 20
+    s = _solver(16, False, rain=rainfall_event(np.array([0.0]), np.array([60.0]), np.array([1.0e46])))
+    try:
+        with pytest.raises(SimulationError, match="Non-finite depth detected at step 20 "):
+            if single:
+                for _ in range(40):
+                    s.run(s.progress().t_s + 1.0e-9)
+            s.run()
+        p = s.progress()
+        assert p.error != 0 and p.error_step == 20
+        with pytest.raises(SimulationError):
+            s.run()
+    finally:
+        s.close()
