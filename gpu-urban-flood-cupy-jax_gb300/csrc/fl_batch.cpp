@@ -21,7 +21,9 @@ namespace fl {
 int set_error(int code, const char *fmt, ...);
 int build_mesh_layout(const FlMeshDesc &m, const FlDrainDesc *d, HostLayout &L);
 cudaError_t batch_configure(int kind, int tile, int smem_bytes, int *per_sm);
-cudaError_t launch_surface_batch(const BatchArgs &a, int kind, int grid, int smem_bytes, cudaStream_t stream);
+int batch_plan_ctas(int tile, int n);
+cudaError_t launch_surface_batch(const BatchArgs &a, const PlanArgs &p, int kind, int slot, int mode, int smem_bytes,
+                                 cudaStream_t stream);
 cudaError_t launch_cfl_batch(const float4 *state0, const float *char_len, const int32_t *tile_valid, float *tile_min,
                              int tiles, int tile, float cfl, float g, float md, cudaStream_t stream);
 cudaError_t launch_plan_batch(const PlanArgs &a, int slot, int init, cudaStream_t stream);
@@ -45,6 +47,8 @@ struct FlBatch {
     int kind = 0;
     int tile = 256;
     int chunk = 32;
+    int interval = 0;  // steps between CFL evaluations where every scenario has the same and a chunk holds whole ones
+    int planning_launches() const { return interval ? chunk / interval : chunk; }
     int grid = 0, smem = 0;
     int64_t cells = 0;  // padded, all scenarios
     int32_t tiles = 0;
@@ -240,12 +244,12 @@ static int batch_create_impl(int32_t n, const FlMeshDesc *meshes, const FlForcin
     FB_CUDA(cudaMemcpy(b->state[0], st0.data(), sizeof(float4) * Cp, cudaMemcpyHostToDevice));
     FB_CUDA(cudaMemcpy(b->state[1], st0.data(), sizeof(float4) * Cp, cudaMemcpyHostToDevice));
     if ((rc = b->alloc(&b->hmax, Cp)) || (rc = b->alloc(&b->wet, Cp)) || (rc = b->alloc(&tile_min, (size_t)b->tiles)) ||
-        (rc = b->alloc(&tile_led, (size_t)b->tiles * SURF_TERMS)) || (rc = b->alloc(&b->run, (size_t)n)) ||
-        (rc = b->alloc(&b->ctrl, (size_t)n * 2)) || (rc = b->alloc(&b->list, 1)) ||
+        (rc = b->alloc(&tile_led, 2 * (size_t)b->tiles * SURF_TERMS)) || (rc = b->alloc(&b->run, (size_t)n)) ||
+        (rc = b->alloc(&b->ctrl, (size_t)n * 2)) || (rc = b->alloc(&b->list, 2)) ||
         (rc = b->alloc(&b->ledger, (size_t)n * SURF_TERMS)))
         return rc;
-    FB_CUDA(cudaMemset(tile_led, 0, sizeof(float) * (size_t)b->tiles * SURF_TERMS));
-    FB_CUDA(cudaMemset(b->list, 0, sizeof(BatchList)));
+    FB_CUDA(cudaMemset(tile_led, 0, 2 * sizeof(float) * (size_t)b->tiles * SURF_TERMS));
+    FB_CUDA(cudaMemset(b->list, 0, 2 * sizeof(BatchList)));
     int32_t largest = 1;
     for (int32_t s = 0; s < n; ++s) largest = std::max(largest, b->cells_s[s]);
     if ((rc = b->alloc(&b->stage_f, (size_t)largest))) return rc;
@@ -323,7 +327,14 @@ static int batch_create_impl(int32_t n, const FlMeshDesc *meshes, const FlForcin
     FB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     if (per_sm < 1) return set_error(FL_E_UNSUPPORTED, "the batch's largest tile needs %d bytes of shared memory", b->smem);
     const int ctas = want_ctas > 0 ? std::min(want_ctas, per_sm) : per_sm;
-    b->grid = std::max(1, std::min(ctas * sms, b->tiles));
+    b->interval = params[0].cfl_update_interval_steps;
+    for (int32_t s = 0; s < n; ++s)
+        if (params[s].cfl_update_interval_steps != b->interval) b->interval = 0;
+    if (b->interval < 2 || b->chunk % b->interval) b->interval = 0;  // (every step evaluates, or steps differ: a planning launch a step)
+    const int planners = b->interval ? batch_plan_ctas(b->tile, n) : 0;
+    b->grid = std::max(1, std::min(std::min(ctas * sms, per_sm * sms - planners), b->tiles));
+    a.ctas = b->grid;
+    a.early = 2 * (b->grid + planners) <= per_sm * sms ? 1 : 0;
     PlanArgs &pa = b->pa;
     pa.run = b->run;
     pa.ctrl = b->ctrl;
@@ -338,6 +349,7 @@ static int batch_create_impl(int32_t n, const FlMeshDesc *meshes, const FlForcin
     pa.list = b->list;
     pa.n = n;
     pa.max_snaps = b->max_snaps;
+    pa.n_tiles = b->tiles;
 
     FB_CUDA(cudaMallocHost((void **)&b->poll_h, sizeof(BatchList) * 2));
     FB_CUDA(cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking));
@@ -383,8 +395,12 @@ static int batch_capture(FlBatch *b) {
     FB_CUDA(cudaStreamBeginCapture(b->cap_stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t e = cudaSuccess;
     for (int j = 0; j < b->chunk && e == cudaSuccess; ++j) {
-        e = launch_surface_batch(b->ba, b->kind, b->grid, b->smem, b->cap_stream);
-        if (e == cudaSuccess) e = launch_plan_batch(b->pa, j & 1, 0, b->cap_stream);
+        // every scenario is at the same step (a batch runs from step 0) or done
+        const int I = b->interval;
+        const bool plan = !I || (j + 1) % I == 0;
+        const int mode = I ? (j % I ? BP_LEDGER : 0) | (plan ? 0 : BP_NEXT) : 0;
+        e = launch_surface_batch(b->ba, b->pa, b->kind, j & 1, mode, b->smem, b->cap_stream);
+        if (e == cudaSuccess && plan) e = launch_plan_batch(b->pa, j & 1, 0, b->cap_stream);
     }
     cudaError_t e2 = cudaStreamEndCapture(b->cap_stream, &g);
     if (e != cudaSuccess || e2 != cudaSuccess) {
@@ -472,7 +488,7 @@ FL_API int fl_batch_run(FlBatch *b, int64_t max_steps, void *stream) {
     int64_t launched = 0;
     while (true) {
         FB_CUDA(cudaGraphLaunch(b->graph, st));
-        add_launches(2 * (int64_t)b->chunk);
+        add_launches((int64_t)b->chunk + b->planning_launches());
         FB_CUDA(cudaMemcpyAsync(b->poll_h[launched & 1].tiles, b->list->tiles, sizeof(int32_t) * b->S, cudaMemcpyDeviceToHost,
                                 st));
         FB_CUDA(cudaEventRecord(b->ev[launched & 1], st));

@@ -29,6 +29,10 @@ struct BatchList {
     BatchEntry e[MAX_SCEN];
 };
 
+// What a step's surface launch plans besides (bits).
+constexpr int BP_LEDGER = 1;  // the previous step's ledger terms into the scenarios' sums
+constexpr int BP_NEXT = 2;    // the next step, which evaluates no CFL minimum
+
 struct BatchArgs {
     const float4 *cinfo;          // [cells] {area, manning, flags, 0}
     const int4 *tile_info;        // [tiles] {first entry, entry count, first halo index, halo count}
@@ -39,14 +43,15 @@ struct BatchArgs {
     float4 *state0, *state1;
     float *hmax;                  // running maximum depth since the last snapshot
     const float *char_len;
-    const BatchList *list;
+    const BatchList *list;        // [2] of even and odd steps
     float *tile_min;              // [tiles] CFL minimum of the tile's output (flagged steps)
-    float *tile_led;              // [tiles * SURF_TERMS] the tile's ledger terms of the step
+    float *tile_led;              // [2 x tiles * SURF_TERMS] the tile's ledger terms of an even, an odd step
     float *snap_h, *snap_hmax;
     float *snap_hu, *snap_hv;     // momentum at each snapshot (same layout)
     const int64_t *snap_base;     // [n] first snapshot element of each scenario
     RunCtrl *run;                 // [n]
     int32_t n_scen, n_tiles, tile, e_cap, h_cap;
+    int32_t ctas, early;          // CTAs with tiles (the others plan); the dependent may start beside this grid
     int32_t off_bar, off_list, off_stage, stage_bytes;
     int32_t so_ci, so_hz, so_wt, so_hm, so_en, so_hs;
     int32_t forcing_kind;
@@ -64,8 +69,8 @@ struct PlanArgs {
     const float *tile_min;
     const float *tile_led;
     float2 *ledger;               // [n * SURF_TERMS] float-float running sums
-    BatchList *list;
-    int32_t n, max_snaps;
+    BatchList *list;              // [2]
+    int32_t n, max_snaps, n_tiles;
 };
 
 }  // namespace fl

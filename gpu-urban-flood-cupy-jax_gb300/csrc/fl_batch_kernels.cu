@@ -14,13 +14,19 @@
 // A tile's warp partials are added up after the next tile's opening barrier,
 // so a tile costs two barriers of the compute warps and none of the CTA.
 //
-// k_plan_batch: one CTA per scenario reduces its tiles' ledger terms and CFL
+// Planning.  A step that follows a CFL evaluation needs the step's minima:
+// k_plan_batch, one CTA per scenario, reduces its tiles' ledger terms and CFL
 // minima, plans its next step with plan_step (the single-scenario planner) and
-// writes the scenario's entry of the step's list.  It sits between two surface
-// launches, so its length counts in full: the run record and the hyetograph
-// are brought to shared memory in one level of loads (read field by field by
-// the one planning thread they made it 12 us a step), and no CTA waits for the
-// others -- the surface CTAs add up the tile counts.
+// writes the scenario's entry of the next step's list.  It sits between two
+// surface launches, so its length counts in full: the run record and the
+// hyetograph are brought to shared memory in one level of loads (read field by
+// field by the one planning thread they made it 12 us a step; 7 here), and no CTA
+// waits for the others -- the surface CTAs add up the tile counts.
+// Any other next step depends on the clock alone.  Where all scenarios evaluate on
+// the same steps, CTAs at the end of the surface launch plan it meanwhile, a warp
+// per scenario, and add up the previous step's ledger terms (lists and terms have
+// two buffers); then only one step in a CFL interval has a planning launch (300 s of 16 scenarios,
+// 1.64 M cells: 41.1 -> 38.0 ms; 90 s of six, 27,000 cells: 2.08 -> 1.59 ms).
 //
 // k_cfl_batch: the CFL minima of every tile's initial state (before step 0).
 #include "fl_batch.cuh"
@@ -109,9 +115,93 @@ __device__ __forceinline__ bool batch_all(bool p) {
     return r != 0;
 }
 
+// A scenario's entry of a list, from its planned step.
+__device__ __forceinline__ void list_entry(const PlanArgs &a, int b, BatchList *list, const StepCtrl &nx, int cfl_interval) {
+    const int t0 = a.scen_tile0[b];
+    list->tiles[b] = nx.active ? a.scen_tile0[b + 1] - t0 : 0;
+    if (nx.active) {
+        BatchEntry e;
+        e.dt = nx.dt_f;
+        e.dtg = nx.dtg_f;
+        e.rain = nx.rain_f;
+        e.infil = a.scen_infil[b];
+        e.scen = b;
+        const bool cfl_next = step_mod(nx.step + 1, cfl_interval) == 0;
+        e.flags = (nx.parity ? BF_PARITY : 0) | (cfl_next ? BF_CFL : 0) | (nx.check_finite ? BF_FINITE : 0) |
+                  (nx.phases << BF_PHASE_SHIFT) | ((nx.snap_slot + 1) << BF_SNAP_SHIFT);
+        e.tile0 = t0;
+        e.cells = a.scen_cells[b];
+        list->e[b] = e;
+    }
+}
+
+// One warp, beside the surface CTAs of the step in `slot`: scenario b's ledger
+// terms of the step before (k_plan_batch's sums, its four warps one after the
+// other) and its next step's record and list entry.  s_run: a run record and a
+// step record of shared memory.  An error that this step's surface CTAs find is
+// seen one step later than by k_plan_batch; the error and its step are theirs.
+__device__ __noinline__ void plan_ahead(const PlanArgs &a, int b, int lane, int slot, int mode, RunCtrl *s_run) {
+    StepCtrl *rec = &a.ctrl[2 * b + (slot ^ 1)], *s_next = (StepCtrl *)(s_run + 1);
+    RunCtrl *run = &a.run[b];
+    for (int i = lane; i < (int)(sizeof(RunCtrl) / 4); i += 32) ((uint32_t *)s_run)[i] = ((const uint32_t *)run)[i];
+    const bool had_step = rec->active != 0;  // (the record of the step before, overwritten below)
+    if (mode & BP_LEDGER) {
+        const float4 *led = (const float4 *)a.tile_led + (size_t)(slot ^ 1) * a.n_tiles;
+        const int t0 = a.scen_tile0[b], t1 = a.scen_tile0[b + 1];
+        float sum[SURF_TERMS] = {0.0f, 0.0f, 0.0f, 0.0f};
+        float l[4][SURF_TERMS];
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+#pragma unroll
+            for (int j = 0; j < SURF_TERMS; ++j) l[w][j] = 0.0f;
+        for (int t = t0 + lane; t < t1; t += 128) {
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                if (t + 32 * w >= t1) break;
+                const float4 v = led[t + 32 * w];
+                l[w][0] += v.x;
+                l[w][1] += v.y;
+                l[w][2] += v.z;
+                l[w][3] += v.w;
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+#pragma unroll
+            for (int j = 0; j < SURF_TERMS; ++j) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) l[w][j] += __shfl_xor_sync(0xffffffffu, l[w][j], o);
+                sum[j] = w == 0 ? l[w][j] : sum[j] + l[w][j];
+            }
+        if (had_step) {
+#pragma unroll
+            for (int j = 0; j < SURF_TERMS; ++j)
+                if (lane == j) ff_accumulate(&a.ledger[b * SURF_TERMS + j], sum[j]);
+        }
+    }
+    __syncwarp();
+    if (!(mode & BP_NEXT)) return;
+    if (lane == 0) {
+        const int before = s_run->error;
+        plan_step(s_run, a.snap_t + (size_t)b * a.max_snaps, a.hy[b], s_next, false, CUDART_INF_F, FL_PHASE_SURFACE | FL_PHASE_CLAMP);
+        list_entry(a, b, a.list + (slot ^ 1), *s_next, s_run->cfl_interval);
+        *rec = *s_next;
+        if (s_run->error != before && atomicCAS(&run->error, 0, s_run->error) == 0) run->error_step = s_run->error_step;
+        run->t = s_run->t;
+        run->next_snap_t = s_run->next_snap_t;
+        run->last_dt = s_run->last_dt;
+        run->step = s_run->step;
+        run->cfl_reused = s_run->cfl_reused;
+        run->parity = s_run->parity;
+        run->snap_count = s_run->snap_count;
+    }
+}
+
 // Four CTAs of 256-cell tiles an SM (seven of 128): 56 registers.
 template <int KIND, int T>
-__global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(const __grid_constant__ BatchArgs a) {
+__global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(const __grid_constant__ BatchArgs a, const __grid_constant__ PlanArgs p,
+                                                                            int slot, int mode) {
     constexpr int W = T / 32;
     extern __shared__ __align__(128) unsigned char smem[];
     float4 *s_flux = (float4 *)smem;  // [T * 3]
@@ -122,6 +212,13 @@ __global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(cons
     int32_t *s_prefix = (int32_t *)(smem + a.off_list);
     BatchEntry *s_ent = (BatchEntry *)(smem + a.off_list + MAX_SCEN * 4 + 16);
     const int tid = threadIdx.x;
+    if ((int)blockIdx.x >= a.ctas) {
+        pdl_wait();
+        if (a.early) pdl_launch_dependents();
+        const int b = ((int)blockIdx.x - a.ctas) * W + (tid >> 5);
+        if (tid < T && b < p.n) plan_ahead(p, b, tid & 31, slot, mode, (RunCtrl *)(smem + (tid >> 5) * 384));
+        return;
+    }
     const uint32_t bar_base = smem_addr(s_bar);
     if (tid < T) {
 #pragma unroll
@@ -136,13 +233,16 @@ __global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(cons
         mbar_fence_init();
     }
     pdl_wait();  // the planner's list (its launch overlaps the set-up above)
+    if (a.early) pdl_launch_dependents();
     const int n = a.n_scen;
-    for (int i = tid; i < n; i += T + 32) s_ent[i] = a.list->e[i];
+    const BatchList *list = a.list + slot;
+    float *tile_led = a.tile_led + (size_t)slot * a.n_tiles * SURF_TERMS;
+    for (int i = tid; i < n; i += T + 32) s_ent[i] = list->e[i];
     if (tid < 32) {  // running sums of the tile counts (an inactive scenario's range is empty)
         constexpr int PER = MAX_SCEN / 32;
         int c[PER], sum = 0;
 #pragma unroll
-        for (int j = 0; j < PER; ++j) c[j] = tid * PER + j < n ? a.list->tiles[tid * PER + j] : 0;
+        for (int j = 0; j < PER; ++j) c[j] = tid * PER + j < n ? list->tiles[tid * PER + j] : 0;
 #pragma unroll
         for (int j = 0; j < PER; ++j) sum += c[j];
         int before = sum;
@@ -161,12 +261,11 @@ __global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(cons
     }
     __syncthreads();  // the last block-wide barrier: the roles split here
     const int total = s_prefix[n];
-    const int G = gridDim.x;
+    const int G = a.ctas;
     const BStage<T> S0 = bstage_at<T>(a, smem, 0), S1 = bstage_at<T>(a, smem, 1);
     auto fail = [&]() {  // (one thread)
         for (int k = 0; k < n; ++k)
-            if (atomicCAS(&a.run[s_ent[k].scen].error, 0, FL_E_TIMEOUT) == 0)
-                a.run[s_ent[k].scen].error_step = a.run[s_ent[k].scen].step - 1;
+            if (atomicCAS(&a.run[k].error, 0, FL_E_TIMEOUT) == 0) a.run[k].error_step = p.ctrl[2 * k + slot].step;
     };
 
     if (tid >= T) {
@@ -222,7 +321,7 @@ __global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(cons
             float sum = 0.0f;
 #pragma unroll
             for (int w = 0; w < W; ++w) sum += s_red[w * 5 + j];
-            a.tile_led[(size_t)t * SURF_TERMS + j] = sum;
+            tile_led[(size_t)t * SURF_TERMS + j] = sum;
         }
         if (cfl) {
             float m = CUDART_INF_F;
@@ -268,7 +367,7 @@ __global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(cons
             const float4 ci = S.ci[tid];
             const uint32_t info = __float_as_uint(ci.z);
             if ((flags & BF_FINITE) && !isfinite(st.x)) {
-                if (atomicCAS(&a.run[E.scen].error, 0, FL_E_NONFINITE) == 0) a.run[E.scen].error_step = a.run[E.scen].step - 1;
+                if (atomicCAS(&a.run[E.scen].error, 0, FL_E_NONFINITE) == 0) a.run[E.scen].error_step = p.ctrl[2 * E.scen + slot].step;
             }
             float wt = 0.0f;
             float4 hz = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
@@ -399,7 +498,7 @@ __global__ void __launch_bounds__(128) k_plan_batch(const __grid_constant__ Plan
     float m = CUDART_INF_F;
     float l[SURF_TERMS] = {0.0f, 0.0f, 0.0f, 0.0f};
     static_assert(SURF_TERMS == 4, "a tile's ledger terms are one float4");
-    const float4 *led = (const float4 *)a.tile_led;
+    const float4 *led = (const float4 *)a.tile_led + (size_t)slot * a.n_tiles;
     for (int t = t0 + tid; t < t1; t += 128 * 4) {  // four tiles' loads in flight (whether or not the step uses them), added in order
         float4 v[4];
         float q[4];
@@ -441,32 +540,17 @@ __global__ void __launch_bounds__(128) k_plan_batch(const __grid_constant__ Plan
         for (int w = 1; w < 4; ++w) mm = fminf(mm, red[w][SURF_TERMS]);
         const bool eval = step_mod(s_run.step, cfl_interval) == 0;
         plan_step(&s_run, a.snap_t + (size_t)b * a.max_snaps, hy, &s_next, eval, mm, FL_PHASE_SURFACE | FL_PHASE_CLAMP);
-        const StepCtrl &nx = s_next;
-        a.list->tiles[b] = nx.active ? t1 - t0 : 0;
-        if (nx.active) {
-            BatchEntry e;
-            e.dt = nx.dt_f;
-            e.dtg = nx.dtg_f;
-            e.rain = nx.rain_f;
-            e.infil = a.scen_infil[b];
-            e.scen = b;
-            const bool cfl_next = step_mod(nx.step + 1, cfl_interval) == 0;
-            e.flags = (nx.parity ? BF_PARITY : 0) | (cfl_next ? BF_CFL : 0) | (nx.check_finite ? BF_FINITE : 0) |
-                      (nx.phases << BF_PHASE_SHIFT) | ((nx.snap_slot + 1) << BF_SNAP_SHIFT);
-            e.tile0 = t0;
-            e.cells = a.scen_cells[b];
-            a.list->e[b] = e;
-        }
+        list_entry(a, b, a.list + (slot ^ 1), s_next, cfl_interval);
     }
     __syncthreads();
     if (tid < (int)(sizeof(RunCtrl) / 4)) ((uint32_t *)run)[tid] = ((const uint32_t *)&s_run)[tid];
     if (tid < (int)(sizeof(StepCtrl) / 4)) ((uint32_t *)&a.ctrl[2 * b + (slot ^ 1)])[tid] = ((const uint32_t *)&s_next)[tid];
 }
 
-template __global__ void k_surface_batch<0, 128>(const __grid_constant__ BatchArgs);
-template __global__ void k_surface_batch<0, 256>(const __grid_constant__ BatchArgs);
-template __global__ void k_surface_batch<1, 128>(const __grid_constant__ BatchArgs);
-template __global__ void k_surface_batch<1, 256>(const __grid_constant__ BatchArgs);
+template __global__ void k_surface_batch<0, 128>(const __grid_constant__ BatchArgs, const __grid_constant__ PlanArgs, int, int);
+template __global__ void k_surface_batch<0, 256>(const __grid_constant__ BatchArgs, const __grid_constant__ PlanArgs, int, int);
+template __global__ void k_surface_batch<1, 128>(const __grid_constant__ BatchArgs, const __grid_constant__ PlanArgs, int, int);
+template __global__ void k_surface_batch<1, 256>(const __grid_constant__ BatchArgs, const __grid_constant__ PlanArgs, int, int);
 
 static const void *surface_batch_fn(int kind, int tile) {
     if (kind) return tile == 128 ? (const void *)k_surface_batch<1, 128> : (const void *)k_surface_batch<1, 256>;
@@ -501,10 +585,14 @@ static cudaError_t launch_dependent(void (*kernel)(Args, Rest...), int grid, int
     return cudaLaunchKernelEx(&cfg, kernel, a, rest...);
 }
 
-cudaError_t launch_surface_batch(const BatchArgs &a, int kind, int grid, int smem_bytes, cudaStream_t stream) {
-    void (*fn)(BatchArgs) = a.tile == 128 ? (kind ? k_surface_batch<1, 128> : k_surface_batch<0, 128>)
-                                          : (kind ? k_surface_batch<1, 256> : k_surface_batch<0, 256>);
-    return launch_dependent(fn, grid, a.tile + 32, smem_bytes, stream, a);
+int batch_plan_ctas(int tile, int n) { return (n + tile / 32 - 1) / (tile / 32); }
+
+cudaError_t launch_surface_batch(const BatchArgs &a, const PlanArgs &p, int kind, int slot, int mode, int smem_bytes,
+                                 cudaStream_t stream) {
+    void (*fn)(BatchArgs, PlanArgs, int, int) = a.tile == 128 ? (kind ? k_surface_batch<1, 128> : k_surface_batch<0, 128>)
+                                                              : (kind ? k_surface_batch<1, 256> : k_surface_batch<0, 256>);
+    return launch_dependent(fn, a.ctas + (mode ? batch_plan_ctas(a.tile, a.n_scen) : 0), a.tile + 32, smem_bytes, stream, a, p, slot,
+                            mode);
 }
 
 cudaError_t launch_cfl_batch(const float4 *state0, const float *char_len, const int32_t *tile_valid, float *tile_min,
