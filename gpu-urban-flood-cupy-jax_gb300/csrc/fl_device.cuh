@@ -399,15 +399,30 @@ __device__ __forceinline__ void warp_add_ledger(const float (&v)[NT], float2 *le
     }
 }
 
-// The same with an explicit warp index (kernels whose warps do not all add).
+// The same in two halves: a warp's slots are fetched where other loads are under
+// way (lane j: term j) and added to at the end.  Fetched there, their round trip
+// was the tail of every kernel of a step.  `warp`: the warp's slot index.
 template <int NT>
-__device__ __forceinline__ void warp_add_ledger_at(const float (&v)[NT], float2 *ledger, int warp) {
+__device__ __forceinline__ float2 ledger_fetch(const float2 *ledger, int warp) {
+    const int lane = threadIdx.x & 31;
+    return lane < NT ? __ldcg(&ledger[(size_t)warp * NT + lane]) : make_float2(0.0f, 0.0f);
+}
+
+template <int NT>
+__device__ __forceinline__ void ledger_add(const float (&v)[NT], float2 slot, float2 *ledger, int warp) {
+    const int lane = threadIdx.x & 31;
+    float mine = 0.0f;
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
         float x = v[j];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        if ((threadIdx.x & 31) == 0) ff_accumulate(&ledger[(size_t)warp * NT + j], x);
+        x = __shfl_sync(0xffffffffu, x, 0);
+        if (lane == j) mine = x;
+    }
+    if (lane < NT) {
+        ff_accumulate(&slot, mine);
+        ledger[(size_t)warp * NT + lane] = slot;
     }
 }
 

@@ -510,12 +510,14 @@ __global__ void __launch_bounds__(128, 7) k_nodes(const __grid_constant__ NodeAr
     pdl_launch_dependents();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const NodeStatic t = node_static(a, n);
+    // (last written by the previous step's launch, which ended before this step's surface kernel began)
+    const float2 slots = ledger_fetch<D1_TERMS>(a.ledger, n >> 5);
     pdl_wait();  // the surface kernel's depths
     const StepCtrl s = a.ctrl[slot];
     if (!s.active || !(s.phases & FL_PHASE_DRAINAGE)) return;
     float led[D1_TERMS] = {0.0f, 0.0f};
     if (n < a.N) node_item(a, s, n, t, led);
-    warp_add_ledger<D1_TERMS>(led, a.ledger);
+    ledger_add<D1_TERMS>(led, slots, a.ledger, n >> 5);
 }
 
 // Link l: the transfer volume from the end volumes after the inlet exchange
@@ -571,12 +573,13 @@ __global__ void __launch_bounds__(128, 7) k_network(const __grid_constant__ NetA
     pdl_launch_dependents();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const GroupStatic t = group_static(a, g);
+    const float2 slots = ledger_fetch<D2_TERMS>(a.ledger, g >> 5);  // (as in k_nodes)
     const StepCtrl s = a.ctrl[slot];
     pdl_wait();  // k_donor's factors (and, through it, every earlier kernel's writes)
     if (!s.active || !(s.phases & FL_PHASE_DRAINAGE)) return;
     float led[D2_TERMS] = {0.0f, 0.0f, 0.0f, 0.0f};
     if (g < a.G) group_item(a, s, t, led);
-    warp_add_ledger<D2_TERMS>(led, a.ledger);
+    ledger_add<D2_TERMS>(led, slots, a.ledger, g >> 5);
 }
 
 // Weighted surcharge return into the table cells (reference

@@ -432,6 +432,8 @@ __global__ void __launch_bounds__(TILE + 32, 3) k_li_tiles(const __grid_constant
     const bool drain_finishes = (s.phases & FL_PHASE_DRAINAGE) != 0;
     const bool recharge_finishes = (s.phases & FL_PHASE_RECHARGE) != 0;
     float led[SURF_TERMS] = {0.0f, 0.0f, 0.0f, 0.0f};
+    const int led_warp = (int)blockIdx.x * (TILE / 32) + (tid >> 5);
+    const float2 slots = ledger_fetch<SURF_TERMS>(q.ledger, led_warp);
     int i = 0;
     for (int t = blockIdx.x; t < a.n_tiles; t += ncta, ++i) {
         const int st_i = i & 1;
@@ -537,7 +539,7 @@ __global__ void __launch_bounds__(TILE + 32, 3) k_li_tiles(const __grid_constant
         __syncwarp();
         if ((tid & 31) == 0) mbar_arrive(bar + 32u + 8u * st_i);
     }
-    warp_add_ledger_at<SURF_TERMS>(led, q.ledger, (int)blockIdx.x * (TILE / 32) + (tid >> 5));
+    ledger_add<SURF_TERMS>(led, slots, q.ledger, led_warp);
 }
 
 // Shared memory layout and grid of k_li_tiles; 0 blocks where fewer than two

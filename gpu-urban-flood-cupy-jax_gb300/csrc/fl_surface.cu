@@ -247,6 +247,9 @@ __global__ void __launch_bounds__(SURF_THREADS, 4) k_surface(const __grid_consta
     const bool drain_finishes = (s.phases & FL_PHASE_DRAINAGE) != 0;
     const bool recharge_finishes = (s.phases & FL_PHASE_RECHARGE) != 0;
     float led[SURF_TERMS] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float2 *ledger = a.ledger + (MEM ? mem * (size_t)a.m_led : 0);
+    const int led_warp = (int)blockIdx.x * (TILE / 32) + (tid >> 5);
+    const float2 slots = ledger_fetch<SURF_TERMS>(ledger, led_warp);
     int i = 0;
     for (int t = blockIdx.x; t < a.n_tiles; t += ncta, ++i) {
         const int st_i = i & 1;
@@ -322,7 +325,7 @@ __global__ void __launch_bounds__(SURF_THREADS, 4) k_surface(const __grid_consta
         __syncwarp();
         if ((tid & 31) == 0) mbar_arrive((bar_base + 32u + 8u * st_i));
     }
-    warp_add_ledger_at<SURF_TERMS>(led, a.ledger + (MEM ? mem * (size_t)a.m_led : 0), (int)blockIdx.x * (TILE / 32) + (tid >> 5));
+    ledger_add<SURF_TERMS>(led, slots, ledger, led_warp);
 }
 
 // Bounded poll: *p has reached v (serial numbers; they may wrap).
