@@ -177,10 +177,9 @@ __device__ __forceinline__ NodeStatic node_static(const NodeArgs &a, int n) {
     return t;
 }
 
-__device__ __forceinline__ void node_item(const NodeArgs &a, const StepCtrl &s, int n, const NodeStatic &t,
+__device__ __forceinline__ void node_item(const NodeArgs &a, const StepCtrl &s, int n, const NodeStatic &t, float2 Vr,
                                           float (&led)[D1_TERMS]) {
     const float4 *hs = s.parity ? a.state0 : a.state1;  // written by the surface step
-    const float2 Vr = a.Va[n];
     float h[DR_PRE];
 #pragma unroll
     for (int u = 0; u < DR_PRE; ++u) h[u] = t.j0 + u < t.j1 ? hs[t.qk[u].y].x : 0.0f;
@@ -300,6 +299,7 @@ __device__ __forceinline__ void group_item(const NetArgs &a, const StepCtrl &s, 
     // one level of loads: the cell's depth, its inlets' exchange, the first
     // node's volume and factor, its transfers and their other ends' factors
     float h = c >= 0 ? hs[c].x : 0.0f;
+    const float wet = c >= 0 && a.forcing_kind == 1 ? a.wet[c] : 0.0f;
     float2 cs[2];
 #pragma unroll
     for (int u = 0; u < 2; ++u) cs[u] = gs.q0 + u < gs.q1 ? __ldcg(&a.capsur[gs.q0 + u]) : make_float2(0.0f, 0.0f);
@@ -444,7 +444,7 @@ __device__ __forceinline__ void group_item(const NetArgs &a, const StepCtrl &s, 
         // a recharge cell is finished by k_recharge
         const bool fin = !(a.has_recharge && (s.phases & FL_PHASE_RECHARGE) && (cflags & CELL_RECHARGE));
         if (fin) {
-            if ((s.phases & FL_PHASE_SURFACE) && a.forcing_kind == 1) a.wet[c] = a.wet[c] + dt * (float)(hf > a.md);
+            if ((s.phases & FL_PHASE_SURFACE) && a.forcing_kind == 1) a.wet[c] = wet + dt * (float)(hf > a.md);
             if (s.snap_slot >= 0) a.snap_h[(size_t)s.snap_slot * (size_t)a.C + c] = hf;
         }
     }
@@ -510,13 +510,15 @@ __global__ void __launch_bounds__(128, 7) k_nodes(const __grid_constant__ NodeAr
     pdl_launch_dependents();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const NodeStatic t = node_static(a, n);
-    // (last written by the previous step's launch, which ended before this step's surface kernel began)
+    // the step record, the volume and the ledger slots: written by kernels that
+    // ended before this step's surface kernel read the record (and let this one start)
+    const StepCtrl s = a.ctrl[slot];
+    const float2 Vr = n < a.N ? a.Va[n] : make_float2(0.0f, 0.0f);
     const float2 slots = ledger_fetch<D1_TERMS>(a.ledger, n >> 5);
     pdl_wait();  // the surface kernel's depths
-    const StepCtrl s = a.ctrl[slot];
     if (!s.active || !(s.phases & FL_PHASE_DRAINAGE)) return;
     float led[D1_TERMS] = {0.0f, 0.0f};
-    if (n < a.N) node_item(a, s, n, t, led);
+    if (n < a.N) node_item(a, s, n, t, Vr, led);
     ledger_add<D1_TERMS>(led, slots, a.ledger, n >> 5);
 }
 
