@@ -113,7 +113,9 @@ __device__ __forceinline__ float node_depth(float2 V, float A) {
 // network of 118,768 nodes needs to hide its scattered sectors.  us per launch
 // before -> after, 960 nodes: k_nodes 5.0 -> 3.8, k_donor 2.0 -> 1.6, k_network
 // 5.2 -> 4.2; 118,768 nodes: 7.0 -> 6.6, 3.0 -> 2.2, 8.8 -> 8.5 (7.9 and 10.7
-// for the first and last at 78 and 96 registers).
+// for the first and last at 78 and 96 registers).  With the step record, the
+// node's volume and the ledger slots before the wait too: k_nodes 3.4 and 6.0,
+// k_network 3.5 and 7.1.
 
 constexpr int DR_PRE = 4;  // list entries held in registers; the rest are read as they come
 

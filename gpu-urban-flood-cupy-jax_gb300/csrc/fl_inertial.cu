@@ -25,7 +25,7 @@
 //               discharge to memory and read it back through scattered slots
 //               (186 MB a step on 981,880 cells, 67.3 us chained); here about a
 //               quarter of the edges are evaluated a second time, beside another
-//               tile, and no discharge leaves the SM: 35.0 us, of which the
+//               tile, and no discharge leaves the SM: 33 us, of which the
 //               compulsory 128 MB take 19 and the IEEE divisions and cube roots
 //               of 1.9 M entries most of the rest.
 //

@@ -271,9 +271,6 @@ static DtArgs dt_args(const FlSolver *s, int m) {
     return d;
 }
 
-// One step: [CFL reduction + plan] surface [inlets network], the CFL and
-// surface launches once per member, each drainage kernel once for all
-// members.
 // The drainage passes of one step.
 static int launch_drainage(FlSolver *s, int slot, cudaStream_t st) {
     FL_CUDA(launch_nodes(s->nd, slot, st));
@@ -291,6 +288,8 @@ static cudaError_t launch_inertial(FlSolver *s, int slot, int plan_next, cudaStr
     return launch_li_tiles(s->lt, s->kind, slot, plan_next, s->lt_grid, s->lt_smem, st);
 }
 
+// One step: [CFL reduction + plan] surface [inlets network], the CFL launch once
+// per member, the surface and each drainage kernel once for all members.
 static int launch_step(FlSolver *s, int slot, bool eval, bool plan_next, cudaStream_t st) {
     if (eval) {
         for (int m = 0; m < s->members; ++m) FL_CUDA(launch_dt(dt_args(s, m), s->dt_blocks, slot, 1, st));

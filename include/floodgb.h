@@ -182,8 +182,8 @@ FL_API void fl_destroy(FlSolver *solver);
  * rain multiplier, scalar infiltration) of forcings[0] apply to every
  * member.  Each member has its own state, adaptive dt, snapshots and
  * ledger and follows exactly the single-instance step of fl_run; per step
- * the surface kernel runs once per member and each drainage kernel once for
- * all members (the members share the static tables).  The calls that take a
+ * the surface kernel and each drainage kernel are launched once for all
+ * members (the members share the static tables).  The calls that take a
  * solver address the selected member (fl_member_select; member 0 after
  * creation), except fl_run, which runs every member to the end of the run
  * (t_target >= the duration, no step cap), and fl_reset_clock, which resets
@@ -287,11 +287,11 @@ FL_API int fl_plan_check(const FlMeshDesc *mesh, const FlDrainDesc *drain, int64
 FL_API int fl_plan_tiles(const FlMeshDesc *mesh, int64_t *tiles);
 
 /* Time `reps` back-to-back launches of one kernel of a step (0 surface (the
- * two local-inertial launches in that mode), 1 node inlet exchange, 2 pipe
+ * local-inertial step in that mode), 1 node inlet exchange, 2 pipe
  * network, 3 CFL reduction, 4 link update, 5 donor factors) between CUDA
  * events on `stream`, at the solver's current state and last dt.  The
  * launches are captured in chains of up to 32 per CUDA graph, each launched
- * as in the step loop (the surface, link, donor and network kernels as
+ * as in the step loop (the surface and the drainage kernels as
  * programmatic dependents of the launch before them), so the time per launch
  * is the kernel's own in-loop cost, not a graph launch's.  The clock is not
  * advanced but the state buffers are overwritten (reset before the next run).
