@@ -483,9 +483,10 @@ __global__ void __launch_bounds__(RUN_THREADS, 4) k_surface_run(const __grid_con
         s_ctrl[0] = first;
         s_run = *a.run;
         s_run.error = 0;  // (a tile that is ahead may have set it)
-        publish(mine, base + steps);  // the run control and the first record are read
     }
     __syncthreads();
+    // every thread has read its serial number and the first record, this one the run control
+    if (tid == 0) publish(mine, base + steps);
     bool ok = mbar_wait_bounded(bar, 0, COPY_WAIT_NS);
     if (!ok) ok = mbar_wait_bounded(bar, 0, COPY_WAIT_NS);  // none may land after the CTA leaves
 
