@@ -36,6 +36,7 @@
 #include <cuda_runtime.h>
 
 #include "fl_device.cuh"
+#include "fl_run.cuh"
 
 namespace fl {
 
@@ -329,6 +330,56 @@ __device__ __forceinline__ float lt_donor_scale(const float4 *slots, float h, fl
     return req > 1.0e-12f ? fmin32(1.0f, vol / req) : 1.0f;
 }
 
+// An active own cell's update from its places and the donor factors: volume change,
+// momentum, then _apply_sources (k_li_cells' arithmetic).  own: its local index.
+template <int KIND>
+__device__ __forceinline__ void lt_cell(const LiArgs &q, const StepCtrl &s, const float4 st, const float4 ci, const float4 hz, float wt,
+                                        float cl, const float4 *slots, const float *scale, int own, float &hn, float &hun, float &hvn,
+                                        float (&led)[SURF_TERMS]) {
+    const float dt = s.dt_f, md = q.md;
+    const float own_scale = scale[own];
+    float hd = 0.0f, qx = 0.0f, qy = 0.0f, bf = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float4 v = slots[k];
+        const uint32_t b = __float_as_uint(v.w);
+        if (!(b & LIS_PRESENT) || v.x == 0.0f) continue;
+        if (b & LIS_INTERIOR) {
+            const bool left = (b & LIS_LEFT) != 0;
+            const float sd = (v.x >= 0.0f) != left ? scale[b >> 8] : own_scale;  // the donor's factor
+            const float lim = v.x * sd * dt;
+            hd += left ? -lim : lim;
+        } else {
+            const float bq = v.x * dt;
+            hd -= bq;
+            bf += bq;
+        }
+        qx += v.y;
+        qy += v.z;
+    }
+    const float area = ci.x;
+    const float h0 = fmax32(st.x + hd / area, 0.0f);
+    const float per = 2.0f * area / fmax32(cl, 1.0e-12f);
+    const bool wet0 = h0 > md;
+    const float hu0 = wet0 ? qx / fmax32(per, 1.0e-12f) : 0.0f;
+    const float hv0 = wet0 ? qy / fmax32(per, 1.0e-12f) : 0.0f;
+    // _apply_sources (reference triangular_backend.py:1330-1379)
+    const float rain = KIND == 1 ? s.rain_f * hz.w : s.rain_f;
+    const float infil = KIND == 1 ? hz.y + (hz.x - hz.y) * __expf(-hz.z * wt) : q.infil_scalar;
+    const float rd = fmax32(rain, 0.0f) * dt;
+    const float h1 = h0 + rd;
+    const float id = fmin32(h1, fmax32(infil, 0.0f) * dt);
+    const float h2 = h1 - id;
+    const float sc = (h1 > md) ? h2 / fmax32(h1, md) : 0.0f;
+    const bool wet2 = h2 > md;
+    hn = h2;
+    hun = wet2 ? hu0 * sc : 0.0f;
+    hvn = wet2 ? hv0 * sc : 0.0f;
+    led[0] += rd * area;
+    led[1] += id * area;
+    led[3] += bf;
+}
+
 // Persistent and warp-specialised as k_surface: a producer warp fills two
 // stages (bulk copies, then the halo states), eight compute warps run the
 // tile's three passes; barriers full[2], halo[2], empty[2], pre (the first
@@ -476,47 +527,7 @@ __global__ void __launch_bounds__(TILE + 32, 3) k_li_tiles(const __grid_constant
             if (!do_surface) {
                 hn = st.x; hun = st.y; hvn = st.z;
             } else if (info & CELL_ACTIVE) {
-                const float own_scale = s_scale[tid];
-                float hd = 0.0f, qx = 0.0f, qy = 0.0f, bf = 0.0f;
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const float4 v = s_slot[tid * 3 + k];
-                    const uint32_t b = __float_as_uint(v.w);
-                    if (!(b & LIS_PRESENT) || v.x == 0.0f) continue;
-                    if (b & LIS_INTERIOR) {
-                        const bool left = (b & LIS_LEFT) != 0;
-                        const float sd = (v.x >= 0.0f) != left ? s_scale[b >> 8] : own_scale;  // the donor's factor
-                        const float lim = v.x * sd * dt;
-                        hd += left ? -lim : lim;
-                    } else {
-                        const float bq = v.x * dt;
-                        hd -= bq;
-                        bf += bq;
-                    }
-                    qx += v.y;
-                    qy += v.z;
-                }
-                const float area = ci.x;
-                const float h0 = fmax32(st.x + hd / area, 0.0f);
-                const float per = 2.0f * area / fmax32(S.cl[tid], 1.0e-12f);
-                const bool wet0 = h0 > md;
-                const float hu0 = wet0 ? qx / fmax32(per, 1.0e-12f) : 0.0f;
-                const float hv0 = wet0 ? qy / fmax32(per, 1.0e-12f) : 0.0f;
-                // _apply_sources (reference triangular_backend.py:1330-1379)
-                const float rain = KIND == 1 ? s.rain_f * hz.w : s.rain_f;
-                const float infil = KIND == 1 ? hz.y + (hz.x - hz.y) * __expf(-hz.z * wt) : q.infil_scalar;
-                const float rd = fmax32(rain, 0.0f) * dt;
-                const float h1 = h0 + rd;
-                const float id = fmin32(h1, fmax32(infil, 0.0f) * dt);
-                const float h2 = h1 - id;
-                const float sc = (h1 > md) ? h2 / fmax32(h1, md) : 0.0f;
-                const bool wet2 = h2 > md;
-                hn = h2;
-                hun = wet2 ? hu0 * sc : 0.0f;
-                hvn = wet2 ? hv0 * sc : 0.0f;
-                led[0] += rd * area;
-                led[1] += id * area;
-                led[3] += bf;
+                lt_cell<KIND>(q, s, st, ci, hz, wt, S.cl[tid], &s_slot[tid * 3], s_scale, tid, hn, hun, hvn, led);
             }
             if (s.phases & FL_PHASE_CLAMP) clamp_velocity_exact(hn, hun, hvn, q.vmax);
             if ((info & CELL_RECEIVER) && (s.phases & FL_PHASE_INFLOW)) hn = __fadd_rn(hn, q.ext_add[c]);
@@ -540,6 +551,138 @@ __global__ void __launch_bounds__(TILE + 32, 3) k_li_tiles(const __grid_constant
         if ((tid & 31) == 0) mbar_arrive(bar + 32u + 8u * st_i);
     }
     ledger_add<SURF_TERMS>(led, slots, q.ledger, led_warp);
+}
+
+// `steps` steps of a run of the local-inertial surface alone in one cooperative
+// launch (fl_run.cuh), a CTA a tile: k_li_tiles' three passes on a tile that stays in
+// shared memory and registers, with its ledger slots and order.  120 s of a run, a
+// launch a step -> here: 1,152 cells 0.74 -> 0.55 ms, 7,200 cells 1.00 -> 0.71, 45,000
+// cells 1.56 -> 0.96; what is left is the halo states' round trip and the three passes.
+template <int KIND>
+__global__ void __launch_bounds__(RUN_THREADS, 3) k_li_run(const __grid_constant__ LiTileArgs a, const RunArgs x, int slot, int steps) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ StepCtrl s_ctrl[2];
+    __shared__ RunCtrl s_run;
+    float4 *s_slot = (float4 *)smem;
+    float *s_scale = (float *)(smem + a.off_scale);
+    const uint32_t bar = smem_addr(smem + a.off_bar);
+    const LiArgs &q = a.c;
+    const int tid = threadIdx.x, tile = blockIdx.x, n_tiles = a.n_tiles;
+    uint32_t *mine = x.serial + (size_t)tile * SYNC_STRIDE;
+    const uint32_t base = *mine;
+    const StepCtrl first = q.ctrl[slot];
+    if (!first.active) {  // (uniform over the grid)
+        if (tid == 0) publish(mine, base + steps);
+        return;
+    }
+    if (tile == n_tiles) {
+        run_last_cta(q.run, q.ctrl, q.snap_t, q.hy, x, n_tiles, base, steps, first, &s_run, &s_ctrl[1]);
+        return;
+    }
+    const LtStage S = lt_stage(a, smem, 0);
+    const int4 ti = a.tile[2 * tile], tj = a.tile[2 * tile + 1];
+    const int n1 = tj.x;
+    for (int i = tid; i < (TILE + n1) * 3; i += RUN_THREADS) s_slot[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        mbar_fence_init();
+        mbar_arrive_expect_tx(bar, lt_static_bytes<KIND>(ti, tj) + lt_step_bytes<KIND>());
+        lt_issue_static<KIND>(a, S, ti, tj, bar, tile);
+        lt_issue_step<KIND>(first.parity ? q.state1 : q.state0, q.wet, S, bar, tile);
+        s_ctrl[0] = first;
+        s_run = *q.run;
+        s_run.error = 0;  // (a tile that is ahead may have set it)
+    }
+    __syncthreads();
+    // every thread has read its serial number and the first record, this one the run control
+    if (tid == 0) publish(mine, base + steps);
+    bool ok = mbar_wait_bounded(bar, 0, LT_WAIT_NS);
+    if (!ok) ok = mbar_wait_bounded(bar, 0, LT_WAIT_NS);  // none may land after the CTA leaves
+    if (tid >= TILE) {
+        run_records(ok, steps, q.hy, &s_run, s_ctrl);
+        return;
+    }
+
+    float2 total[SURF_TERMS];  // lane 0 of a warp: its ledger sums
+    float2 *ledger = q.ledger + (size_t)(tile * (TILE / 32) + (tid >> 5)) * SURF_TERMS;
+#pragma unroll
+    for (int j = 0; j < SURF_TERMS; ++j) total[j] = (tid & 31) == 0 ? ledger[j] : make_float2(0.0f, 0.0f);
+    const int c = tile * TILE + tid;
+    const float4 ci = S.ci[tid];
+    const uint32_t info = __float_as_uint(ci.z);
+    const bool sent = (x.sent[c >> 5] >> (c & 31) & 1u) != 0;  // another tile reads the cell
+    const float cl = S.cl[tid];
+    float wt = 0.0f;
+    float4 hz = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+    if (KIND == 1) {
+        wt = S.wt[tid];
+        hz = S.hz[tid];
+    }
+    int k = 0;
+    for (; k < steps; ++k) {
+        ok = run_halo(ok, k, first.parity ? q.state1 : q.state0, x, base, S.hs, ti.w, S.st);
+        if (!run_all(ok)) {  // the halo states and the step record are in place
+            if (tid == 0 && atomicCAS(&q.run->error, 0, FL_E_TIMEOUT) == 0) q.run->error_step = first.step + k;
+            break;
+        }
+        const StepCtrl s = s_ctrl[k & 1];
+        if (!s.active) break;  // (uniform over the grid)
+        const float dt = s.dt_f;
+        const bool do_surface = (s.phases & FL_PHASE_SURFACE) != 0;
+        float led[SURF_TERMS] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (do_surface) {
+#pragma unroll 1
+            for (int e = tid; e < ti.y; e += TILE) lt_entry(S.en[e], S.dm[e], S.st, s_slot, q.g, dt);
+            lt_sync();  // the discharges are in place
+            s_scale[tid] = lt_donor_scale(&s_slot[tid * 3], S.st[tid].x, ci.x, dt);
+            for (int j = tid; j < n1; j += TILE)
+                s_scale[TILE + j] = lt_donor_scale(&s_slot[(TILE + j) * 3], S.st[TILE + j].x, S.ha[j], dt);
+        }
+        lt_sync();  // the donor factors are in place
+        if (c < q.C) {
+            const float4 st = S.st[tid];
+            if (s.check_finite && !isfinite(st.x)) {
+                if (atomicCAS(&q.run->error, 0, FL_E_NONFINITE) == 0) q.run->error_step = s.step;
+            }
+            float hn = 0.0f, hun = 0.0f, hvn = 0.0f;
+            if (!do_surface) {
+                hn = st.x; hun = st.y; hvn = st.z;
+            } else if (info & CELL_ACTIVE) {
+                lt_cell<KIND>(q, s, st, ci, hz, wt, cl, &s_slot[tid * 3], s_scale, tid, hn, hun, hvn, led);
+            }
+            if (s.phases & FL_PHASE_CLAMP) clamp_velocity_exact(hn, hun, hvn, q.vmax);
+            if (sent) send_state(x.exchange + (size_t)((base + k + 1) & 1u) * x.cells + c, hn, hun, hvn, base + k + 1);
+            S.st[tid] = make_float4(hn, hun, hvn, st.w);
+            if (KIND == 1 && do_surface) wt = wt + dt * (float)(hn > q.md);
+            if (s.snap_slot >= 0) {
+                const size_t o = (size_t)s.snap_slot * (size_t)q.C + (size_t)c;
+                q.snap_h[o] = hn;
+                q.snap_hu[o] = hun;
+                q.snap_hv[o] = hvn;
+            }
+        }
+        // the places are empty again for the next step (its entries are written after
+        // the barrier that follows its halo)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) s_slot[tid * 3 + j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int j = tid; j < n1 * 3; j += TILE) s_slot[TILE * 3 + j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int j = 0; j < SURF_TERMS; ++j) {
+            float y = led[j];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) y += __shfl_down_sync(0xffffffffu, y, o);
+            if ((tid & 31) == 0) ff_accumulate(&total[j], y);
+        }
+    }
+    // k steps were run: the states go where the next launch reads them
+    if (c < q.C) {
+        if (k > 0) (((first.parity ^ k) & 1) ? q.state1 : q.state0)[c] = S.st[tid];
+        if (KIND == 1) q.wet[c] = wt;
+    }
+    if ((tid & 31) == 0) {
+#pragma unroll
+        for (int j = 0; j < SURF_TERMS; ++j) ledger[j] = total[j];
+    }
 }
 
 // Shared memory layout and grid of k_li_tiles; 0 blocks where fewer than two
@@ -597,6 +740,21 @@ cudaError_t launch_li_tiles(const LiTileArgs &a, int kind, int slot, int plan_ne
     cfg.numAttrs = 1;
     return kind == 1 ? cudaLaunchKernelEx(&cfg, k_li_tiles<1>, a, slot, plan_next)
                      : cudaLaunchKernelEx(&cfg, k_li_tiles<0>, a, slot, plan_next);
+}
+
+// Whether k_li_run can run the mesh: a CTA per tile of k_li_tiles' grid and all
+// resident at once.  *smem_bytes 0: it cannot.
+cudaError_t plan_li_run(const LiTileArgs &a, int kind, int tiles_grid, int device, int *smem_bytes, size_t *serial_words) {
+    const void *fn = kind ? (const void *)k_li_run<1> : (const void *)k_li_run<0>;
+    const int bytes = a.off_stage + a.stage_bytes;
+    *smem_bytes = 0;
+    *serial_words = (size_t)(a.n_tiles + 1) * SYNC_STRIDE;
+    if (a.n_tiles + 1 != tiles_grid) return cudaSuccess;
+    return run_fits(fn, a.n_tiles + 1, bytes, device, smem_bytes);
+}
+
+cudaError_t launch_li_run(const LiTileArgs &a, int kind, const RunArgs &x, int slot, int steps, int smem_bytes, cudaStream_t stream) {
+    return launch_run(kind ? k_li_run<1> : k_li_run<0>, a, x, slot, steps, a.n_tiles + 1, smem_bytes, stream);
 }
 
 int li_edge_blocks(int32_t E, int sms) { return std::max(1, std::min(sms * 8, (E + 255) / 256)); }

@@ -72,6 +72,8 @@ cudaError_t plan_li_tiles(LiTileArgs &a, int kind, int device, int *grid, int *s
 cudaError_t plan_surface_run(const SurfArgs &a, int kind, int device, int *smem_bytes, size_t *serial_words);
 cudaError_t launch_surface_run(const SurfArgs &a, int kind, const RunArgs &x, int slot, int steps, int smem_bytes,
                                cudaStream_t stream);
+cudaError_t plan_li_run(const LiTileArgs &a, int kind, int tiles_grid, int device, int *smem_bytes, size_t *serial_words);
+cudaError_t launch_li_run(const LiTileArgs &a, int kind, const RunArgs &x, int slot, int steps, int smem_bytes, cudaStream_t stream);
 cudaError_t launch_li_tiles(const LiTileArgs &a, int kind, int slot, int plan_next, int grid, int smem_bytes,
                             cudaStream_t stream);
 int node_blocks(int32_t N);
@@ -145,11 +147,11 @@ struct FlSolver {
     bool li_mode = false;     // surface_step_mode = local_inertial
     LiTileArgs lt{};          // its tiles (lt_grid 0: the two launches over edges and cells)
     int lt_grid = 0, lt_smem = 0;
-    int run_smem = 0;         // k_surface_run's (0: a launch a step)
+    int run_smem = 0;         // k_surface_run's or k_li_run's (0: a launch a step)
     RunArgs run_args{};
     // a run's steps up to the next CFL evaluation in one launch: the surface alone, one member
     bool run_kernel() const {
-        return run_smem > 0 && members == 1 && !li_mode && !has_inflow() && !has_drain() && !has_table() && !has_recharge();
+        return run_smem > 0 && members == 1 && !has_inflow() && !has_drain() && !has_table() && !has_recharge();
     }
     int launches_per_chunk() const {
         const int interval = params.cfl_update_interval_steps, evals = (chunk + interval - 1) / interval;
@@ -382,9 +384,12 @@ static int capture_graph(FlSolver *s) {
     int rc = FL_OK;
     for (int j = 0; j < s->chunk && rc == FL_OK && s->run_kernel(); j += interval) {
         cudaError_t e = launch_dt(dt_args(s, 0), s->dt_blocks, j & 1, 1, s->cap_stream);
-        if (e == cudaSuccess) e = launch_surface_run(s->sa, s->kind, s->run_args, j & 1, interval, s->run_smem, s->cap_stream);
+        s->lt.c = s->li;
+        if (e == cudaSuccess)
+            e = s->li_mode ? launch_li_run(s->lt, s->kind, s->run_args, j & 1, interval, s->run_smem, s->cap_stream)
+                           : launch_surface_run(s->sa, s->kind, s->run_args, j & 1, interval, s->run_smem, s->cap_stream);
         g_launches += 2;
-        if (e != cudaSuccess) rc = set_error(FL_E_CUDA, "launch_surface_run: %s", cudaGetErrorString(e));
+        if (e != cudaSuccess) rc = set_error(FL_E_CUDA, "run launch: %s", cudaGetErrorString(e));
     }
     for (int j = 0; j < s->chunk && rc == FL_OK && !s->run_kernel(); ++j) {
         const bool eval = (j % interval) == 0;
@@ -498,6 +503,41 @@ FL_API void fl_destroy(FlSolver *s) {
     if (s->poll_h) cudaFreeHost(s->poll_h);
     delete s;
 }
+
+// The exchange of a run in one launch (s->run_args) for tiles with these halo cells,
+// halo[first] .. of tile t; `words` serial words.  s->run_smem stays 0 unless every
+// tile whose cells a tile reads reads cells of that tile (a tile waits only for the
+// tiles that it reads).
+static int setup_run(FlSolver *s, const std::vector<std::pair<int32_t, int32_t>> &ranges, const std::vector<int32_t> &halo,
+                     int smem_bytes, size_t words) {
+    std::vector<std::pair<int32_t, int32_t>> reads;
+    std::vector<uint32_t> sent((size_t)s->Cp / 32, 0u);
+    for (size_t t = 0; t < ranges.size(); ++t)
+        for (int32_t j = 0; j < ranges[t].second; ++j) {
+            const int32_t c = halo[(size_t)ranges[t].first + j];
+            reads.emplace_back((int32_t)t, c / TILE);
+            sent[c / 32] |= 1u << (c % 32);
+        }
+    std::sort(reads.begin(), reads.end());
+    reads.erase(std::unique(reads.begin(), reads.end()), reads.end());
+    for (const auto &r : reads)
+        if (!std::binary_search(reads.begin(), reads.end(), std::make_pair(r.second, r.first))) return FL_OK;
+    uint32_t *d_sent = nullptr;
+    RunArgs &x = s->run_args;
+    int rc;
+    x.cells = s->Cp;
+    if ((rc = s->alloc(&x.serial, words)) || (rc = s->upload(&d_sent, sent)) || (rc = s->alloc(&x.exchange, 2 * (size_t)s->Cp)))
+        return rc;
+    x.sent = d_sent;
+    FL_CUDA(cudaMemset(x.serial, 0, words * sizeof(uint32_t)));
+    FL_CUDA(cudaMemset(x.exchange, 0, 2 * (size_t)s->Cp * sizeof(float4)));
+    s->run_smem = smem_bytes;
+    return FL_OK;
+}
+
+// With a few steps between CFL evaluations there is little to keep resident, and a
+// run that meets a non-finite depth goes on up to the next evaluation.
+static bool run_interval(int32_t steps) { return steps >= 8 && steps <= 256; }
 
 // Tiles of the one-launch local-inertial step: entries, rings and areas per
 // tile of 256 cells (s->lt; s->lt_grid stays 0 where they do not fit).  lr, geo
@@ -617,20 +657,13 @@ static int build_li_tiles(FlSolver *s, const HostLayout &L, const std::vector<in
     a.halo_src = d_halo;
     a.harea = d_area;
     a.char_len = d_len;
-    return FL_OK;
-}
-
-// Every tile whose cells a tile reads reads cells of that tile.
-static bool halos_mutual(const HostLayout &L) {
-    std::vector<std::pair<int32_t, int32_t>> reads;
-    for (size_t t = 0; t < L.tile_info.size(); ++t)
-        for (int32_t j = 0; j < L.tile_info[t].w; ++j)
-            reads.emplace_back((int32_t)t, L.halo_src[(size_t)L.tile_info[t].z + j] / TILE);
-    std::sort(reads.begin(), reads.end());
-    reads.erase(std::unique(reads.begin(), reads.end()), reads.end());
-    for (const auto &r : reads)
-        if (!std::binary_search(reads.begin(), reads.end(), std::make_pair(r.second, r.first))) return false;
-    return true;
+    if (s->members > 1 || s->N > 0 || !run_interval(s->params.cfl_update_interval_steps)) return FL_OK;
+    size_t words = 0;
+    int bytes = 0;
+    FL_CUDA(plan_li_run(a, s->kind, s->lt_grid, s->device, &bytes, &words));
+    std::vector<std::pair<int32_t, int32_t>> ranges;
+    for (int32_t t = 0; t < tiles; ++t) ranges.emplace_back(info[2 * t].z, info[2 * t].w);
+    return bytes ? setup_run(s, ranges, halo, bytes, words) : FL_OK;
 }
 
 // forcings: M entries (the members' rainfall); the per-cell fields come from
@@ -762,30 +795,13 @@ static int create_impl(const FlMeshDesc *mesh, const FlDrainDesc *drain, const F
     s->li_mode = p.surface_step_mode == 1;
     // the surface ledger: per warp of the surface kernel (or of the local-inertial cell kernel)
     s->n_led_s = (size_t)std::max(surface_warps(s->surf_grid), s->li_mode ? li_cell_blocks(C) * 8 : 0) * SURF_TERMS;
-    // (a tile waits only for the tiles that it reads, so these have to read it too;
-    // with a few steps between CFL evaluations there is little to keep resident, and
-    // a run that meets a non-finite depth goes on up to the next evaluation)
-    if (!s->li_mode && M == 1 && !drain && p.cfl_update_interval_steps >= 8 && p.cfl_update_interval_steps <= 256 &&
-        halos_mutual(L)) {
+    if (!s->li_mode && M == 1 && !drain && run_interval(p.cfl_update_interval_steps)) {
         size_t words = 0;
-        FL_CUDA(plan_surface_run(s->sa, s->kind, device, &s->run_smem, &words));
-        if (s->run_smem) {
-            std::vector<uint32_t> sent((size_t)L.Cp / 32, 0u);
-            for (const int4 &ti : L.tile_info)
-                for (int32_t j = 0; j < ti.w; ++j) {
-                    const int32_t c = L.halo_src[(size_t)ti.z + j];
-                    sent[c / 32] |= 1u << (c % 32);
-                }
-            uint32_t *d_sent = nullptr;
-            RunArgs &x = s->run_args;
-            x.cells = L.Cp;
-            if ((rc = s->alloc(&x.serial, words)) || (rc = s->upload(&d_sent, sent)) ||
-                (rc = s->alloc(&x.exchange, 2 * (size_t)L.Cp)))
-                return rc;
-            x.sent = d_sent;
-            FL_CUDA(cudaMemset(x.serial, 0, words * sizeof(uint32_t)));
-            FL_CUDA(cudaMemset(x.exchange, 0, 2 * (size_t)L.Cp * sizeof(float4)));
-        }
+        int bytes = 0;
+        FL_CUDA(plan_surface_run(s->sa, s->kind, device, &bytes, &words));
+        std::vector<std::pair<int32_t, int32_t>> ranges;
+        for (const int4 &ti : L.tile_info) ranges.emplace_back(ti.z, ti.w);
+        if (bytes && (rc = setup_run(s, ranges, L.halo_src, bytes, words))) return rc;
     }
     s->dt_blocks = std::max(1, std::min(sms * 4, (C + 255) / 256));
     float *dt_partial = nullptr;

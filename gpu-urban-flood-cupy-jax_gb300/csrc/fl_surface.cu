@@ -35,6 +35,7 @@
 #include <algorithm>
 
 #include "fl_device.cuh"
+#include "fl_run.cuh"
 
 namespace fl {
 
@@ -328,108 +329,15 @@ __global__ void __launch_bounds__(SURF_THREADS, 4) k_surface(const __grid_consta
     ledger_add<SURF_TERMS>(led, slots, ledger, led_warp);
 }
 
-// Bounded poll: *p has reached v (serial numbers; they may wrap).
-__device__ __forceinline__ bool poll_reached(const uint32_t *p, uint32_t v) {
-    uint64_t t0 = 0;
-    for (int i = 0;; ++i) {
-        uint32_t x;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(p) : "memory");
-        if ((int32_t)(x - v) >= 0) return true;
-        if ((i & 63) == 63) {
-            if (t0 == 0) t0 = global_ns();
-            else if (global_ns() - t0 > COPY_WAIT_NS) return false;
-        }
-    }
-}
-
-__device__ __forceinline__ void publish(uint32_t *p, uint32_t v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// A state and the serial number of its step, as one 16-byte access each way.
-__device__ __forceinline__ void send_state(float4 *p, float h, float hu, float hv, uint32_t serial) {
-    const uint64_t lo = (uint64_t)__float_as_uint(h) | (uint64_t)__float_as_uint(hu) << 32;
-    const uint64_t hi = (uint64_t)__float_as_uint(hv) | (uint64_t)serial << 32;
-    asm volatile(
-        "{\n"
-        ".reg .b128 t;\n"
-        "mov.b128 t, {%1, %2};\n"
-        "st.relaxed.gpu.global.b128 [%0], t;\n"
-        "}\n" ::"l"(p), "l"(lo), "l"(hi)
-        : "memory");
-}
-
-// Bounded poll for the state with this serial number.
-__device__ __forceinline__ bool receive_state(const float4 *p, uint32_t serial, float4 &v) {
-    uint64_t t0 = 0;
-    for (int i = 0;; ++i) {
-        uint64_t lo, hi;
-        asm volatile(
-            "{\n"
-            ".reg .b128 t;\n"
-            "ld.relaxed.gpu.global.b128 t, [%2];\n"
-            "mov.b128 {%0, %1}, t;\n"
-            "}\n"
-            : "=l"(lo), "=l"(hi)
-            : "l"(p)
-            : "memory");
-        if ((uint32_t)(hi >> 32) == serial) {
-            v.x = __uint_as_float((uint32_t)lo);
-            v.y = __uint_as_float((uint32_t)(lo >> 32));
-            v.z = __uint_as_float((uint32_t)hi);
-            return true;
-        }
-        if ((i & 63) == 63) {
-            if (t0 == 0) t0 = global_ns();
-            else if (global_ns() - t0 > COPY_WAIT_NS) return false;
-        }
-    }
-}
-
-// `steps` steps of a run of the surface alone in one cooperative launch, a CTA a
-// tile: the tile's entries, halo list, cell data, wet time and states stay in
-// shared memory and registers.  After a step a CTA sends the states of the cells
-// that other tiles read, each with its step's serial number in one 16-byte store,
-// and polls its halo cells for theirs: one L2 round trip, no fence.  The exchange
-// has two buffers in turn; a tile's step k + 2 overwrites what its step k sent, and
-// starts after its neighbours' step k + 1, which read that (halos are mutual).
-//
-// Every CTA plans for itself: its ninth warp advances a copy of the run control by
-// plan_step during the step before (the records depend on times alone, so all CTAs
-// get the same ones), and the last CTA, which has no tile, writes the run control's
-// end back when every other CTA has copied its start.  (One planner for all put two
-// more L2 round trips across the dies into every step: 4.9 instead of 3.0 us on
-// 20,000 cells.)  An error that a tile finds ends the run at the next CFL
-// evaluation.  The ledger sums keep k_surface's slots and order: the same bits,
+// `steps` steps of a run of the surface alone in one cooperative launch (fl_run.cuh):
+// a tile's entries, halo list, cell data, wet time and states stay in shared memory
+// and registers.  The ledger sums keep k_surface's slots and order: the same bits,
 // step by step.
 //
 // A launch a step costs a small mesh more than its work.  us a step with 32 (8)
 // steps between CFL evaluations, a launch a step -> here: 1,800 cells 5.4 -> 3.0
 // (6.0 -> 3.9), 20,000 cells 5.7 -> 3.0 (6.7 -> 3.8), 154,568 cells 8.7 -> 4.5
 // (9.6 -> 5.8); what is left is the halo states' round trip and the two phases.
-//
-// Serial numbers: SYNC_STRIDE words a tile, then the last CTA's.  All of them hold
-// the same number between launches (each CTA adds `steps`, also when the run ends
-// early or a wait gives up), so nothing has to be reset.  Co-residency comes from
-// the cooperative launch; every wait is bounded.
-constexpr int SYNC_STRIDE = 8;      // words: a sector each
-constexpr int RUN_THREADS = TILE + 32;
-
-__device__ __forceinline__ bool run_all(bool p) {
-    uint32_t r;
-    asm volatile(
-        "{\n"
-        ".reg .pred pi, po;\n"
-        "setp.ne.u32 pi, %1, 0;\n"
-        "bar.red.and.pred po, 2, %2, pi;\n"
-        "selp.u32 %0, 1, 0, po;\n"
-        "}\n"
-        : "=r"(r)
-        : "r"((uint32_t)p), "n"(RUN_THREADS)
-        : "memory");
-    return r != 0;
-}
-
 template <int KIND>
 __global__ void __launch_bounds__(RUN_THREADS, 4) k_surface_run(const __grid_constant__ SurfArgs a, const RunArgs x, int slot, int steps) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -445,30 +353,8 @@ __global__ void __launch_bounds__(RUN_THREADS, 4) k_surface_run(const __grid_con
         if (tid == 0) publish(mine, base + steps);
         return;
     }
-    if (tile == n_tiles) {  // the run control after the last step
-        if (tid == 0) {
-            s_run = *a.run;
-            s_run.error = 0;  // (first is active; a tile that is ahead may have set it since)
-            s_ctrl[1] = first;
-            for (int k = 1; k < steps && s_ctrl[1].active; ++k)
-                plan_step(&s_run, a.snap_t, a.hy, &s_ctrl[1], false, 0.0f, FL_PHASE_ALL);
-        }
-        bool ok = true;
-        for (int t = tid; t < n_tiles; t += RUN_THREADS) ok = ok && poll_reached(x.serial + (size_t)t * SYNC_STRIDE, base + steps);
-        ok = __syncthreads_and(ok);
-        if (tid == 0) {
-            const int err = ok ? s_run.error : FL_E_TIMEOUT;
-            if (err && atomicCAS(&a.run->error, 0, err) == 0) a.run->error_step = s_run.error ? s_run.error_step : first.step;
-            a.run->t = s_run.t;
-            a.run->next_snap_t = s_run.next_snap_t;
-            a.run->step = s_run.step;
-            a.run->last_dt = s_run.last_dt;
-            a.run->cfl_reused = s_run.cfl_reused;
-            a.run->parity = s_run.parity;
-            a.run->snap_count = s_run.snap_count;
-            if (!s_ctrl[1].active) a.ctrl[0] = a.ctrl[1] = s_ctrl[1];
-            publish(mine, base + steps);
-        }
+    if (tile == n_tiles) {
+        run_last_cta(a.run, a.ctrl, a.snap_t, a.hy, x, n_tiles, base, steps, first, &s_run, &s_ctrl[1]);
         return;
     }
     const TileStage S = stage_at(a, smem, 0);
@@ -490,13 +376,8 @@ __global__ void __launch_bounds__(RUN_THREADS, 4) k_surface_run(const __grid_con
     bool ok = mbar_wait_bounded(bar, 0, COPY_WAIT_NS);
     if (!ok) ok = mbar_wait_bounded(bar, 0, COPY_WAIT_NS);  // none may land after the CTA leaves
 
-    if (tid >= TILE) {  // the ninth warp: the next step's record
-        for (int k = 0; k < steps; ++k) {
-            if (!run_all(ok) || !s_ctrl[k & 1].active) break;
-            if (tid == TILE && k + 1 < steps)
-                plan_step(&s_run, nullptr, a.hy, &s_ctrl[(k + 1) & 1], false, 0.0f, FL_PHASE_ALL);
-            __syncwarp();
-        }
+    if (tid >= TILE) {
+        run_records(ok, steps, a.hy, &s_run, s_ctrl);
         return;
     }
 
@@ -517,19 +398,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 4) k_surface_run(const __grid_con
     const float md = a.md;
     int k = 0;
     for (; k < steps; ++k) {
-        if (k == 0) {
-            const float4 *in = first.parity ? a.state1 : a.state0;
-            for (int j = tid; j < ti.w && ok; j += TILE) S.st[TILE + j] = in[S.hs[j]];
-        } else {  // (a halo cell's bed, the fourth word, stays)
-            const float4 *in = x.exchange + (size_t)((base + k) & 1u) * x.cells;
-            for (int j = tid; j < ti.w && ok; j += TILE) {
-                float4 v;
-                ok = receive_state(in + S.hs[j], base + k, v);
-                S.st[TILE + j].x = v.x;
-                S.st[TILE + j].y = v.y;
-                S.st[TILE + j].z = v.z;
-            }
-        }
+        ok = run_halo(ok, k, first.parity ? a.state1 : a.state0, x, base, S.hs, ti.w, S.st);
         if (!run_all(ok)) {  // the halo states and the step record are in place
             if (tid == 0 && atomicCAS(&a.run->error, 0, FL_E_TIMEOUT) == 0) a.run->error_step = first.step + k;
             break;
@@ -821,36 +690,14 @@ cudaError_t plan_surface_launch(SurfArgs &a, int kind, int device, int *grid, in
 // serial_words: the zeroed words of RunArgs::serial.
 cudaError_t plan_surface_run(const SurfArgs &a, int kind, int device, int *smem_bytes, size_t *serial_words) {
     const void *fn = kind ? (const void *)k_surface_run<1> : (const void *)k_surface_run<0>;
-    const int bytes = a.off_stage + a.stage_bytes;
     *smem_bytes = 0;
     *serial_words = (size_t)(a.n_tiles + 1) * SYNC_STRIDE;
-    int per_sm = 0, sms = 0, most = 0, coop = 0;
-    cudaError_t e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    cudaFuncAttributes at{};
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, fn);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)at.sharedSizeBytes);
-    if (e != cudaSuccess || !coop || bytes > most - (int)at.sharedSizeBytes) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, RUN_THREADS, (size_t)bytes);
-    if (e == cudaSuccess && a.n_tiles + 1 <= per_sm * sms) *smem_bytes = bytes;
-    return e;
+    return run_fits(fn, a.n_tiles + 1, a.off_stage + a.stage_bytes, device, smem_bytes);
 }
 
 cudaError_t launch_surface_run(const SurfArgs &a, int kind, const RunArgs &x, int slot, int steps, int smem_bytes,
                                cudaStream_t stream) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)a.n_tiles + 1);
-    cfg.blockDim = dim3(RUN_THREADS);
-    cfg.dynamicSmemBytes = (size_t)smem_bytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return kind ? cudaLaunchKernelEx(&cfg, k_surface_run<1>, a, x, slot, steps)
-                : cudaLaunchKernelEx(&cfg, k_surface_run<0>, a, x, slot, steps);
+    return launch_run(kind ? k_surface_run<1> : k_surface_run<0>, a, x, slot, steps, a.n_tiles + 1, smem_bytes, stream);
 }
 
 int surface_warps(int grid) { return grid * (TILE / 32); }

@@ -16,9 +16,9 @@ from floodgb.solver import FloodSolver
 from floodgb.synthetic import make_grid_city
 
 
-def _solver(n, per_cell, max_snapshots=None, rain=None):
+def _solver(n, per_cell, max_snapshots=None, rain=None, mode="full_swe"):
     sc = make_grid_city(n=n, size_m=10.0 * n, seed=n, duration_min=3.0)
-    cfg = load_config(None, dict(sc.overrides, **{"solver.snapshot_interval_min": 1.0,
+    cfg = load_config(None, dict(sc.overrides, **{"solver.snapshot_interval_min": 1.0, "solver.surface_step_mode": mode,
                                                "solver.finite_check_interval_steps": 20}))
     topo = sc.city.topologies.surface_topology
     rng = np.random.default_rng(n)
@@ -38,11 +38,13 @@ def _solver(n, per_cell, max_snapshots=None, rain=None):
 
 
 # 32 cells (one partial tile), 512 (two whole tiles), 3,200 (13 tiles, a remainder),
-# 33,800 (133 tiles), 160,178 (626 tiles: more than fit, a launch a step both ways)
+# 33,800 (133 tiles), 160,178 (626 tiles: more than fit, a launch a step both ways);
+# the local-inertial tiles read two rings of neighbours
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [4, 16, 40, 130, 283])
 @pytest.mark.parametrize("per_cell", [False, True])
-def test_a_run_equals_the_same_run_step_by_step(n, per_cell):
+@pytest.mark.parametrize("mode", ["full_swe", "local_inertial"])
+def test_a_run_equals_the_same_run_step_by_step(n, per_cell, mode):
     from floodgb.build import build_library
 
     build_library()
@@ -51,7 +53,7 @@ def test_a_run_equals_the_same_run_step_by_step(n, per_cell):
         pytest.skip("no CUDA device")
     out = []
     for single in (False, True):
-        s = _solver(n, per_cell)
+        s = _solver(n, per_cell, mode=mode)
         try:
             if single:
                 for _ in range(70):  # past two CFL evaluations
