@@ -69,7 +69,7 @@ cudaError_t launch_surcharge(const SurchargeArgs &a, int slot, cudaStream_t stre
 cudaError_t launch_li(const LiArgs &a, int kind, int slot, int plan_next, int sms, cudaStream_t stream);
 int li_cell_blocks(int32_t C);
 cudaError_t plan_li_tiles(LiTileArgs &a, int kind, int device, int *grid, int *smem_bytes);
-cudaError_t plan_surface_run(const SurfArgs &a, int kind, int device, int *smem_bytes, size_t *serial_words);
+cudaError_t plan_surface_run(const SurfArgs &a, int kind, int surf_grid, int device, int *smem_bytes, size_t *serial_words);
 cudaError_t launch_surface_run(const SurfArgs &a, int kind, const RunArgs &x, int slot, int steps, int smem_bytes,
                                cudaStream_t stream);
 cudaError_t plan_li_run(const LiTileArgs &a, int kind, int tiles_grid, int device, int *smem_bytes, size_t *serial_words);
@@ -798,7 +798,7 @@ static int create_impl(const FlMeshDesc *mesh, const FlDrainDesc *drain, const F
     if (!s->li_mode && M == 1 && !drain && run_interval(p.cfl_update_interval_steps)) {
         size_t words = 0;
         int bytes = 0;
-        FL_CUDA(plan_surface_run(s->sa, s->kind, device, &bytes, &words));
+        FL_CUDA(plan_surface_run(s->sa, s->kind, s->surf_grid, device, &bytes, &words));
         std::vector<std::pair<int32_t, int32_t>> ranges;
         for (const int4 &ti : L.tile_info) ranges.emplace_back(ti.z, ti.w);
         if (bytes && (rc = setup_run(s, ranges, L.halo_src, bytes, words))) return rc;

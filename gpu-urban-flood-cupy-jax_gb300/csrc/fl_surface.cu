@@ -686,12 +686,17 @@ cudaError_t plan_surface_launch(SurfArgs &a, int kind, int device, int *grid, in
 }
 
 // Whether k_surface_run can run the mesh: every tile's CTA and the planner resident
-// at once (on 152 SMs up to 607 tiles, 155,000 cells).  *smem_bytes 0: it cannot.
-// serial_words: the zeroed words of RunArgs::serial.
-cudaError_t plan_surface_run(const SurfArgs &a, int kind, int device, int *smem_bytes, size_t *serial_words) {
+// at once (on 152 SMs up to 607 tiles, 155,000 cells), and a CTA per tile of
+// k_surface's grid too.  The ledger has a slot per warp of that grid, and a single
+// step adds a CTA's tiles up before its slot: with fewer CTAs than tiles (k_surface
+// keeps two stages in shared memory, so wide halos cost it a CTA an SM that the run
+// kernel still has) the run kernel would have slots that do not exist.
+// *smem_bytes 0: it cannot.  serial_words: the zeroed words of RunArgs::serial.
+cudaError_t plan_surface_run(const SurfArgs &a, int kind, int surf_grid, int device, int *smem_bytes, size_t *serial_words) {
     const void *fn = kind ? (const void *)k_surface_run<1> : (const void *)k_surface_run<0>;
     *smem_bytes = 0;
     *serial_words = (size_t)(a.n_tiles + 1) * SYNC_STRIDE;
+    if (a.n_tiles + 1 != surf_grid) return cudaSuccess;
     return run_fits(fn, a.n_tiles + 1, a.off_stage + a.stage_bytes, device, smem_bytes);
 }
 
