@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 3) k_li_run(const __grid_constant
     bool ok = mbar_wait_bounded(bar, 0, LT_WAIT_NS);
     if (!ok) ok = mbar_wait_bounded(bar, 0, LT_WAIT_NS);  // none may land after the CTA leaves
     if (tid >= TILE) {
-        run_records(ok, steps, q.hy, &s_run, s_ctrl);
+        run_records(ok, steps, q.hy, q.run, n_tiles, &s_run, s_ctrl);
         return;
     }
 
@@ -641,9 +641,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 3) k_li_run(const __grid_constant
         lt_sync();  // the donor factors are in place
         if (c < q.C) {
             const float4 st = S.st[tid];
-            if (s.check_finite && !isfinite(st.x)) {
-                if (atomicCAS(&q.run->error, 0, FL_E_NONFINITE) == 0) q.run->error_step = s.step;
-            }
+            if (s.check_finite && !isfinite(st.x)) run_non_finite(q.run, s.step);
             float hn = 0.0f, hun = 0.0f, hvn = 0.0f;
             if (!do_surface) {
                 hn = st.x; hun = st.y; hvn = st.z;

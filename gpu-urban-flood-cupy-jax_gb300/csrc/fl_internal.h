@@ -85,6 +85,10 @@ struct RunCtrl {
     int32_t cfl_interval, finite_interval;
     int32_t hyeto_n;
     int32_t pad;
+    // runs in one launch (fl_run.cuh): finite checks that a tile has finished, counted over
+    // all tiles, at the start of the launch and now; ~step of the first failed one (0: none)
+    uint32_t checks_base, checks;
+    uint64_t first_bad;
 };
 
 struct HyetoView {

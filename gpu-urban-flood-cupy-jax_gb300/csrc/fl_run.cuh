@@ -13,8 +13,12 @@
 // get the same ones), and the last CTA, which has no tile, writes the run control's
 // end back when every other CTA has copied its start.  (One planner for all put two
 // more L2 round trips across the dies into every step: 4.9 instead of 3.0 us on
-// 20,000 cells.)  An error that a tile finds ends the run at the next CFL
-// evaluation.
+// 20,000 cells.)
+//
+// A step that checks for non-finite depths ends the run as a launch a step does, the
+// step after it still done: each CTA counts its finished check, and the record of
+// the step after next is planned when all have (a step later, so the wait is rarely
+// one), on the first failed check by then -- the same in every CTA.
 //
 // Serial numbers: SYNC_STRIDE words a tile, then the last CTA's.  All of them hold
 // the same number between launches (each CTA adds `steps`, also when the run ends
@@ -89,6 +93,23 @@ __device__ __forceinline__ bool receive_state(const float4 *p, uint32_t serial, 
     }
 }
 
+// A thread found a non-finite depth in a step's finite check.
+__device__ __forceinline__ void run_non_finite(RunCtrl *run, int64_t step) {
+    atomicMax((unsigned long long *)&run->first_bad, ~(unsigned long long)step);
+    atomicCAS(&run->error, 0, FL_E_NONFINITE);
+}
+
+// Bounded wait until all tiles' checks up to `step` are finished (`count` in all); a
+// failed one among them goes into the run control that plans (a later step's, which
+// a tile that is ahead may have recorded, does not: some CTAs would see it, others not).
+__device__ __forceinline__ bool run_checked(RunCtrl *run, uint32_t count, int64_t step, RunCtrl *s_run) {
+    if (!poll_reached(&run->checks, count)) return false;
+    unsigned long long bad;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(bad) : "l"(&run->first_bad) : "memory");
+    if (bad >= ~(unsigned long long)step) s_run->error = FL_E_NONFINITE;
+    return true;
+}
+
 __device__ __forceinline__ bool run_all(bool p) {
     uint32_t r;
     asm volatile(
@@ -110,13 +131,25 @@ __device__ __forceinline__ void run_last_cta(RunCtrl *run, StepCtrl *ctrl, doubl
                                              int n_tiles, uint32_t base, int steps, const StepCtrl &first, RunCtrl *s_run,
                                              StepCtrl *s_rec) {
     const int tid = threadIdx.x;
+    bool ok = true;
     if (tid == 0) {
         *s_run = *run;
         s_run->error = 0;  // (first is active; a tile that is ahead may have set it since)
         *s_rec = first;
-        for (int k = 1; k < steps && s_rec->active; ++k) plan_step(s_run, snap_t, hy, s_rec, false, 0.0f, FL_PHASE_ALL);
+        uint32_t count = s_run->checks_base;
+        bool check = first.check_finite != 0, before = false;  // of the records k - 1 and k - 2
+        int64_t at = first.step, at_before = 0;
+        for (int k = 1; k < steps && s_rec->active && ok; ++k) {  // (as run_records)
+            if (before) ok = run_checked(run, count += n_tiles, at_before, s_run);
+            before = check;
+            at_before = at;
+            plan_step(s_run, snap_t, hy, s_rec, false, 0.0f, FL_PHASE_ALL);
+            check = s_rec->check_finite != 0;
+            at = s_rec->step;
+        }
+        if (before && s_rec->active) count += n_tiles;  // counted in the last step, which plans none
+        s_run->checks_base = count;
     }
-    bool ok = true;
     for (int t = tid; t < n_tiles; t += RUN_THREADS) ok = ok && poll_reached(x.serial + (size_t)t * SYNC_STRIDE, base + steps);
     ok = __syncthreads_and(ok);
     if (tid == 0) {
@@ -129,17 +162,32 @@ __device__ __forceinline__ void run_last_cta(RunCtrl *run, StepCtrl *ctrl, doubl
         run->cfl_reused = s_run->cfl_reused;
         run->parity = s_run->parity;
         run->snap_count = s_run->snap_count;
+        run->checks_base = s_run->checks_base;
         if (!s_rec->active) ctrl[0] = ctrl[1] = *s_rec;
         publish(x.serial + (size_t)n_tiles * SYNC_STRIDE, base + steps);
     }
 }
 
 // A tile's ninth warp: the next step's record during each step.
-__device__ __forceinline__ void run_records(bool ok, int steps, const HyetoView &hy, RunCtrl *s_run, StepCtrl *s_ctrl) {
+__device__ __forceinline__ void run_records(bool ok, int steps, const HyetoView &hy, RunCtrl *run, int n_tiles, RunCtrl *s_run,
+                                            StepCtrl *s_ctrl) {
+    uint32_t count = s_run->checks_base;
+    bool check = false;  // of the step before
+    int64_t at = 0;
     for (int k = 0; k < steps; ++k) {
-        if (!run_all(ok) || !s_ctrl[k & 1].active) break;
-        if (threadIdx.x == TILE && k + 1 < steps)
-            plan_step(s_run, nullptr, hy, &s_ctrl[(k + 1) & 1], false, 0.0f, FL_PHASE_ALL);
+        if (!run_all(ok) || !s_ctrl[k & 1].active) break;  // (the CTA has finished step k - 1)
+        if (threadIdx.x == TILE) {
+            if (check) {
+                count += n_tiles;
+                asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&run->checks) : "memory");
+            }
+            if (k + 1 < steps) {
+                if (check) ok = run_checked(run, count, at, s_run);
+                check = s_ctrl[k & 1].check_finite != 0;
+                at = s_ctrl[k & 1].step;
+                plan_step(s_run, nullptr, hy, &s_ctrl[(k + 1) & 1], false, 0.0f, FL_PHASE_ALL);
+            }
+        }
         __syncwarp();
     }
 }

@@ -251,6 +251,8 @@ struct FlSolver {
 static int sync_run(FlSolver *s, cudaStream_t st) {
     FL_CUDA(cudaMemcpyAsync(s->run_h, s->run, sizeof(RunCtrl), cudaMemcpyDeviceToHost, st));
     FL_CUDA(cudaStreamSynchronize(st));
+    RunCtrl &r = *s->run_h;  // (a run in one launch records the first failed check only there)
+    if (r.error == FL_E_NONFINITE && r.first_bad) r.error_step = (int64_t)~r.first_bad;
     return FL_OK;
 }
 
@@ -535,8 +537,7 @@ static int setup_run(FlSolver *s, const std::vector<std::pair<int32_t, int32_t>>
     return FL_OK;
 }
 
-// With a few steps between CFL evaluations there is little to keep resident, and a
-// run that meets a non-finite depth goes on up to the next evaluation.
+// With a few steps between CFL evaluations there is little to keep resident.
 static bool run_interval(int32_t steps) { return steps >= 8 && steps <= 256; }
 
 // Tiles of the one-launch local-inertial step: entries, rings and areas per

@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 4) k_surface_run(const __grid_con
     if (!ok) ok = mbar_wait_bounded(bar, 0, COPY_WAIT_NS);  // none may land after the CTA leaves
 
     if (tid >= TILE) {
-        run_records(ok, steps, a.hy, &s_run, s_ctrl);
+        run_records(ok, steps, a.hy, a.run, n_tiles, &s_run, s_ctrl);
         return;
     }
 
@@ -416,9 +416,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 4) k_surface_run(const __grid_con
         compute_sync();
         if (c < a.C) {
             const float4 st = S.st[tid];
-            if (s.check_finite && !isfinite(st.x)) {
-                if (atomicCAS(&a.run->error, 0, FL_E_NONFINITE) == 0) a.run->error_step = s.step;
-            }
+            if (s.check_finite && !isfinite(st.x)) run_non_finite(a.run, s.step);
             float hn = 0.0f, hun = 0.0f, hvn = 0.0f;
             if (!do_surface) {
                 hn = st.x; hun = st.y; hvn = st.z;

@@ -213,7 +213,9 @@ FL_API int fl_reset_clock(FlSolver *solver, void *stream);
 /* Advance the adaptive loop of run_simulation (engine.py:219-344) until the
  * simulated time reaches min(t_target_s, duration) or max_steps more steps
  * ran (FL_E_STEP_CAP).  The loop runs on the device as CUDA-graph chunks of
- * cfl_update_interval_steps steps; the host only polls progress. */
+ * cfl_update_interval_steps steps; the host only polls progress.  A finite
+ * check that fails in step s (counted from 0; FL_E_NONFINITE, error_step s)
+ * ends the run; step s + 1 may have been planned beside it and is then done. */
 FL_API int fl_run(FlSolver *solver, double t_target_s, int64_t max_steps, void *stream);
 
 /* One step with an explicit dt and a phase set: step_triangular_surface
