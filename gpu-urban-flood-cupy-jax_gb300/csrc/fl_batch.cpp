@@ -246,8 +246,9 @@ static int batch_create_impl(int32_t n, const FlMeshDesc *meshes, const FlForcin
     if ((rc = b->alloc(&b->hmax, Cp)) || (rc = b->alloc(&b->wet, Cp)) || (rc = b->alloc(&tile_min, (size_t)b->tiles)) ||
         (rc = b->alloc(&tile_led, 2 * (size_t)b->tiles * SURF_TERMS)) || (rc = b->alloc(&b->run, (size_t)n)) ||
         (rc = b->alloc(&b->ctrl, (size_t)n * 2)) || (rc = b->alloc(&b->list, 2)) ||
-        (rc = b->alloc(&b->ledger, (size_t)n * SURF_TERMS)))
+        (rc = b->alloc(&b->ledger, (size_t)n * SURF_TERMS)) || (rc = b->alloc(&b->pa.arrived, 1)))
         return rc;
+    FB_CUDA(cudaMemset(b->pa.arrived, 0, sizeof(uint32_t)));
     FB_CUDA(cudaMemset(tile_led, 0, 2 * sizeof(float) * (size_t)b->tiles * SURF_TERMS));
     FB_CUDA(cudaMemset(b->list, 0, 2 * sizeof(BatchList)));
     int32_t largest = 1;

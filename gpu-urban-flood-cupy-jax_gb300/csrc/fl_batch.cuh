@@ -70,6 +70,7 @@ struct PlanArgs {
     const float *tile_led;
     float2 *ledger;               // [n * SURF_TERMS] float-float running sums
     BatchList *list;              // [2]
+    uint32_t *arrived;            // CTAs that are done with a step that checks for non-finite depths
     int32_t n, max_snaps, n_tiles;
 };
 

@@ -27,6 +27,9 @@
 // per scenario, and add up the previous step's ledger terms (lists and terms have
 // two buffers); then only one step in a CFL interval has a planning launch (300 s of 16 scenarios,
 // 1.64 M cells: 41.1 -> 38.0 ms; 90 s of six, 27,000 cells: 2.08 -> 1.59 ms).
+// A scenario whose step checks for non-finite depths ends with that step if the
+// check fails, so its next step is planned when the step is done: by the launch's
+// last CTA, without a wait of any other.
 //
 // k_cfl_batch: the CFL minima of every tile's initial state (before step 0).
 #include "fl_batch.cuh"
@@ -132,18 +135,22 @@ __device__ __forceinline__ void list_entry(const PlanArgs &a, int b, BatchList *
         e.tile0 = t0;
         e.cells = a.scen_cells[b];
         list->e[b] = e;
+    } else {
+        list->e[b].flags = 0;
     }
 }
 
 // One warp, beside the surface CTAs of the step in `slot`: scenario b's ledger
 // terms of the step before (k_plan_batch's sums, its four warps one after the
 // other) and its next step's record and list entry.  s_run: a run record and a
-// step record of shared memory.  An error that this step's surface CTAs find is
-// seen one step later than by k_plan_batch; the error and its step are theirs.
+// step record of shared memory.
+constexpr int PLAN_SMEM = 384;
+static_assert(sizeof(RunCtrl) % 8 == 0 && sizeof(RunCtrl) + sizeof(StepCtrl) <= PLAN_SMEM, "a warp's records in shared memory");
+
 __device__ __noinline__ void plan_ahead(const PlanArgs &a, int b, int lane, int slot, int mode, RunCtrl *s_run) {
     StepCtrl *rec = &a.ctrl[2 * b + (slot ^ 1)], *s_next = (StepCtrl *)(s_run + 1);
     RunCtrl *run = &a.run[b];
-    for (int i = lane; i < (int)(sizeof(RunCtrl) / 4); i += 32) ((uint32_t *)s_run)[i] = ((const uint32_t *)run)[i];
+    for (int i = lane; i < (int)(sizeof(RunCtrl) / 4); i += 32) ((uint32_t *)s_run)[i] = __ldcg((const uint32_t *)run + i);
     const bool had_step = rec->active != 0;  // (the record of the step before, overwritten below)
     if (mode & BP_LEDGER) {
         const float4 *led = (const float4 *)a.tile_led + (size_t)(slot ^ 1) * a.n_tiles;
@@ -198,6 +205,28 @@ __device__ __noinline__ void plan_ahead(const PlanArgs &a, int b, int lane, int 
     }
 }
 
+// The first T threads of a CTA that is done with a step in which some scenario
+// checks for non-finite depths: the last CTA plans those scenarios' next step.
+// smem: T / 32 records of PLAN_SMEM bytes and a word.
+template <int T>
+__device__ __noinline__ void plan_checked(const PlanArgs &a, int slot, unsigned char *smem) {
+    volatile uint32_t *s_last = (volatile uint32_t *)(smem + T / 32 * PLAN_SMEM);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        __threadfence();  // (this CTA's errors, ordered by the barrier before the call)
+        const bool last = atomicAdd(a.arrived, 1u) == gridDim.x - 1;
+        __threadfence();
+        if (last) *a.arrived = 0u;
+        *s_last = last;
+    }
+    batch_sync<T>();
+    if (!*s_last) return;
+    for (int b = warp; b < a.n; b += T / 32) {
+        if (a.list[slot].e[b].flags & BF_FINITE) plan_ahead(a, b, lane, slot, BP_NEXT, (RunCtrl *)(smem + warp * PLAN_SMEM));
+        __syncwarp();
+    }
+}
+
 // Four CTAs of 256-cell tiles an SM (seven of 128): 56 registers.
 template <int KIND, int T>
 __global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(const __grid_constant__ BatchArgs a, const __grid_constant__ PlanArgs p,
@@ -216,7 +245,17 @@ __global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(cons
         pdl_wait();
         if (a.early) pdl_launch_dependents();
         const int b = ((int)blockIdx.x - a.ctas) * W + (tid >> 5);
-        if (tid < T && b < p.n) plan_ahead(p, b, tid & 31, slot, mode, (RunCtrl *)(smem + (tid >> 5) * 384));
+        int check = 0;
+        for (int i = tid; i < p.n; i += T + 32) check |= a.list[slot].e[i].flags & BF_FINITE;
+        const bool checked = __syncthreads_or(check) && (mode & BP_NEXT);
+        if (tid >= T) return;
+        if (b < p.n)
+            plan_ahead(p, b, tid & 31, slot, a.list[slot].e[b].flags & BF_FINITE ? mode & ~BP_NEXT : mode,
+                       (RunCtrl *)(smem + (tid >> 5) * PLAN_SMEM));
+        if (checked) {
+            batch_sync<T>();
+            plan_checked<T>(p, slot, smem);
+        }
         return;
     }
     const uint32_t bar_base = smem_addr(s_bar);
@@ -237,7 +276,11 @@ __global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(cons
     const int n = a.n_scen;
     const BatchList *list = a.list + slot;
     float *tile_led = a.tile_led + (size_t)slot * a.n_tiles * SURF_TERMS;
-    for (int i = tid; i < n; i += T + 32) s_ent[i] = list->e[i];
+    int check = 0;
+    for (int i = tid; i < n; i += T + 32) {
+        s_ent[i] = list->e[i];
+        check |= s_ent[i].flags & BF_FINITE;
+    }
     if (tid < 32) {  // running sums of the tile counts (an inactive scenario's range is empty)
         constexpr int PER = MAX_SCEN / 32;
         int c[PER], sum = 0;
@@ -259,7 +302,7 @@ __global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(cons
         }
         if (tid == 31 && n == MAX_SCEN) s_prefix[n] = before;
     }
-    __syncthreads();  // the last block-wide barrier: the roles split here
+    const bool checked = __syncthreads_or(check) && (mode & BP_NEXT);  // the last block-wide barrier: the roles split here
     const int total = s_prefix[n];
     const int G = a.ctas;
     const BStage<T> S0 = bstage_at<T>(a, smem, 0), S1 = bstage_at<T>(a, smem, 1);
@@ -341,7 +384,8 @@ __global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(cons
                  mbar_wait_bounded(bar_base + 16u + 8u * st_i, (i >> 1) & 1u, BATCH_WAIT_NS);
         if (!batch_all<T>(ok)) {  // also: every warp's partials of the previous tile are in place
             if (tid == 0) fail();
-            return;  // the producer waits out its own copies
+            done_t = -1;
+            break;  // the producer waits out its own copies
         }
         if (tid == 0 && done_t >= 0) finish_tile(done_t, done_cfl);
         const BatchEntry &E = s_ent[s_kt[2 * st_i]];
@@ -430,10 +474,11 @@ __global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(cons
         done_t = t;
         done_cfl = (flags & BF_CFL) != 0;
     }
-    if (done_t >= 0) {
+    if (done_t >= 0 || checked) {
         batch_sync<T>();
-        if (tid == 0) finish_tile(done_t, done_cfl);
+        if (tid == 0 && done_t >= 0) finish_tile(done_t, done_cfl);
     }
+    if (checked) plan_checked<T>(p, slot, smem);
 }
 
 // CFL minima of every tile's state before the first step (all scenarios'
