@@ -351,12 +351,14 @@ class MPNN:
 
         ws = self.ws
         C, E, L = g.C, g.E, self.n_layers
+        x_bf, dy = ops.node_inputs(x_bf, g, ws.y.device), ops.output_gradients(dy, g, ws.y.device)
         if max(getattr(g, "max_in", MAX_IN + 1), getattr(g, "max_out", MAX_IN + 1)) <= MAX_IN and L <= MAX_LAYERS:
             ops.mpnn_backward(self, g, x_bf, dy, ws.fused())
             for (_, e2), dagg in zip(self.edge, ws.dagg_f32):
                 e2.gb.add_(dagg.sum(0))
             return
         ws.products()
+        dy = dy if dy.stride(1) == 1 else dy.contiguous()
         # decoder
         a, b = self.dec
         ops.cast_bf16(dy, ws.dy_bf)

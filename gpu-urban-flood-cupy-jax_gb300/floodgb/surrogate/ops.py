@@ -84,16 +84,50 @@ def _pointers(tensors, n):
     return (C.c_void_p * max(n, 1))(*[ts[k % len(ts)] for k in range(n)])
 
 
-def mpnn_forward(net, g, x, ws):
-    """The network's forward pass over graph g (at most three edges into a
-    cell) into workspace ws; hidden activations are kept where ws has them."""
+def _padded_rows(t, rows, cols, dtype, device, name):
+    """t as `cols` wide rows in memory: a narrower view of rows that are (the
+    padding belongs to its storage) is widened.  Anything else is refused."""
+
+    if t.dtype != dtype or t.dim() != 2:
+        raise ValueError(f"{name} must be a matrix of {dtype}, got {t.dtype} with {t.dim()} dimensions")
+    if t.device != device:
+        raise ValueError(f"{name} are on {t.device}, expected {device}")
+    if t.shape == (rows, cols):
+        return t
+    if t.shape[0] == rows and t.shape[1] < cols and t.stride(1) == 1 and t.stride(0) >= cols:
+        held = t.untyped_storage().nbytes() // t.element_size() - t.storage_offset()
+        if (rows - 1) * t.stride(0) + cols <= held:
+            return t.as_strided((rows, cols), t.stride())
+    if t.shape[0] < rows or t.shape[1] < cols:
+        raise ValueError(f"{name} have shape {tuple(t.shape)}, expected ({rows}, {cols})")
+    return t[:rows, :cols]
+
+
+def node_inputs(x, g, device):
+    """x checked as bf16 node inputs of graph g."""
 
     import torch
 
     if x.dtype != torch.bfloat16 or x.dim() != 2 or x.stride(1) != 1:
         raise ValueError("A segments must be row-major bf16 matrices")
-    if x.shape[0] != g.C or x.shape[1] < 64:
+    if x.shape[0] != g.C:
         raise ValueError(f"inputs have shape {tuple(x.shape)}, expected ({g.C}, 64)")
+    return _padded_rows(x, g.C, 64, torch.bfloat16, device, "inputs")
+
+
+def output_gradients(dy, g, device):
+    """dy checked as fp32 gradients of graph g's outputs."""
+
+    import torch
+
+    return _padded_rows(dy, g.C, 64, torch.float32, device, "output gradients")
+
+
+def mpnn_forward(net, g, x, ws):
+    """The network's forward pass over graph g (at most three edges into a
+    cell) into workspace ws; hidden activations are kept where ws has them."""
+
+    x = node_inputs(x, g, ws.y.device)
     L = net.n_layers
     d = N.FlMpnnForwardDesc()
     d.cells, d.edges, d.layers = g.C, g.E, L
@@ -129,9 +163,9 @@ def _dense_grads(layers):
 
 def mpnn_backward(net, g, x, dy, ws):
     """Add the parameter gradients for the output gradient dy (fp32 [C, 64])
-    of the forward pass whose activations ws holds."""
+    of the forward pass whose activations ws holds (x, dy: checked by the caller)."""
 
-    if dy.stride(1) != 1 or dy.stride(0) % 8 or dy.data_ptr() % 32:
+    if dy.stride(1) != 1 or dy.stride(0) < 64 or dy.stride(0) % 8 or dy.data_ptr() % 32:
         ws.dy_f32.copy_(dy)
         dy = ws.dy_f32
     L = net.n_layers
