@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstring>
 #include <limits>
+#include <memory>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -1615,13 +1616,32 @@ FL_API int fl_time_kernel(FlSolver *s, int32_t kernel, int32_t reps, void *strea
     c.phases = FL_PHASE_ALL;
     c.step = r.step;
     FL_CUDA(cudaMemcpyAsync(&s->ctrl[0], &c, sizeof(StepCtrl), cudaMemcpyHostToDevice, st));
-    auto launch = [&](cudaStream_t ls) -> cudaError_t {
+    const int chain = std::min(reps, 32);
+    // k_nodes and k_network fetch their ledger slots before their wait for the kernel
+    // before them.  In a step that is another kernel; here each launch of a chain gets
+    // slots of its own, or it would read those that the one before still adds to.
+    const size_t n_led = kernel == 1 ? s->n_led_1 : kernel == 2 ? s->n_led_2 : 0;
+    float2 *slots = nullptr;
+    if (n_led) {
+        FL_CUDA(cudaMalloc((void **)&slots, sizeof(float2) * n_led * chain));
+        FL_CUDA(cudaMemsetAsync(slots, 0, sizeof(float2) * n_led * chain, st));
+    }
+    std::unique_ptr<float2, cudaError_t (*)(void *)> slots_owner(slots, cudaFree);
+    auto launch = [&](cudaStream_t ls, int i) -> cudaError_t {
         switch (kernel) {
             case 0:
                 return s->li_mode ? launch_inertial(s, 0, 0, ls)
                                   : launch_surface(s->sa, s->kind, 0, 0, s->surf_grid, s->surf_smem, ls);
-            case 1: return launch_nodes(s->nd, 0, ls);
-            case 2: return launch_network(s->nw, 0, ls);
+            case 1: {
+                NodeArgs a = s->nd;
+                a.ledger = slots + n_led * i;
+                return launch_nodes(a, 0, ls);
+            }
+            case 2: {
+                NetArgs a = s->nw;
+                a.ledger = slots + n_led * i;
+                return launch_network(a, 0, ls);
+            }
             case 4: return launch_links(s->lk, 0, ls);
             case 5: return launch_donor(s->dn, 0, ls);
             default: {
@@ -1635,13 +1655,12 @@ FL_API int fl_time_kernel(FlSolver *s, int32_t kernel, int32_t reps, void *strea
     // A chain of launches captured as one graph and replayed, as in the step
     // loop: the time is the kernels' own, not the host's launch rate or a
     // graph launch's.
-    const int chain = std::min(reps, 32);
     const int replays = (reps + chain - 1) / chain;
     cudaGraph_t g = nullptr;
     cudaGraphExec_t ge = nullptr;
     FL_CUDA(cudaStreamBeginCapture(s->cap_stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t le = cudaSuccess;
-    for (int i = 0; i < chain && le == cudaSuccess; ++i) le = launch(s->cap_stream);
+    for (int i = 0; i < chain && le == cudaSuccess; ++i) le = launch(s->cap_stream, i);
     const cudaError_t ce = cudaStreamEndCapture(s->cap_stream, &g);
     cudaError_t err = le != cudaSuccess ? le : ce;
     if (err == cudaSuccess) err = cudaGraphInstantiate(&ge, g, 0);

@@ -296,7 +296,8 @@ FL_API int fl_plan_tiles(const FlMeshDesc *mesh, int64_t *tiles);
  * as in the step loop (the surface and the drainage kernels as
  * programmatic dependents of the launch before them), so the time per launch
  * is the kernel's own in-loop cost, not a graph launch's.  The clock is not
- * advanced but the state buffers are overwritten (reset before the next run).
+ * advanced but the state buffers are overwritten (reset before the next run),
+ * and kernel 0 adds to the surface terms of the ledger.
  * No reference counterpart: it is the measurement hook for the roofline. */
 FL_API int fl_time_kernel(FlSolver *solver, int32_t kernel, int32_t reps, void *stream, double *ms_per_launch);
 
