@@ -17,6 +17,7 @@
 #include <mutex>
 
 #include "fl_device.cuh"
+#include "fl_run.cuh"
 
 namespace fl {
 
@@ -120,23 +121,38 @@ extern "C" FL_API int fl_stable_timestep_noalloc(const float *char_len, const fl
 // ------------------------------------------------------------------ wait self-test
 namespace fl {
 
-// One warp waits on an mbarrier that nothing arrives on, with the same bounded
-// wait the surface, batch and GEMM kernels use; it must give up after
-// limit_ns and report FL_E_TIMEOUT (the context stays usable).
-__global__ void k_wait_selftest(uint64_t limit_ns, int32_t *status, uint64_t *elapsed_ns) {
+// A warp a kind of bounded wait: on an mbarrier that nothing arrives on (as the
+// surface, batch and tensor-core kernels wait for copies), on a serial number that is
+// not reached and for a state that is not sent (as a run in one launch waits for other
+// tiles).  Each must give up after limit_ns and say so; the context stays usable.
+constexpr int WAIT_KINDS = 3;
+
+struct WaitResult {
+    float4 state;
+    uint64_t ns;
+    uint32_t serial;
+    int32_t status;
+};
+
+__global__ void k_wait_selftest(uint64_t limit_ns, WaitResult *r) {
     __shared__ __align__(8) uint64_t bar;
     const uint32_t b = smem_addr(&bar);
     if (threadIdx.x == 0) {
         mbar_init(b, 1);
         mbar_fence_init();
     }
-    __syncwarp();
+    __syncthreads();
+    const int kind = threadIdx.x >> 5;
+    WaitResult *mine = r + kind;
+    float4 v;
     const uint64_t t0 = global_ns();
-    const bool ok = mbar_wait_bounded(b, 0, limit_ns);
+    const bool ok = kind == 0   ? mbar_wait_bounded(b, 0, limit_ns)
+                    : kind == 1 ? poll_reached(&mine->serial, 1u, limit_ns)
+                                : receive_state(&mine->state, 1u, v, limit_ns);
     const uint64_t t1 = global_ns();
-    if (threadIdx.x == 0) {
-        *status = ok ? FL_OK : FL_E_TIMEOUT;
-        *elapsed_ns = t1 - t0;
+    if ((threadIdx.x & 31) == 0) {
+        mine->status = ok ? FL_OK : FL_E_TIMEOUT;
+        mine->ns = t1 - t0;
     }
 }
 
@@ -146,22 +162,23 @@ extern "C" FL_API int fl_wait_selftest(double limit_s, int32_t *status, double *
     using namespace fl;
     if (!status || !elapsed_s || !(limit_s > 0.0) || limit_s > 5.0)
         return set_error(FL_E_INVALID, "fl_wait_selftest: limit must be in (0, 5] s");
-    int32_t *d_status = nullptr;
-    uint64_t *d_el = nullptr;
-    cudaError_t e = cudaMalloc(&d_status, sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&d_el, sizeof(uint64_t));
-    if (e != cudaSuccess) {
-        cudaFree(d_status);
-        return set_error(FL_E_NOMEM, "fl_wait_selftest: %s", cudaGetErrorString(e));
+    WaitResult *d = nullptr, h[WAIT_KINDS];
+    cudaError_t e = cudaMalloc(&d, sizeof(h));
+    if (e != cudaSuccess) return set_error(FL_E_NOMEM, "fl_wait_selftest: %s", cudaGetErrorString(e));
+    e = cudaMemset(d, 0, sizeof(h));
+    if (e == cudaSuccess) {
+        k_wait_selftest<<<1, 32 * WAIT_KINDS>>>((uint64_t)(limit_s * 1e9), d);
+        e = cudaGetLastError();
     }
-    k_wait_selftest<<<1, 32>>>((uint64_t)(limit_s * 1e9), d_status, d_el);
-    uint64_t el = 0;
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpy(status, d_status, sizeof(int32_t), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(&el, d_el, sizeof(uint64_t), cudaMemcpyDeviceToHost);
-    cudaFree(d_status);
-    cudaFree(d_el);
+    if (e == cudaSuccess) e = cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost);
+    cudaFree(d);
     if (e != cudaSuccess) return set_error(FL_E_CUDA, "fl_wait_selftest: %s", cudaGetErrorString(e));
+    *status = FL_E_TIMEOUT;
+    uint64_t el = h[0].ns;
+    for (const WaitResult &r : h) {
+        if (r.status != FL_E_TIMEOUT) *status = r.status;
+        if (r.ns < el) el = r.ns;
+    }
     *elapsed_s = (double)el * 1e-9;
     return FL_OK;
 }

@@ -36,7 +36,7 @@ constexpr int RUN_THREADS = TILE + 32;
 
 
 // Bounded poll: *p has reached v (serial numbers; they may wrap).
-__device__ __forceinline__ bool poll_reached(const uint32_t *p, uint32_t v) {
+__device__ __forceinline__ bool poll_reached(const uint32_t *p, uint32_t v, uint64_t limit_ns = RUN_WAIT_NS) {
     uint64_t t0 = 0;
     for (int i = 0;; ++i) {
         uint32_t x;
@@ -44,7 +44,7 @@ __device__ __forceinline__ bool poll_reached(const uint32_t *p, uint32_t v) {
         if ((int32_t)(x - v) >= 0) return true;
         if ((i & 63) == 63) {
             if (t0 == 0) t0 = global_ns();
-            else if (global_ns() - t0 > RUN_WAIT_NS) return false;
+            else if (global_ns() - t0 > limit_ns) return false;
         }
     }
 }
@@ -67,7 +67,7 @@ __device__ __forceinline__ void send_state(float4 *p, float h, float hu, float h
 }
 
 // Bounded poll for the state with this serial number.
-__device__ __forceinline__ bool receive_state(const float4 *p, uint32_t serial, float4 &v) {
+__device__ __forceinline__ bool receive_state(const float4 *p, uint32_t serial, float4 &v, uint64_t limit_ns = RUN_WAIT_NS) {
     uint64_t t0 = 0;
     for (int i = 0;; ++i) {
         uint64_t lo, hi;
@@ -88,7 +88,7 @@ __device__ __forceinline__ bool receive_state(const float4 *p, uint32_t serial, 
         }
         if ((i & 63) == 63) {
             if (t0 == 0) t0 = global_ns();
-            else if (global_ns() - t0 > RUN_WAIT_NS) return false;
+            else if (global_ns() - t0 > limit_ns) return false;
         }
     }
 }

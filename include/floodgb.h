@@ -524,9 +524,10 @@ FL_API int fl_adam_all(const FlAdamTensor *tensors, int32_t n, float lr, float b
                        float weight_decay, void *stream);
 
 /* Self-test of the bounded device waits (no reference counterpart): one
- * warp waits on an mbarrier that nothing arrives on; *status receives
- * FL_E_TIMEOUT once the wait gives up after limit_s (at most 5 s), and the
- * device stays usable. */
+ * warp waits on an mbarrier that nothing arrives on, one on a serial number
+ * that is not reached, one for a state that is not sent; *status receives
+ * FL_E_TIMEOUT once all have given up after limit_s (at most 5 s), *elapsed_s
+ * the shortest wait, and the device stays usable. */
 FL_API int fl_wait_selftest(double limit_s, int32_t *status, double *elapsed_s);
 
 /* Number of kernel launches the library has issued in this process. */
