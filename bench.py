@@ -604,8 +604,8 @@ def members_measure(hours: float = 3.0, members: int = 8) -> dict:
     """Config-4 ensemble: `members` production-sized coupled members on the
     981,880-triangle city with seeded variants of the 160 mm / 24 h event
     (intensity x U(0.7, 1.3), peak shifted by up to +-3 h), run for `hours`
-    simulated hours as one member solver (the surface kernel once per member
-    and each drainage kernel once for all members per step), against the
+    simulated hours as one member solver (the surface kernel and each drainage
+    kernel once for all members per step), against the
     same members run one after another by the single-instance solver."""
 
     import numpy as np

@@ -1,8 +1,9 @@
 // Batched-ensemble runtime behind the fl_batch_* entry points of
 // include/floodgb.h: per-scenario layouts built with the single-scenario
 // planner and concatenated tile by tile, device memory, the lockstep step
-// loop as CUDA-graph chunks (surface launch + planning launch per step), and
-// state / snapshot / ledger readout per scenario.
+// loop as CUDA-graph chunks (a surface launch per step, planning launches where
+// a step's plan needs the step before), and state / snapshot / ledger readout per
+// scenario.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -93,15 +93,13 @@ __device__ __forceinline__ float node_depth(float2 V, float A) {
 // record arrives, so its latency overlaps theirs instead of adding to the
 // dependent-load chain.
 //
-// All four are launched as programmatic dependents of the kernel before them: each kernel lets its dependent launch as soon as
-// its own blocks run (griddepcontrol.launch_dependents), and the dependent
-// loads its static tables, then waits for the whole previous grid to finish
-// and its writes to be visible (griddepcontrol.wait) before it reads them.
-// The launch latency and the static loads of each kernel overlap the
-// previous one.  (A surface grid that fills the device lets k_nodes start only
-// at its end.)
-
-
+// All four are launched as programmatic dependents of the kernel before them:
+// each kernel lets its dependent launch as soon as its own blocks run
+// (griddepcontrol.launch_dependents), and the dependent loads its static tables,
+// then waits for the whole previous grid to finish and its writes to be visible
+// (griddepcontrol.wait) before it reads them.  The launch latency and the static
+// loads of each kernel overlap the previous one.  (A surface grid that fills the
+// device lets k_nodes start only at its end.)
 //
 // An item's static records (list ranges, the first four list entries, their
 // parameters) are loaded into registers before the wait; after it, everything

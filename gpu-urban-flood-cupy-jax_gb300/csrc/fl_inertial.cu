@@ -555,9 +555,10 @@ __global__ void __launch_bounds__(TILE + 32, 3) k_li_tiles(const __grid_constant
 
 // `steps` steps of a run of the local-inertial surface alone in one cooperative
 // launch (fl_run.cuh), a CTA a tile: k_li_tiles' three passes on a tile that stays in
-// shared memory and registers, with its ledger slots and order.  120 s of a run, a
-// launch a step -> here: 1,152 cells 0.74 -> 0.55 ms, 7,200 cells 1.00 -> 0.71, 45,000
-// cells 1.56 -> 0.96; what is left is the halo states' round trip and the three passes.
+// shared memory and registers, with its ledger slots and order.  us a step of a whole
+// run with 32 steps between CFL evaluations, a launch a step -> here: 1,800 cells 4.7
+// -> 3.4, 20,000 cells 5.0 -> 3.8, 105,800 cells 6.6 -> 4.8; what is left is the halo
+// states' round trip and the three passes.
 template <int KIND>
 __global__ void __launch_bounds__(RUN_THREADS, 3) k_li_run(const __grid_constant__ LiTileArgs a, const RunArgs x, int slot, int steps) {
     extern __shared__ __align__(128) unsigned char smem[];

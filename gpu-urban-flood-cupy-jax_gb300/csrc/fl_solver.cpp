@@ -263,8 +263,8 @@ static int push_run(FlSolver *s, cudaStream_t st) {
     return FL_OK;
 }
 
-// The surface / CFL kernel arguments of member m: the solver's arguments
-// (the shared tables and settings) with that member's arrays.
+// The CFL kernel's arguments for member m: the solver's (the shared tables and
+// settings) with that member's arrays.
 static DtArgs dt_args(const FlSolver *s, int m) {
     DtArgs d = s->da;
     d.state0 = s->mb.state[0] + (size_t)m * s->Cp;
@@ -538,7 +538,13 @@ static int setup_run(FlSolver *s, const std::vector<std::pair<int32_t, int32_t>>
     return FL_OK;
 }
 
-// With a few steps between CFL evaluations there is little to keep resident.
+// A launch's set-up and last round trip have to be spread over its steps.  us a step, a
+// launch a step -> one launch, at 2 / 4 / 8 / 32 steps between CFL evaluations: full
+// scheme, 1,800 cells 6.3 -> 6.9 / 5.3 -> 5.1 / 4.5 -> 4.0 / 3.8 -> 3.0, 153,458 cells
+// 9.1 -> 9.1 / 7.5 -> 6.8 / 6.6 -> 5.7 / 5.6 -> 4.5; local-inertial, 20,000 cells 7.9
+// -> 8.4 / 6.6 -> 6.1 / 5.8 -> 5.2 / 5.0 -> 3.8.  So 2 is too few, and 8 is on the safe
+// side of the line (4 already gains 4 to 17 %).  Past 256 steps (512: 4.8 -> 2.5) a
+// launch would hold its CTA slots for more than a millisecond against other streams.
 static bool run_interval(int32_t steps) { return steps >= 8 && steps <= 256; }
 
 // Tiles of the one-launch local-inertial step: entries, rings and areas per

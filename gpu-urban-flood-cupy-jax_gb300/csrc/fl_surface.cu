@@ -334,10 +334,10 @@ __global__ void __launch_bounds__(SURF_THREADS, 4) k_surface(const __grid_consta
 // and registers.  The ledger sums keep k_surface's slots and order: the same bits,
 // step by step.
 //
-// A launch a step costs a small mesh more than its work.  us a step with 32 (8)
-// steps between CFL evaluations, a launch a step -> here: 1,800 cells 5.4 -> 3.0
-// (6.0 -> 3.9), 20,000 cells 5.7 -> 3.0 (6.7 -> 3.8), 154,568 cells 8.7 -> 4.5
-// (9.6 -> 5.8); what is left is the halo states' round trip and the two phases.
+// A launch a step costs a small mesh more than its work.  us a step of a whole run
+// with 32 (8) steps between CFL evaluations, a launch a step -> here: 1,800 cells
+// 3.8 -> 3.0 (4.5 -> 4.0), 20,000 cells 3.8 -> 3.0 (4.5 -> 3.8), 153,458 cells 5.6 ->
+// 4.5 (6.6 -> 5.7); what is left is the halo states' round trip and the two phases.
 template <int KIND>
 __global__ void __launch_bounds__(RUN_THREADS, 4) k_surface_run(const __grid_constant__ SurfArgs a, const RunArgs x, int slot, int steps) {
     extern __shared__ __align__(128) unsigned char smem[];

@@ -2,7 +2,8 @@
 
 Scenarios are cities (any mesh sizes) with their own rainfall, forcing,
 duration and adaptive dt.  The library concatenates their tiles and runs one
-persistent surface launch plus one planning launch per lockstep step, so a
+persistent surface launch per lockstep step (plus a planning launch after each CFL
+evaluation's step, or after every step where scenarios evaluate apart), so a
 64-scenario ensemble costs about what one mesh of the combined size costs,
 instead of 64 runs of launch-bound small meshes.  Each scenario follows the
 single-instance step exactly (``FloodSolver.run`` gives bitwise the same
