@@ -92,8 +92,6 @@ def _padded_rows(t, rows, cols, dtype, device, name):
         raise ValueError(f"{name} must be a matrix of {dtype}, got {t.dtype} with {t.dim()} dimensions")
     if t.device != device:
         raise ValueError(f"{name} are on {t.device}, expected {device}")
-    if t.shape == (rows, cols):
-        return t
     if t.shape[0] == rows and t.shape[1] < cols and t.stride(1) == 1 and t.stride(0) >= cols:
         held = t.untyped_storage().nbytes() // t.element_size() - t.storage_offset()
         if (rows - 1) * t.stride(0) + cols <= held:
@@ -110,6 +108,8 @@ def node_inputs(x, g, device):
 
     if x.dtype != torch.bfloat16 or x.dim() != 2 or x.stride(1) != 1:
         raise ValueError("A segments must be row-major bf16 matrices")
+    if x.shape == (g.C, 64) and x.device == device:
+        return x
     if x.shape[0] != g.C:
         raise ValueError(f"inputs have shape {tuple(x.shape)}, expected ({g.C}, 64)")
     return _padded_rows(x, g.C, 64, torch.bfloat16, device, "inputs")
@@ -120,6 +120,8 @@ def output_gradients(dy, g, device):
 
     import torch
 
+    if dy.dtype == torch.float32 and dy.shape == (g.C, 64) and dy.device == device:
+        return dy
     return _padded_rows(dy, g.C, 64, torch.float32, device, "output gradients")
 
 
