@@ -331,7 +331,9 @@ static int batch_create_impl(int32_t n, const FlMeshDesc *meshes, const FlForcin
     const int ctas = want_ctas > 0 ? std::min(want_ctas, per_sm) : per_sm;
     b->interval = params[0].cfl_update_interval_steps;
     for (int32_t s = 0; s < n; ++s)
-        if (params[s].cfl_update_interval_steps != b->interval) b->interval = 0;
+        if (params[s].cfl_update_interval_steps != b->interval ||
+            (params[s].finite_check_interval_steps > 0 && params[s].finite_check_interval_steps < BP_CHECK_STEPS))
+            b->interval = 0;
     if (b->interval < 2 || b->chunk % b->interval) b->interval = 0;  // (every step evaluates, or steps differ: a planning launch a step)
     const int planners = b->interval ? batch_plan_ctas(b->tile, n) : 0;
     b->grid = std::max(1, std::min(std::min(ctas * sms, per_sm * sms - planners), b->tiles));

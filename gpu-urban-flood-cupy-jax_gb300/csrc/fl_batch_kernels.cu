@@ -29,7 +29,8 @@
 // 1.64 M cells: 41.1 -> 38.0 ms; 90 s of six, 27,000 cells: 2.08 -> 1.59 ms).
 // A scenario whose step checks for non-finite depths ends with that step if the
 // check fails, so its next step is planned when the step is done: by the launch's
-// last CTA, without a wait of any other.
+// last CTA, without a wait of any other.  (Where checks come every few steps, a
+// planning launch a step is cheaper.)
 //
 // k_cfl_batch: the CFL minima of every tile's initial state (before step 0).
 #include "fl_batch.cuh"
@@ -147,14 +148,21 @@ __device__ __forceinline__ void list_entry(const PlanArgs &a, int b, BatchList *
 constexpr int PLAN_SMEM = 384;
 static_assert(sizeof(RunCtrl) % 8 == 0 && sizeof(RunCtrl) + sizeof(StepCtrl) <= PLAN_SMEM, "a warp's records in shared memory");
 
+// A scenario whose step checks for non-finite depths is left to plan_checked, when
+// the step is done (CHECKED: its record has been written by other SMs meanwhile).
+// Its flag is loaded with the rest, not in front of it, and the two are separate
+// code: on small batches this planner is the step.
+template <bool CHECKED>
 __device__ __noinline__ void plan_ahead(const PlanArgs &a, int b, int lane, int slot, int mode, RunCtrl *s_run) {
     StepCtrl *rec = &a.ctrl[2 * b + (slot ^ 1)], *s_next = (StepCtrl *)(s_run + 1);
     RunCtrl *run = &a.run[b];
-    for (int i = lane; i < (int)(sizeof(RunCtrl) / 4); i += 32) ((uint32_t *)s_run)[i] = __ldcg((const uint32_t *)run + i);
+    const int flags = a.list[slot].e[b].flags, t0 = a.scen_tile0[b], t1 = a.scen_tile0[b + 1];
+    for (int i = lane; i < (int)(sizeof(RunCtrl) / 4); i += 32)
+        ((uint32_t *)s_run)[i] = CHECKED ? __ldcg((const uint32_t *)run + i) : ((const uint32_t *)run)[i];
     const bool had_step = rec->active != 0;  // (the record of the step before, overwritten below)
+    if (((flags & BF_FINITE) != 0 && (mode & BP_NEXT)) != CHECKED) return;
     if (mode & BP_LEDGER) {
         const float4 *led = (const float4 *)a.tile_led + (size_t)(slot ^ 1) * a.n_tiles;
-        const int t0 = a.scen_tile0[b], t1 = a.scen_tile0[b + 1];
         float sum[SURF_TERMS] = {0.0f, 0.0f, 0.0f, 0.0f};
         float l[4][SURF_TERMS];
 #pragma unroll
@@ -205,16 +213,16 @@ __device__ __noinline__ void plan_ahead(const PlanArgs &a, int b, int lane, int 
     }
 }
 
-// The first T threads of a CTA that is done with a step in which some scenario
-// checks for non-finite depths: the last CTA plans those scenarios' next step.
-// smem: T / 32 records of PLAN_SMEM bytes and a word.
+// The compute threads of a CTA that is done with a step in which some scenario
+// checks for non-finite depths: the last of the `ctas` CTAs with tiles plans for those
+// scenarios.  smem: T / 32 records of PLAN_SMEM bytes and a word.
 template <int T>
-__device__ __noinline__ void plan_checked(const PlanArgs &a, int slot, unsigned char *smem) {
+__device__ __noinline__ void plan_checked(const PlanArgs &a, int ctas, int slot, int mode, unsigned char *smem) {
     volatile uint32_t *s_last = (volatile uint32_t *)(smem + T / 32 * PLAN_SMEM);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         __threadfence();  // (this CTA's errors, ordered by the barrier before the call)
-        const bool last = atomicAdd(a.arrived, 1u) == gridDim.x - 1;
+        const bool last = atomicAdd(a.arrived, 1u) == (uint32_t)ctas - 1;
         __threadfence();
         if (last) *a.arrived = 0u;
         *s_last = last;
@@ -222,7 +230,7 @@ __device__ __noinline__ void plan_checked(const PlanArgs &a, int slot, unsigned 
     batch_sync<T>();
     if (!*s_last) return;
     for (int b = warp; b < a.n; b += T / 32) {
-        if (a.list[slot].e[b].flags & BF_FINITE) plan_ahead(a, b, lane, slot, BP_NEXT, (RunCtrl *)(smem + warp * PLAN_SMEM));
+        plan_ahead<true>(a, b, lane, slot, mode, (RunCtrl *)(smem + warp * PLAN_SMEM));
         __syncwarp();
     }
 }
@@ -245,17 +253,7 @@ __global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(cons
         pdl_wait();
         if (a.early) pdl_launch_dependents();
         const int b = ((int)blockIdx.x - a.ctas) * W + (tid >> 5);
-        int check = 0;
-        for (int i = tid; i < p.n; i += T + 32) check |= a.list[slot].e[i].flags & BF_FINITE;
-        const bool checked = __syncthreads_or(check) && (mode & BP_NEXT);
-        if (tid >= T) return;
-        if (b < p.n)
-            plan_ahead(p, b, tid & 31, slot, a.list[slot].e[b].flags & BF_FINITE ? mode & ~BP_NEXT : mode,
-                       (RunCtrl *)(smem + (tid >> 5) * PLAN_SMEM));
-        if (checked) {
-            batch_sync<T>();
-            plan_checked<T>(p, slot, smem);
-        }
+        if (tid < T && b < p.n) plan_ahead<false>(p, b, tid & 31, slot, mode, (RunCtrl *)(smem + (tid >> 5) * PLAN_SMEM));
         return;
     }
     const uint32_t bar_base = smem_addr(s_bar);
@@ -276,11 +274,7 @@ __global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(cons
     const int n = a.n_scen;
     const BatchList *list = a.list + slot;
     float *tile_led = a.tile_led + (size_t)slot * a.n_tiles * SURF_TERMS;
-    int check = 0;
-    for (int i = tid; i < n; i += T + 32) {
-        s_ent[i] = list->e[i];
-        check |= s_ent[i].flags & BF_FINITE;
-    }
+    for (int i = tid; i < n; i += T + 32) s_ent[i] = list->e[i];
     if (tid < 32) {  // running sums of the tile counts (an inactive scenario's range is empty)
         constexpr int PER = MAX_SCEN / 32;
         int c[PER], sum = 0;
@@ -302,7 +296,7 @@ __global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(cons
         }
         if (tid == 31 && n == MAX_SCEN) s_prefix[n] = before;
     }
-    const bool checked = __syncthreads_or(check) && (mode & BP_NEXT);  // the last block-wide barrier: the roles split here
+    __syncthreads();  // the last block-wide barrier: the roles split here
     const int total = s_prefix[n];
     const int G = a.ctas;
     const BStage<T> S0 = bstage_at<T>(a, smem, 0), S1 = bstage_at<T>(a, smem, 1);
@@ -357,6 +351,11 @@ __global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(cons
 
     // ------------------------------------------------------------- compute
     const float md = a.md;
+    // whether some scenario checks for non-finite depths (while the first tile's copies are under way)
+    bool check = false;
+    if (mode & BP_NEXT)
+        for (int k = tid; k < n; k += T) check = check || (s_ent[k].flags & BF_FINITE);
+    const bool checked = (mode & BP_NEXT) && !batch_all<T>(!check);
     // the tile's ledger terms and CFL minimum from its warp partials (one thread)
     auto finish_tile = [&](int t, bool cfl) {
 #pragma unroll
@@ -478,7 +477,7 @@ __global__ void __launch_bounds__(T + 32, T == 256 ? 4 : 7) k_surface_batch(cons
         batch_sync<T>();
         if (tid == 0 && done_t >= 0) finish_tile(done_t, done_cfl);
     }
-    if (checked) plan_checked<T>(p, slot, smem);
+    if (checked) plan_checked<T>(p, G, slot, mode, smem);
 }
 
 // CFL minima of every tile's state before the first step (all scenarios'

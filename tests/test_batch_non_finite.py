@@ -35,7 +35,7 @@ def _member(n, seed, interval, finite, failing=False):
 # checks on every step, inside an interval, on its last two steps, on the first two of the
 # next one; tiles on few CTAs (the next launch sets up early) and on every slot of the device
 @pytest.mark.gpu
-@pytest.mark.parametrize("finite", [1, 5, 30, 31, 32, 33])
+@pytest.mark.parametrize("finite", [1, 5, 10, 30, 31, 32, 33])
 @pytest.mark.parametrize("tile", [128, 256])
 @pytest.mark.parametrize("others", [3, 20])
 def test_a_failed_check_ends_its_scenario(finite, tile, others):
